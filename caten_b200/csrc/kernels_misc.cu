@@ -301,37 +301,95 @@ int launch_embed(caten_b200_ctx *ctx, const float *ids_f32, const int64_t *ids_i
 // ---------------------------------------------------------------------------------------------
 // arg-max with the reference's tie rule: the lowest index among the maxima
 // (source/api/high-level-ops.lisp:321-325).
+//
+// Bound by latency: a row is 128-200 KB, and one block of 256 threads that walked it kept a step of 64 rows waiting for
+// 20 us.  So the row is cut into 2 or 4 parts per CTA and, while that leaves the GPU room, over a cluster of 2 or 4
+// CTAs; every part keeps one candidate per index residue mod 256, part after part.  The candidates of a residue are
+// merged in index order and the residues by a tree, which is the order of comparisons of a single block of 256 threads
+// that walks the row, so a NaN (which no comparison admits unless it is the first value of its residue) is treated alike
+// however the row is cut.  V = 50257, one block of 256 threads per row -> this, us a call in a row of
+// calls: 1 row 12.3 -> 5.5, 64 rows 13.0 -> 6.4, 128 rows 13.3 -> 7.6, 256 rows 14.6 -> 12.0.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ x, int64_t V, int64_t *__restrict__ out) {
+constexpr int AM_CLASSES = 256, AM_PARTS = 4;   // residues; parts per CTA at most
+
+struct ArgmaxCand {
+  float v;
+  int64_t i;
+};
+
+__global__ void __launch_bounds__(AM_CLASSES * AM_PARTS) argmax_kernel(const float *__restrict__ x, int64_t V, int64_t *__restrict__ out, int cluster) {
+  __shared__ ArgmaxCand sub[AM_PARTS * AM_CLASSES];
+  extern __shared__ ArgmaxCand all[];   // cluster x 256, of the first CTA of the cluster: one candidate per CTA and residue
+  if (cluster > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "my shared memory may be written to"
   pdl_enter();
-  const float *xr = x + (int64_t)blockIdx.x * V;
+  const int tid = threadIdx.x, lane = tid & 31, r = tid & (AM_CLASSES - 1), cta_parts = blockDim.x / AM_CLASSES;
+  const int rank = (int)(blockIdx.x % cluster);
+  const int64_t row = blockIdx.x / cluster;
+  const float *xr = x + row * V;
+  const int64_t steps = (V + AM_CLASSES - 1) / AM_CLASSES, parts = (int64_t)cta_parts * cluster, part = (int64_t)rank * cta_parts + (tid >> 8);
+  const int mine = r < V ? (int)((V - r + AM_CLASSES - 1) / AM_CLASSES) : 0;   // values of this residue
+  const int j0 = (int)(steps * part / parts), j1 = min(mine, (int)(steps * (part + 1) / parts));
   float best = -INFINITY;
-  int64_t bi = V;  // V = "nothing seen"
-  for (int64_t v = threadIdx.x; v < V; v += blockDim.x) {
-    const float f = xr[v];
-    if (f > best || bi == V) {
-      if (f > best || bi == V) { best = f; bi = v; }
-    }
+  int at = -1;
+  if (part == 0 && mine > 0) { best = xr[r]; at = 0; }   // (a NaN here stays)
+  for (int j = j0; j < j1; j += 8) {
+    float f[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) f[u] = j + u < j1 ? xr[r + (int64_t)(j + u) * AM_CLASSES] : -INFINITY;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (f[u] > best) { best = f[u]; at = j + u; }
   }
-  __shared__ float sv[256];
-  __shared__ int64_t si[256];
-  sv[threadIdx.x] = best;
-  si[threadIdx.x] = bi;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      const float ov = sv[threadIdx.x + o];
-      const int64_t oi = si[threadIdx.x + o];
-      const float mv = sv[threadIdx.x];
-      const int64_t mi = si[threadIdx.x];
-      if (oi < V && (mi == V || ov > mv || (ov == mv && oi < mi))) {
-        sv[threadIdx.x] = ov;
-        si[threadIdx.x] = oi;
-      }
-    }
+  if (at < 0)   // nothing above minus infinity: its first place, if there is one
+    for (int j = j0; j < j1 && at < 0; ++j)
+      if (xr[r + (int64_t)j * AM_CLASSES] == -INFINITY) at = j;
+  ArgmaxCand c = {best, at < 0 ? V : r + (int64_t)at * AM_CLASSES};   // V = "nothing seen"
+  // candidates of later parts replace an earlier one only when they are greater: ties keep the lowest index
+  auto merge = [&](ArgmaxCand &m, const ArgmaxCand &o) {
+    if (o.i < V && (m.i == V || o.v > m.v)) m = o;
+  };
+  if (cta_parts > 1) {
+    if (tid >= AM_CLASSES) sub[tid] = c;
     __syncthreads();
+    if (tid < AM_CLASSES)
+      for (int p = 1; p < cta_parts; ++p) merge(c, sub[p * AM_CLASSES + tid]);
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = si[0] == V ? 0 : si[0];
+  if (cluster > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < AM_CLASSES && rank > 0) {
+      uint32_t at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&all[rank * AM_CLASSES + tid])), "r"(0));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(c.v) : "memory");
+      asm volatile("st.shared::cluster.s64 [%0], %1;" ::"r"(at + 8), "l"(c.i) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank != 0) return;
+    if (tid < AM_CLASSES)
+      for (int q = 1; q < cluster; ++q) merge(c, all[q * AM_CLASSES + tid]);
+  }
+  if (tid >= AM_CLASSES) return;
+  // the tree over residues: t with t + 128, with t + 64, ...
+  auto join = [&](ArgmaxCand &m, const ArgmaxCand &n) {
+    if (n.i < V && (m.i == V || n.v > m.v || (n.v == m.v && n.i < m.i))) m = n;
+  };
+  sub[tid] = c;
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  if (tid >= 32) return;
+  ArgmaxCand k[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) k[u] = sub[tid + 32 * u];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int u = 0; u < o; ++u) join(k[u], k[u + o]);
+  c = k[0];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const ArgmaxCand n = {__shfl_down_sync(0xffffffffu, c.v, o), (int64_t)__shfl_down_sync(0xffffffffu, (long long)c.i, o)};
+    if (lane + o < 32) join(c, n);
+  }
+  if (tid == 0) out[row] = c.i == V ? 0 : c.i;
 }
 
 // End of a graph-replayed decode step: the new ids become the next step's input, are recorded in
@@ -382,7 +440,26 @@ int launch_finish_step(caten_b200_ctx *ctx, const int64_t *out_ids, int64_t *ids
 int launch_argmax(caten_b200_ctx *ctx, const float *x, int64_t rows, int64_t V, int64_t *out) {
   if (rows <= 0) return 0;
   if (V <= 0) return fail(ctx, CATEN_B200_EINVAL, "argmax: V <= 0");
-  launch_k(ctx, argmax_kernel, dim3((unsigned)rows), dim3(256), 0, x, V, out);
+  // CTAs of 1024 threads while one per SM holds all rows, and a cluster per row while there are SMs to spare; above that two
+  // parts per CTA, so that more CTAs are resident.  (us at V = 50257 for cluster x parts, a first version: 1 row 4x4 6.1, 2x4 7.5, 8x4 6.3;
+  // 64 rows 2x4 8.0, 4x4 12.2, 1x4 10.3; 128 rows 1x4 10.4, 2x4 15.1; 256 rows 1x2 17.7, 1x4 20.0.)
+  const int cluster = rows * 8 <= ctx->sm_count ? 4 : rows * 2 <= ctx->sm_count ? 2 : 1, parts = rows <= ctx->sm_count ? 4 : 2;
+  if (V > (int64_t)AM_CLASSES * 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "argmax: rows of %lld", (long long)V);
+  if (rows * cluster > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "argmax: %lld rows", (long long)rows);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(rows * cluster));
+  cfg.blockDim = dim3(AM_CLASSES * parts);
+  cfg.dynamicSmemBytes = cluster > 1 ? (size_t)cluster * AM_CLASSES * sizeof(ArgmaxCand) : 0;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = take_pdl(ctx) ? 2 : 1;
+  CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, argmax_kernel, x, V, out, cluster));
   CB_LAUNCH_CHECK(ctx, "argmax_kernel");
   return 0;
 }

@@ -119,6 +119,39 @@ def test_argmax(rt, oracle):
     assert got[0] == 100 and got[1] == 0 and got[2] == 50256 and got[3] == 0
 
 
+def _argmax_of_256_walkers(row):
+    """One walker per index residue mod 256 that keeps its first value and then greater ones, and a tree over the walkers."""
+    V = row.size
+    c = []
+    for r in range(256):
+        v, i = -np.inf, V
+        for k in range(r, V, 256):
+            if i == V or row[k] > v: v, i = row[k], k
+        c.append((v, i))
+    o = 128
+    while o:
+        for t in range(o):
+            (mv, mi), (ov, oi) = c[t], c[t + o]
+            if oi < V and (mi == V or ov > mv or (ov == mv and oi < mi)): c[t] = c[t + o]
+        o >>= 1
+    return c[0][1]
+
+
+@pytest.mark.parametrize("rows,V", [(1, 1), (2, 255), (3, 2048), (5, 16385), (74, 8193), (149, 4100)])
+def test_argmax_however_a_row_is_cut(rt, rows, V):
+    """One, two and four CTAs per row, two and four parts in them; ties, minus infinity only, and NaNs, which stand where no comparison admits them."""
+    rng = np.random.Generator(np.random.PCG64(V))
+    x = rng.integers(-40, 40, (rows, V)).astype(np.float32)
+    x[0] = -np.inf
+    x[-1, rng.integers(0, V, 5)] = np.nan
+    x[-1, 0] = np.nan
+    got = rt.argmax(rt.transfer_from_array(x)).numpy()
+    at = sorted({0, 1 % rows, rows // 2, rows - 1})
+    np.testing.assert_array_equal(got[at], [_argmax_of_256_walkers(x[r]) for r in at])
+    finite = np.isfinite(x).all(1)
+    np.testing.assert_array_equal(got[finite], x[finite].argmax(1))
+
+
 GEMV_SHAPES = [(96, 128), (200, 768), (1000, 1600), (130, 3072), (77, 6400)]
 
 
