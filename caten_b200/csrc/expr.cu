@@ -3,14 +3,14 @@
 // Schedule-Item (source/byoc/clang.lisp:163-205, op by op as in source/codegen/renderer.lisp:331-410)
 // and compiles it with gcc at run time; here nothing is compiled on the host.
 //
-// One thread owns four output elements of the innermost kept loop (32 apart, so that a warp's
+// One thread owns up to eight output elements of the innermost kept loop (32 apart, so that a warp's
 // accesses are coalesced).  It decodes its multi-index once, then walks the reduced loops (if
 // any) in loop order, exactly like the rendered loop nest, so a float sum is added in the
-// reference's order.  The program is postfix over a small value stack whose slots hold the four
-// elements side by side, so decoding a program word is paid once per four elements; the top of
+// reference's order.  The program is postfix over a small value stack whose slots hold the
+// elements side by side, so decoding a program word is paid once for all of them; the top of
 // the stack is in registers, the rest in shared memory, the program and the views in the
 // kernel's constant parameter space.  Contiguous row reductions use a second kernel with the
-// lanes along the reduced loop and an in-order accumulation across lanes.
+// lanes along the reduced loop and an in-order accumulation of tiles in shared memory.
 #include "common.cuh"
 
 namespace cb {
@@ -45,35 +45,69 @@ __device__ __forceinline__ uint32_t expr_cast(uint32_t v, int from, int to) {
   return to == CATEN_B200_CLS_BOOL ? (v != 0u ? 1u : 0u) : v;                          // I32 <-> BOOL
 }
 
-constexpr int EV = 4;          // output elements per thread (32 apart along the strip)
 constexpr int EXPR_THREADS = 256;
 constexpr int MAXD = CATEN_B200_EXPR_MAX_DIMS;
 
+// Words as the kernels see them (expr_fuse writes them from the caller's program): bits 24..26 say where a word's right
+// operand comes from, so that `LOAD b; ADD` or `CONST c; MUL` is one word that touches no stack slot; bit 27 / 28: the right
+// operand is negated / replaced by its reciprocal first (`LOAD b; NEG; ADD` and `LOAD b; RECIP; MUL`, floats).
+enum ExprMode : uint32_t { EXPR_POP = 0, EXPR_WITH_CONST = 1u << 24, EXPR_WITH_LOAD = 2u << 24, EXPR_MODES = 7u << 24, EXPR_NEG_B = 1u << 27, EXPR_RECIP_B = 1u << 28 };
+
 // Per-thread state is kept out of local memory: with 2048 threads per SM a few hundred bytes of
 // local arrays each overflow L1 and turn every stack access into L2 traffic.  The loop indices
-// are MAXD registers (all loops over them are fully unrolled), operand offsets are recomputed
-// from them at each LOAD (strides come from the kernel's parameter space), the top of the value
+// are ND registers (all loops over them are fully unrolled; the strides of loops that are not there are 0), operand
+// offsets are recomputed from them at each LOAD (strides come from the kernel's parameter space), the top of the value
 // stack is EV registers and the values under it live in shared memory, [slot][element][thread].
-struct ExprIx {
-  int v[MAXD];
+template <int ND> struct ExprIx {
+  int v[ND];
 };
 
-// Runs the program for EV elements at once: the decode of a word is shared.  Element j of the
-// thread is 32 j further along loop `vec_axis` (vec_axis < 0: a single element); for j >= lanes
-// element 0 is re-read, so nothing outside the views is touched.
-__device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx &ix, const int vec_axis, const int lanes, uint32_t *tos,
-                                         uint32_t *sm) {
-  int sp = 0;  // values on the stack, the top one (registers) included
-  auto slot = [&](int s, int j) -> uint32_t & { return sm[(s * EV + j) * EXPR_THREADS]; };
-#define EXPR_PUSH(VALUE)                                                           \
-  {                                                                                \
-    if (sp > 0) {                                                                  \
-      _Pragma("unroll") for (int j = 0; j < EV; ++j) slot(sp - 1, j) = tos[j];     \
-    }                                                                              \
-    _Pragma("unroll") for (int j = 0; j < EV; ++j) tos[j] = (VALUE);               \
-    ++sp;                                                                          \
-    break;                                                                         \
+// EV values of operand `arg`: element j is 32 j further along loop `va`; for j >= lanes the last element is re-read, so
+// nothing outside the views is touched.
+template <int ND, int EV>
+__device__ __forceinline__ void expr_load_ev(const caten_b200_expr &e, const int arg, const ExprIx<ND> &ix, const int va, const int lanes, uint32_t *out) {
+  const int dt = e.operand_dtype[arg];
+  int64_t o = e.operand_offset[arg];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) o += (int64_t)ix.v[d] * e.operand_stride[arg][d];
+  const int64_t step = va >= 0 ? 32 * e.operand_stride[arg][va] : 0;
+  const int last = lanes > 0 ? lanes - 1 : 0;
+  if (dt == CATEN_B200_DT_F32) {  // the common case without the per-element type switch
+    const float *p = reinterpret_cast<const float *>(e.operand[arg]) + o;
+    if (step == 0) {
+      const uint32_t v = __float_as_uint(*p);
+#pragma unroll
+      for (int j = 0; j < EV; ++j) out[j] = v;
+      return;
+    }
+    if (step == 32) {   // the strip is contiguous
+#pragma unroll
+      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * 32]);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * step]);
+    return;
   }
+#pragma unroll
+  for (int j = 0; j < EV; ++j) out[j] = expr_load(e.operand[arg], dt, o + (j < last ? j : last) * step);
+}
+
+// Runs the program for EV elements at once: the decode of a word is shared.  Element j of the
+// thread is 32 j further along loop `va` (va < 0: a single element).  HEAVY: with the words whose code takes twice the
+// registers (sines and logarithms in double, integer division); programs without them run in the lean form, of which twice
+// as many warps are resident (exp2 and division items over 12800 x 511: 50 us before, 36 us without the split, 27 us with it).
+template <int ND, int EV, int THREADS, bool HEAVY>
+__device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx<ND> &ix, const int va, const int lanes, uint32_t *tos, uint32_t *sm) {
+  int sp = 0;  // values on the stack, the top one (registers) included
+  auto slot = [&](int s, int j) -> uint32_t & { return sm[(s * EV + j) * THREADS]; };
+  auto push = [&]() {
+    if (sp > 0) {
+#pragma unroll
+      for (int j = 0; j < EV; ++j) slot(sp - 1, j) = tos[j];
+    }
+    ++sp;
+  };
 #define EXPR_UN(EXPR_F, EXPR_I)                                                    \
   {                                                                                \
     _Pragma("unroll") for (int j = 0; j < EV; ++j) {                               \
@@ -87,9 +121,8 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx 
   }
 #define EXPR_BIN(EXPR_F, EXPR_I)                                                   \
   {                                                                                \
-    --sp;                                                                          \
     _Pragma("unroll") for (int j = 0; j < EV; ++j) {                               \
-      const uint32_t b = tos[j], a = slot(sp - 1, j);                              \
+      const uint32_t a = tos[j], b = r[j];                                         \
       const float fa = __uint_as_float(a), fb = __uint_as_float(b);                \
       const int32_t ia = (int32_t)a, ib = (int32_t)b;                              \
       (void)fa; (void)fb; (void)ia; (void)ib;                                      \
@@ -101,35 +134,54 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx 
     const uint32_t w = e.code[pc];
     const int op = w & 255, arg = (w >> 8) & 255, cls = (w >> 16) & 255;
     const bool f = cls == CATEN_B200_CLS_F32;
-    switch (op) {
-      case CATEN_B200_OP_LOAD: {
-        const void *p = e.operand[arg];
-        const int dt = e.operand_dtype[arg];
-        int64_t o = e.operand_offset[arg];
+    uint32_t r[EV];   // right operand of a binary word; tos becomes the left one
+    if (op >= CATEN_B200_OP_ADD && op <= CATEN_B200_OP_LT) {
+      const uint32_t mode = w & EXPR_MODES;
+      if (mode == EXPR_WITH_LOAD) {
+        expr_load_ev<ND, EV>(e, arg, ix, va, lanes, r);
+      } else if (mode == EXPR_WITH_CONST) {
 #pragma unroll
-        for (int d = 0; d < MAXD; ++d)
-          if (d < e.ndim) o += (int64_t)ix.v[d] * e.operand_stride[arg][d];
-        const int64_t step = vec_axis >= 0 ? 32 * e.operand_stride[arg][vec_axis] : 0;
-        if (dt == CATEN_B200_DT_F32) {  // the common case without the per-element type switch
-          const float *fp = reinterpret_cast<const float *>(p) + o;
-          EXPR_PUSH(__float_as_uint(fp[(j < lanes ? j : 0) * step]))
-        }
-        EXPR_PUSH(expr_load(p, dt, o + (j < lanes ? j : 0) * step))
+        for (int j = 0; j < EV; ++j) r[j] = e.consts[arg];
+      } else {
+        --sp;
+#pragma unroll
+        for (int j = 0; j < EV; ++j) { r[j] = tos[j]; tos[j] = slot(sp - 1, j); }
       }
-      case CATEN_B200_OP_CONST: EXPR_PUSH(e.consts[arg])
+      if (w & EXPR_NEG_B) {
+#pragma unroll
+        for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(-__uint_as_float(r[j]));
+      }
+      if (w & EXPR_RECIP_B) {
+#pragma unroll
+        for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(1.0f / __uint_as_float(r[j]));
+      }
+    }
+    switch (op) {
+      case CATEN_B200_OP_LOAD:
+        push();
+        expr_load_ev<ND, EV>(e, arg, ix, va, lanes, tos);
+        break;
+      case CATEN_B200_OP_CONST:
+        push();
+#pragma unroll
+        for (int j = 0; j < EV; ++j) tos[j] = e.consts[arg];
+        break;
       case CATEN_B200_OP_INDEX: {
+        push();
         int base = 0;
 #pragma unroll
-        for (int d = 0; d < MAXD; ++d)
+        for (int d = 0; d < ND; ++d)
           if (d == arg) base = ix.v[d];
-        EXPR_PUSH((uint32_t)(base + (arg == vec_axis ? 32 * j : 0)))
+#pragma unroll
+        for (int j = 0; j < EV; ++j) tos[j] = (uint32_t)(base + (arg == va ? 32 * j : 0));
+        break;
       }
       case CATEN_B200_OP_NEG: EXPR_UN(__float_as_uint(-fa), (uint32_t)(-ia))
-      case CATEN_B200_OP_RECIP: EXPR_UN(__float_as_uint(1.0f / fa), (ia == 0 ? 0u : (uint32_t)(1 / ia)))
-      case CATEN_B200_OP_SIN: EXPR_UN(__float_as_uint((float)sin((double)fa)), a)
+      case CATEN_B200_OP_RECIP: EXPR_UN(__float_as_uint(1.0f / fa), (ia == 1 || ia == -1 ? (uint32_t)ia : 0u))
+      case CATEN_B200_OP_SIN: EXPR_UN(HEAVY ? __float_as_uint((float)sin((double)fa)) : a, a)
       case CATEN_B200_OP_EXP2: EXPR_UN(__float_as_uint((float)exp2((double)fa)), a)
-      case CATEN_B200_OP_LOG2: EXPR_UN(__float_as_uint((float)log2((double)fa)), a)
-      case CATEN_B200_OP_SQRT: EXPR_UN(__float_as_uint((float)sqrt((double)fa)), a)
+      case CATEN_B200_OP_LOG2: EXPR_UN(HEAVY ? __float_as_uint((float)log2((double)fa)) : a, a)
+      case CATEN_B200_OP_SQRT: EXPR_UN(HEAVY ? __float_as_uint((float)sqrt((double)fa)) : a, a)
       case CATEN_B200_OP_NOT: EXPR_UN((fa == 0.0f ? 1u : 0u), (a == 0u ? 1u : 0u))
       case CATEN_B200_OP_CAST: {
 #pragma unroll
@@ -138,8 +190,8 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx 
       }
       case CATEN_B200_OP_ADD: EXPR_BIN(__float_as_uint(fa + fb), (uint32_t)(ia + ib))
       case CATEN_B200_OP_MUL: EXPR_BIN(__float_as_uint(fa * fb), (uint32_t)(ia * ib))
-      case CATEN_B200_OP_MOD: EXPR_BIN(a, (ib == 0 ? 0u : (uint32_t)(ia % ib)))
-      case CATEN_B200_OP_IDIV: EXPR_BIN(a, (ib == 0 ? 0u : (uint32_t)(ia / ib)))
+      case CATEN_B200_OP_MOD: EXPR_BIN(a, (!HEAVY || ib == 0 ? 0u : (uint32_t)(ia % ib)))
+      case CATEN_B200_OP_IDIV: EXPR_BIN(a, (!HEAVY || ib == 0 ? 0u : (uint32_t)(ia / ib)))
       case CATEN_B200_OP_AND: EXPR_BIN(a & b, a & b)
       case CATEN_B200_OP_OR: EXPR_BIN(a | b, a | b)
       case CATEN_B200_OP_XOR: EXPR_BIN(a ^ b, a ^ b)
@@ -154,15 +206,15 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx 
       }
     }
   }
-#undef EXPR_PUSH
 #undef EXPR_UN
 #undef EXPR_BIN
 }
 
 // loop indices of flat position `pos` over loops [first, last) -> ix (innermost fastest)
-__device__ __forceinline__ void expr_decode(const caten_b200_expr &e, int64_t pos, const int first, const int last, ExprIx &ix) {
+template <int ND>
+__device__ __forceinline__ void expr_decode(const caten_b200_expr &e, int64_t pos, const int first, const int last, ExprIx<ND> &ix) {
 #pragma unroll
-  for (int d = MAXD - 1; d >= 0; --d) {
+  for (int d = ND - 1; d >= 0; --d) {
     if (d >= first && d < last) {
       ix.v[d] = (int)(pos % e.shape[d]);
       pos /= e.shape[d];
@@ -170,10 +222,11 @@ __device__ __forceinline__ void expr_decode(const caten_b200_expr &e, int64_t po
   }
 }
 
-__device__ __forceinline__ int64_t expr_out_at(const caten_b200_expr &e, const ExprIx &ix, const int nd_out) {
+template <int ND>
+__device__ __forceinline__ int64_t expr_out_at(const caten_b200_expr &e, const ExprIx<ND> &ix, const int nd_out) {
   int64_t at = e.out_offset;
 #pragma unroll
-  for (int d = 0; d < MAXD; ++d)
+  for (int d = 0; d < ND; ++d)
     if (d < nd_out) at += (int64_t)ix.v[d] * e.out_stride[d];
   return at;
 }
@@ -211,7 +264,8 @@ __device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const
 // warp takes `spw` consecutive strips of one row, so the index decoding (64-bit divisions) is
 // paid once per warp.  Reduced loops (if any) are walked by each thread in loop order, exactly
 // like the rendered loop nest, so a float sum is added in the reference's order.
-__global__ void __launch_bounds__(EXPR_THREADS) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int spw,
+template <int ND, int EV, bool HEAVY>
+__global__ void __launch_bounds__(EXPR_THREADS, HEAVY ? 2 : 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int spw,
                                                             const int64_t n_red, const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
   pdl_enter();
@@ -224,9 +278,9 @@ __global__ void __launch_bounds__(EXPR_THREADS) expr_kernel(const __grid_constan
   const int64_t vlen = va >= 0 ? e.shape[va] : 1;
   const int64_t strips_per_row = (vlen + 32 * EV - 1) / (32 * EV);
   const int64_t groups_per_row = (strips_per_row + spw - 1) / spw;
-  ExprIx ix;
+  ExprIx<ND> ix;
 #pragma unroll
-  for (int d = 0; d < MAXD; ++d) ix.v[d] = 0;
+  for (int d = 0; d < ND; ++d) ix.v[d] = 0;
   expr_decode(e, group / groups_per_row, 0, va, ix);
   int64_t j0 = (group % groups_per_row) * spw * (32 * EV) + lane;  // this thread's first element; the others follow 32 apart
   const bool is_f = result_cls == CATEN_B200_CLS_F32, is_sum = e.reduce_op == CATEN_B200_RED_SUM;
@@ -234,12 +288,12 @@ __global__ void __launch_bounds__(EXPR_THREADS) expr_kernel(const __grid_constan
   for (int s = 0; s < spw && j0 < vlen; ++s, j0 += 32 * EV) {
     const int lanes = (int)((vlen - j0 + 31) / 32 < EV ? (vlen - j0 + 31) / 32 : EV);  // elements of this thread in this strip
 #pragma unroll
-    for (int d = 0; d < MAXD; ++d)
+    for (int d = 0; d < ND; ++d)
       if (d == va) ix.v[d] = (int)j0;
     const int64_t out_at = expr_out_at(e, ix, nd_out);
     uint32_t val[EV];
     if (e.n_reduce == 0) {
-      expr_run(e, ix, va, lanes, val, sm);
+      expr_run<ND, EV, EXPR_THREADS, HEAVY>(e, ix, va, lanes, val, sm);
 #pragma unroll
       for (int j = 0; j < EV; ++j)
         if (j < lanes) expr_store(e.out, e.out_dtype, out_at + j * ovs, val[j], result_cls);
@@ -250,7 +304,7 @@ __global__ void __launch_bounds__(EXPR_THREADS) expr_kernel(const __grid_constan
     for (int j = 0; j < EV; ++j) acc[j] = expr_acc_init(e, is_f, out_at + j * ovs, j < lanes);
     for (int64_t r = 0; r < n_red; ++r) {
       expr_decode(e, r, nd_out, e.ndim, ix);
-      expr_run(e, ix, va, lanes, val, sm);
+      expr_run<ND, EV, EXPR_THREADS, HEAVY>(e, ix, va, lanes, val, sm);
 #pragma unroll
       for (int j = 0; j < EV; ++j) expr_acc_add(acc[j], val[j], is_f, is_sum, !e.accumulate && r == 0);
     }
@@ -260,56 +314,85 @@ __global__ void __launch_bounds__(EXPR_THREADS) expr_kernel(const __grid_constan
   }
 }
 
-// Reduction whose single reduced loop is the contiguous one (row sums, softmax statistics): one
-// warp per output element, lanes along the reduced loop so that loads are coalesced.  The warp
-// evaluates 32 * EV elements at a time and then adds them in loop order - element r0, r0 + 1, ... -
-// by walking the lanes with shuffles, so the result has the reference's order of additions
-// although the loads are parallel.
-__global__ void __launch_bounds__(EXPR_THREADS) expr_rowreduce_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out,
-                                                                      const int result_cls) {
+// Reduction whose single reduced loop is the contiguous one (row sums, softmax statistics).  Loads want lanes along the
+// reduced loop, the reference's order of additions wants one adder per output element, and walking the lanes of a warp with
+// shuffles spends a warp's instructions on a single sum.  So a CTA takes R output elements: eight warps evaluate tiles of
+// R x C values with lanes along the reduced loop and leave them in shared memory (rows C + 1 apart, no bank conflicts), and a
+// ninth warp, one lane per output element, adds the tile before in loop order meanwhile.  12800 rows of 511: 50 us with
+// the shuffles (issue-bound: 8 instructions per value and row), 17 us with the tiles; 16 rows of 2048: 26 -> 14 us.
+constexpr int RR_EV = 8, RR_WARPS = 8, RR_THREADS = (RR_WARPS + 1) * 32;
+// columns of a tile: one strip, more where there are too few rows to give every warp one
+__host__ __device__ constexpr int rr_cols(int R) { return R >= RR_WARPS ? 32 * RR_EV : 32 * RR_EV * RR_WARPS / R; }
+
+template <int ND, bool HEAVY>
+__global__ void __launch_bounds__(RR_THREADS, HEAVY ? 1 : 3) expr_rowreduce_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out, const int R,
+                                                                    const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
   pdl_enter();
-  const int64_t o_idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (o_idx >= n_out) return;  // whole warps leave together
-  uint32_t *sm = expr_smem + threadIdx.x;
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int C = rr_cols(R), strips = C / (32 * RR_EV);   // per row of a tile
+  uint32_t *tile = expr_smem;                              // 2 x R x (C + 1)
+  uint32_t *sm = expr_smem + 2 * R * (C + 1) + tid;
   const int nd_out = e.ndim - 1, ra = e.ndim - 1;
-  const int64_t n_red = e.shape[ra];
-  ExprIx ix;
-#pragma unroll
-  for (int d = 0; d < MAXD; ++d) ix.v[d] = 0;
-  expr_decode(e, o_idx, 0, nd_out, ix);
-  const int64_t out_at = expr_out_at(e, ix, nd_out);
+  const int n_red = (int)e.shape[ra];
+  const int64_t o0 = (int64_t)blockIdx.x * R;
+  const int rows = n_out - o0 < R ? (int)(n_out - o0) : R;
   const bool is_f = result_cls == CATEN_B200_CLS_F32, is_sum = e.reduce_op == CATEN_B200_RED_SUM;
-  ExprAcc acc = expr_acc_init(e, is_f, out_at, true);
-  uint32_t val[EV];
-  for (int64_t r0 = 0; r0 < n_red; r0 += 32 * EV) {
-    const int64_t mine = r0 + lane;  // this lane's elements: mine, mine + 32, ...
-    // elements of this lane in this round; a lane past the end re-reads element 0 of the row
-    const int mine_n = mine >= n_red ? 0 : (int)((n_red - mine + 31) / 32 < EV ? (n_red - mine + 31) / 32 : EV);
+  ExprAcc acc = {0.0f, 0};
+  int64_t out_at = 0;
+  ExprIx<ND> ix;
 #pragma unroll
-    for (int d = 0; d < MAXD; ++d)
-      if (d == ra) ix.v[d] = mine_n > 0 ? (int)mine : 0;
-    expr_run(e, ix, ra, mine_n, val, sm);
+  for (int d = 0; d < ND; ++d) ix.v[d] = 0;
+  if (warp == RR_WARPS && lane < rows) {
+    expr_decode(e, o0 + lane, 0, nd_out, ix);
+    out_at = expr_out_at(e, ix, nd_out);
+    acc = expr_acc_init(e, is_f, out_at, true);
+  }
+  const int tiles = n_red / C + (n_red % C != 0);
+  for (int t = 0; t <= tiles; ++t) {
+    if (warp < RR_WARPS) {
+      if (t < tiles) {
+        uint32_t *dst = tile + (t & 1) * R * (C + 1);
+        for (int s = warp; s < R * strips; s += RR_WARPS) {
+          const int row = s / strips;
+          const int64_t at = (int64_t)t * C + (s - row * strips) * (32 * RR_EV);   // first element of the strip along the reduced loop
+          if (row >= rows || at >= n_red) continue;
+          const int64_t mine = at + lane;
+          const int n = mine >= n_red ? 0 : (int)((n_red - mine + 31) / 32 < RR_EV ? (n_red - mine + 31) / 32 : RR_EV);
+          expr_decode(e, o0 + row, 0, nd_out, ix);
 #pragma unroll
-    for (int j = 0; j < EV; ++j) {
-      const int64_t first = r0 + 32 * j;  // element of lane 0 in this round
-      if (first >= n_red) break;
-      const int n_here = (int)(n_red - first < 32 ? n_red - first : 32);
+          for (int d = 0; d < ND; ++d)
+            if (d == ra) ix.v[d] = n > 0 ? (int)mine : 0;   // a lane past the end reads element 0 of the row
+          uint32_t val[RR_EV];
+          expr_run<ND, RR_EV, RR_THREADS, HEAVY>(e, ix, ra, n, val, sm);
+          uint32_t *to = dst + row * (C + 1) + (int)(mine - (int64_t)t * C);
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {       // loop order: lane 0, 1, ..., 31
-        const uint32_t x = __shfl_sync(0xffffffffu, val[j], k);
-        if (k < n_here) expr_acc_add(acc, x, is_f, is_sum, !e.accumulate && first + k == 0);
+          for (int j = 0; j < RR_EV; ++j)
+            if (j < n) to[32 * j] = val[j];
+        }
+      }
+    } else if (t > 0 && lane < rows) {
+      const uint32_t *src = tile + ((t - 1) & 1) * R * (C + 1) + lane * (C + 1);
+      const int64_t left = n_red - (int64_t)(t - 1) * C;
+      const int n = left < C ? (int)left : C;
+      int i = 0;
+      if (t == 1) { expr_acc_add(acc, src[0], is_f, is_sum, !e.accumulate); i = 1; }
+      if (is_f && is_sum) {
+#pragma unroll 16
+        for (; i < n; ++i) acc.f = acc.f + __uint_as_float(src[i]);
+      } else {
+#pragma unroll 8
+        for (; i < n; ++i) expr_acc_add(acc, src[i], is_f, is_sum, false);
       }
     }
+    __syncthreads();
   }
-  if (lane == 0) expr_store(e.out, e.out_dtype, out_at, is_f ? __float_as_uint(acc.f) : (uint32_t)acc.i, result_cls);
+  if (warp == RR_WARPS && lane < rows) expr_store(e.out, e.out_dtype, out_at, is_f ? __float_as_uint(acc.f) : (uint32_t)acc.i, result_cls);
 }
 
 // Checks the program on the host (operand indices, stack discipline, classes) and returns the
 // class of the value it leaves.
-static int expr_validate(caten_b200_ctx *ctx, const caten_b200_expr *e, int *result_cls, int *max_depth) {
-  *max_depth = 1;
+static int expr_validate(caten_b200_ctx *ctx, const caten_b200_expr *e, int *result_cls) {
   if (e->ndim < 1 || e->ndim > CATEN_B200_EXPR_MAX_DIMS) return fail(ctx, CATEN_B200_EINVAL, "eval_expr: ndim %d outside 1..%d", e->ndim, CATEN_B200_EXPR_MAX_DIMS);
   if (e->n_reduce < 0 || e->n_reduce > e->ndim) return fail(ctx, CATEN_B200_EINVAL, "eval_expr: n_reduce %d", e->n_reduce);
   if ((e->n_reduce > 0) != (e->reduce_op != CATEN_B200_RED_NONE) || e->reduce_op < 0 || e->reduce_op > CATEN_B200_RED_MAX)
@@ -338,7 +421,6 @@ static int expr_validate(caten_b200_ctx *ctx, const caten_b200_expr *e, int *res
       }
       if (sp >= 16) return fail(ctx, CATEN_B200_EINVAL, "eval_expr: stack deeper than 16");
       cls_stack[sp++] = cls;
-      if (sp > *max_depth) *max_depth = sp;
     } else if (op >= CATEN_B200_OP_NEG && op <= CATEN_B200_OP_CAST) {
       if (sp < 1) return fail(ctx, CATEN_B200_EINVAL, "eval_expr: word %d: empty stack", pc);
       const int have = cls_stack[sp - 1];
@@ -412,18 +494,87 @@ static void expr_collapse(caten_b200_expr *c) {
   }
 }
 
-int launch_expr(caten_b200_ctx *ctx, const caten_b200_expr *given) {
-  int result_cls = 0, max_depth = 1;
-  if (int rc = expr_validate(ctx, given, &result_cls, &max_depth)) return rc;
-  // values under the top of the stack: [slot][element][thread] in shared memory
-  const size_t smem = (size_t)(max_depth > 1 ? max_depth - 1 : 1) * EV * EXPR_THREADS * sizeof(uint32_t);
-  if (smem > 48 * 1024) {
-    CB_CUDA(ctx, cudaFuncSetAttribute(expr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CB_CUDA(ctx, cudaFuncSetAttribute(expr_rowreduce_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// Joins `LOAD b` / `CONST c` (and a NEG or RECIP of a float after it) with the binary word that uses it, and returns the
+// depth of the stack that is left.  Values and the order of operations are those of the program given.
+static int expr_fuse(caten_b200_expr *c) {
+  int n = 0;
+  for (int pc = 0; pc < c->n_code; ++pc) {
+    uint32_t w = c->code[pc] & 0xffffffu;   // the bits above are the kernels' own
+    const int op = w & 255, cls = (w >> 16) & 255;
+    if (op >= CATEN_B200_OP_ADD && op <= CATEN_B200_OP_LT && n > 0) {
+      uint32_t extra = 0;
+      int from = n - 1, prev = c->code[from] & 255;
+      if (cls == CATEN_B200_CLS_F32 && from > 0 && (prev == CATEN_B200_OP_NEG || prev == CATEN_B200_OP_RECIP)) {
+        extra = prev == CATEN_B200_OP_NEG ? EXPR_NEG_B : EXPR_RECIP_B;
+        prev = c->code[--from] & 255;
+      }
+      if (prev == CATEN_B200_OP_LOAD || prev == CATEN_B200_OP_CONST) {
+        w = (w & 0xff00ffu) | (c->code[from] & 0xff00u) | (prev == CATEN_B200_OP_LOAD ? EXPR_WITH_LOAD : EXPR_WITH_CONST) | extra;
+        n = from;
+      }
+    }
+    c->code[n++] = w;
   }
+  c->n_code = n;
+  int sp = 0, depth = 1;
+  for (int pc = 0; pc < n; ++pc) {
+    const int op = c->code[pc] & 255;
+    if (op == CATEN_B200_OP_LOAD || op == CATEN_B200_OP_CONST || op == CATEN_B200_OP_INDEX) ++sp;
+    else if (op >= CATEN_B200_OP_ADD && op <= CATEN_B200_OP_LT) sp -= (c->code[pc] & EXPR_MODES) == EXPR_POP ? 1 : 0;
+    else if (op == CATEN_B200_OP_WHERE) sp -= 2;
+    if (sp > depth) depth = sp;
+  }
+  return depth;
+}
+
+template <int ND, int EV, bool HEAVY>
+static int launch_expr_elements(caten_b200_ctx *ctx, const caten_b200_expr &e, int depth, int64_t rows, int64_t vlen, int64_t n_red, int result_cls) {
+  // values under the top of the stack: [slot][element][thread] in shared memory
+  const size_t smem = (size_t)(depth > 1 ? depth - 1 : 1) * EV * EXPR_THREADS * sizeof(uint32_t);
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(expr_kernel<ND, EV, HEAVY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t strips_per_row = (vlen + 32 * EV - 1) / (32 * EV);
+  // strips per warp: as many as still leave every SM a full complement of warps, at most 16
+  int64_t spw = (rows * strips_per_row) / ((int64_t)ctx->sm_count * 64);
+  spw = spw < 1 ? 1 : spw > 16 ? 16 : spw;
+  if (spw > strips_per_row) spw = strips_per_row;
+  const int64_t n_groups = rows * ((strips_per_row + spw - 1) / spw);  // one warp each
+  const int64_t blocks = (n_groups + 7) / 8;
+  if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)(rows * vlen));
+  launch_k(ctx, expr_kernel<ND, EV, HEAVY>, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_groups, (int)spw, n_red, result_cls);
+  CB_LAUNCH_CHECK(ctx, "expr_kernel");
+  return 0;
+}
+
+template <int ND, bool HEAVY>
+static int launch_expr_rows(caten_b200_ctx *ctx, const caten_b200_expr &e, int depth, int64_t n_out, int result_cls) {
+  // output elements per CTA: 32 keep the adding warp full; fewer when that would leave SMs without a CTA
+  int R = 32;
+  while (R > 1 && (n_out + R - 1) / R < 2 * ctx->sm_count) R >>= 1;
+  const int64_t blocks = (n_out + R - 1) / R;
+  if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
+  const size_t smem = (2 * (size_t)R * (rr_cols(R) + 1) + (size_t)(depth > 1 ? depth - 1 : 1) * RR_EV * RR_THREADS) * sizeof(uint32_t);
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(expr_rowreduce_kernel<ND, HEAVY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_k(ctx, expr_rowreduce_kernel<ND, HEAVY>, dim3((unsigned)blocks), dim3(RR_THREADS), smem, e, n_out, R, result_cls);
+  CB_LAUNCH_CHECK(ctx, "expr_rowreduce_kernel");
+  return 0;
+}
+
+int launch_expr(caten_b200_ctx *ctx, const caten_b200_expr *given) {
+  int result_cls = 0;
+  if (int rc = expr_validate(ctx, given, &result_cls)) return rc;
   caten_b200_expr collapsed = *given;
   expr_collapse(&collapsed);
+  const int depth = expr_fuse(&collapsed);
   const caten_b200_expr *e = &collapsed;
+  for (int d = e->ndim; d < MAXD; ++d) {   // loops that are not there do not move
+    collapsed.out_stride[d] = 0;
+    for (int i = 0; i < e->n_operands; ++i) collapsed.operand_stride[i][d] = 0;
+  }
+  bool heavy = false;
+  for (int pc = 0; pc < e->n_code; ++pc) {
+    const int op = e->code[pc] & 255;
+    heavy = heavy || op == CATEN_B200_OP_SIN || op == CATEN_B200_OP_LOG2 || op == CATEN_B200_OP_SQRT || op == CATEN_B200_OP_MOD || op == CATEN_B200_OP_IDIV;
+  }
   const int nd_out = e->ndim - e->n_reduce;
   int64_t n_out = 1, n_red = 1;
   for (int d = 0; d < nd_out; ++d) n_out *= e->shape[d];
@@ -439,25 +590,22 @@ int launch_expr(caten_b200_ctx *ctx, const caten_b200_expr *given) {
       if (nd_out > 0 && e->operand_stride[i][nd_out - 1] == 1) unit_kept = true;
     }
     if (nd_out == 0 || (unit_red && !unit_kept)) {
-      const int64_t blocks = (n_out + 7) / 8;  // one warp per output element
-      if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
-      launch_k(ctx, expr_rowreduce_kernel, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, *e, n_out, result_cls);
-      CB_LAUNCH_CHECK(ctx, "expr_rowreduce_kernel");
-      return 0;
+      if (heavy) return launch_expr_rows<MAXD, true>(ctx, *e, depth, n_out, result_cls);
+      return e->ndim <= 2 ? launch_expr_rows<2, false>(ctx, *e, depth, n_out, result_cls) : launch_expr_rows<MAXD, false>(ctx, *e, depth, n_out, result_cls);
     }
   }
-  const int64_t vlen = nd_out > 0 ? e->shape[nd_out - 1] : 1;
-  const int64_t strips_per_row = (vlen + 32 * EV - 1) / (32 * EV), rows = n_out / vlen;
-  // strips per warp: as many as still leave every SM a full complement of warps, at most 16
-  int64_t spw = (rows * strips_per_row) / ((int64_t)ctx->sm_count * 64);
-  spw = spw < 1 ? 1 : spw > 16 ? 16 : spw;
-  if (spw > strips_per_row) spw = strips_per_row;
-  const int64_t n_groups = rows * ((strips_per_row + spw - 1) / spw);  // one warp each
-  const int64_t blocks = (n_groups + 7) / 8;
-  if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
-  launch_k(ctx, expr_kernel, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, *e, n_groups, (int)spw, n_red, result_cls);
-  CB_LAUNCH_CHECK(ctx, "expr_kernel");
-  return 0;
+  const int64_t vlen = nd_out > 0 ? e->shape[nd_out - 1] : 1, rows = n_out / vlen;
+  if (heavy) return launch_expr_elements<MAXD, 4, true>(ctx, *e, depth, rows, vlen, n_red, result_cls);
+  // Elements per thread: decoding a word costs about as much as applying it to four values, so eight, where that pads the
+  // rows no further than four would and still gives every SM 16 warps; one where a row fits the lanes of a warp.
+  const bool wide = (vlen + 255) / 256 * 256 == (vlen + 127) / 128 * 128 && rows * (vlen / 256) >= (int64_t)ctx->sm_count * 16;
+  const int ev = vlen <= 32 ? 1 : wide ? 8 : 4;
+#define EXPR_ELEMENTS(ND)                                                                              \
+  ev == 1   ? launch_expr_elements<ND, 1, false>(ctx, *e, depth, rows, vlen, n_red, result_cls)        \
+  : ev == 4 ? launch_expr_elements<ND, 4, false>(ctx, *e, depth, rows, vlen, n_red, result_cls)        \
+            : launch_expr_elements<ND, 8, false>(ctx, *e, depth, rows, vlen, n_red, result_cls)
+  return e->ndim <= 2 ? (EXPR_ELEMENTS(2)) : (EXPR_ELEMENTS(MAXD));
+#undef EXPR_ELEMENTS
 }
 
 }  // namespace cb

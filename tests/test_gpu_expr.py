@@ -201,6 +201,32 @@ def test_empty_and_large(rt):
     check(rt, E.load(big.view) * E.load(big.view) + 1.0, res, pairs=(big,))
 
 
+@pytest.mark.parametrize("rows,cols,op", [(1, 64, "sum"), (1, 9000, "sum"), (33, 129, "max"), (700, 1025, "sum"), (9500, 127, "max"), (9500, 128, "sum")])
+def test_row_reductions_at_tile_edges(rt, rows, cols, op):
+    """Output elements per CTA from 1 to 32, tiles and rows of CTAs that end early, values no comparison admits."""
+    rng = np.random.Generator(np.random.PCG64(rows + cols))
+    a = rng.standard_normal((rows, cols), dtype=np.float32)
+    a[0, cols // 2], a[-1, 0], a[rows // 2, -1] = np.nan, -np.inf, np.inf
+    x, s = Pair(rt, a), Pair(rt, rng.standard_normal((rows, 1), dtype=np.float32), strides=(1, 0))
+    check(rt, E.load(x.view) * 0.5, s, shape=(rows, cols), n_reduce=1, reduce_op=op, pairs=(x,))
+    s.host[:] = s.dev.numpy()
+    check(rt, E.load(x.view) - 1.0, s, shape=(rows, cols), n_reduce=1, reduce_op=op, accumulate=True, pairs=(x,))
+
+
+@pytest.mark.parametrize("shape", [(3, 32), (2400, 511), (2400, 256), (5, 7, 300)])
+def test_words_joined_with_their_right_operand(rt, shape):
+    """A load or a constant, negated or reciprocal, on either side of a binary word; one, four and eight elements a thread."""
+    rng = np.random.Generator(np.random.PCG64(len(shape) + shape[-1]))
+    x, y = (Pair(rt, rng.standard_normal(shape, dtype=np.float32)) for _ in range(2))
+    z = Pair(rt, rng.standard_normal(shape[:-1] + (1,), dtype=np.float32), strides=tuple(int(np.prod(shape[i + 1:-1])) for i in range(len(shape) - 1)) + (0,))
+    i = Pair(rt, rng.integers(-9, 9, shape, dtype=np.int32))
+    lx, ly, lz = E.load(x.view), E.load(y.view), E.load(z.view)
+    out = Pair(rt, np.zeros(shape, np.float32))
+    check(rt, (lx - lz) * 1.5 / ly + lx / lz, out, pairs=(x, y, z))
+    check(rt, E.const(2.0) - lx * ly + (-(lx + 1.0)) * E.recip(lz * 0.5), out, pairs=(x, y, z))
+    check(rt, E.where(lx < lz, E.maximum(ly, lz), E.cast(E.load(i.view) * E.const(3) + E.index(len(shape) - 1), E.F32)), out, pairs=(x, y, z, i))
+
+
 def test_malformed_programs_are_refused(rt):
     from caten_b200 import _lib as L
     x = Pair(rt, np.zeros(8, np.float32))
