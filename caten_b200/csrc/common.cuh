@@ -248,10 +248,13 @@ struct WSrc {
 };
 constexpr int WT_F32_T = 100;  // pseudo weight type: fp32 operand given as [K, N] row-major (relu_matmul's b)
 // many-row GEMM with both operands from shared memory (gemm_dense.cu)
-bool gemm_dense_applies(const caten_b200_ctx *ctx, int64_t M, int64_t N, int64_t K);
+bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K);
 int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo,
                       const float *bias, const float *res, int act, float *y, BfOut ybf, int64_t M, int64_t N, int64_t K, int nsplit,
-                      LinGroups grp = LinGroups());
+                      LinGroups grp = LinGroups(), PartIn *defer = nullptr);
+// sums partial tiles part[split][tile][row of x][128 features] and applies the linear's epilogue
+int launch_splitk_reduce(caten_b200_ctx *ctx, const float *part, int splits, int tiles_x, int tiles, int bnx, const float *bias, const float *res, float *y,
+                         BfOut ybf, int act, int M, int N, int group_rows, int tiles_per_group, int ygroup, int ldy);
 // the Linear of a model: GEMV for up to 4 rows, otherwise the GEMM of `prec`; with a tensor-core precision the input is
 // xbf when it is set (written by its producer), and the output can be requested the same way (ybf)
 int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, const float *x, BfOut xbf, const float *bias, const float *res,

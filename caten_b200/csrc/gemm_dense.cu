@@ -7,7 +7,7 @@
 //   warp 0      one lane issues the TMA loads of the W and x tiles into a ring of stages
 //   warp 1      issues tcgen05.mma (A = W tile, B = x tile, both K-major with 128-byte swizzle)
 //               into one of TWO accumulators in tensor memory (2 x 256 columns)
-//   warps 2..9  epilogue: read the other accumulator with tcgen05.ld, add bias, apply the
+//   warps 2..17 epilogue: read the other accumulator with tcgen05.ld, add bias, apply the
 //               activation and the residual, store — while the next tile's MMAs run
 // Tile = 128 output features (TMEM lanes) x 256 rows (TMEM columns); a stage holds 64 k (bf16) or 32 k (split bf16).
 // Split-bf16 (NSPLIT = 3) issues W_hi.x_hi + W_lo.x_hi + W_hi.x_lo per k-step, as the decode GEMM.
@@ -30,7 +30,7 @@ constexpr int GD_BK = 64;    // k granularity of the operands (K % 64 == 0)
 // k per stage: 64 (128-byte rows, 128-byte swizzle) in bf16; 32 (64-byte rows, 64-byte swizzle) in split bf16, where a
 // 64-k stage of hi and lo tiles is 96 KB and only two would fit: four 48 KB stages keep three loads in flight
 template <int NSPLIT> struct GdStage { static constexpr int BK = NSPLIT == 3 ? 32 : 64; };
-constexpr int GD_EPI_WARPS = 8;
+constexpr int GD_EPI_WARPS = 16;
 constexpr int GD_THREADS = (2 + GD_EPI_WARPS) * 32;
 
 struct GdArgs {
@@ -45,11 +45,18 @@ struct GdArgs {
   // [g * ygroup, ..) of rows of ldy; a group has tiles_per_group feature tiles, the last one possibly partial
   int group_rows, xplane, ygroup, ldy, tiles_per_group;
   uint32_t idesc;
-  int bn;                     // EXPERTS: activation rows per tile (GD_BN otherwise)
+  int bn;                     // activation rows per tile, 16 or a multiple of 32
+  int splits, cps;            // split-K: `splits` work items per tile, each of cps k-stages; their sums go to part
+  float *part;                // [split][tile][row of x][feature]; summed by the consumer or splitk_reduce_kernel
+  int static_w;               // W depends on no kernel in flight: its first stages are loaded before the wait for x
+  uint32_t tmem_cols;         // allocated: the accumulators, rounded up to a power of two
   ExpertRows er;
 };
 
 constexpr int GD_MAX_EXPERTS = 1024;
+constexpr int GD_EXPAND_ROWS = 1536;   // expanded weights: rows from which every shape runs here
+constexpr size_t GD_STAGE_BYTES = 227 * 1024 - 2048 - GD_EPI_WARPS * 2048;
+constexpr int GD_SPLIT_ROWS = 512;     // rows up to which k is shared among CTAs
 
 // One output tile: features [f0, f_end), activation rows [m0, m_end), first row of its x tile
 struct GdTile {
@@ -74,7 +81,7 @@ __device__ __forceinline__ GdTile gd_tile(const GdArgs &a, int tile, const int *
     const int f = tile % a.tiles_f, g = f / a.tiles_per_group;
     t.f0 = g * a.group_rows + (f % a.tiles_per_group) * GD_BM;
     t.f_end = min(a.N, (g + 1) * a.group_rows);
-    t.m0 = (tile / a.tiles_f) * GD_BN;
+    t.m0 = (tile / a.tiles_f) * a.bn;
     t.m_end = a.M;
     t.x0 = t.m0 + g * a.xplane;
     t.shift = g * (a.group_rows - a.ygroup);
@@ -225,14 +232,13 @@ __device__ __forceinline__ uint64_t gd_desc(uint32_t saddr) {
   return d;
 }
 
-template <int NSPLIT, bool EXPERTS>
+template <int NSPLIT, bool EXPERTS, bool WLO>
 __global__ void __launch_bounds__(GD_THREADS, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_constant__ CUtensorMap tw_lo,
                   const __grid_constant__ CUtensorMap tx_hi, const __grid_constant__ CUtensorMap tx_lo, const GdArgs a) {
   constexpr int BK = GdStage<NSPLIT>::BK;
   constexpr uint32_t ROW_BYTES = BK * 2u;
-  constexpr bool WLO = NSPLIT == 3 && !EXPERTS;   // (experts' weights are bf16: no low part)
-  const int BN = EXPERTS ? a.bn : GD_BN;
+  const int BN = a.bn;
   constexpr uint32_t W_BYTES = GD_BM * ROW_BYTES;
   const uint32_t X_BYTES = (uint32_t)BN * ROW_BYTES;
   const uint32_t STAGE_BYTES = W_BYTES * (WLO ? 2u : 1u) + X_BYTES * (NSPLIT == 3 ? 2u : 1u);
@@ -258,6 +264,11 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int num_k = a.K / BK;
+  // work item i: tile i % tiles, k-stages [i / tiles * cps, ..) of it
+  auto k_of = [&](int z, int *k0) {
+    *k0 = z * a.cps;
+    return min(num_k - *k0, a.cps);
+  };
 
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -273,7 +284,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(a.tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -289,7 +300,19 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       tma_prefetch_map(&tx_lo);
     }
   }
-  // both operands and the residual were written by preceding kernels
+  // Weights that no kernel writes are on their way before the wait below: in a decode step that is most of what this CTA
+  // reads, and it arrives while the kernel that produces x still runs.
+  int ahead = 0;   // stages whose W tiles have been asked for
+  if (!EXPERTS && a.static_w && warp == 0 && lane == 0) {
+    const GdTile t = gd_tile<EXPERTS>(a, (int)(blockIdx.x % a.tiles), nullptr);
+    int k0;
+    const int nk = k_of(blockIdx.x / a.tiles, &k0);
+    for (; ahead < nk && ahead < S; ++ahead) {
+      mbar_expect_tx(full(ahead), STAGE_BYTES);
+      tma_load_2d(st_whi(ahead), &tw_hi, full(ahead), (k0 + ahead) * BK, t.f0);
+    }
+  }
+  // the activations, the residual and (otherwise) the weights were written by preceding kernels
   pdl_wait();
   int tiles = a.tiles;
   int *first = reinterpret_cast<int *>(smem + (size_t)S * STAGE_BYTES + GD_EPI_WARPS * 2048);   // EXPERTS: [experts + 1]
@@ -313,6 +336,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     __syncthreads();
     tiles = first[a.er.experts];
   }
+  const int items = tiles * a.splits;
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -320,16 +344,21 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       int issued = 0, s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        const int tile = item % tiles;
         const GdTile t = gd_tile<EXPERTS>(a, tile, first);
-        for (int kc = 0; kc < num_k; ++kc) {
+        int k0;
+        const int nk = k_of(item / tiles, &k0);
+        for (int kc = k0; kc < k0 + nk; ++kc) {
           if (!mbar_wait(empty(s), ph ^ 1u, abort_flag)) {
             if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 11; a.status[2] = tile; }
             ok = false;
             break;
           }
-          mbar_expect_tx(full(s), STAGE_BYTES);
-          tma_load_2d(st_whi(s), &tw_hi, full(s), kc * BK, t.f0);
+          if (issued >= ahead) {
+            mbar_expect_tx(full(s), STAGE_BYTES);
+            tma_load_2d(st_whi(s), &tw_hi, full(s), kc * BK, t.f0);
+          }
           if (WLO) tma_load_2d(st_wlo(s), &tw_lo, full(s), kc * BK, t.f0);
           tma_load_2d(st_xhi(s), &tx_hi, full(s), kc * BK, t.x0);
           if (NSPLIT == 3) tma_load_2d(st_xlo(s), &tx_lo, full(s), kc * BK, t.x0);
@@ -347,8 +376,10 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     int s = 0, it = 0;
     uint32_t ph = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
-      const int b = it & 1;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+      const int b = it & 1, tile = item % tiles;
+      int k0;
+      const int nk = k_of(item / tiles, &k0);
       // the epilogue has drained this accumulator (first use of each passes at once)
       if (!mbar_wait(acc_empty(b), (((uint32_t)it >> 1) & 1u) ^ 1u, abort_flag)) {
         if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 12; a.status[2] = tile; }
@@ -356,8 +387,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
         break;
       }
       tc_fence_after();
-      const uint32_t acc = tmem_base + (uint32_t)b * GD_BN;
-      for (int kc = 0; kc < num_k; ++kc) {
+      const uint32_t acc = tmem_base + (uint32_t)(b * BN);
+      for (int kc = 0; kc < nk; ++kc) {
         if (!mbar_wait(full(s), ph, abort_flag)) {
           if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 13; a.status[2] = tile; }
           ok = false;
@@ -386,14 +417,22 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     }
   } else {
     // ---------------- epilogue ----------------
-    // a warp reaches the TMEM lanes of quadrant (warp % 4); the two warps of a quadrant split the columns
-    const int quad = warp & 3, half = (warp - 2) >> 2;
+    // a warp reaches the TMEM lanes of quadrant (warp % 4); the four warps of a quadrant take blocks of 16 columns in turns
+    // (with two warps per quadrant the epilogue was the longest part of a launch of one or two tiles per CTA: the linears of
+    // 1665 rows of width 1024 took 25.8 us each, with four 21.4 us)
+    const int quad = warp & 3, turn = (warp - 2) >> 2;
     float *stg = reinterpret_cast<float *>(smem + (size_t)S * STAGE_BYTES) + (warp - 2) * 512;  // 16 rows x 32 features
     int it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
-      const int b = it & 1;
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+      const int b = it & 1, tile = item % tiles;
       const GdTile t = gd_tile<EXPERTS>(a, tile, first);
+      // after the transpose a lane owns features o0 .. o0 + 3 (N % 4 == 0: all inside or all outside)
+      const int64_t o0 = (int64_t)t.f0 + quad * 32 + 4 * (lane & 7);
+      const bool o_ok = o0 < t.f_end;
+      const int64_t oc = o0 - t.shift;   // output column
+      float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (a.bias && o_ok) bias4 = *reinterpret_cast<const float4 *>(a.bias + o0);
       int got = 0;
       if (lane == 0) {
         got = mbar_wait(acc_full(b), ((uint32_t)it >> 1) & 1u, abort_flag) ? 1 : 0;
@@ -402,16 +441,18 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) { ok = false; break; }
       tc_fence_after();
-      // after the transpose a lane owns features o0 .. o0 + 3 (N % 4 == 0: all inside or all outside)
-      const int64_t o0 = (int64_t)t.f0 + quad * 32 + 4 * (lane & 7);
-      const bool o_ok = o0 < t.f_end;
-      const int64_t oc = o0 - t.shift;   // output column
-      const int cols = EXPERTS ? (BN >= 32 ? BN / 2 : half == 0 ? 16 : 0) : GD_BN / 2;
-      float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (a.bias && o_ok) bias4 = *reinterpret_cast<const float4 *>(a.bias + o0);
-      const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * GD_BN + half * (BN / 2));
-      for (int c = 0; c < cols; c += 16) {
-        if (EXPERTS && t.m0 + half * (BN / 2) + c >= t.m_end) break;
+      const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
+      for (int c = 16 * turn; c < BN; c += 4 * GD_EPI_WARPS) {
+        if (t.m0 + c >= t.m_end) break;
+        if (!EXPERTS && a.part) {   // sums of this share of k: a warp stores 32 features of one row of x at a time
+          uint32_t r[16];
+          tmem_ld16(trow + (uint32_t)c, r);
+          tmem_ld_wait();
+          float *dst = a.part + ((int64_t)item * BN + c) * GD_BM + quad * 32 + lane;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) dst[i * GD_BM] = __uint_as_float(r[i]);
+          continue;
+        }
         uint32_t r[16];
         tmem_ld16(trow + (uint32_t)c, r);
         tmem_ld_wait();
@@ -419,7 +460,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 16; ++i) stg[i * 32 + lane] = __uint_as_float(r[i]);
         __syncwarp();
-        const int m_first = t.m0 + half * (BN / 2) + c;
+        const int m_first = t.m0 + c;
         if (a.act == CATEN_B200_ACT_SILU_GLU) gd_store_block<CATEN_B200_ACT_SILU_GLU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
         else if (a.act == CATEN_B200_ACT_RELU_GLU) gd_store_block<CATEN_B200_ACT_RELU_GLU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
         else if (!EXPERTS && a.act == CATEN_B200_ACT_GELU) gd_store_block<CATEN_B200_ACT_GELU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
@@ -435,7 +476,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols) : "memory");
   }
 }
 
@@ -467,31 +508,73 @@ static int launch_wsplit(caten_b200_ctx *ctx, const WSrc &ws, int64_t N, int64_t
   return 0;
 }
 
-bool gemm_dense_applies(const caten_b200_ctx *ctx, int64_t M, int64_t N, int64_t K) {
-  // enough rows that expanding the weights once is cheap next to the GEMM and the tiles fill the GPU
-  return ctx->dense_gemm && M >= 1024 && N % 4 == 0 && K % GD_BK == 0 && K >= GD_BK && (M + GD_BN - 1) / GD_BN * ((N + GD_BM - 1) / GD_BM) >= ctx->sm_count;
+// How a launch is cut: rows of x per tile and shares of k.
+struct GdPlan {
+  int bn, splits, cps;
+};
+
+// The cut with the shortest expected time.  A CTA's stage takes as long as its MMAs (bn / 2 cycles each, at least 40) or as
+// long as its operands need from L2 (about 60 bytes a cycle and SM with every SM at work; measured: 128 x 256 tiles of
+// plain bf16 run at 0.85 of the burst rate of the tensor cores, 48 KB in 870 cycles).  Wide tiles read least, narrow ones
+// leave no SM without work and the last wave short; shares of k pay for a pass over their partial sums.
+static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums) {
+  GdPlan best = {256, 1, (int)(K / bk)};
+  double least = 1e30;
+  const int nk = (int)(K / bk), products = nsplit == 1 ? 1 : wlo ? 3 : 2, parts = nsplit == 1 ? 1 : 2;
+  for (int bn = 16; bn <= GD_BN; bn = bn < 32 ? 32 : bn + 32) {
+    if (bn == 16 && M > 16) continue;
+    const int64_t tiles = (M + bn - 1) / bn * tiles_f;
+    const double mma = (double)(bk / 16) * products * (bn > 80 ? bn / 2 : 40);
+    const double bytes = (double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)bn * parts);
+    const double epilogue = 500 + 8.0 * bn;
+    for (int splits = 1; splits <= 32; ++splits) {
+      const int cps = (nk + splits - 1) / splits, s = (nk + cps - 1) / cps;
+      if (splits > 1 && (!can_split || tiles * s > sm || cps * bk < 256)) break;
+      if (s != splits) continue;
+      const int64_t items = tiles * s;
+      const double busy = items < sm ? (double)items : (double)sm, rate = 60.0 * sm / busy < 100.0 ? 60.0 * sm / busy : 100.0;
+      const double stage = mma > bytes / rate ? mma : bytes / rate, body = cps * stage;
+      const int64_t waves = (items + sm - 1) / sm;
+      double t = 1500 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
+      if (s > 1) t += (consumer_sums ? 500.0 : 5000.0) + (double)M * N * 4 * s / (sm * 30.0);
+      t *= 1.0 + 0.0003 * (GD_BN - bn);   // traffic costs power too, which is what limits long launches
+      if (t < least) { least = t; best = {bn, s, cps}; }
+    }
+    if (bn >= M) break;
+  }
+  return best;
+}
+
+// Which linears run here.  bf16 weights are the operand as they are: every one whose shape fits (us a call, other kernel ->
+// this, plain bf16, 11264 x 2048: 16 rows 29 -> 13, 256 rows 42 -> 27, 777 rows 108 -> 39; 1024 x 4096: 1665 rows 45 -> 28).
+// Other formats are expanded once per call, which pays when the converting producers of the other kernel (one per output
+// tile) repeat it often: with full waves of the widest tiles from 1024 rows on, otherwise from 1536 (split bf16, Q4_0,
+// 1600 x 6400: 777 rows 65 here 87, 1024 rows 69 here 90, 1665 rows 113 here 106; 1600 x 1600: 1665 rows 38 here 32).
+bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K) {
+  if (!ctx->dense_gemm || N % 4 || K % GD_BK || K < GD_BK) return false;
+  if (wt == CATEN_B200_BF16 || M >= GD_EXPAND_ROWS) return true;
+  return M >= 1024 && (M + GD_BN - 1) / GD_BN * ((N + GD_BM - 1) / GD_BM) >= ctx->sm_count;
 }
 
 // wt: a ggml type or WT_F32_T (then ws.qs is b[K, N] fp32).  x: fp32 [M, K], or its split bf16 copy when xhi is given.
 int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo,
                       const float *bias, const float *res, int act, float *y, BfOut ybf, int64_t M, int64_t N, int64_t K, int nsplit,
-                      LinGroups grp) {
+                      LinGroups grp, PartIn *defer) {
   if (!ctx->encode_tiled) return fail(ctx, CATEN_B200_ECUDA, "gemm_dense: cuTensorMapEncodeTiled is not available");
   if (K % GD_BK || M > 0x7fffffff || N > 0x7fffffff || K > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: shape %lldx%lldx%lld", (long long)M, (long long)N, (long long)K);
   if (nsplit != 1 && nsplit != 3) return fail(ctx, CATEN_B200_EINVAL, "gemm_dense: nsplit must be 1 or 3");
   const int parts = nsplit == 3 ? 2 : 1;
   // bf16 copy of the weights
-  const bool as_is = wt == CATEN_B200_BF16 && parts == 1;  // the weight is the operand: no copy
+  const bool as_is = wt == CATEN_B200_BF16;  // the weight is the operand: no copy, and no low part
   const size_t wb = ((size_t)N * K * 2 + 1023) & ~(size_t)1023;
   if (!as_is)
     if (int rc = scratch_reserve(ctx, &ctx->wbf, wb * parts)) return rc;
-  __nv_bfloat16 *whi = (__nv_bfloat16 *)ctx->wbf.ptr, *wlo = parts == 2 ? (__nv_bfloat16 *)((uint8_t *)ctx->wbf.ptr + wb) : nullptr;
+  __nv_bfloat16 *whi = (__nv_bfloat16 *)ctx->wbf.ptr, *wlo = parts == 2 && !as_is ? (__nv_bfloat16 *)((uint8_t *)ctx->wbf.ptr + wb) : nullptr;
   int rc = 0;
   if (as_is) whi = (__nv_bfloat16 *)ws.qs;
   else switch (wt) {
     case CATEN_B200_F32: rc = launch_wsplit<CATEN_B200_F32>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_F16: rc = launch_wsplit<CATEN_B200_F16>(ctx, ws, N, K, whi, wlo); break;
-    case CATEN_B200_BF16: rc = launch_wsplit<CATEN_B200_BF16>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_Q4_0: rc = launch_wsplit<CATEN_B200_Q4_0>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_Q4_1: rc = launch_wsplit<CATEN_B200_Q4_1>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_Q5_0: rc = launch_wsplit<CATEN_B200_Q5_0>(ctx, ws, N, K, whi, wlo); break;
@@ -522,10 +605,9 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   CUtensorMap twh, twl, txh, txl;
   const int bk = nsplit == 3 ? GdStage<3>::BK : GdStage<1>::BK;
   if ((rc = make_map(ctx, &twh, whi, N, K, GD_BM, bk))) return rc;
-  if ((rc = make_map(ctx, &twl, wlo ? wlo : whi, N, K, GD_BM, bk))) return rc;
+  twl = twh;
+  if (wlo && (rc = make_map(ctx, &twl, wlo, N, K, GD_BM, bk))) return rc;
   const int64_t xrows = grp.group_rows ? (N - 1) / grp.group_rows * grp.xplane + M : M;  // all planes of x
-  if ((rc = make_map(ctx, &txh, xhi, xrows, K, GD_BN, bk))) return rc;
-  if ((rc = make_map(ctx, &txl, nsplit == 3 ? xlo : xhi, xrows, K, GD_BN, bk))) return rc;
 
   GdArgs a;
   a.bias = bias; a.res = res; a.y = y; a.yhi = ybf.hi; a.ylo = ybf.lo; a.status = ctx->d_status;
@@ -535,18 +617,35 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   a.tiles_f = (int)((N + a.group_rows - 1) / a.group_rows) * a.tiles_per_group;
   a.ygroup = grp.ygroup ? (int)grp.ygroup : a.group_rows;
   a.ldy = grp.ldy ? (int)grp.ldy : (int)(act_is_glu(act) ? N / 2 : N);
-  a.bn = GD_BN;
   if (res && !grp.plain_output()) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: a residual needs the plain output layout");
-  const int64_t tiles = (int64_t)a.tiles_f * ((M + GD_BN - 1) / GD_BN);
-  if (tiles > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: too many tiles");
+  const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && grp.plain_output() && grp.group_rows % GD_BM == 0;
+  const GdPlan p = gd_plan(ctx->sm_count, M, N, a.tiles_f, K, nsplit, wlo != nullptr, bk, M <= GD_SPLIT_ROWS, can_defer);
+  a.bn = p.bn; a.splits = p.splits; a.cps = p.cps; a.part = nullptr;
+  a.static_w = as_is && !ctx->weights_pending;
+  if ((rc = make_map(ctx, &txh, xhi, xrows, K, p.bn, bk))) return rc;
+  txl = txh;
+  if (nsplit == 3 && (rc = make_map(ctx, &txl, xlo, xrows, K, p.bn, bk))) return rc;
+  const int64_t tiles = (int64_t)a.tiles_f * ((M + p.bn - 1) / p.bn), items = tiles * p.splits;
+  if (items > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: too many tiles");
   a.tiles = (int)tiles;
-  const size_t stage = (size_t)(GD_BM + GD_BN) * (size_t)bk * 2 * parts;
-  int stages = (int)((200 * 1024) / stage);  // 1 KB slack + 1 KB barriers + stages + 16 KB of epilogue staging fit 227 KB
-  if (stages > 6) stages = 6;
+  if (p.splits > 1) {
+    if ((rc = scratch_reserve(ctx, &ctx->wtmp, (size_t)items * p.bn * GD_BM * sizeof(float)))) return rc;
+    a.part = (float *)ctx->wtmp.ptr;
+  }
+  const size_t stage = (size_t)(GD_BM * (wlo ? 2 : 1) + p.bn * parts) * (size_t)bk * 2;
+  const int grid = items < ctx->sm_count ? (int)items : ctx->sm_count;
+  // A CTA with one item leaves room on its SM for one of the next linear, which starts to load its weights meanwhile; a
+  // CTA that walks over items takes what there is: 1 KB slack + 1 KB barriers + stages + 32 KB of staging fit 227 KB.
+  const size_t staging = 2048 * 4 * (size_t)(p.bn < 64 ? p.bn / 16 : 4);   // of the epilogue warps that have columns to store
+  int stages = (int)((items <= ctx->sm_count && M <= GD_SPLIT_ROWS ? 108 * 1024 - staging : GD_STAGE_BYTES) / stage);
+  if (stages > 8) stages = 8;
+  if (stages > p.cps) stages = p.cps;
+  if (stages < 2) stages = 2;
   a.stages = stages;
-  a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GD_BN >> 3) << 17) | ((uint32_t)(GD_BM >> 4) << 24);
-  const size_t smem = 2048 + stage * stages + (size_t)GD_EPI_WARPS * 2048;
-  const int grid = tiles < ctx->sm_count ? (int)tiles : ctx->sm_count;
+  a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(GD_BM >> 4) << 24);
+  a.tmem_cols = 32;
+  while (a.tmem_cols < (uint32_t)(p.bn * (items > grid ? 2 : 1))) a.tmem_cols *= 2;
+  const size_t smem = 2048 + stage * stages + staging;
 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
@@ -558,15 +657,17 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = take_pdl(ctx) ? 1 : 0;
-  if (nsplit == 3) {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_dense_kernel<3, false>, twh, twl, txh, txl, a));
-  } else {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_dense_kernel<1, false>, twh, twl, txh, txl, a));
-  }
+  auto kernel = nsplit == 1 ? gemm_dense_kernel<1, false, false> : wlo ? gemm_dense_kernel<3, false, true> : gemm_dense_kernel<3, false, false>;
+  CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, twh, twl, txh, txl, a));
   CB_LAUNCH_CHECK(ctx, "gemm_dense_kernel");
-  return 0;
+  if (p.splits == 1) return 0;
+  if (can_defer) {   // the consumer of this linear sums the shares itself (and adds bias and residual)
+    defer->part = a.part; defer->bias = bias; defer->splits = p.splits; defer->tiles_x = a.tiles_f; defer->bnx = p.bn;
+    defer->zstride = (long long)tiles * p.bn * GD_BM;
+    return 0;
+  }
+  return launch_splitk_reduce(ctx, a.part, p.splits, a.tiles_f, a.tiles, p.bn, bias, res, y, ybf, act, a.M, a.N, a.group_rows, a.tiles_per_group, a.ygroup, a.ldy);
 }
 
 int launch_gemm_experts(caten_b200_ctx *ctx, const caten_b200_weight *w, const ExpertRows &er, BfOut x, int act, float *y, BfOut ybf, int nsplit) {
@@ -586,15 +687,17 @@ int launch_gemm_experts(caten_b200_ctx *ctx, const caten_b200_weight *w, const E
   // twice the rows an expert has on average, so that most experts need one row tile
   int bn = 16;
   while (bn < GD_BN && (int64_t)bn * er.experts < 2 * er.pairs) bn *= 2;
-  a.bn = bn;
+  a.bn = bn; a.splits = 1; a.part = nullptr; a.static_w = 0;
+  a.tmem_cols = 512;
   a.er = er;
   const int bk = nsplit == 3 ? GdStage<3>::BK : GdStage<1>::BK;
+  a.cps = (int)(K / bk);
   CUtensorMap tw, txh, txl;
   if (int rc = make_map(ctx, &tw, w->qs, N, K, GD_BM, bk)) return rc;
   if (int rc = make_map(ctx, &txh, x.hi, er.pairs, K, bn, bk)) return rc;
   if (int rc = make_map(ctx, &txl, nsplit == 3 ? x.lo : x.hi, er.pairs, K, bn, bk)) return rc;
   const size_t stage = (size_t)bk * 2 * (GD_BM + (size_t)bn * (nsplit == 3 ? 2 : 1));
-  int stages = (int)((196 * 1024) / stage);
+  int stages = (int)((GD_STAGE_BYTES - (GD_MAX_EXPERTS + 1) * sizeof(int)) / stage);
   if (stages > 10) stages = 10;
   a.stages = stages;
   a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(GD_BM >> 4) << 24);
@@ -602,11 +705,11 @@ int launch_gemm_experts(caten_b200_ctx *ctx, const caten_b200_weight *w, const E
   const int64_t most = (er.pairs / bn + (er.pairs < er.experts ? er.pairs : er.experts)) * a.tiles_f;
   const int grid = most < ctx->sm_count ? (int)most : ctx->sm_count;
   if (nsplit == 3) {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_k(ctx, gemm_dense_kernel<3, true>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
+    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<3, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(ctx, gemm_dense_kernel<3, true, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
   } else {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_k(ctx, gemm_dense_kernel<1, true>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
+    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(ctx, gemm_dense_kernel<1, true, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
   }
   CB_LAUNCH_CHECK(ctx, "gemm_dense_kernel");
   return 0;

@@ -744,6 +744,15 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restr
   }
 }
 
+int launch_splitk_reduce(caten_b200_ctx *ctx, const float *part, int splits, int tiles_x, int tiles, int bnx, const float *bias, const float *res, float *y,
+                         BfOut ybf, int act, int M, int N, int group_rows, int tiles_per_group, int ygroup, int ldy) {
+  const int64_t total = (int64_t)tiles * bnx * (TC_BM / 4);
+  launch_k(ctx, splitk_reduce_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, part, splits, tiles_x, tiles, bnx, bias, res, y, ybf.hi, ybf.lo, act, M, N,
+           group_rows, tiles_per_group, ygroup, ldy);
+  CB_LAUNCH_CHECK(ctx, "splitk_reduce_kernel");
+  return 0;
+}
+
 // x -> bf16 hi (and lo) copies, row-major [M, K]
 __global__ void split_bf16_kernel(const float4 *__restrict__ x, uint2 *__restrict__ hi, uint2 *__restrict__ lo, int64_t n4) {
   pdl_enter();
@@ -875,7 +884,7 @@ static int run_tc(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x,
   // thousands of rows (prefill): expand the weights once, both operands through TMA
   // (its epilogue moves 16 bytes at a time: bias, residual and outputs must be aligned for that)
   const uintptr_t align_bits = (uintptr_t)bias | (uintptr_t)res | (uintptr_t)y | (uintptr_t)ybf.hi | (uintptr_t)ybf.lo;
-  if (gemm_dense_applies(ctx, M, N, K) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp);
+  if (gemm_dense_applies(ctx, wt, M, N, K) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp, defer);
   TcPlan p;
   // reduce inside a cluster: always (mode 1) or only when this launch needs its own epilogue (mode 2)
   const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && N % 4 == 0 && grp.plain_output() && grp.group_rows % TC_BM == 0;
@@ -933,11 +942,7 @@ static int run_tc(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x,
     defer->zstride = (long long)p.tiles * p.bnx * TC_BM;
     return 0;
   }
-  const int64_t total = p.tiles * p.bnx * (TC_BM / 4);
-  launch_k(ctx, splitk_reduce_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, a.part, p.splits, (int)p.gx, (int)p.tiles, p.bnx, bias,
-                                                                              res, y, a.yhi, a.ylo, act, (int)M, (int)N, a.group_rows, a.tiles_per_group, a.ygroup, a.ldy);
-  CB_LAUNCH_CHECK(ctx, "splitk_reduce_kernel");
-  return 0;
+  return launch_splitk_reduce(ctx, a.part, p.splits, (int)p.gx, (int)p.tiles, p.bnx, bias, res, y, ybf, act, (int)M, (int)N, a.group_rows, a.tiles_per_group, a.ygroup, a.ldy);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1005,11 +1010,7 @@ int launch_gemm_tc_noalloc(caten_b200_ctx *ctx, const caten_b200_weight *w, cons
   const dim3 grid((unsigned)p.gx, (unsigned)p.gy, (unsigned)p.splits);
   const int rc = launch_tc(ctx, w->type, nsplit, mh, ml, a, grid, smem);
   if (rc || p.splits == 1) return rc;
-  const int64_t total = p.tiles * p.bnx * (TC_BM / 4);
-  launch_k(ctx, splitk_reduce_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, a.part, p.splits, (int)p.gx, (int)p.tiles, p.bnx, bias,
-                                                                              res, y, a.yhi, a.ylo, act, (int)M, (int)N, a.group_rows, a.tiles_per_group, a.ygroup, a.ldy);
-  CB_LAUNCH_CHECK(ctx, "splitk_reduce_kernel");
-  return 0;
+  return launch_splitk_reduce(ctx, a.part, p.splits, (int)p.gx, (int)p.tiles, p.bnx, bias, res, y, BfOut(), act, (int)M, (int)N, a.group_rows, a.tiles_per_group, a.ygroup, a.ldy);
 }
 
 int launch_gemm_tc(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
