@@ -392,11 +392,7 @@ int caten_b200_linear(caten_b200_ctx *ctx, const caten_b200_weight *w, const flo
   if (!aligned16(d_x) || !aligned16(d_y)) return fail(ctx, CATEN_B200_EINVAL, "linear: x and y must be 16-byte aligned");
   ProfScope prof(ctx, M <= 4 ? CATEN_B200_K_GEMV : CATEN_B200_K_GEMM);
   if (M <= 4) {
-    for (int64_t m = 0; m < M; ++m)
-      if (int rc = launch_gemv(ctx, w, d_x + m * w->cols, d_bias, d_residual ? d_residual + m * ny : nullptr, act,
-                               d_y + m * ny))
-        return rc;
-    return 0;
+    return launch_gemv(ctx, w, d_x, d_bias, d_residual, act, d_y, M);
   }
   switch (precision) {
     case CATEN_B200_PREC_FP32: return launch_gemm_simt(ctx, w, d_x, d_bias, d_residual, act, d_y, M);
@@ -418,11 +414,7 @@ int caten_b200_linear_noalloc(caten_b200_ctx *ctx, const caten_b200_weight *w, c
   if (!aligned16(d_x) || !aligned16(d_y)) return fail(ctx, CATEN_B200_EINVAL, "linear_noalloc: x and y must be 16-byte aligned");
   ProfScope prof(ctx, M <= 4 ? CATEN_B200_K_GEMV : CATEN_B200_K_GEMM);
   if (M <= 4) {  // the dequant-GEMV uses no scratch memory
-    for (int64_t m = 0; m < M; ++m)
-      if (int rc = launch_gemv(ctx, w, d_x + m * w->cols, d_bias, d_residual ? d_residual + m * ny : nullptr, act,
-                               d_y + m * ny))
-        return rc;
-    return 0;
+    return launch_gemv(ctx, w, d_x, d_bias, d_residual, act, d_y, M);
   }
   switch (precision) {
     case CATEN_B200_PREC_FP32: return launch_gemm_simt(ctx, w, d_x, d_bias, d_residual, act, d_y, M);  // no scratch either
@@ -522,9 +514,7 @@ int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, cons
   if (res && !grp.plain_output()) return fail(ctx, CATEN_B200_EUNSUPPORTED, "linear: a residual needs the plain output layout");
   ProfScope prof(ctx, M <= 4 ? CATEN_B200_K_GEMV : CATEN_B200_K_GEMM);
   if (M <= 4) {
-    for (int64_t m = 0; m < M; ++m)
-      if (int rc = launch_gemv(ctx, w, x + m * w->cols, bias, res ? res + m * ny : nullptr, act, y + m * ny, grp)) return rc;
-    return 0;
+    return launch_gemv(ctx, w, x, bias, res, act, y, M, grp);
   }
   if (prec == CATEN_B200_PREC_FP32) return launch_gemm_simt(ctx, w, x, bias, res, act, y, M, grp);
   const int nsplit = prec == CATEN_B200_PREC_BF16X3 ? 3 : 1;

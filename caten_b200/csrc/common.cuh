@@ -210,7 +210,7 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
 int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, const float *kc, const float *vc, float *out, int64_t B,
                         int64_t s, int64_t n, int64_t H, int64_t T, cb::BfOut bf);
 int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
-                const float *res, int act, float *y, LinGroups grp = LinGroups());
+                const float *res, int act, float *y, int64_t M = 1, LinGroups grp = LinGroups());   // M: 1 to 4 rows of x
 int launch_gemm_simt(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
                      const float *res, int act, float *y, int64_t M, LinGroups grp = LinGroups());
 int launch_gemm_tc(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,

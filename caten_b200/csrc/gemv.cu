@@ -14,35 +14,37 @@ struct GemvArgs {
   const uint32_t *qh;    // fifth code bits (Q5_0, Q5_1)
   const float *x, *bias, *res;
   float *y;
-  int act, N, nkb, G;
+  int act, N, nkb, G, M;
 };
 
 constexpr int GEMV_MAX_THREADS = 512;
+constexpr int GEMV_XPAD = 36;   // floats between the 32-wide blocks of x in shared memory: eight threads' 16-byte reads cover all banks
 
 __device__ __forceinline__ uint4 ld_stream(const uint4 *p) { return __ldcs(p); }
 
-// Thread t < G*nkb owns column block kb = t % nkb and row offset ro = t / nkb; a CTA iteration
-// covers G*RI consecutive rows (RI independent 16/32-byte loads in flight per thread).  The
+// Thread t < G*nkb owns column block kb = t % nkb and row offset ro = t / nkb; a CTA covers G*RI consecutive rows (RI
+// independent 16/32-byte loads in flight per thread), once, or (LOOP) again and again with the next rows' loads ahead.  The
 // per-(row, block) partial sums go through shared memory and are added in a fixed order (lane
 // strided, then a butterfly), so results do not depend on scheduling.
-template <class BLK, int RI>
-__global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_blocked_kernel(GemvArgs a) {
-  extern __shared__ float red[];
-  // The packed weights depend on no other kernel: the first loads of this CTA's rows are issued
-  // before waiting for the kernel that produces x, so their HBM latency overlaps its tail.
+// A launch is a few microseconds of dependent latencies, so: the packed weights, which depend on no other kernel, are in
+// registers before the wait for x; x comes through shared memory (thread by thread from global memory, 128 bytes apart, it
+// took 256 L1 wavefronts a warp); small CTAs, three to an SM, leave the next launch room to load its own weights.
+// GPT-2 XL Q4_0, one sequence, us a linear inside a step: 6.3 to 7.6 -> 3.0 to 5.0.
+template <class BLK, int RI, bool LOOP, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK::WORDS > 16 ? 2 : 3) gemv_blocked_kernel(const GemvArgs a) {
+  extern __shared__ float gemv_smem[];
   pdl_launch_dependents();
   constexpr int W = BLK::WORDS;
   const int tid = threadIdx.x, nkb = a.nkb, G = a.G;
+  float *xs = gemv_smem;                              // [M][nkb][GEMV_XPAD]
+  float *red = gemv_smem + a.M * nkb * GEMV_XPAD;     // two buffers of [G * RI][nkb]
   const bool active = tid < G * nkb;
   const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
   const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
   const int rows_per_iter = G * RI;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = (blockDim.x + 31) >> 5;
+  const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   const int64_t stride = (int64_t)gridDim.x * rows_per_iter;
 
-  // The loads of iteration i+1 are issued before iteration i is reduced, and the partial sums
-  // alternate between two shared-memory buffers, so there is one barrier per iteration and the
-  // packed stream stays in flight across it.
   uint32_t qn[RI][W];
   float scn[RI], mnn[RI];
   uint32_t qhn[RI];
@@ -63,21 +65,23 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_blocked_kernel(GemvArgs
     }
   };
   int64_t base = (int64_t)blockIdx.x * rows_per_iter;
-  if (base < a.N) load(base);
+  load(base);
   pdl_wait();
+  for (int i = tid; i < a.M * nkb * 8; i += blockDim.x)
+    *reinterpret_cast<float4 *>(xs + (i >> 3) * GEMV_XPAD + (i & 7) * 4) = reinterpret_cast<const float4 *>(a.x)[i];
+  // what the warp adds to its rows (lane i: its i-th) is asked for before their sums are formed
+  auto addends = [&](int m, float *b, float *r) {
+    const int at = warp + lane * nwarps;
+    const bool has = at < rows_per_iter && base + at < a.N;
+    *b = has && a.bias ? a.bias[base + at] : 0.0f;
+    *r = has && a.res ? a.res[(int64_t)m * a.N + base + at] : 0.0f;
+  };
+  float bz, rz;
+  addends(0, &bz, &rz);
+  __syncthreads();
   BLK blk;
-  {
-    float xv[32];
-    const float4 *xp = reinterpret_cast<const float4 *>(a.x + (int64_t)kb * 32);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 v = xp[i];
-      xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
-    }
-    blk.prep(xv);
-  }
   int buf = 0;
-  for (; base < a.N; base += stride) {
+  for (bool again = false; base < a.N; base += stride, again = true) {
     uint32_t q[RI][W], qhc[RI];
     float sc[RI], mn[RI];
 #pragma unroll
@@ -88,48 +92,68 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_blocked_kernel(GemvArgs
 #pragma unroll
       for (int j = 0; j < W; ++j) q[i][j] = qn[i][j];
     }
-    if (base + stride < a.N) load(base + stride);
-    float *rb = red + buf * rows_per_iter * nkb;
-    if (active) {
+    if (LOOP && base + stride < a.N) load(base + stride);
+    for (int m = 0; m < a.M; ++m) {   // rows of x share the packed blocks
 #pragma unroll
       for (int i = 0; i < RI; ++i) {
-        float r;
-        if constexpr (BLK::HAS_M || BLK::HAS_QH) r = blk.dotx(q[i], sc[i], mn[i], qhc[i]);
-        else r = blk.dot(q[i], sc[i]);
-        rb[(i * G + ro) * nkb + kb] = r;
+        if (BLK::HAS_QH) asm volatile("" : "+r"(qhc[i]));
+#pragma unroll
+        for (int j = 0; j < W; ++j) asm volatile("" : "+r"(q[i][j]));   // unpacked again for every m: the codes would not fit unpacked
       }
-    }
-    __syncthreads();
-    for (int r = warp; r < rows_per_iter; r += nwarps) {
-      const int64_t row = base + r;
-      if (row >= a.N) break;
-      float s = 0.0f;
-      for (int k = lane; k < nkb; k += 32) s += rb[r * nkb + k];
-      s = warp_sum(s);
-      if (lane == 0) {
-        if (a.bias) s = s + a.bias[row];
-        s = apply_act(s, a.act);
-        if (a.res) s = a.res[row] + s;
-        a.y[row] = s;
+      if (again || m > 0) addends(m, &bz, &rz);
+      if (!again || a.M > 1) {
+        float xv[32];
+        const float4 *xp = reinterpret_cast<const float4 *>(xs + (m * nkb + kb) * GEMV_XPAD);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 v = xp[i];
+          xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
+        }
+        blk.prep(xv);
       }
+      float *rb = red + buf * rows_per_iter * nkb;
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < RI; ++i) {
+          float r;
+          if constexpr (BLK::HAS_M || BLK::HAS_QH) r = blk.dotx(q[i], sc[i], mn[i], qhc[i]);
+          else r = blk.dot(q[i], sc[i]);
+          rb[(i * G + ro) * nkb + kb] = r;
+        }
+      }
+      __syncthreads();
+      int t = 0;
+      for (int r = warp; r < rows_per_iter; r += nwarps, ++t) {
+        const int64_t row = base + r;
+        if (row >= a.N) break;
+        float s = 0.0f;
+        for (int k = lane; k < nkb; k += 32) s += rb[r * nkb + k];
+        s = warp_sum(s);
+        const float bt = __shfl_sync(0xffffffffu, bz, t & 31), rt = __shfl_sync(0xffffffffu, rz, t & 31);
+        if (lane == 0) {
+          if (a.bias) s = s + (t < 32 ? bt : a.bias[row]);
+          s = apply_act(s, a.act);
+          if (a.res) s = (t < 32 ? rt : a.res[(int64_t)m * a.N + row]) + s;
+          a.y[(int64_t)m * a.N + row] = s;
+        }
+      }
+      buf ^= 1;
     }
-    buf ^= 1;
+    if (!LOOP) break;
   }
 }
 
-// fp32 / fp16 / bf16 weights: one warp per row, RI rows in flight, x in shared memory.
+// fp32 / fp16 / bf16 weights.  16 bytes of a row as they are stored, and their fp32 values.
 template <typename T> struct DenseLoad;
 template <> struct DenseLoad<float> {
   static constexpr int VEC = 4;
-  __device__ static __forceinline__ void load(const float *p, float *o) {
-    const float4 v = __ldcs(reinterpret_cast<const float4 *>(p));
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+  __device__ static __forceinline__ void expand(const uint4 &v, float *o) {
+    o[0] = __uint_as_float(v.x); o[1] = __uint_as_float(v.y); o[2] = __uint_as_float(v.z); o[3] = __uint_as_float(v.w);
   }
 };
 template <> struct DenseLoad<__half> {
   static constexpr int VEC = 8;
-  __device__ static __forceinline__ void load(const __half *p, float *o) {
-    const uint4 v = __ldcs(reinterpret_cast<const uint4 *>(p));
+  __device__ static __forceinline__ void expand(const uint4 &v, float *o) {
     const __half2 *h = reinterpret_cast<const __half2 *>(&v);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -138,11 +162,9 @@ template <> struct DenseLoad<__half> {
     }
   }
 };
-
 template <> struct DenseLoad<__nv_bfloat16> {
   static constexpr int VEC = 8;
-  __device__ static __forceinline__ void load(const __nv_bfloat16 *p, float *o) {
-    const uint4 v = __ldcs(reinterpret_cast<const uint4 *>(p));
+  __device__ static __forceinline__ void expand(const uint4 &v, float *o) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -152,203 +174,261 @@ template <> struct DenseLoad<__nv_bfloat16> {
   }
 };
 
+// A launch of these lasts a few microseconds whatever the matrix, so what counts is the chain after the wait for x.  RI rows
+// are shared by `ks` warps (vectors of 16 bytes dealt out in turns), as many as let a lane hold its whole part of them:
+// GEMV_PRE loads, all asked for before the wait, and the next rows' before the sums of these are reduced.  Up to NR
+// rows of x are multiplied with a weight row read once.  Bias and residual are asked for beside x.  GPT-2 small fp32, one
+// sequence, us a linear inside a step: one load per lane before the wait and one launch per row of x 6.2, this 3.4.
 // blockIdx.y = group of `group_rows` output rows with an input plane of its own (one group: N rows).  EXPERTS: blockIdx.y
 // is a (token, expert) pair; expert[pair] says which group of rows it uses, its input is row pair / xplane, its products
 // are scaled by weight[pair].
-template <typename T, int RI, bool EXPERTS>
-__global__ void __launch_bounds__(256) gemv_dense_kernel(const T *__restrict__ W, const float *__restrict__ x,
-                                                         const float *__restrict__ bias, const float *__restrict__ res,
-                                                         float *__restrict__ y, int act, int N, int K, int group_rows, int64_t xplane, int64_t ygroup,
-                                                         const int *__restrict__ expert, const float *__restrict__ weight) {
-  extern __shared__ float xs[];
+constexpr int GEMV_PRE = 8;
+
+struct GemvDense {
+  const void *W;
+  const float *x, *bias, *res;
+  float *y;
+  int act, N, K, M, ks, group_rows;
+  int64_t xplane, ygroup, ldy;   // ldy: between the outputs of two rows of x
+  const int *expert;
+  const float *weight;
+};
+
+template <typename T, int RI, int NR, bool EXPERTS>
+__global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const GemvDense a) {
+  constexpr int PRE = GEMV_PRE;
+  extern __shared__ float xs[];   // [NR][K]
+  __shared__ float part[8][RI * NR];
+  const T *W = reinterpret_cast<const T *>(a.W);
+  const float *x = a.x, *bias = a.bias, *res = a.res;
+  float *y = a.y;
+  const int K = a.K;
+  int N = a.group_rows;
   float wt = 1.0f;
   if (EXPERTS) {
     pdl_enter();   // which rows to read comes from the kernel before
-    W += (int64_t)expert[blockIdx.y] * group_rows * K;
-    x += (int64_t)(blockIdx.y / xplane) * K;
-    y += (int64_t)blockIdx.y * ygroup;
-    if (weight) wt = weight[blockIdx.y];
-    N = group_rows;
+    W += (int64_t)a.expert[blockIdx.y] * a.group_rows * K;
+    x += (int64_t)(blockIdx.y / a.xplane) * K;
+    y += (int64_t)blockIdx.y * a.ygroup;
+    if (a.weight) wt = a.weight[blockIdx.y];
   } else {
-    const int64_t r0 = (int64_t)blockIdx.y * group_rows;
+    const int64_t r0 = (int64_t)blockIdx.y * a.group_rows;
     W += r0 * K;
-    x += (int64_t)blockIdx.y * xplane * K;
-    y += (int64_t)blockIdx.y * ygroup;
+    x += (int64_t)blockIdx.y * a.xplane * K;
+    y += (int64_t)blockIdx.y * a.ygroup;
     if (bias) bias += r0;
     if (res) res += r0;
-    N = N - r0 < group_rows ? (int)(N - r0) : group_rows;
+    if (a.N - r0 < N) N = (int)(a.N - r0);
+    pdl_launch_dependents();
   }
-  // weights depend on no other kernel: the first tile of this warp's rows is loaded before the
-  // wait for the producer of x
-  if (!EXPERTS) pdl_launch_dependents();
   constexpr int VEC = DenseLoad<T>::VEC;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nvec = K / VEC;
-  const int64_t first = ((int64_t)blockIdx.x * 8 + warp) * RI;
-  float w0[RI][VEC];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = a.ks;
+  const int slot = warp / ks, share = warp - slot * ks, slots = 8 / ks;
+  const int nvec = K / VEC, step = 32 * ks, c0 = share * 32 + lane;
+  uint4 w[RI][PRE];
+  auto load = [&](int64_t row, int c) {
 #pragma unroll
-  for (int i = 0; i < RI; ++i) {
-    if (first + i < N && lane < nvec) DenseLoad<T>::load(W + (first + i) * K + (int64_t)lane * VEC, w0[i]);
-    else {
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) w0[i][j] = 0.0f;
-    }
-  }
+      for (int u = 0; u < PRE; ++u)
+        w[i][u] = row + i < N && c + u * step < nvec ? __ldcs(reinterpret_cast<const uint4 *>(W + (row + i) * K) + c + u * step) : make_uint4(0, 0, 0, 0);
+  };
+  int64_t base = ((int64_t)blockIdx.x * slots + slot) * RI;
+  const int64_t stride = (int64_t)gridDim.x * slots * RI;
+  load(base, c0);
   if (!EXPERTS) pdl_wait();
-  for (int i = threadIdx.x; i < K; i += blockDim.x) xs[i] = x[i];
+  // the lane that finishes output (row base + i, row m of x) is lane i * NR + m of the slot's first warp
+  const int fi = lane / NR, fm = lane % NR;
+  const bool glu_rows = RI == 2 && act_is_glu(a.act);
+  const bool fin = share == 0 && lane < RI * NR && fm < a.M;
+  auto addends = [&](int64_t row, float *b, float *r) {
+    *b = fin && bias && row + fi < N ? bias[row + fi] : 0.0f;
+    *r = fin && res && row + fi < N ? res[fm * a.ldy + row + fi] : 0.0f;
+  };
+  float bz, rz;
+  addends(base, &bz, &rz);
+  for (int i = threadIdx.x; i < NR * K / 4; i += 256)
+    reinterpret_cast<float4 *>(xs)[i] = NR == 1 || i < a.M * K / 4 ? reinterpret_cast<const float4 *>(x)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
-  for (int64_t base = first; base < N; base += (int64_t)gridDim.x * 8 * RI) {
-    float acc[RI];
+  const int64_t rounds = ((int64_t)N + stride - 1) / stride;   // the same for every warp: the slots' warps meet at barriers
+  for (int64_t it = 0; it < rounds; ++it) {
+    float acc[RI][NR];
 #pragma unroll
-    for (int i = 0; i < RI; ++i) acc[i] = 0.0f;
-    int c = lane;
-    if (base == first && c < nvec) {  // the tile fetched before the wait
+    for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const float xv = xs[c * VEC + j];
+      for (int m = 0; m < NR; ++m) acc[i][m] = 0.0f;
+    for (int c = c0; c - c0 < nvec; c += PRE * step) {
+      if (c != c0) load(base, c);
 #pragma unroll
-        for (int i = 0; i < RI; ++i) acc[i] = fmaf(xv, w0[i][j], acc[i]);
-      }
-      c += 32;
-    }
-    // four tiles per lane in flight; the products are still added in increasing k
-    for (; c < nvec; c += 32 * 4) {
-      float wv[4][RI][VEC];
+      for (int u = 0; u < PRE; ++u) {
+        if (c + u * step >= nvec) break;
+        float wv[RI][VEC];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+        for (int i = 0; i < RI; ++i) DenseLoad<T>::expand(w[i][u], wv[i]);
 #pragma unroll
-        for (int i = 0; i < RI; ++i) {
-          if (c + 32 * u < nvec && base + i < N) {
-            DenseLoad<T>::load(W + (base + i) * K + (int64_t)(c + 32 * u) * VEC, wv[u][i]);
-          } else {
+        for (int m = 0; m < NR; ++m)
 #pragma unroll
-            for (int j = 0; j < VEC; ++j) wv[u][i][j] = 0.0f;
+          for (int q = 0; q < VEC / 4; ++q) {
+            const float4 xv = reinterpret_cast<const float4 *>(xs + (size_t)m * K)[(c + u * step) * (VEC / 4) + q];
+            const float xe[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int i = 0; i < RI; ++i) acc[i][m] = fmaf(xe[j], wv[i][4 * q + j], acc[i][m]);
           }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (c + 32 * u < nvec) {
-#pragma unroll
-          for (int j = 0; j < VEC; ++j) {
-            const float xv = xs[(c + 32 * u) * VEC + j];
-#pragma unroll
-            for (int i = 0; i < RI; ++i) acc[i] = fmaf(xv, wv[u][i][j], acc[i]);
-          }
-        }
       }
     }
-    if (RI == 2 && act_is_glu(act)) {  // rows (base, base + 1) are a (gate, up) pair: base is even
-      float g = warp_sum(acc[0]), u = warp_sum(acc[RI - 1]);
-      if (lane == 0 && base < N) {
-        if (bias) { g = g + bias[base]; u = u + bias[base + 1]; }
-        if (EXPERTS) { g = g * wt; u = u * wt; }
-        y[base >> 1] = glu(act, g, u);
-      }
-      continue;
+    const int64_t row = base + fi;
+    const float b = bz, r = rz;
+    base += stride;
+    if (it + 1 < rounds) {
+      load(base, c0);
+      addends(base, &bz, &rz);
     }
+    float mine = 0.0f;
 #pragma unroll
-    for (int i = 0; i < RI; ++i) {
-      float s = warp_sum(acc[i]);
-      const int64_t row = base + i;
-      if (lane == 0 && row < N) {
-        if (bias) s = s + bias[row];
-        if (EXPERTS) s = s * wt;
-        s = apply_act(s, act);
-        if (res) s = res[row] + s;
-        y[row] = s;
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+      for (int m = 0; m < NR; ++m) {
+        const float s = warp_sum(acc[i][m]);
+        if (lane == i * NR + m) mine = s;
+      }
+    if (ks > 1) {
+      if (lane < RI * NR) part[warp][lane] = mine;
+      __syncthreads();
+      if (share == 0 && lane < RI * NR)
+        for (int q = 1; q < ks; ++q) mine += part[warp + q][lane];
+    }
+    if (share == 0) {   // (whole warps)
+      float s = bias ? mine + b : mine;
+      if (EXPERTS) s = s * wt;
+      if (glu_rows) {  // rows (base, base + 1) are a (gate, up) pair: base is even
+        const float up = __shfl_sync(0xffffffffu, s, (lane + NR) & 31);
+        if (lane < NR && fin && row < N) y[fm * a.ldy + (row >> 1)] = glu(a.act, s, up);
+      } else if (fin && row < N) {
+        s = apply_act(s, a.act);
+        if (res) s = r + s;
+        y[fm * a.ldy + row] = s;
       }
     }
+    if (ks > 1) __syncthreads();   // before the partial sums are written again
   }
 }
 
-template <class BLK, int RI>
-static int launch_blocked(caten_b200_ctx *ctx, const GemvArgs &a) {
-  const int threads = ((a.G * a.nkb + 31) / 32) * 32;
-  const size_t smem = 2 * (size_t)a.G * RI * a.nkb * sizeof(float);
-  int occ = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemv_blocked_kernel<BLK, RI>, threads, smem);
-  if (occ < 1) occ = 1;
-  const int64_t slabs = ((int64_t)a.N + a.G * RI - 1) / (a.G * RI);
-  int64_t grid = (int64_t)ctx->sm_count * occ;
-  if (grid > slabs) grid = slabs;
-  launch_k(ctx, gemv_blocked_kernel<BLK, RI>, dim3((unsigned)grid), dim3(threads), smem, a);
+template <class BLK, int RI, bool LOOP, int THREADS>
+static int launch_blocked_t(caten_b200_ctx *ctx, GemvArgs a) {
+  a.G = THREADS / a.nkb;
+  const int threads = (a.G * a.nkb + 31) / 32 * 32;
+  const size_t smem = ((size_t)a.M * a.nkb * GEMV_XPAD + 2 * (size_t)a.G * RI * a.nkb) * sizeof(float);
+  auto kernel = gemv_blocked_kernel<BLK, RI, LOOP, THREADS>;
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int64_t grid = ((int64_t)a.N + a.G * RI - 1) / (a.G * RI);
+  if (LOOP) {
+    const int occ = THREADS > 256 || smem > 100 * 1024 ? 1 : 2;
+    if (grid > (int64_t)ctx->sm_count * occ) grid = (int64_t)ctx->sm_count * occ;
+  }
+  launch_k(ctx, kernel, dim3((unsigned)grid), dim3(threads), smem, a);
   CB_LAUNCH_CHECK(ctx, "gemv_blocked_kernel");
   return 0;
 }
 
+template <class BLK>
+static int launch_blocked(caten_b200_ctx *ctx, const GemvArgs &a) {
+  if (a.nkb > 256) return launch_blocked_t<BLK, 1, true, 512>(ctx, a);
+  // one pass while the rows fit the resident CTAs (three to an SM where the blocks in flight leave the registers for it) with
+  // up to eight loads per thread; more rows: CTAs that go on
+  const int64_t slab = (int64_t)(256 / a.nkb) * ctx->sm_count;
+  const bool small = (size_t)a.M * a.nkb * GEMV_XPAD * sizeof(float) < 60 * 1024;
+  const int deep = 16 / BLK::WORDS;   // loads per thread with three CTAs
+  if (a.N <= (small ? 3 : 1) * slab) return launch_blocked_t<BLK, 1, false, 256>(ctx, a);
+  if (a.N <= (small ? 3 : 1) * 2 * slab) return launch_blocked_t<BLK, 2, false, 256>(ctx, a);
+  if (a.N <= (small ? deep >= 4 ? 3 : 2 : 1) * 4 * slab) return launch_blocked_t<BLK, 4, false, 256>(ctx, a);
+  return launch_blocked_t<BLK, 4, true, 256>(ctx, a);
+}
+
+template <typename T, int RI, int NR, bool EXPERTS>
+static int launch_dense_t(caten_b200_ctx *ctx, GemvDense g, int groups) {
+  const int nvec = g.K / DenseLoad<T>::VEC;
+  // warps per RI rows: so many that a lane's share of a row is loaded at once, and more while the CTAs do not fill the
+  // GPU twice and every lane still has two vectors
+  int ks = 1;
+  while (ks < 8 && (nvec > 32 * GEMV_PRE * ks || (nvec > 64 * ks && ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI) * groups < 2 * ctx->sm_count))) ks *= 2;
+  g.ks = ks;
+  const int64_t ctas = ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI);
+  const size_t smem = (size_t)NR * g.K * sizeof(float);
+  auto kernel = gemv_dense_kernel<T, RI, NR, EXPERTS>;
+  if (smem > 47 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int64_t grid = ((int64_t)ctx->sm_count * (smem > 72 * 1024 || RI == 2 ? 2 : 3) + groups - 1) / groups;   // resident at once
+  if (grid > ctas) grid = ctas;
+  launch_k(ctx, kernel, dim3((unsigned)grid, (unsigned)groups), dim3(256), smem, g);
+  CB_LAUNCH_CHECK(ctx, "gemv_dense_kernel");
+  return 0;
+}
+
+template <typename T, bool EXPERTS>
+static int launch_dense(caten_b200_ctx *ctx, const GemvDense &g, int groups) {
+  if (g.K % DenseLoad<T>::VEC) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols %d not a multiple of %d", g.K, DenseLoad<T>::VEC);
+  // two rows per warp when they are a pair or one row per warp would need more CTAs than are resident
+  const bool two = act_is_glu(g.act) || ((int64_t)g.group_rows + 7) / 8 * groups > 4 * ctx->sm_count;
+  if constexpr (EXPERTS) return two ? launch_dense_t<T, 2, 1, true>(ctx, g, groups) : launch_dense_t<T, 1, 1, true>(ctx, g, groups);
+  else {
+    if (g.M == 1) return two ? launch_dense_t<T, 2, 1, false>(ctx, g, groups) : launch_dense_t<T, 1, 1, false>(ctx, g, groups);
+    if (g.M == 2) return two ? launch_dense_t<T, 2, 2, false>(ctx, g, groups) : launch_dense_t<T, 1, 2, false>(ctx, g, groups);
+    return two ? launch_dense_t<T, 2, 4, false>(ctx, g, groups) : launch_dense_t<T, 1, 4, false>(ctx, g, groups);
+  }
+}
+
+// M rows of x, 1 to 4
 int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
-                const float *res, int act, float *y, LinGroups grp) {
+                const float *res, int act, float *y, int64_t M, LinGroups grp) {
   if (w->rows > 0x7fffffff || w->cols > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: dimension too large");
   const int N = (int)w->rows, K = (int)w->cols;
+  if (!type_is_packed(w->type) && (size_t)K * sizeof(float) > 160 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide", K);
+  if (M > 1 && (M > 4 || (size_t)K * 4 * sizeof(float) > 160 * 1024)) {   // rows of x that do not fit shared memory together: one by one
+    const int64_t ny = grp.ldy ? grp.ldy : act_is_glu(act) ? N / 2 : N;
+    for (int64_t m = 0; m < M; ++m)
+      if (int rc = launch_gemv(ctx, w, x + m * K, bias, res ? res + m * ny : nullptr, act, y + m * ny, 1, grp)) return rc;
+    return 0;
+  }
   if (type_is_packed(w->type)) {
     if (grp.group_rows || act_is_glu(act)) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: input groups and the gated activation take dense weights");
     GemvArgs a;
     a.qs = w->qs; a.d = w->d; a.m = w->m; a.qh = w->qh; a.x = x; a.bias = bias; a.res = res; a.y = y; a.act = act; a.N = N;
-    a.nkb = (int)w->nkb;
+    a.nkb = (int)w->nkb; a.M = (int)M;
     if (a.nkb > GEMV_MAX_THREADS) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide (max %d)", K, GEMV_MAX_THREADS * 32);
-    a.G = GEMV_MAX_THREADS / a.nkb;
-    // few rows: keep every SM busy with single-row-group iterations; many rows: 4 loads in flight
-    const bool deep = (int64_t)N >= (int64_t)a.G * 4 * ctx->sm_count;
     switch (w->type) {
-      case CATEN_B200_Q4_0: return deep ? launch_blocked<BlkQ4, 4>(ctx, a) : launch_blocked<BlkQ4, 1>(ctx, a);
-      case CATEN_B200_Q4_1: return deep ? launch_blocked<BlkQ41, 4>(ctx, a) : launch_blocked<BlkQ41, 1>(ctx, a);
-      case CATEN_B200_Q5_0: return deep ? launch_blocked<BlkQ5<false>, 4>(ctx, a) : launch_blocked<BlkQ5<false>, 1>(ctx, a);
-      case CATEN_B200_Q5_1: return deep ? launch_blocked<BlkQ5<true>, 4>(ctx, a) : launch_blocked<BlkQ5<true>, 1>(ctx, a);
-      default: return deep ? launch_blocked<BlkQ8, 4>(ctx, a) : launch_blocked<BlkQ8, 1>(ctx, a);
+      case CATEN_B200_Q4_0: return launch_blocked<BlkQ4>(ctx, a);
+      case CATEN_B200_Q4_1: return launch_blocked<BlkQ41>(ctx, a);
+      case CATEN_B200_Q5_0: return launch_blocked<BlkQ5<false>>(ctx, a);
+      case CATEN_B200_Q5_1: return launch_blocked<BlkQ5<true>>(ctx, a);
+      default: return launch_blocked<BlkQ8>(ctx, a);
     }
   }
-  const size_t smem = (size_t)K * sizeof(float);
-  if (smem > 160 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide", K);
+  GemvDense g;
+  g.W = w->qs; g.x = x; g.bias = bias; g.res = res; g.y = y; g.act = act; g.N = N; g.K = K; g.M = (int)M;
+  g.group_rows = grp.group_rows > 0 ? (int)grp.group_rows : N;
+  g.xplane = grp.xplane; g.ygroup = grp.ygroup ? grp.ygroup : act_is_glu(act) ? g.group_rows / 2 : g.group_rows;
+  g.ldy = grp.ldy ? grp.ldy : act_is_glu(act) ? N / 2 : N;
+  g.expert = nullptr; g.weight = nullptr;
   const int ng = grp.group_rows > 0 ? (int)((N + grp.group_rows - 1) / grp.group_rows) : 1;
-  const int rows = grp.group_rows > 0 ? (int)grp.group_rows : N;  // per group
-  // two rows per warp when that still gives every SM a CTA (or the rows are pairs), else one row per warp (more CTAs)
-  const int64_t ygroup = grp.ygroup ? grp.ygroup : rows;
-  const bool two = act_is_glu(act) || ((int64_t)rows + 15) / 16 * ng >= ctx->sm_count;
-  const int64_t groups = two ? ((int64_t)rows + 15) / 16 : ((int64_t)rows + 7) / 8;
-  int64_t grid = ((int64_t)ctx->sm_count * 4 + ng - 1) / ng;
-  if (grid > groups) grid = groups;
-#define GEMV_DENSE(T, CT)                                                                                                        \
-  do {                                                                                                                           \
-    if (K % DenseLoad<CT>::VEC) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv " T ": cols %% %d != 0", DenseLoad<CT>::VEC);    \
-    if (smem > 48 * 1024) {                                                                                                      \
-      cudaFuncSetAttribute(gemv_dense_kernel<CT, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
-      cudaFuncSetAttribute(gemv_dense_kernel<CT, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);             \
-    }                                                                                                                            \
-    const dim3 g((unsigned)grid, (unsigned)ng);                                                                                  \
-    if (two) launch_k(ctx, gemv_dense_kernel<CT, 2, false>, g, dim3(256), smem, (const CT *)w->qs, x, bias, res, y, act, N, K, rows, grp.xplane, ygroup, nullptr, nullptr); \
-    else launch_k(ctx, gemv_dense_kernel<CT, 1, false>, g, dim3(256), smem, (const CT *)w->qs, x, bias, res, y, act, N, K, rows, grp.xplane, ygroup, nullptr, nullptr);     \
-  } while (0)
   switch (w->type) {
-    case CATEN_B200_F32: GEMV_DENSE("f32", float); break;
-    case CATEN_B200_F16: GEMV_DENSE("f16", __half); break;
-    case CATEN_B200_BF16: GEMV_DENSE("bf16", __nv_bfloat16); break;
+    case CATEN_B200_F32: return launch_dense<float, false>(ctx, g, ng);
+    case CATEN_B200_F16: return launch_dense<__half, false>(ctx, g, ng);
+    case CATEN_B200_BF16: return launch_dense<__nv_bfloat16, false>(ctx, g, ng);
     default: return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: weight type %d", w->type);
   }
-#undef GEMV_DENSE
-  CB_LAUNCH_CHECK(ctx, "gemv_dense_kernel");
-  return 0;
 }
 
 int launch_gemv_experts(caten_b200_ctx *ctx, const caten_b200_weight *w, int64_t rows, const float *x, const int *expert, const float *weight,
                         int64_t pairs, int xdiv, int act, float *y) {
   if (pairs <= 0) return 0;
   const int64_t K = w->cols;
-  const size_t smem = (size_t)K * sizeof(float);
   if (w->type != CATEN_B200_BF16 || K % 8 || rows % 2) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: experts take BF16 weights");
-  if (smem > 160 * 1024 || pairs > 65535) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%lld or %lld pairs", (long long)K, (long long)pairs);
-  const bool two = act_is_glu(act) || (rows + 15) / 16 * pairs >= ctx->sm_count;
-  const int64_t groups = two ? (rows + 15) / 16 : (rows + 7) / 8;
-  int64_t grid = ((int64_t)ctx->sm_count * 4 + pairs - 1) / pairs;
-  if (grid > groups) grid = groups;
-  const dim3 g((unsigned)grid, (unsigned)pairs);
-  const float *none = nullptr;
-  const int64_t ld = act_is_glu(act) ? rows / 2 : rows;
-  auto kernel = two ? gemv_dense_kernel<__nv_bfloat16, 2, true> : gemv_dense_kernel<__nv_bfloat16, 1, true>;
-  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_k(ctx, kernel, g, dim3(256), smem, (const __nv_bfloat16 *)w->qs, x, none, none, y, act, (int)rows, (int)K, (int)rows, (int64_t)xdiv, ld, expert, weight);
-  CB_LAUNCH_CHECK(ctx, "gemv_dense_kernel");
-  return 0;
+  if (K > 40 * 1024 || pairs > 65535) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%lld or %lld pairs", (long long)K, (long long)pairs);
+  GemvDense g;
+  g.W = w->qs; g.x = x; g.bias = g.res = nullptr; g.y = y; g.act = act; g.N = g.group_rows = (int)rows; g.K = (int)K; g.M = 1;
+  g.xplane = xdiv; g.ygroup = g.ldy = act_is_glu(act) ? rows / 2 : rows; g.expert = expert; g.weight = weight;
+  return launch_dense<__nv_bfloat16, true>(ctx, g, (int)pairs);
 }
 
 }  // namespace cb
