@@ -403,9 +403,9 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     return 0;
   }
   if (d_n) return fail(ctx, CATEN_B200_EINVAL, "attention: a device-side position is only supported for single-token steps");
+  if (tensor_cores) return launch_attention_tc(ctx, qkv, kc, vc, out, B, s, n, H, T, bf);
   launch_k(ctx, kv_append_kernel, dim3((unsigned)(B * s)), dim3(128), 0, qkv, kc, vc, (int)s, (int)n, (int)H, (int)T);
   CB_LAUNCH_CHECK(ctx, "kv_append_kernel");
-  if (tensor_cores) return launch_attention_tc(ctx, qkv, kc, vc, out, B, s, n, H, T, bf);
   const size_t smem = 4 * 64 * PF_LD * sizeof(float);
   CB_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_k(ctx, attn_prefill_kernel, dim3((unsigned)((s + 63) / 64), (unsigned)H, (unsigned)B), dim3(256), smem, 

@@ -8,32 +8,28 @@
 // q.K^T keeps all four products, P.V drops only lo*lo), so the result stays within about 2^-16
 // of the fp32 one.
 //
-// One CTA = 128 queries of one (sequence, head) = the 128 lanes of tensor memory; keys go in
-// steps of 64 (with a window: from the step that holds the first key any of the tile's queries sees).
-// With NQ = NE = 1 a CTA uses 256 of the 512 TMEM columns and under half of the shared memory, so two
-// CTAs share an SM and one's MMAs overlap the other's softmax.  Per step:
-//   all 8 warps  copy the NEXT step's K (and V) rows from the cache into a staging buffer in shared
-//                memory (cp.async, 16 bytes per thread, coalesced; in flight during this step's
-//                MMAs and softmax), and split the current step's staged rows into bf16 hi/lo,
-//                stored as 128-byte-swizzled K-major tiles in shared memory:
-//                K tiles  = 64 keys x 64 dims, hi and lo, per block  (K-major B operands of S = Q.K^T)
-//                V tiles  = 64 keys x 64 dims, hi and lo, per block  (MN-major B operands of O += P.V)
-//   one thread   issues S[128 x 64] = (Q_hi + Q_lo) . (K_hi + K_lo)^T as four MMAs per 16 dims into
-//                the same 64 columns (Q tile in shared memory)
-//   all 8 warps  read their query's scores from tensor memory (warps w and w+4 share lanes and
-//                take 32 keys each), mask, and
-//                p = exp2((s - max)/ln2), accumulate the row sum, split p into bf16 hi/lo and
-//                write it back to tensor memory as the A operand of the second product
-//   one thread   issues O[128 x 64] += P_hi.V_hi + P_lo.V_hi + P_hi.V_lo, accumulating over the
-//                key steps in tensor memory
+// Two kernels.  attn_tiles_kernel splits the visible keys and values into bf16 hi/lo once per call and leaves them as the
+// operand tiles of the second kernel, 64 keys each, byte for byte as they lie in shared memory (128-byte swizzle), so that a
+// tile is one contiguous bulk copy; for GPT-2 it also appends the step's keys and values to the cache.  (Every query tile of
+// every query head used to convert the same rows again: 32 times for grouped heads at 1024 tokens.)
+// attn_prefill_tc_kernel: one CTA = 128 queries of one (sequence, head) = the 128 lanes of tensor memory; keys go in steps
+// of 64 (with a window: from the step that holds the first key any of the tile's queries sees).  By warp:
+//   warp 8       one lane asks for the K and V tiles of the steps ahead (two stages each)
+//   warp 9       issues S[128 x 64] = (Q_hi + Q_lo) . (K_hi + K_lo)^T, four MMAs per 16 dims, into one of TWO blocks of
+//                tensor memory, a step ahead of the softmax, and O[128 x 64 NE] += P_hi.V_hi + P_lo.V_hi + P_hi.V_lo
+//   warps 0..7   read their query's scores (warps w and w + 4 share lanes and take 32 keys each), mask, take
+//                p = exp2((s - max)/ln2), accumulate the row sum, split p into bf16 hi/lo and write it back to tensor
+//                memory as the A operand of the second product
+// so that the scores of step i + 1 and the output of step i - 1 are computed while the softmax of step i runs.  The softmax is
+// what a step waits for (about 2.5 k cycles against 1.8 k of MMAs); with the phases one after the other, conversion included,
+// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 183 us and 13 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
+// 40 us for the append -> 136 us and 72 us for append and tiles.
 // The softmax is single-pass with a lazily moved reference maximum: each step exchanges the
 // maximum of its visible scores between the row's two threads; the reference only moves (and O and
 // the row sum are rescaled, O by a TMEM load / multiply / store) when a step exceeds it by more
 // than AT_TAU, which in causal attention happens in the first steps and then rarely.  Softmax is
-// invariant to the reference, so this equals the reference's two-pass form up to rounding.  The
-// phases of a step are sequential within the CTA (block-wide barriers + one mbarrier the MMAs
-// commit to).
-// TMEM columns: [0,64) S, [128,192) P (hi 32, lo 32), [192, 192 + 64 NE) O.
+// invariant to the reference, so this equals the reference's two-pass form up to rounding.
+// TMEM columns: [0,64) and [64,128) S, [128,192) P (hi 32, lo 32), [192, 192 + 64 NE) O.
 //
 // The mbarrier waits are bounded; when one runs out the CTA records it in the context's status
 // word, skips the remaining work and its output, frees its tensor memory and returns.
@@ -49,26 +45,19 @@ constexpr int AT_Q = 128;                        // queries per CTA (MMA M)
 constexpr int AT_K = 64;                         // keys per step
 constexpr float AT_TAU = 8.0f;                   // slack of the running maximum, in units of the score
 constexpr uint32_t AT_COL_S = 0, AT_COL_P = 128, AT_COL_O = 192;
+constexpr int AT_SOFTMAX_WARPS = 8, AT_THREADS = (AT_SOFTMAX_WARPS + 2) * 32;
+constexpr size_t AT_TILES_BYTES = (size_t)256 << 20;   // tiles of as many sequences as fit here are made at a time
 template <int NQ, int NE> struct AtLayout {
   static constexpr uint32_t COLS = NE == 1 ? 256 : 512;  // TMEM columns per CTA (a power of two)
-  // Q: per block 128 rows hi, 128 rows lo (16 KB each); K, V: per block 64 rows hi, 64 rows lo (8 KB each)
-  static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * 32768, OFF_V = OFF_K + NQ * 16384, OFF_SK = OFF_V + NE * 16384;
-  // staging of the raw fp32 rows: 256 bytes per block and row, padded by 16, so that threads reading one
-  // row each (16 bytes at a time) spread over all banks
-  static constexpr uint32_t LD_K = NQ * 256 + 16, LD_V = NE * 256 + 16;
-  static constexpr uint32_t OFF_SV = OFF_SK + AT_K * LD_K, OFF_MISC = OFF_SV + AT_K * LD_V;
-  // tiles + staging + exchange buffer + barrier / TMEM slot / abort flag + alignment slack
-  static constexpr size_t SMEM = OFF_MISC + 1024 + 64 + 1024;
+  // Q: per block 128 rows hi, 128 rows lo (16 KB each); K, V: per block 64 rows hi, 64 rows lo (8 KB each), two stages
+  static constexpr uint32_t K_BYTES = NQ * 16384, V_BYTES = NE * 16384, TILE = K_BYTES + V_BYTES;
+  static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * 32768, OFF_V = OFF_K + 2 * K_BYTES, OFF_MISC = OFF_V + 2 * V_BYTES;
+  // tiles + exchange of the rows' maxima (2 steps) + barriers, TMEM slot, abort flag + alignment slack
+  static constexpr size_t SMEM = OFF_MISC + 2048 + 160 + 1024;
   static constexpr int CTAS = NQ == 1 && NE == 1 ? 2 : 1;  // per SM
 };
 static_assert(2 * (AtLayout<1, 1>::SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
 static_assert(AtLayout<2, 2>::SMEM <= 227 * 1024, "one CTA per SM");
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes) {  // src_bytes 0: zero fill
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // byte offset of 16-byte chunk `chunk` (0..7) of row `row` in a K-major tile with 128-byte rows
 // and the 128-byte swizzle (8-row groups of 1024 bytes)
@@ -97,107 +86,119 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-template <int N> struct IntC { static constexpr int value = N; };
-
 __device__ __forceinline__ float4 scale4(float4 v, float c) { return make_float4(v.x * c, v.y * c, v.z * c, v.w * c); }
+
+// first 64-key tile that a query of the step sees
+__host__ __device__ inline int at_first_tile(const AttnArgs &p) {
+  const int first = p.window > 0 ? p.n - p.window + 1 : 0;
+  return first > 0 ? first / AT_K : 0;
+}
 
 }  // namespace
 
-// PLAIN: heads of exactly 64, no window, a cache that never wraps (GPT-2): the masks' lower ends, the ring arithmetic and
+// One CTA = one tile of one key/value head: 64 rows of K and V -> hi and lo operand tiles; rows past the context and
+// columns past the head are zero.  PLAIN (GPT-2): rows of this step come from the projections and go to the cache as well.
+template <int NQ, int NE, bool PLAIN>
+__global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b0, uint8_t *__restrict__ tiles) {
+  using Lay = AtLayout<NQ, NE>;
+  pdl_enter();
+  const int g = blockIdx.y, b = b0 + blockIdx.z, t = p.n + p.s, j0 = (at_first_tile(p) + blockIdx.x) * AT_K;
+  uint8_t *dst = tiles + (((int64_t)blockIdx.z * p.G + g) * gridDim.x + blockIdx.x) * Lay::TILE;
+  const int64_t head = (int64_t)b * p.G + g;
+  const float *kx = !PLAIN && p.kx ? p.kx + b * p.cap * p.kx_ld - p.kx_from : nullptr;   // column c of the key, c >= kx_from
+  constexpr int KP = AT_K * NQ * 8, PIECES = KP + AT_K * NE * 8;   // pieces of eight floats
+#pragma unroll
+  for (int i0 = 0; i0 < PIECES; i0 += 256) {
+    const int i = i0 + threadIdx.x;
+    const bool key = i < KP;
+    const int nb = key ? NQ : NE, at = key ? i : i - KP;
+    const int row = at / (8 * nb), c8 = at % (8 * nb), j = j0 + row;
+    float4 v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int c = 8 * c8 + 4 * u;
+      const float *src = nullptr;
+      float *keep = nullptr;
+      if (PLAIN) {
+        if (j < t) {
+          keep = (key ? p.kc : p.vc) + (head * p.cap + j) * 64 + c;
+          src = keep;
+          if (j >= p.n) src = p.qkv + ((int64_t)b * p.s + j - p.n) * p.ld + (key ? p.k_off : p.v_off) + g * 64 + c;
+          else keep = nullptr;
+        }
+      } else if (j < t && c < (key ? p.Dp : p.Ep)) {
+        const int64_t slot = j % p.cap;
+        if (key && c >= p.kx_from) src = kx + slot * p.kx_ld + c;
+        else src = key ? p.kc + b * p.k_seq + g * p.k_head + slot * p.k_ld + c : p.vc + b * p.v_seq + g * p.v_head + slot * p.v_ld + c;
+      }
+      v[u] = src ? *reinterpret_cast<const float4 *>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (PLAIN && keep) *reinterpret_cast<float4 *>(keep) = v[u];
+    }
+    st_split8(dst + (key ? 0 : Lay::K_BYTES) + (c8 >> 3) * 16384, row, AT_K + row, c8 & 7, v[0], v[1]);
+  }
+}
+
+// PLAIN: heads of exactly 64, no window, a cache that never wraps (GPT-2): the masks' lower ends and
 // the zero-filled head columns compile away.
 template <int NQ, int NE, bool PLAIN>
-__global__ void __launch_bounds__(256, AtLayout<NQ, NE>::CTAS) attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t idesc_n64) {
+__global__ void __launch_bounds__(AT_THREADS, AtLayout<NQ, NE>::CTAS)
+attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t idesc_n64, int b0, const uint8_t *__restrict__ tiles, int ntiles) {
   using Lay = AtLayout<NQ, NE>;
-  constexpr uint32_t AT_OFF_Q = Lay::OFF_Q, AT_OFF_K = Lay::OFF_K, AT_OFF_V = Lay::OFF_V, AT_OFF_SK = Lay::OFF_SK, AT_OFF_SV = Lay::OFF_SV, AT_OFF_MISC = Lay::OFF_MISC;
   extern __shared__ unsigned char at_raw[];
   unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(at_raw) + 1023) & ~(uintptr_t)1023);
-  float *red = reinterpret_cast<float *>(sm + AT_OFF_MISC);
-  const uint32_t bar = smem_u32(sm + AT_OFF_MISC + 1024);
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + AT_OFF_MISC + 1024 + 8);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + AT_OFF_MISC + 1024 + 12);
+  float *red = reinterpret_cast<float *>(sm + Lay::OFF_MISC);   // [step & 1][half][row]
+  const uint32_t bars = smem_u32(sm + Lay::OFF_MISC + 2048);
+  auto k_full = [&](int i) { return bars + 8u * i; };
+  auto k_empty = [&](int i) { return bars + 16u + 8u * i; };
+  auto v_full = [&](int i) { return bars + 32u + 8u * i; };
+  auto v_empty = [&](int i) { return bars + 48u + 8u * i; };
+  auto s_full = [&](int i) { return bars + 64u + 8u * i; };
+  auto s_empty = [&](int i) { return bars + 80u + 8u * i; };
+  const uint32_t p_full = bars + 96u, pv_done = bars + 104u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + Lay::OFF_MISC + 2048 + 112);
+  // [0] some role gave up a wait; [1] never set (for waits that must run their full limit)
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Lay::OFF_MISC + 2048 + 120);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int quad = warp & 3;  // 32-lane quadrant of tensor memory this warp may access
   const int hf = warp >> 2;   // which half (of a step's keys / of a block's head dims) this thread takes
   const int r = quad * 32 + lane;  // query row within the tile = TMEM lane
-  const int ck = tid & 63, cq = tid >> 6;  // conversion: key row of the step, and which 16 of a block's 64 dims
-  const int q0 = (int)(gridDim.x - 1 - blockIdx.x) * AT_Q;  // tiles with the longest history first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int q0 = (int)(gridDim.z - 1 - blockIdx.z) * AT_Q;  // of all heads, the tiles with the longest history first
+  const int h = blockIdx.x, b = b0 + blockIdx.y;
   const int s = p.s, n = p.n, t = n + s;
 
   if (tid == 0) {
-    mbar_init(bar, 1);
-    *abort_flag = 0;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(k_full(i), 1);
+      mbar_init(k_empty(i), 1);
+      mbar_init(v_full(i), 1);
+      mbar_init(v_empty(i), 1);
+      mbar_init(s_full(i), 1);
+      mbar_init(s_empty(i), AT_SOFTMAX_WARPS);
+    }
+    mbar_init(p_full, AT_SOFTMAX_WARPS);
+    mbar_init(pv_done, 1);
+    abort_flag[0] = 0;
+    abort_flag[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
+  if (warp == 9) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(Lay::COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
-  pdl_enter();
+  pdl_wait();
 
   const int Dp = PLAIN ? 64 : p.Dp, Ep = PLAIN ? 64 : p.Ep;
-  const int64_t head = (int64_t)b * p.G + (PLAIN ? h : h / (p.H / p.G));  // the key/value head this query head reads
-  const int64_t kv_head = head - (int64_t)b * p.G;
-  const float *kb = PLAIN ? p.kc + head * p.cap * 64 : p.kc + b * p.k_seq + kv_head * p.k_head;
-  const float *vb = PLAIN ? p.vc + head * p.cap * 64 : p.vc + b * p.v_seq + kv_head * p.v_head;
-  const float *kx = !PLAIN && p.kx ? p.kx + b * p.cap * p.kx_ld - p.kx_from : nullptr;   // column c of the key, c >= kx_from
   const int W = !PLAIN && p.window > 0 ? p.window : 0x3fffffff;
   const int kend = min(t, n + q0 + AT_Q);  // keys beyond the last query of this tile are masked
   const int kfirst = PLAIN ? 0 : n + q0 - W + 1;       // first key the tile's first query sees
-  const int kbeg = kfirst > 0 ? kfirst / AT_K * AT_K : 0;
-  const int nblk = (kend - kbeg + AT_K - 1) / AT_K;
-  const int qi = min(q0 + r, s - 1);  // rows past the end of the step mask like the last row (their output is dropped)
-  const int jmax = n + qi;            // last visible key of this query (< t)
-  const int jmin = jmax - W + 1;      // first visible key (may be negative)
-
-  const uint64_t dq = umma_desc(smem_u32(sm + AT_OFF_Q)), dk = umma_desc(smem_u32(sm + AT_OFF_K)), dv = umma_desc(smem_u32(sm + AT_OFF_V));
-  const uint32_t idesc_pv = idesc_n64 | (1u << 16);  // B operand MN-major: V rows (keys) with the dims contiguous
-  const int ksteps = Dp / 16;
-  uint32_t ph = 0;
-  int ok = 1;
-
-  // copy the 64 rows [j0, j0+64) of one head's K or V history into a staging buffer; rows past
-  // the end of the context and columns past the head are zero-filled
-  auto prefetch = [&](const float *base, int64_t ld, int j0, uint32_t stage_off, auto nb, int width, bool key) {
-    constexpr int NB = decltype(nb)::value;
-    const int slot0 = PLAIN ? j0 : (int)(j0 % p.cap);
-#pragma unroll
-    for (int i = 0; i < 4 * NB; ++i) {
-      const int piece = tid + 256 * i, row = piece / (16 * NB), c16 = piece % (16 * NB);
-      const bool okk = j0 + row < t && (PLAIN || c16 * 4 < width);
-      int slot = slot0 + row;
-      if (!PLAIN && slot >= (int)p.cap) slot -= (int)p.cap;
-      const float *src = base + (okk ? (int64_t)slot * (PLAIN ? 64 : ld) + c16 * 4 : 0);
-      if (!PLAIN && key && okk && c16 * 4 >= p.kx_from) src = kx + (int64_t)slot * p.kx_ld + c16 * 4;
-      cp_async16(smem_u32(sm + stage_off + row * (NB * 256 + 16) + c16 * 16), src, okk ? 16u : 0u);
-    }
-  };
-  auto staged_row = [&](uint32_t row_off, int block, float4 *v) {  // this thread's 16 dims of its key row
-    const float4 *src = reinterpret_cast<const float4 *>(sm + row_off + 256 * block + 64 * cq);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = src[i];
-  };
-  // one warp polls the mbarrier; the others park at the block barrier instead of spinning (their
-  // issue slots go to the other CTA of the SM)
-  auto wait_mma = [&]() {
-    if (warp == 0 && !mbar_wait(bar, ph, abort_flag)) {
-      ok = 0;
-      *abort_flag = 1;
-    }
-    ph ^= 1u;
-    ok = __syncthreads_and(ok);
+  const int tile0 = kfirst > 0 ? kfirst / AT_K : 0, kbeg = tile0 * AT_K;
+  const int nblk = (kend - kbeg + AT_K - 1) / AT_K;    // at least 1
+  auto give_up = [&](int code) {
+    if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, DEV_WAIT_TIMEOUT); status[1] = code; }
   };
 
-  prefetch(kb, p.k_ld, kbeg, AT_OFF_SK, IntC<NQ>(), Dp, true);
-  prefetch(vb, p.v_ld, kbeg, AT_OFF_SV, IntC<NE>(), Ep, false);
-  cp_async_commit();
   // Q tiles: rows [0,128) hi, [128,256) lo per block; GPT-2's 1/8 score scale is folded in (a power of two: exact)
-  {
+  if (warp < AT_SOFTMAX_WARPS) {
     const bool okq = q0 + r < s;
     const float4 *src = reinterpret_cast<const float4 *>(p.qkv + ((int64_t)b * s + (okq ? q0 + r : 0)) * p.ld + p.q_off + (int64_t)h * Dp);
 #pragma unroll
@@ -209,103 +210,144 @@ __global__ void __launch_bounds__(256, AtLayout<NQ, NE>::CTAS) attn_prefill_tc_k
         v[i] = okq && (PLAIN || 4 * c4 < Dp) ? scale4(src[c4], qscale) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) st_split8(sm + AT_OFF_Q + kb_ * 32768, r, 128 + r, 4 * hf + c, v[2 * c], v[2 * c + 1]);
-    }
-  }
-  cp_async_wait_all();
-  __syncthreads();  // step 0 of K and V is staged (and the Q tile is written)
-
-  // ---- key steps: scores, running maximum, probabilities, row sums, O ---------------------------------
-  float m = -INFINITY;  // the row's reference maximum: the same value in both threads of a row
-  float lsum = 0.0f;    // this thread's part of the row sum, relative to m
-  for (int blk = 0; blk < nblk && ok; ++blk) {
-    const int j0 = kbeg + blk * AT_K;
-    {
-      // split this thread's part of the staged rows in registers, then (once the previous step's
-      // P.V has read the V^T tile and P) store it into the tiles
-      uint4 khi[NQ][2], klo[NQ][2], vhi[NE][2], vlo[NE][2];
-#pragma unroll
-      for (int w = 0; w < NQ; ++w) {
-        float4 kv[4];
-        staged_row(AT_OFF_SK + ck * Lay::LD_K, w, kv);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          khi[w][c] = pack8(kv[2 * c], kv[2 * c + 1]);
-          klo[w][c] = pack8_lo(kv[2 * c], kv[2 * c + 1]);
-        }
-      }
-#pragma unroll
-      for (int w = 0; w < NE; ++w) {
-        float4 vv[4];
-        staged_row(AT_OFF_SV + ck * Lay::LD_V, w, vv);
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          vhi[w][c] = pack8(vv[2 * c], vv[2 * c + 1]);
-          vlo[w][c] = pack8_lo(vv[2 * c], vv[2 * c + 1]);
-        }
-      }
-      if (blk > 0) wait_mma();
-#pragma unroll
-      for (int w = 0; w < NQ; ++w)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          *reinterpret_cast<uint4 *>(sm + AT_OFF_K + w * 16384 + sw128(ck, 2 * cq + c)) = khi[w][c];
-          *reinterpret_cast<uint4 *>(sm + AT_OFF_K + w * 16384 + sw128(64 + ck, 2 * cq + c)) = klo[w][c];
-        }
-      // V tiles (hi, then lo): rows = keys, 64 dims contiguous: the MMA reads them as an MN-major B operand
-#pragma unroll
-      for (int w = 0; w < NE; ++w)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          *reinterpret_cast<uint4 *>(sm + AT_OFF_V + w * 16384 + sw128(ck, 2 * cq + c)) = vhi[w][c];
-          *reinterpret_cast<uint4 *>(sm + AT_OFF_V + w * 16384 + 8192 + sw128(ck, 2 * cq + c)) = vlo[w][c];
-        }
+      for (int c = 0; c < 4; ++c) st_split8(sm + Lay::OFF_Q + kb_ * 32768, r, 128 + r, 4 * hf + c, v[2 * c], v[2 * c + 1]);
     }
     fence_proxy_async();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);  // tiles complete, staging buffers free
-    if (!ok) break;
-    if (warp == 0) {  // converged warp, one elected lane: the descriptors stay in uniform registers
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();   // not before this CTA has its tensor memory: the next kernel's CTAs ask for theirs and then wait for this grid
+
+  float m = -INFINITY;  // the row's reference maximum: the same value in both threads of a row
+  float lsum = 0.0f;    // this thread's part of the row sum, relative to m
+  bool ok = true;
+  if (warp == 8) {
+    // ---------------- tiles ----------------
+    if (lane == 0) {
+      const int64_t kv = (int64_t)blockIdx.y * p.G + (PLAIN ? h : h / (p.H / p.G));  // the key/value head this query head reads
+      const uint8_t *src = tiles + (kv * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;
+      int ki = 0, vi = 0;   // copies asked for
+      for (int i = 0; i < nblk; ++i, src += Lay::TILE) {
+        const int st = i & 1;
+        const uint32_t ph = ((uint32_t)(i >> 1) & 1u) ^ 1u;   // (the first use of a stage passes at once)
+        if (!mbar_wait(k_empty(st), ph, abort_flag)) break;
+        mbar_expect_tx(k_full(st), Lay::K_BYTES);
+        bulk_load(smem_u32(sm + Lay::OFF_K) + st * Lay::K_BYTES, src, Lay::K_BYTES, k_full(st));
+        ++ki;
+        if (!mbar_wait(v_empty(st), ph, abort_flag)) break;
+        mbar_expect_tx(v_full(st), Lay::V_BYTES);
+        bulk_load(smem_u32(sm + Lay::OFF_V) + st * Lay::V_BYTES, src + Lay::K_BYTES, Lay::V_BYTES, v_full(st));
+        ++vi;
+      }
+      if (vi < nblk) give_up(16);
+      // the copies this thread started land before the CTA's shared memory is released, whoever gives up
+      for (int k = ki > 2 ? ki - 2 : 0; k < ki; ++k) mbar_wait(k_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
+      for (int k = vi > 2 ? vi - 2 : 0; k < vi; ++k) mbar_wait(v_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
+    }
+  } else if (warp == 9) {
+    // ---------------- MMAs (uniform control flow, one elected lane issues) ----------------
+    const uint64_t dq = umma_desc(smem_u32(sm + Lay::OFF_Q)), dk0 = umma_desc(smem_u32(sm + Lay::OFF_K)), dv0 = umma_desc(smem_u32(sm + Lay::OFF_V));
+    const uint32_t idesc_pv = idesc_n64 | (1u << 16);  // B operand MN-major: V rows (keys) with the dims contiguous
+    const int ksteps = Dp / 16;
+    auto scores = [&](int i) {   // S of step i
+      const int st = i & 1;
+      const uint32_t ph = (uint32_t)(i >> 1) & 1u;
+      if (!mbar_wait(k_full(st), ph, abort_flag) || !mbar_wait(s_empty(st), ph ^ 1u, abort_flag)) return false;
       tc_fence_after();
       if (elect_one()) {
+        const uint64_t dk = dk0 + (uint64_t)(st * (Lay::K_BYTES >> 4));
+        const uint32_t acc = tmem_base + AT_COL_S + 64u * st;
 #pragma unroll
         for (int k = 0; k < 4 * NQ; ++k) {
           if (NQ == 1 || k < ksteps) {
             // 16 bf16 = 32 bytes = 2 descriptor units; a Q block is 32 KB = 2048 units, a K block 16 KB = 1024
             const uint64_t aq = dq + (uint64_t)((k >> 2) * 2048 + 2 * (k & 3)), ak = dk + (uint64_t)((k >> 2) * 1024 + 2 * (k & 3));
-            umma_bf16(tmem_base + AT_COL_S, aq, ak, idesc_n64, k > 0 ? 1u : 0u);
-            umma_bf16(tmem_base + AT_COL_S, aq + 1024, ak, idesc_n64, 1u);
-            umma_bf16(tmem_base + AT_COL_S, aq, ak + 512, idesc_n64, 1u);
-            umma_bf16(tmem_base + AT_COL_S, aq + 1024, ak + 512, idesc_n64, 1u);
+            umma_bf16(acc, aq, ak, idesc_n64, k > 0 ? 1u : 0u);
+            umma_bf16(acc, aq + 1024, ak, idesc_n64, 1u);
+            umma_bf16(acc, aq, ak + 512, idesc_n64, 1u);
+            umma_bf16(acc, aq + 1024, ak + 512, idesc_n64, 1u);
           }
         }
-        umma_commit(bar);
+        umma_commit(k_empty(st));
+        umma_commit(s_full(st));
+      }
+      __syncwarp();
+      return true;
+    };
+    ok = scores(0);
+    for (int i = 0; i < nblk && ok; ++i) {
+      if (i + 1 < nblk && !(ok = scores(i + 1))) break;
+      const int st = i & 1;
+      ok = mbar_wait(v_full(st), (uint32_t)(i >> 1) & 1u, abort_flag) && mbar_wait(p_full, (uint32_t)i & 1u, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int w = 0; w < NE; ++w) {
+          const uint32_t acc = tmem_base + AT_COL_O + 64 * w;
+          const uint64_t dv_hi = dv0 + (uint64_t)(st * (Lay::V_BYTES >> 4) + 1024 * w), dv_lo = dv_hi + 512;
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4) {
+            const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
+            const uint32_t p_hi = tmem_base + AT_COL_P + 8 * k4, p_lo = p_hi + 32;
+            umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u);
+            umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u);
+            umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u);
+          }
+        }
+        umma_commit(v_empty(st));
+        umma_commit(pv_done);
       }
       __syncwarp();
     }
-    // the next step's rows start to arrive while the MMAs run (issued after them: the MMAs are the critical path)
-    if (blk + 1 < nblk) {
-      prefetch(kb, p.k_ld, j0 + AT_K, AT_OFF_SK, IntC<NQ>(), Dp, true);
-      prefetch(vb, p.v_ld, j0 + AT_K, AT_OFF_SV, IntC<NE>(), Ep, false);
-      cp_async_commit();
-    }
-    wait_mma();
-    tc_fence_after();
-    {
-      // this thread's 32 keys in one round trip to tensor memory
+    if (!ok && lane == 0) give_up(17);
+    // the last products are awaited here too: tensor memory is freed below
+    if (ok && !mbar_wait(pv_done, (uint32_t)(nblk - 1) & 1u, abort_flag) && lane == 0) give_up(18);
+    __syncwarp();
+  } else {
+    // ---------------- softmax ----------------
+    const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const int qi = min(q0 + r, s - 1);  // rows past the end of the step mask like the last row (their output is dropped)
+    const int jmax = n + qi;            // last visible key of this query (< t)
+    const int jmin = jmax - W + 1;      // first visible key (may be negative)
+    // the warp's view of a wait; a warp whose wait ran out goes on through the pair barriers and touches nothing else
+    auto wait = [&](uint32_t bar, uint32_t ph) {
+      if (!ok) return;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_flag));
+      if (!ok && lane == 0) give_up(10);
+    };
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };   // warps quad and quad + 4
+    for (int i = 0; i < nblk; ++i) {
+      const int st = i & 1, j0 = kbeg + i * AT_K;
       uint32_t a[32];
-      tmem_ld16(tlane + AT_COL_S + 32 * hf, a);
-      tmem_ld16(tlane + AT_COL_S + 32 * hf + 16, a + 16);
-      tmem_ld_wait();
-      // maximum of the visible scores of this step: over this thread's 32 keys, then over the row's two threads
-      const int lim = jmax - j0 - 32 * hf, low = jmin - j0 - 32 * hf;  // key e of this thread is visible iff low <= e <= lim
+      wait(s_full(st), (uint32_t)(i >> 1) & 1u);
       float mloc = -INFINITY;
+      // key e of this thread is visible iff low <= e <= lim
+      const int lim = jmax - j0 - 32 * hf, low = jmin - j0 - 32 * hf;
+      const bool whole = lim >= 31 && (PLAIN || low <= 0);
+      if (ok) {
+        tc_fence_after();
+        tmem_ld16(tlane + AT_COL_S + 64 * st + 32 * hf, a);
+        tmem_ld16(tlane + AT_COL_S + 64 * st + 32 * hf + 16, a + 16);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty(st));
+        if (!__all_sync(0xffffffffu, whole)) {   // (only the tiles at the ends of what is visible)
 #pragma unroll
-      for (int e = 0; e < 32; ++e)
-        if (e <= lim && (PLAIN || e >= low)) mloc = fmaxf(mloc, __uint_as_float(a[e]));
-      red[hf * 128 + r] = mloc;
-      __syncthreads();
-      const float mstep = fmaxf(red[r], red[128 + r]);
+          for (int e = 0; e < 32; ++e)
+            if (e > lim || (!PLAIN && e < low)) a[e] = __float_as_uint(-INFINITY);
+        }
+#pragma unroll
+        for (int e = 0; e < 32; ++e) mloc = fmaxf(mloc, __uint_as_float(a[e]));
+      }
+      float *rd = red + st * 256;
+      rd[hf * 128 + r] = mloc;
+      pair_sync();
+      if (!ok) continue;
+      const float mstep = fmaxf(rd[r], rd[128 + r]);
       // The reference maximum only moves when the step's maximum exceeds it by more than AT_TAU
       // (probabilities then stay below e^AT_TAU, harmless in fp32 / split bf16); when it moves, O and
       // the row sum accumulated so far are rescaled.  Softmax is invariant to the shift, so this is
@@ -313,113 +355,89 @@ __global__ void __launch_bounds__(256, AtLayout<NQ, NE>::CTAS) attn_prefill_tc_k
       // -inf (and every probability zero) until the row's first visible key.
       const bool move = mstep > m + AT_TAU;  // also true at the first visible key (m = -inf)
       const float m_new = move ? mstep : m;
-      if (blk > 0 && __any_sync(0xffffffffu, move)) {
-        const float scale = move ? exp2f((m - m_new) * kAtInvLn2) : 1.0f;
-        lsum *= scale;
-#pragma unroll
-        for (int w = 0; w < NE; ++w) {
-          uint32_t o[32];
-          tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
-          tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * scale);
-          tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
-          tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
-        }
-      }
+      const float scale = move ? exp2f((m - m_new) * kAtInvLn2) : 1.0f;
+      lsum *= scale;
       m = m_new;
+      const float m_ref = m == -INFINITY ? 0.0f : m;   // (nothing visible yet: every score is -inf)
+      uint32_t phi[16], plo[16];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        float pr[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const float val = __uint_as_float(a[16 * c + e]);
-          pr[e] = (16 * c + e <= lim && (PLAIN || 16 * c + e >= low)) ? ex2_approx((val - m) * kAtInvLn2) : 0.0f;
-          lsum += pr[e];
-        }
-        uint32_t phi[8], plo[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          phi[e] = pack_bf16(pr[2 * e], pr[2 * e + 1]);
-          plo[e] = pack_bf16(bf16_lo(pr[2 * e]), bf16_lo(pr[2 * e + 1]));
-        }
-        // 16 keys = 8 columns; key k of the step sits in column k / 2
-        tmem_st8(tlane + AT_COL_P + 16 * hf + 8 * c, phi);
-        tmem_st8(tlane + AT_COL_P + 32 + 16 * hf + 8 * c, plo);
+      for (int e = 0; e < 16; ++e) {
+        const float p0 = ex2_approx((__uint_as_float(a[2 * e]) - m_ref) * kAtInvLn2), p1 = ex2_approx((__uint_as_float(a[2 * e + 1]) - m_ref) * kAtInvLn2);
+        lsum += p0;
+        lsum += p1;
+        phi[e] = pack_bf16(p0, p1);
+        plo[e] = pack_bf16(bf16_lo(p0), bf16_lo(p1));
       }
-    }
-    tmem_st_wait();
-    tc_fence_before();
-    cp_async_wait_all();
-    ok = __syncthreads_and(ok);  // P is written; the next step's rows are staged
-    if (!ok) break;
-    if (warp == 0) {  // converged warp, one elected lane: the descriptors stay in uniform registers
-      tc_fence_after();
-      if (elect_one()) {
+      if (i > 0) {   // the step before has read P and added to O
+        wait(pv_done, (uint32_t)(i - 1) & 1u);
+        if (!ok) continue;
+        tc_fence_after();
+        if (__any_sync(0xffffffffu, move)) {
 #pragma unroll
-        for (int w = 0; w < NE; ++w) {
-          const uint32_t acc = tmem_base + AT_COL_O + 64 * w;
-          const uint64_t dv_hi = dv + (uint64_t)(1024 * w), dv_lo = dv_hi + 512;
+          for (int w = 0; w < NE; ++w) {
+            uint32_t o[32];
+            tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
+            tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
+            tmem_ld_wait();
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
-            const uint32_t p_hi = tmem_base + AT_COL_P + 8 * k4, p_lo = p_hi + 32;
-            umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u);
-            umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u);
-            umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u);
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * scale);
+            tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
+            tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
           }
         }
-        umma_commit(bar);
       }
+      // key k of the step sits in column k / 2
+      tmem_st16(tlane + AT_COL_P + 16 * hf, phi);
+      tmem_st16(tlane + AT_COL_P + 32 + 16 * hf, plo);
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
     }
-  }
-  if (ok && nblk > 0) wait_mma();
-  tc_fence_after();
-  red[hf * 128 + r] = lsum;
-  ok = __syncthreads_and(ok);
-  if (ok) {
-    float inv = 1.0f / (red[r] + red[128 + r]);
-    const int64_t orow = (int64_t)b * s + q0 + r;
-    if (!PLAIN && p.gate_off >= 0 && q0 + r < s) inv *= 1.0f / (1.0f + expf(-p.qkv[orow * p.ld + p.gate_off + h]));
+    wait(pv_done, (uint32_t)(nblk - 1) & 1u);
+    tc_fence_after();
+    float *rd = red + (nblk & 1) * 256;
+    rd[hf * 128 + r] = lsum;
+    pair_sync();
+    if (ok) {
+      float inv = 1.0f / (rd[r] + rd[128 + r]);
+      const int64_t orow = (int64_t)b * s + q0 + r;
+      if (!PLAIN && p.gate_off >= 0 && q0 + r < s) inv *= 1.0f / (1.0f + expf(-p.qkv[orow * p.ld + p.gate_off + h]));
 #pragma unroll
-    for (int w = 0; w < NE; ++w) {
-      uint32_t a[32];
-      tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, a);
-      tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, a + 16);
-      tmem_ld_wait();
-      float o[32];
+      for (int w = 0; w < NE; ++w) {
+        uint32_t a[32];
+        tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, a);
+        tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, a + 16);
+        tmem_ld_wait();
+        float o[32];
 #pragma unroll
-      for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(a[e]) * inv;
-      if (q0 + r < s) {
-        const int c0 = 64 * w + 32 * hf;
-        const int64_t at = orow * p.out_ld + (int64_t)h * Ep + c0;
+        for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(a[e]) * inv;
+        if (q0 + r < s) {
+          const int c0 = 64 * w + 32 * hf;
+          const int64_t at = orow * p.out_ld + (int64_t)h * Ep + c0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (!PLAIN && c0 + 8 * i >= Ep) continue;
-          const float *v = o + 8 * i;
-          if (p.bf.hi) {
-            *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) =
-                make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-            if (p.bf.lo)
-              *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) =
-                  make_uint4(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])),
-                             pack_bf16(bf16_lo(v[4]), bf16_lo(v[5])), pack_bf16(bf16_lo(v[6]), bf16_lo(v[7])));
-          } else {
-            *reinterpret_cast<float4 *>(p.out + at + 8 * i) = make_float4(v[0], v[1], v[2], v[3]);
-            *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+          for (int i = 0; i < 4; ++i) {
+            if (!PLAIN && c0 + 8 * i >= Ep) continue;
+            const float *v = o + 8 * i;
+            if (p.bf.hi) {
+              *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) =
+                  make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+              if (p.bf.lo)
+                *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) =
+                    make_uint4(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])),
+                               pack_bf16(bf16_lo(v[4]), bf16_lo(v[5])), pack_bf16(bf16_lo(v[6]), bf16_lo(v[7])));
+            } else {
+              *reinterpret_cast<float4 *>(p.out + at + 8 * i) = make_float4(v[0], v[1], v[2], v[3]);
+              *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            }
           }
         }
       }
     }
-  } else if (tid == 0) {
-    atomicCAS(status, 0, DEV_WAIT_TIMEOUT);
-    status[1] = 10;
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 9) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(Lay::COLS) : "memory");
   }
@@ -427,13 +445,29 @@ __global__ void __launch_bounds__(256, AtLayout<NQ, NE>::CTAS) attn_prefill_tc_k
 
 template <int NQ, int NE, bool PLAIN = false>
 static int launch_at(caten_b200_ctx *ctx, const AttnArgs &a, float qscale) {
+  using Lay = AtLayout<NQ, NE>;
   const uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_Q >> 4) << 24);  // fp32 accumulate, bf16 x bf16, M = 128
   const uint32_t idesc_n64 = base | ((uint32_t)(64 >> 3) << 17);
-  constexpr size_t smem = AtLayout<NQ, NE>::SMEM;
+  constexpr size_t smem = Lay::SMEM;
   CB_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_tc_kernel<NQ, NE, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)((a.s + AT_Q - 1) / AT_Q), (unsigned)a.H, (unsigned)a.B), dim3(256), smem, a, qscale,
-           ctx->d_status, idesc_n64);
-  CB_LAUNCH_CHECK(ctx, "attn_prefill_tc_kernel");
+  const int ntiles = (a.n + a.s + AT_K - 1) / AT_K - at_first_tile(a);
+  // The tiles are as large as the visible keys and values in fp32.  Sequences are taken in groups whose tiles stay within
+  // AT_TILES_BYTES (a prompt of 8192 tokens of GPT-2 XL, the largest portion by default, needs 105 MB), one at least.
+  const size_t per_seq = (size_t)a.G * ntiles * Lay::TILE;
+  int group = per_seq < AT_TILES_BYTES ? (int)(AT_TILES_BYTES / per_seq) : 1;
+  if (group > a.B) group = a.B;
+  if (int rc = scratch_reserve(ctx, &ctx->attn_tiles, per_seq * group)) return rc;
+  uint8_t *tiles = (uint8_t *)ctx->attn_tiles.ptr;
+  const unsigned qtiles = (unsigned)((a.s + AT_Q - 1) / AT_Q);
+  if (qtiles > 65535) return fail(ctx, CATEN_B200_EUNSUPPORTED, "attention: %d tokens in one step", a.s);
+  for (int b0 = 0; b0 < a.B; b0 += group) {
+    const int nb = a.B - b0 < group ? a.B - b0 : group;
+    launch_k(ctx, attn_tiles_kernel<NQ, NE, PLAIN>, dim3((unsigned)ntiles, (unsigned)a.G, (unsigned)nb), dim3(256), 0, a, b0, tiles);
+    CB_LAUNCH_CHECK(ctx, "attn_tiles_kernel");
+    launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)a.H, (unsigned)nb, qtiles), dim3(AT_THREADS), smem, a, qscale, ctx->d_status, idesc_n64, b0,
+             (const uint8_t *)tiles, ntiles);
+    CB_LAUNCH_CHECK(ctx, "attn_prefill_tc_kernel");
+  }
   return 0;
 }
 
@@ -448,13 +482,16 @@ int launch_attention_tc_ex(caten_b200_ctx *ctx, const AttnArgs &args, float qsca
   return launch_at<1, 1>(ctx, a, qscale);
 }
 
-int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, const float *kc, const float *vc, float *out, int64_t B, int64_t s,
+// the step's keys and values are appended to the cache here
+int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B, int64_t s,
                         int64_t n, int64_t H, int64_t T, BfOut bf) {
   AttnArgs a;
   a.qkv = const_cast<float *>(qkv);
   a.ld = 3 * H * 64;
-  a.kc = const_cast<float *>(kc);
-  a.vc = const_cast<float *>(vc);
+  a.k_off = H * 64;
+  a.v_off = 2 * H * 64;
+  a.kc = kc;
+  a.vc = vc;
   a.cap = T;
   a.out = out; a.bf = bf; a.out_ld = H * 64;
   a.B = (int)B; a.s = (int)s; a.n = (int)n; a.H = a.G = (int)H;

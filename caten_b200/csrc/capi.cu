@@ -139,6 +139,7 @@ int caten_b200_destroy(caten_b200_ctx *ctx) {
   if (ctx->wbf.ptr) cudaFree(ctx->wbf.ptr);
   if (ctx->wkv_tmp.ptr) cudaFree(ctx->wkv_tmp.ptr);
   if (ctx->chunk_states.ptr) cudaFree(ctx->chunk_states.ptr);
+  if (ctx->attn_tiles.ptr) cudaFree(ctx->attn_tiles.ptr);
   if (ctx->upload_stage.ptr) cudaFree(ctx->upload_stage.ptr);
   for (int k = 0; k < 2; ++k) {
     if (ctx->pin[k]) cudaFreeHost(ctx->pin[k]);

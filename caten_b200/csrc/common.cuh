@@ -119,6 +119,7 @@ struct caten_b200_ctx {
   cb::Scratch wbf;           // bf16 copy (hi, lo) of the weight operand of the many-row GEMM
   cb::Scratch chunk_states;    // per-chunk states of a recurrent layer's prompt
   cb::Scratch wkv_tmp;       // intermediates of a stand-alone time-mixing call
+  cb::Scratch attn_tiles;    // keys and values of a multi-token step as operand tiles
   cb::Scratch upload_stage;  // raw blocks of the weight being uploaded, before their re-layout
   void *pin[2] = {nullptr, nullptr};          // pinned bounce buffers for large copies from pageable host memory
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
@@ -207,7 +208,7 @@ int launch_sample(caten_b200_ctx *ctx, const float *logits, int64_t rows, int64_
 int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B,
                      int64_t s, int64_t n, int64_t H, int64_t T, const int *d_n = nullptr, cb::BfOut bf = cb::BfOut(),
                      const cb::PartIn *pending_qkv = nullptr, int tensor_cores = 0);
-int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, const float *kc, const float *vc, float *out, int64_t B,
+int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B,
                         int64_t s, int64_t n, int64_t H, int64_t T, cb::BfOut bf);
 int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
                 const float *res, int act, float *y, int64_t M = 1, LinGroups grp = LinGroups());   // M: 1 to 4 rows of x
