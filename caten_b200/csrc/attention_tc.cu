@@ -15,21 +15,20 @@
 // attn_prefill_tc_kernel: one CTA = 128 queries of one (sequence, head) = the 128 lanes of tensor memory; keys go in steps
 // of 64 (with a window: from the step that holds the first key any of the tile's queries sees).  By warp:
 //   warp 8       one lane asks for the K and V tiles of the steps ahead (two stages each)
-//   warp 9       issues S[128 x 64] = (Q_hi + Q_lo) . (K_hi + K_lo)^T, four MMAs per 16 dims, into one of TWO blocks of
-//                tensor memory, a step ahead of the softmax, and O[128 x 64 NE] += P_hi.V_hi + P_lo.V_hi + P_hi.V_lo
+//   warp 9       issues the scores (Q_hi + Q_lo) . (K_hi + K_lo)^T, into one of two blocks of tensor memory and a step ahead
+//                of the softmax, and O[128 x 64 NE] += P_hi.V_hi + P_lo.V_hi + P_hi.V_lo, all dims in one MMA
 //   warps 0..7   read their query's scores (warps w and w + 4 share lanes and take 32 keys each), mask, take
 //                p = exp2((s - max)/ln2), accumulate the row sum, split p into bf16 hi/lo and write it back to tensor
 //                memory as the A operand of the second product
 // so that the scores of step i + 1 and the output of step i - 1 are computed while the softmax of step i runs.  The softmax is
 // what a step waits for (about 2.5 k cycles against 1.8 k of MMAs); with the phases one after the other, conversion included,
-// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 183 us and 13 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
-// 40 us for the append -> 136 us and 72 us for append and tiles.
+// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 166 us and 13 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
+// 40 us for the append -> 136 us and 67 us for append and tiles.
 // The softmax is single-pass with a lazily moved reference maximum: each step exchanges the
 // maximum of its visible scores between the row's two threads; the reference only moves (and O and
 // the row sum are rescaled, O by a TMEM load / multiply / store) when a step exceeds it by more
 // than AT_TAU, which in causal attention happens in the first steps and then rarely.  Softmax is
 // invariant to the reference, so this equals the reference's two-pass form up to rounding.
-// TMEM columns: [0,64) and [64,128) S, [128,192) P (hi 32, lo 32), [192, 192 + 64 NE) O.
 //
 // The mbarrier waits are bounded; when one runs out the CTA records it in the context's status
 // word, skips the remaining work and its output, frees its tensor memory and returns.
@@ -44,17 +43,22 @@ constexpr float kAtInvLn2 = 1.0f / 0.6931472f;  // (/ (log 2)) in single float, 
 constexpr int AT_Q = 128;                        // queries per CTA (MMA M)
 constexpr int AT_K = 64;                         // keys per step
 constexpr float AT_TAU = 8.0f;                   // slack of the running maximum, in units of the score
-constexpr uint32_t AT_COL_S = 0, AT_COL_P = 128, AT_COL_O = 192;
 constexpr int AT_SOFTMAX_WARPS = 8, AT_THREADS = (AT_SOFTMAX_WARPS + 2) * 32;
 constexpr size_t AT_TILES_BYTES = (size_t)256 << 20;   // tiles of as many sequences as fit here are made at a time
 template <int NQ, int NE> struct AtLayout {
-  static constexpr uint32_t COLS = NE == 1 ? 256 : 512;  // TMEM columns per CTA (a power of two)
+  static constexpr int CTAS = NQ == 1 && NE == 1 ? 2 : 1;  // per SM
+  // Where one CTA has the SM and its tensor memory to itself the rows of K_hi and K_lo are one operand of 128 rows: two MMAs of
+  // 128 columns per 16 dims (an MMA of 64 columns takes hardly less time), whose two halves the softmax adds (16 heads of 128,
+  // 8 x 1024 tokens: 183 -> 166 us).  Two CTAs share an SM otherwise, and a block of 128 columns each would leave them one
+  // block instead of two (25 heads of 64, 16 x 512 tokens: 136 us with two of 64 columns, 161 us with one of 128).
+  static constexpr bool STACK = CTAS == 1;
+  // TMEM columns: two blocks of scores, P (hi 32, lo 32), O (64 NE); allocated: a power of two
+  static constexpr uint32_t COLS = STACK ? 512 : 256, S_COLS = STACK ? 128 : 64, COL_P = 2 * S_COLS, COL_O = COL_P + 64;
   // Q: per block 128 rows hi, 128 rows lo (16 KB each); K, V: per block 64 rows hi, 64 rows lo (8 KB each), two stages
   static constexpr uint32_t K_BYTES = NQ * 16384, V_BYTES = NE * 16384, TILE = K_BYTES + V_BYTES;
   static constexpr uint32_t OFF_Q = 0, OFF_K = NQ * 32768, OFF_V = OFF_K + 2 * K_BYTES, OFF_MISC = OFF_V + 2 * V_BYTES;
   // tiles + exchange of the rows' maxima (2 steps) + barriers, TMEM slot, abort flag + alignment slack
   static constexpr size_t SMEM = OFF_MISC + 2048 + 160 + 1024;
-  static constexpr int CTAS = NQ == 1 && NE == 1 ? 2 : 1;  // per SM
 };
 static_assert(2 * (AtLayout<1, 1>::SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
 static_assert(AtLayout<2, 2>::SMEM <= 227 * 1024, "one CTA per SM");
@@ -107,34 +111,40 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b
   const int64_t head = (int64_t)b * p.G + g;
   const float *kx = !PLAIN && p.kx ? p.kx + b * p.cap * p.kx_ld - p.kx_from : nullptr;   // column c of the key, c >= kx_from
   constexpr int KP = AT_K * NQ * 8, PIECES = KP + AT_K * NE * 8;   // pieces of eight floats
+  constexpr int IT = PIECES / 256;
+  float4 v[IT][2];   // all of this thread's loads are in flight together: the stores below may alias them
 #pragma unroll
-  for (int i0 = 0; i0 < PIECES; i0 += 256) {
-    const int i = i0 + threadIdx.x;
+  for (int it = 0; it < IT; ++it) {
+    const int i = it * 256 + threadIdx.x;
     const bool key = i < KP;
     const int nb = key ? NQ : NE, at = key ? i : i - KP;
     const int row = at / (8 * nb), c8 = at % (8 * nb), j = j0 + row;
-    float4 v[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int c = 8 * c8 + 4 * u;
       const float *src = nullptr;
-      float *keep = nullptr;
       if (PLAIN) {
-        if (j < t) {
-          keep = (key ? p.kc : p.vc) + (head * p.cap + j) * 64 + c;
-          src = keep;
-          if (j >= p.n) src = p.qkv + ((int64_t)b * p.s + j - p.n) * p.ld + (key ? p.k_off : p.v_off) + g * 64 + c;
-          else keep = nullptr;
-        }
+        if (j < t) src = j >= p.n ? p.qkv + ((int64_t)b * p.s + j - p.n) * p.ld + (key ? p.k_off : p.v_off) + g * 64 + c : (key ? p.kc : p.vc) + (head * p.cap + j) * 64 + c;
       } else if (j < t && c < (key ? p.Dp : p.Ep)) {
         const int64_t slot = j % p.cap;
         if (key && c >= p.kx_from) src = kx + slot * p.kx_ld + c;
         else src = key ? p.kc + b * p.k_seq + g * p.k_head + slot * p.k_ld + c : p.vc + b * p.v_seq + g * p.v_head + slot * p.v_ld + c;
       }
-      v[u] = src ? *reinterpret_cast<const float4 *>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (PLAIN && keep) *reinterpret_cast<float4 *>(keep) = v[u];
+      v[it][u] = src ? *reinterpret_cast<const float4 *>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    st_split8(dst + (key ? 0 : Lay::K_BYTES) + (c8 >> 3) * 16384, row, AT_K + row, c8 & 7, v[0], v[1]);
+  }
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int i = it * 256 + threadIdx.x;
+    const bool key = i < KP;
+    const int nb = key ? NQ : NE, at = key ? i : i - KP;
+    const int row = at / (8 * nb), c8 = at % (8 * nb), j = j0 + row;
+    if (PLAIN && j >= p.n && j < t) {
+      float4 *keep = reinterpret_cast<float4 *>((key ? p.kc : p.vc) + (head * p.cap + j) * 64 + 8 * c8);
+      keep[0] = v[it][0];
+      keep[1] = v[it][1];
+    }
+    st_split8(dst + (key ? 0 : Lay::K_BYTES) + (c8 >> 3) * 16384, row, AT_K + row, c8 & 7, v[it][0], v[it][1]);
   }
 }
 
@@ -142,7 +152,7 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b
 // the zero-filled head columns compile away.
 template <int NQ, int NE, bool PLAIN>
 __global__ void __launch_bounds__(AT_THREADS, AtLayout<NQ, NE>::CTAS)
-attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t idesc_n64, int b0, const uint8_t *__restrict__ tiles, int ntiles) {
+attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t idesc, int b0, const uint8_t *__restrict__ tiles, int ntiles) {
   using Lay = AtLayout<NQ, NE>;
   extern __shared__ unsigned char at_raw[];
   unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(at_raw) + 1023) & ~(uintptr_t)1023);
@@ -248,8 +258,10 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
     }
   } else if (warp == 9) {
     // ---------------- MMAs (uniform control flow, one elected lane issues) ----------------
-    const uint64_t dq = umma_desc(smem_u32(sm + Lay::OFF_Q)), dk0 = umma_desc(smem_u32(sm + Lay::OFF_K)), dv0 = umma_desc(smem_u32(sm + Lay::OFF_V));
-    const uint32_t idesc_pv = idesc_n64 | (1u << 16);  // B operand MN-major: V rows (keys) with the dims contiguous
+    const uint64_t dq = umma_desc(smem_u32(sm + Lay::OFF_Q)), dk0 = umma_desc(smem_u32(sm + Lay::OFF_K)), dv0 = umma_desc(smem_u32(sm + Lay::OFF_V)) - (1ull << 16) + ((uint64_t)(16384 >> 4) << 16);
+    const uint32_t idesc_s = idesc | ((Lay::S_COLS >> 3) << 17);
+    // B operand MN-major: V rows (keys) with the dims contiguous; blocks of 64 dims are 16 KB apart (the leading offset)
+    const uint32_t idesc_pv = idesc | (1u << 16) | ((uint32_t)(64 * NE >> 3) << 17);
     const int ksteps = Dp / 16;
     auto scores = [&](int i) {   // S of step i
       const int st = i & 1;
@@ -258,16 +270,18 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       tc_fence_after();
       if (elect_one()) {
         const uint64_t dk = dk0 + (uint64_t)(st * (Lay::K_BYTES >> 4));
-        const uint32_t acc = tmem_base + AT_COL_S + 64u * st;
+        const uint32_t acc = tmem_base + Lay::S_COLS * st;
 #pragma unroll
         for (int k = 0; k < 4 * NQ; ++k) {
           if (NQ == 1 || k < ksteps) {
             // 16 bf16 = 32 bytes = 2 descriptor units; a Q block is 32 KB = 2048 units, a K block 16 KB = 1024
             const uint64_t aq = dq + (uint64_t)((k >> 2) * 2048 + 2 * (k & 3)), ak = dk + (uint64_t)((k >> 2) * 1024 + 2 * (k & 3));
-            umma_bf16(acc, aq, ak, idesc_n64, k > 0 ? 1u : 0u);
-            umma_bf16(acc, aq + 1024, ak, idesc_n64, 1u);
-            umma_bf16(acc, aq, ak + 512, idesc_n64, 1u);
-            umma_bf16(acc, aq + 1024, ak + 512, idesc_n64, 1u);
+            umma_bf16(acc, aq, ak, idesc_s, k > 0 ? 1u : 0u);
+            umma_bf16(acc, aq + 1024, ak, idesc_s, 1u);
+            if (!Lay::STACK) {
+              umma_bf16(acc, aq, ak + 512, idesc_s, 1u);
+              umma_bf16(acc, aq + 1024, ak + 512, idesc_s, 1u);
+            }
           }
         }
         umma_commit(k_empty(st));
@@ -284,18 +298,15 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       if (!ok) break;
       tc_fence_after();
       if (elect_one()) {
+        const uint32_t acc = tmem_base + Lay::COL_O;
+        const uint64_t dv_hi = dv0 + (uint64_t)(st * (Lay::V_BYTES >> 4)), dv_lo = dv_hi + 512;
 #pragma unroll
-        for (int w = 0; w < NE; ++w) {
-          const uint32_t acc = tmem_base + AT_COL_O + 64 * w;
-          const uint64_t dv_hi = dv0 + (uint64_t)(st * (Lay::V_BYTES >> 4) + 1024 * w), dv_lo = dv_hi + 512;
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
-            const uint32_t p_hi = tmem_base + AT_COL_P + 8 * k4, p_lo = p_hi + 32;
-            umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u);
-            umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u);
-            umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u);
-          }
+        for (int k4 = 0; k4 < 4; ++k4) {
+          const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
+          const uint32_t p_hi = tmem_base + Lay::COL_P + 8 * k4, p_lo = p_hi + 32;
+          umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u);
+          umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u);
+          umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u);
         }
         umma_commit(v_empty(st));
         umma_commit(pv_done);
@@ -329,9 +340,22 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       const bool whole = lim >= 31 && (PLAIN || low <= 0);
       if (ok) {
         tc_fence_after();
-        tmem_ld16(tlane + AT_COL_S + 64 * st + 32 * hf, a);
-        tmem_ld16(tlane + AT_COL_S + 64 * st + 32 * hf + 16, a + 16);
-        tmem_ld_wait();
+        const uint32_t block = tlane + Lay::S_COLS * st + 32 * hf;
+        if constexpr (Lay::STACK) {
+#pragma unroll
+          for (int c = 0; c < 32; c += 16) {
+            uint32_t lo[16];
+            tmem_ld16(block + c, a + c);
+            tmem_ld16(block + 64 + c, lo);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) a[c + e] = __float_as_uint(__uint_as_float(a[c + e]) + __uint_as_float(lo[e]));
+          }
+        } else {
+          tmem_ld16(block, a);
+          tmem_ld16(block + 16, a + 16);
+          tmem_ld_wait();
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(s_empty(st));
@@ -376,19 +400,19 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
 #pragma unroll
           for (int w = 0; w < NE; ++w) {
             uint32_t o[32];
-            tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
-            tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
+            tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf, o);
+            tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf + 16, o + 16);
             tmem_ld_wait();
 #pragma unroll
             for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * scale);
-            tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf, o);
-            tmem_st16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, o + 16);
+            tmem_st16(tlane + Lay::COL_O + 64 * w + 32 * hf, o);
+            tmem_st16(tlane + Lay::COL_O + 64 * w + 32 * hf + 16, o + 16);
           }
         }
       }
       // key k of the step sits in column k / 2
-      tmem_st16(tlane + AT_COL_P + 16 * hf, phi);
-      tmem_st16(tlane + AT_COL_P + 32 + 16 * hf, plo);
+      tmem_st16(tlane + Lay::COL_P + 16 * hf, phi);
+      tmem_st16(tlane + Lay::COL_P + 32 + 16 * hf, plo);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -406,8 +430,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
 #pragma unroll
       for (int w = 0; w < NE; ++w) {
         uint32_t a[32];
-        tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf, a);
-        tmem_ld16(tlane + AT_COL_O + 64 * w + 32 * hf + 16, a + 16);
+        tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf, a);
+        tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf + 16, a + 16);
         tmem_ld_wait();
         float o[32];
 #pragma unroll
@@ -446,8 +470,7 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
 template <int NQ, int NE, bool PLAIN = false>
 static int launch_at(caten_b200_ctx *ctx, const AttnArgs &a, float qscale) {
   using Lay = AtLayout<NQ, NE>;
-  const uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_Q >> 4) << 24);  // fp32 accumulate, bf16 x bf16, M = 128
-  const uint32_t idesc_n64 = base | ((uint32_t)(64 >> 3) << 17);
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_Q >> 4) << 24);  // fp32 accumulate, bf16 x bf16, M = 128
   constexpr size_t smem = Lay::SMEM;
   CB_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_tc_kernel<NQ, NE, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ntiles = (a.n + a.s + AT_K - 1) / AT_K - at_first_tile(a);
@@ -464,7 +487,7 @@ static int launch_at(caten_b200_ctx *ctx, const AttnArgs &a, float qscale) {
     const int nb = a.B - b0 < group ? a.B - b0 : group;
     launch_k(ctx, attn_tiles_kernel<NQ, NE, PLAIN>, dim3((unsigned)ntiles, (unsigned)a.G, (unsigned)nb), dim3(256), 0, a, b0, tiles);
     CB_LAUNCH_CHECK(ctx, "attn_tiles_kernel");
-    launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)a.H, (unsigned)nb, qtiles), dim3(AT_THREADS), smem, a, qscale, ctx->d_status, idesc_n64, b0,
+    launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)a.H, (unsigned)nb, qtiles), dim3(AT_THREADS), smem, a, qscale, ctx->d_status, idesc, b0,
              (const uint8_t *)tiles, ntiles);
     CB_LAUNCH_CHECK(ctx, "attn_prefill_tc_kernel");
   }

@@ -48,6 +48,22 @@ def test_linear_bf16_weight(rt, M_, N, Kd, precision):
     assert np.abs(got - x @ wf.T).max() < (3e-2 if precision == "bf16" else 1e-4)
 
 
+@pytest.mark.parametrize("M_", [5, 16, 17, 33, 255, 257, 513, 1537])
+@pytest.mark.parametrize("N,Kd", [(4, 64), (132, 4096), (1540, 1088)])
+@pytest.mark.parametrize("precision", ["bf16", "bf16x3"])
+def test_linear_bf16_weight_tiles_and_shares_of_k(rt, M_, N, Kd, precision):
+    """Row tiles of every width, shares of k with and without a summing kernel, partial tiles; bias, activation, residual.  A
+    sum of Kd products of unit variance over sqrt(Kd) has rounding errors of a few 2^-9 (operands in bf16) or 2^-16."""
+    rng = np.random.default_rng(M_ + N)
+    w, wf = bf16_weight(rt, rng, N, Kd)
+    x, bias, res = rng.standard_normal((M_, Kd), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M_, N), dtype=np.float32)
+    dx, db, dr = (rt.transfer_from_array(a) for a in (x, bias, res))
+    y = x @ wf.T + bias
+    tol = 3e-2 if precision == "bf16" else 1e-4
+    assert np.abs(rt.linear(w, dx, db, dr, precision=L.PRECISIONS[precision]).numpy() - (y + res)).max() < tol
+    assert np.abs(rt.linear(w, dx, db, act=L.ACT_RELU, precision=L.PRECISIONS[precision]).numpy() - np.maximum(y, 0)).max() < tol
+
+
 @pytest.mark.parametrize("M_,N,Kd", [(m, n + n % 2, k) for m, n, k in SHAPES])
 @pytest.mark.parametrize("precision", ["fp32", "bf16", "bf16x3"])
 def test_gated_linear(rt, M_, N, Kd, precision):

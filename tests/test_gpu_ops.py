@@ -189,6 +189,20 @@ def test_gemv_up_to_four_rows(rt, oracle):
     w.close()
 
 
+@pytest.mark.parametrize("wtype", ["q4_0", "q8_0", "f32", "f16"])
+@pytest.mark.parametrize("M,N,K", [(2, 77, 3072), (3, 1301, 768), (4, 6402, 64), (4, 5000, 1600), (1, 9001, 1600)])
+def test_gemv_rows_share_the_weights(rt, oracle, wtype, M, N, K):
+    """One to four rows of x; a CTA's rows once, several loads deep and walked, the last ones partial."""
+    rng = np.random.Generator(np.random.PCG64(M * N + K))
+    up, t, raw = make_weight(rng, N, K, wtype)
+    Wf = oracle.dequant(t, raw, N * K).reshape(N, K)
+    x, bias, res = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M, N), dtype=np.float32)
+    w = rt.upload_weight(up)
+    got = rt.linear(w, rt.transfer_from_array(x), rt.transfer_from_array(bias), rt.transfer_from_array(res), L.ACT_GELU).numpy()
+    np.testing.assert_allclose(got, oracle.linear(x, Wf, bias, res, L.ACT_GELU, mode=0), atol=1e-4, rtol=1e-4)
+    w.close()
+
+
 def test_gemv_large_activations_and_zero_scale(rt, oracle):
     """The Q4_0 path pre-scales x by powers of two: large and tiny activations must survive."""
     rng = np.random.Generator(np.random.PCG64(9))
@@ -387,6 +401,27 @@ def test_attention_decode_steps(rt, oracle, B, H, T):
         np.testing.assert_allclose(got, want, atol=1e-5, rtol=1e-5)
     np.testing.assert_array_equal(dk.numpy(), _to_gpu_cache(kc))
     np.testing.assert_array_equal(dv.numpy(), _to_gpu_cache(vc))
+
+
+@pytest.mark.parametrize("B,H,T", [(1, 2, 1030), (1, 25, 515), (2, 3, 259), (5, 30, 130)])
+def test_attention_decode_shared_histories(rt, oracle, B, H, T):
+    """One to eight CTAs per history, around the lengths where their number changes."""
+    test_attention_decode_steps(rt, oracle, B, H, T)
+
+
+def test_attention_prefill_tensor_cores_in_groups(rt):
+    """Histories so long that the operand tiles of one sequence fill the memory they are given."""
+    torch = pytest.importorskip("torch")
+    B, H, s, n = 2, 20, 65, 16300
+    g = torch.Generator().manual_seed(5)
+    k, v = (torch.randn(B, H, n + s, 64, generator=g) for _ in range(2))
+    q = torch.randn(B, H, s, 64, generator=g)
+    rows = torch.cat([a.transpose(1, 2).reshape(B * s, H * 64) for a in (q, k[:, :, n:], v[:, :, n:])], 1)
+    want = torch.nn.functional.scaled_dot_product_attention(q, k, v, attn_mask=torch.ones(s, n + s, dtype=torch.bool).tril(n))
+    kc, vc = (rt.transfer_from_array(torch.cat([a[:, :, :n], torch.zeros(B, H, s, 64)], 2).numpy()) for a in (k, v))
+    got = rt.attention(rt.transfer_from_array(rows.numpy()), kc, vc, B, s, n, precision=L.PREC_BF16X3).numpy()
+    np.testing.assert_allclose(got, want.transpose(1, 2).reshape(B * s, H * 64).numpy(), atol=2e-5, rtol=2e-5)
+    np.testing.assert_array_equal(kc.numpy(), k.numpy())
 
 
 @pytest.mark.parametrize("B,H,T,s,n", [(2, 2, 64, 5, 0), (1, 3, 200, 64, 0), (2, 1, 200, 70, 9), (1, 2, 300, 130, 40), (1, 1, 8, 2, 6)])
