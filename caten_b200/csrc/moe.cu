@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) moe_choose_kernel(const RouteArgs a) {
 // its first place in every expert, and the warps then place their pairs in order.
 __global__ void __launch_bounds__(MR_THREADS) moe_sort_kernel(const RouteArgs a, int fused) {
   extern __shared__ int counts[];   // [MR_WARPS][experts]
-  __shared__ int warp_total[MR_WARPS];
+  __shared__ int warp_total[MR_WARPS], first[MR_MAX_EXPERTS];   // first: pairs of each expert, then its first place
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, E = a.experts;
   const int pairs = a.rows * a.top;
@@ -83,13 +83,20 @@ __global__ void __launch_bounds__(MR_THREADS) moe_sort_kernel(const RouteArgs a,
     }
   }
   __syncthreads();
-  int total = 0;
-  if (tid < E)
-    for (int w = 0; w < MR_WARPS; ++w) {
-      const int c = counts[w * E + tid];
-      counts[w * E + tid] = total;
-      total += c;
+  // counts[w][e] -> pairs of expert e in the warps before w: one warp per expert, a lane per warp of the CTA
+  for (int e = warp; e < E; e += MR_WARPS) {
+    const int c = counts[lane * E + e];
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += up;
     }
+    counts[lane * E + e] = inc - c;
+    if (lane == 31) first[e] = inc;
+  }
+  __syncthreads();
+  const int total = tid < E ? first[tid] : 0;
   int inc = total;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -98,12 +105,12 @@ __global__ void __launch_bounds__(MR_THREADS) moe_sort_kernel(const RouteArgs a,
   }
   if (lane == 31) warp_total[warp] = inc;
   __syncthreads();
-  int before = inc - total;
-  for (int w = 0; w < warp; ++w) before += warp_total[w];
-  if (tid < E) {
-    a.offsets[tid] = before;
-    if (tid == E - 1) a.offsets[E] = pairs;
-    for (int w = 0; w < MR_WARPS; ++w) counts[w * E + tid] += before;
+  if (warp * 32 < E) {
+    const int before = inc - total + __reduce_add_sync(0xffffffffu, lane < warp ? warp_total[lane] : 0);
+    if (tid < E) {
+      a.offsets[tid] = first[tid] = before;
+      if (tid == E - 1) a.offsets[E] = pairs;
+    }
   }
   __syncthreads();
   for (int q = p0; q < p1; q += 32 * MR_U) {
@@ -120,7 +127,7 @@ __global__ void __launch_bounds__(MR_THREADS) moe_sort_kernel(const RouteArgs a,
       const int p = q + 32 * u + lane;
       const unsigned same = __match_any_sync(0xffffffffu, e[u]);
       int at = 0;
-      if (e[u] >= 0) at = mine[e[u]] + __popc(same & ((1u << lane) - 1u));
+      if (e[u] >= 0) at = first[e[u]] + mine[e[u]] + __popc(same & ((1u << lane) - 1u));
       __syncwarp();
       if (e[u] >= 0) {
         a.pos[p] = at;

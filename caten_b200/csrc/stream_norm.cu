@@ -60,10 +60,33 @@ __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(
 template <int IN, int OUT, int MAXV>
 __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArgs a) {
   __shared__ float red[SN_THREADS / 32];
+  const int d4 = a.d4;
+  // The kernel is a chain of latencies when the rows are few, so what does not depend on the kernels before it (gains and the
+  // pass's step, written at load) is asked for before the wait, and the places of the experts' rows beside the row itself.
+  constexpr bool EARLY = OUT == SN_NORM2 && MAXV <= 2;
+  float4 g1[EARLY ? MAXV : 1], g2[EARLY ? MAXV : 1], st[EARLY ? MAXV : 1];
+  if (EARLY) {
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+      const int c = threadIdx.x + SN_THREADS * i;
+      if (c < d4) {
+        g1[i] = reinterpret_cast<const float4 *>(a.w1)[c];
+        if (a.w2) g2[i] = reinterpret_cast<const float4 *>(a.w2)[c];
+        if (a.step) st[i] = reinterpret_cast<const float4 *>(a.step)[c];
+      }
+    }
+  }
   pdl_enter();
   const int64_t row = blockIdx.x;
   const int64_t src = a.rows ? a.rows[row] : (a.src_stride > 1 ? (row + 1) * a.src_stride - 1 : row);
-  const int d4 = a.d4;
+  constexpr int SUM_U = 4;   // experts' rows in flight
+  int64_t place[SUM_U];
+  auto places = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < SUM_U; ++u)
+      if (k0 + u < a.top) place[u] = a.pos ? a.pos[src * a.top + k0 + u] : src * a.top + k0 + u;
+  };
+  if (IN == SN_SUM) places(0);
   float4 v[MAXV];
   if (IN == SN_EMBED) {
     const int64_t tok = a.ids[(src / a.s) * a.ids_ld + src % a.s];
@@ -111,13 +134,21 @@ __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArg
       }
     }
     if (IN == SN_SUM) {
-      for (int k = 0; k < a.top; ++k) {
-        const int64_t p = a.pos ? a.pos[src * a.top + k] : src * a.top + k;
+      for (int k0 = 0; k0 < a.top; k0 += SUM_U) {
+        if (k0) places(k0);
+        float4 t[SUM_U][MAXV];
 #pragma unroll
-        for (int i = 0; i < MAXV; ++i) {
-          const int c = threadIdx.x + SN_THREADS * i;
-          if (c < d4) v[i] = add4(v[i], reinterpret_cast<const float4 *>(a.ye)[p * d4 + c]);
-        }
+        for (int u = 0; u < SUM_U; ++u)
+#pragma unroll
+          for (int i = 0; i < MAXV; ++i) {
+            const int c = threadIdx.x + SN_THREADS * i;
+            if (k0 + u < a.top && c < d4) t[u][i] = reinterpret_cast<const float4 *>(a.ye)[place[u] * d4 + c];
+          }
+#pragma unroll
+        for (int u = 0; u < SUM_U; ++u)
+#pragma unroll
+          for (int i = 0; i < MAXV; ++i)
+            if (k0 + u < a.top && threadIdx.x + SN_THREADS * i < d4) v[i] = add4(v[i], t[u][i]);
       }
 #pragma unroll
       for (int i = 0; i < MAXV; ++i)
@@ -137,7 +168,7 @@ __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArg
       const int c = threadIdx.x + SN_THREADS * i;
       if (c < d4) {
         if (a.add_x0) v[i] = add4(v[i], reinterpret_cast<const float4 *>(a.x0)[src * d4 + c]);
-        v[i] = add4(v[i], reinterpret_cast<const float4 *>(a.step)[c]);
+        v[i] = add4(v[i], EARLY ? st[i] : reinterpret_cast<const float4 *>(a.step)[c]);
       }
     }
   }
@@ -186,8 +217,8 @@ __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArg
       const int c = threadIdx.x + SN_THREADS * i;
       if (c < d4) {
         const float4 u = make_float4(v[i].x * rs, v[i].y * rs, v[i].z * rs, v[i].w * rs);
-        sn_store(a.h, a.hb, row * d4 + c, mul4(u, reinterpret_cast<const float4 *>(a.w1)[c]));
-        if (a.w2) sn_store(a.h, a.hb, (a.plane + row) * d4 + c, mul4(u, reinterpret_cast<const float4 *>(a.w2)[c]));
+        sn_store(a.h, a.hb, row * d4 + c, mul4(u, EARLY ? g1[i] : reinterpret_cast<const float4 *>(a.w1)[c]));
+        if (a.w2) sn_store(a.h, a.hb, (a.plane + row) * d4 + c, mul4(u, EARLY ? g2[i] : reinterpret_cast<const float4 *>(a.w2)[c]));
       }
     }
   }
