@@ -2,8 +2,8 @@
 
     python -m caten_b200.build [--force] [--verbose] [--timing]
 
-``--timing`` builds a second library, ``libcaten_b200_timing.so``, whose single-kernel decode step
-records per-phase timestamps of CTA 0 (``-DDS_TIMING``; read by ``microbench.py decode_step``).
+``--timing`` builds a second library, ``libcaten_b200_timing.so``, whose tensor-core GEMM over packed weights records
+timestamps of CTA 0's roles (``-DDS_TIMING``; ``cb_debug_tc_marks``).
 It is a development aid: load it with ``CATEN_B200_LIB=caten_b200/libcaten_b200_timing.so``.
 
 ``-fmad=false``: multiply-add contraction is off so that element-wise formulas round exactly as
@@ -22,7 +22,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libcaten_b200.so")
-SOURCES = ["capi.cu", "decode_small.cu", "kernels_misc.cu", "gemv.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_dense.cu", "attention.cu", "attention_tc.cu", "gguf.cu", "expr.cu", "dequant_extra.cu", "sample.cu", "dist.cu", "llama_ops.cu",
+SOURCES = ["capi.cu", "kernels_misc.cu", "gemv.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_dense.cu", "attention.cu", "attention_tc.cu", "gguf.cu", "expr.cu", "dequant_extra.cu", "sample.cu", "dist.cu", "llama_ops.cu",
            "stream_norm.cu", "attn_window.cu", "wkv.cu", "latent.cu", "retention.cu", "moe.cu", "decoder.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-fmad=false", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -45,7 +45,7 @@ def _deps():
 def build(force: bool = False, verbose: bool = False, timing: bool = False) -> str:
     lib = LIB.replace(".so", "_timing.so") if timing else LIB
     obj_dir = OBJ_DIR + ("_timing" if timing else "")
-    flags = NVCC_FLAGS + (["-DDS_TIMING", "-DDS_TIMING_CTA=0"] if timing else [])
+    flags = NVCC_FLAGS + (["-DDS_TIMING"] if timing else [])
     newest = max(os.path.getmtime(p) for p in _deps())
     if not force and os.path.exists(lib) and os.path.getmtime(lib) >= newest:
         return lib

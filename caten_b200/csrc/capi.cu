@@ -310,7 +310,7 @@ int caten_b200_weight_upload_device(caten_b200_ctx *ctx, int type, const void *d
     const size_t qbytes = (size_t)nblocks * cb::type_code_bytes(type);
     auto drop = [&]() { cudaFree(w->qs); cudaFree(w->d); cudaFree(w->m); cudaFree(w->qh); delete w; };
     if ((e = cudaMalloc(&w->qs, qbytes)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight codes)"); }
-    // 16 spare bytes: the single-kernel decode step fetches scales in whole 16-byte pieces
+    // 16 spare bytes: scales may be fetched in whole 16-byte pieces
     if ((e = cudaMalloc((void **)&w->d, (size_t)nblocks * 2 + 16)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight scales)"); }
     cudaMemsetAsync((uint8_t *)w->d + (size_t)nblocks * 2, 0, 16, ctx->stream);
     w->device_bytes = (int64_t)qbytes + nblocks * 2;
@@ -507,7 +507,7 @@ int caten_b200_eval_expr(caten_b200_ctx *ctx, const caten_b200_expr *e) {
 namespace cb {
 
 int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, const float *x, BfOut xbf, const float *bias, const float *res,
-                 int act, float *y, BfOut ybf, int64_t M, PartIn *defer, LinGroups grp) {
+                 int act, float *y, BfOut ybf, int64_t M, PartIn *defer, LinGroups grp, GemvNorm norm) {
   if (defer) *defer = PartIn();
   if (M <= 0) return 0;
   if (int rc = check_glu(ctx, "linear", w, act, res)) return rc;
@@ -515,7 +515,7 @@ int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, cons
   if (res && !grp.plain_output()) return fail(ctx, CATEN_B200_EUNSUPPORTED, "linear: a residual needs the plain output layout");
   ProfScope prof(ctx, M <= 4 ? CATEN_B200_K_GEMV : CATEN_B200_K_GEMM);
   if (M <= 4) {
-    return launch_gemv(ctx, w, x, bias, res, act, y, M, grp);
+    return launch_gemv(ctx, w, x, bias, res, act, y, M, grp, norm);
   }
   if (prec == CATEN_B200_PREC_FP32) return launch_gemm_simt(ctx, w, x, bias, res, act, y, M, grp);
   const int nsplit = prec == CATEN_B200_PREC_BF16X3 ? 3 : 1;
@@ -544,16 +544,15 @@ struct caten_b200_gpt2 {
   // decode replayed from a CUDA graph: position and ids live on the device
   cb::StepLoop loop;
   int *h_pos_pinned = nullptr;
-  // 1..4 sequences: the whole single-token step is one kernel (decode_small.cu); CATEN_B200_PERSISTENT=0 keeps
-  // the kernel-per-operation path
-  cb::DecodeSmall *ds = nullptr;
-  int64_t ds_failures_seen = 0;
+  // 1..4 sequences over Q4_0 / Q8_0 layers: profiling times a single-token step as a whole (class DECODE_STEP), and the
+  // device entry replays the captured step too.  CATEN_B200_PERSISTENT=0: per kernel, and launch by launch
+  bool whole_step = false;
   bool defer_reduce = true;  // CATEN_B200_DEFER_REDUCE=0 keeps a reduction kernel behind every split-K linear
 };
 
 static int model_linear(caten_b200_gpt2 *m, const caten_b200_weight *w, const float *x, cb::BfOut xbf, const float *bias,
-                        const float *res, int act, float *y, cb::BfOut ybf, int64_t M, cb::PartIn *defer = nullptr) {
-  return cb::model_linear(m->ctx, m->desc.precision, w, x, xbf, bias, res, act, y, ybf, M, defer);
+                        const float *res, int act, float *y, cb::BfOut ybf, int64_t M, cb::PartIn *defer = nullptr, cb::GemvNorm norm = cb::GemvNorm()) {
+  return cb::model_linear(m->ctx, m->desc.precision, w, x, xbf, bias, res, act, y, ybf, M, defer, cb::LinGroups(), norm);
 }
 
 extern "C" {
@@ -626,14 +625,11 @@ int caten_b200_gpt2_create(caten_b200_ctx *ctx, const caten_b200_gpt2_desc *dsc,
   if (!rc && cudaMallocHost(&m->h_pos_pinned, sizeof(int)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(pos)");
   if (!rc && cudaMallocHost(&m->h_ids_pinned, (size_t)B * T * sizeof(float)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(ids)");
   if (!rc && cudaMallocHost(&m->h_out_pinned, (size_t)B * sizeof(int64_t)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(out ids)");
-  bool persistent = true;
-  if (const char *e = getenv("CATEN_B200_PERSISTENT")) persistent = atoi(e) != 0;
-  if (!rc && persistent && cb::decode_small_supported(m->desc, m->attn_w.data(), m->proj_w.data(), m->fc_w.data(), m->mproj_w.data())) {
-    const std::vector<const float *> vecs[8] = {m->ln1_g, m->ln1_b, m->attn_b, m->proj_b, m->ln2_g, m->ln2_b, m->fc_b, m->mproj_b};
-    rc = cb::decode_small_create(ctx, m->desc, m->attn_w, m->proj_w, m->fc_w, m->mproj_w, vecs, m->kc, m->vc, m->loop.ids_io, m->loop.out_ids,
-                                 m->loop.hist, m->loop.d_pos, m->logits, &m->ds);
-    m->ds_failures_seen = ctx->device_failures;
-  }
+  m->whole_step = B <= 4;
+  for (int64_t l = 0; l < L; ++l)
+    for (const caten_b200_weight *w : {m->attn_w[l], m->proj_w[l], m->fc_w[l], m->mproj_w[l]})
+      m->whole_step = m->whole_step && (w->type == CATEN_B200_Q4_0 || w->type == CATEN_B200_Q8_0);
+  if (const char *e = getenv("CATEN_B200_PERSISTENT")) m->whole_step = m->whole_step && atoi(e) != 0;
   if (rc) { caten_b200_gpt2_destroy(m); return rc; }
   m->launches0 = ctx->launches;
   *out = m;
@@ -650,7 +646,6 @@ int caten_b200_gpt2_destroy(caten_b200_gpt2 *m) {
   float *bufs[] = {m->h, m->h2, m->xn, m->qkv, m->att, m->ff, m->last, m->logits, m->ids_f32};
   for (float *p : bufs) if (p) cudaFree(p);
   cb::step_loop_free(&m->loop);
-  cb::decode_small_destroy(m->ds);
   if (m->bf_arena) cudaFree(m->bf_arena);
   if (m->h_pos_pinned) cudaFreeHost(m->h_pos_pinned);
   if (m->h_ids_pinned) cudaFreeHost(m->h_ids_pinned);
@@ -658,6 +653,9 @@ int caten_b200_gpt2_destroy(caten_b200_gpt2 *m) {
   delete m;
   return 0;
 }
+
+// Single-token steps of up to four sequences: lm_head normalises its input rows, which are the stream itself
+static bool head_norms(const caten_b200_gpt2 *m, int64_t s) { return s == 1 && m->desc.batch <= 4; }
 
 // Runs the Transformer (external/llm/layers.lisp:81-90) on `nb` sequences [b0, b0+nb) of s tokens.
 static int run_chunk(caten_b200_gpt2 *m, const float *ids_f32, const int64_t *ids_i64, int64_t b0, int64_t nb, int64_t s,
@@ -690,13 +688,16 @@ static int run_chunk(caten_b200_gpt2 *m, const float *ids_f32, const int64_t *id
     return pin.splits > 0 ? launch_layernorm_pending(ctx, pin, res, x, g, b, y, rows, d, eps, stride, o)
                           : launch_layernorm_strided(ctx, x, g, b, y, rows, d, eps, stride, o);
   };
+  const bool few = R <= 4;   // rows for the GEMV, which normalises its input itself
   for (int64_t l = 0; l < L; ++l) {
-    int rc = layernorm(pend_h, m->h2, m->h, m->ln1_g[l], m->ln1_b[l], m->xn, R, 1, bf(m->xn_bf));
-    if (!rc) rc = model_linear(m, m->attn_w[l], m->xn, m->xn_bf, m->attn_b[l], nullptr, CATEN_B200_ACT_NONE, m->qkv, none, R, defer_ok ? &pend_qkv : nullptr);
+    cb::GemvNorm n1, n2;
+    if (few) { n1.g = m->ln1_g[l]; n1.b = m->ln1_b[l]; n2.g = m->ln2_g[l]; n2.b = m->ln2_b[l]; n1.eps = n2.eps = eps; }
+    int rc = few ? 0 : layernorm(pend_h, m->h2, m->h, m->ln1_g[l], m->ln1_b[l], m->xn, R, 1, bf(m->xn_bf));
+    if (!rc) rc = model_linear(m, m->attn_w[l], few ? m->h : m->xn, m->xn_bf, m->attn_b[l], nullptr, CATEN_B200_ACT_NONE, m->qkv, none, R, defer_ok ? &pend_qkv : nullptr, n1);
     if (!rc) { ProfScope prof(ctx, s == 1 ? CATEN_B200_K_ATTN_DECODE : CATEN_B200_K_ATTN_PREFILL); rc = launch_attention(ctx, m->qkv, m->kc[l] + kv_off, m->vc[l] + kv_off, m->att, nb, s, n, H, T, d_n, bf(m->att_bf), &pend_qkv, prec != CATEN_B200_PREC_FP32 && ctx->attn_tc); }
     if (!rc) rc = model_linear(m, m->proj_w[l], m->att, m->att_bf, m->proj_b[l], m->h, CATEN_B200_ACT_NONE, m->h2, none, R, defer_ok ? &pend_h2 : nullptr);
-    if (!rc) rc = layernorm(pend_h2, m->h, m->h2, m->ln2_g[l], m->ln2_b[l], m->xn, R, 1, bf(m->xn_bf));
-    if (!rc) rc = model_linear(m, m->fc_w[l], m->xn, m->xn_bf, m->fc_b[l], nullptr, CATEN_B200_ACT_GELU, m->ff, bf(m->ff_bf), R);
+    if (!rc && !few) rc = layernorm(pend_h2, m->h, m->h2, m->ln2_g[l], m->ln2_b[l], m->xn, R, 1, bf(m->xn_bf));
+    if (!rc) rc = model_linear(m, m->fc_w[l], few ? m->h2 : m->xn, m->xn_bf, m->fc_b[l], nullptr, CATEN_B200_ACT_GELU, m->ff, bf(m->ff_bf), R, nullptr, n2);
     if (!rc) rc = model_linear(m, m->mproj_w[l], m->ff, m->ff_bf, m->mproj_b[l], m->h2, CATEN_B200_ACT_NONE, m->h, none, R, defer_ok ? &pend_h : nullptr);
     if (rc) return rc;
   }
@@ -704,10 +705,19 @@ static int run_chunk(caten_b200_gpt2 *m, const float *ids_f32, const int64_t *id
   // logits, layers.lisp:90), gathered into rows [b0, b0+nb) of `last`
   cb::BfOut lb;
   if (prec != CATEN_B200_PREC_FP32 && c.batch > 4) { lb.hi = m->last_bf.hi + b0 * d; lb.lo = x3 ? m->last_bf.lo + b0 * d : nullptr; }
+  if (head_norms(m, s)) return 0;   // lm_head does it
   return layernorm(pend_h, m->h2, m->h, c.lnf_g, c.lnf_b, m->last + b0 * d, nb, s, lb);
 }
 
-static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host);
+// logits of the last positions (lm_head has no bias, layers.lisp:79)
+static int head(caten_b200_gpt2 *m, int64_t s) {
+  const caten_b200_gpt2_desc &c = m->desc;
+  cb::GemvNorm norm;
+  if (head_norms(m, s)) { norm.g = c.lnf_g; norm.b = c.lnf_b; norm.eps = c.eps; }
+  return model_linear(m, c.lm_head, norm.g ? m->h : m->last, m->last_bf, nullptr, nullptr, CATEN_B200_ACT_NONE, m->logits, cb::BfOut(), c.batch, nullptr, norm);
+}
+
+static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps);
 
 int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, const int64_t *d_ids_i64, int64_t s, int64_t n,
                                 int64_t *d_out_ids) {
@@ -720,10 +730,9 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
   if (s < 1 || n < 0 || n + s > c.max_seq_len)
     return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: s=%lld n=%lld outside the cache (max_seq_len=%d)", (long long)s, (long long)n, c.max_seq_len);
   const int64_t B = c.batch;
-  if (s == 1 && m->ds) {
-    // single-token step of a few sequences: the one-kernel path, fed from the device-side state
+  if (s == 1 && m->whole_step) {
     if (int rc = launch_begin_steps(ctx, d_ids_f32, d_ids_i64, m->loop.ids_io, m->loop.d_pos, n, B)) return rc;
-    if (int rc = decode_step_device_pos(m, n)) return rc;
+    if (int rc = decode_run(m, n, 1)) return rc;
     if (d_out_ids != m->loop.out_ids)
       CB_CUDA(ctx, cudaMemcpyAsync(d_out_ids, m->loop.out_ids, (size_t)B * sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
     return 0;
@@ -735,13 +744,12 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
     const int64_t nb = B - b0 < per ? B - b0 : per;
     if (int rc = run_chunk(m, d_ids_f32, d_ids_i64, b0, nb, s, n)) return rc;
   }
-  // lm_head (no bias, layers.lisp:79) + argmax over the vocabulary
-  if (int rc = model_linear(m, c.lm_head, m->last, m->last_bf, nullptr, nullptr, CATEN_B200_ACT_NONE, m->logits, cb::BfOut(), B)) return rc;
+  // lm_head + argmax over the vocabulary
+  if (int rc = head(m, s)) return rc;
   ProfScope prof(ctx, CATEN_B200_K_ARGMAX);
   return launch_argmax(ctx, m->logits, B, c.vocab, d_out_ids);
 }
 
-static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps);
 
 int caten_b200_gpt2_step(caten_b200_gpt2 *m, const float *h_ids_f32, int64_t s, int64_t n, int64_t *h_out_ids) {
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "gpt2_step: model is NULL");
@@ -773,24 +781,24 @@ int caten_b200_gpt2_step(caten_b200_gpt2 *m, const float *h_ids_f32, int64_t s, 
 static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host) {
   caten_b200_ctx *ctx = m->ctx;
   const caten_b200_gpt2_desc &c = m->desc;
-  if (m->ds) {
-    if (m->ds_failures_seen != ctx->device_failures) {   // an interrupted step left half-written exchange words
-      if (int rc = cb::decode_small_reset(ctx, m->ds)) return rc;
-      m->ds_failures_seen = ctx->device_failures;
-    }
-    ProfScope prof(ctx, CATEN_B200_K_DECODE_STEP);
-    return cb::decode_small_launch(ctx, m->ds);
-  }
-  if (int rc = run_chunk(m, nullptr, m->loop.ids_io, 0, c.batch, 1, n_host, m->loop.d_pos)) return rc;
-  if (int rc = model_linear(m, c.lm_head, m->last, m->last_bf, nullptr, nullptr, CATEN_B200_ACT_NONE, m->logits, cb::BfOut(), c.batch)) return rc;
-  if (int rc = launch_argmax(ctx, m->logits, c.batch, c.vocab, m->loop.out_ids)) return rc;
-  return launch_finish_step(ctx, m->loop.out_ids, m->loop.ids_io, m->loop.hist, m->loop.d_pos, c.batch);
+  auto step = [&]() {
+    if (int rc = run_chunk(m, nullptr, m->loop.ids_io, 0, c.batch, 1, n_host, m->loop.d_pos)) return rc;
+    if (int rc = head(m, 1)) return rc;
+    if (int rc = launch_argmax(ctx, m->logits, c.batch, c.vocab, m->loop.out_ids)) return rc;
+    return launch_finish_step(ctx, m->loop.out_ids, m->loop.ids_io, m->loop.hist, m->loop.d_pos, c.batch);
+  };
+  if (!m->whole_step || !(ctx->prof_mask & (1u << CATEN_B200_K_DECODE_STEP))) return step();
+  ProfScope prof(ctx, CATEN_B200_K_DECODE_STEP);
+  const unsigned mask = ctx->prof_mask;
+  ctx->prof_mask = 0;   // the step's kernels are part of it
+  const int rc = step();
+  ctx->prof_mask = mask;
+  return rc;
 }
 
 // Runs `steps` single-token steps from the device-side state.
 static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps) {
-  // event brackets cannot be placed inside a graph; a step that is one kernel already gains nothing from one
-  const bool use_graph = m->ctx->prof_mask == 0 && !m->ds;
+  const bool use_graph = m->ctx->prof_mask == 0;   // event brackets cannot be placed inside a graph
   return cb::step_loop_run(m->ctx, &m->loop, n, steps, m->desc.max_seq_len, use_graph, [m](int64_t pos) { return decode_step_device_pos(m, pos); });
 }
 

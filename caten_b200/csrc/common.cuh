@@ -210,8 +210,14 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
                      const cb::PartIn *pending_qkv = nullptr, int tensor_cores = 0);
 int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B,
                         int64_t s, int64_t n, int64_t H, int64_t T, cb::BfOut bf);
+// LayerNorm of a linear's input rows, done by the linear itself (up to four rows)
+struct GemvNorm {
+  const float *g = nullptr, *b = nullptr;   // g NULL: x as it is
+  float eps = 0.0f;
+};
+
 int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
-                const float *res, int act, float *y, int64_t M = 1, LinGroups grp = LinGroups());   // M: 1 to 4 rows of x
+                const float *res, int act, float *y, int64_t M = 1, LinGroups grp = LinGroups(), GemvNorm norm = GemvNorm());   // M: 1 to 4 rows of x
 int launch_gemm_simt(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
                      const float *res, int act, float *y, int64_t M, LinGroups grp = LinGroups());
 int launch_gemm_tc(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
@@ -259,7 +265,7 @@ int launch_splitk_reduce(caten_b200_ctx *ctx, const float *part, int splits, int
 // the Linear of a model: GEMV for up to 4 rows, otherwise the GEMM of `prec`; with a tensor-core precision the input is
 // xbf when it is set (written by its producer), and the output can be requested the same way (ybf)
 int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, const float *x, BfOut xbf, const float *bias, const float *res,
-                 int act, float *y, BfOut ybf, int64_t M, PartIn *defer = nullptr, LinGroups grp = LinGroups());
+                 int act, float *y, BfOut ybf, int64_t M, PartIn *defer = nullptr, LinGroups grp = LinGroups(), GemvNorm norm = GemvNorm());
 
 // Whether the next launch may be a programmatic dependent launch; clears the pending-upload mark.
 inline bool take_pdl(caten_b200_ctx *ctx) {
@@ -267,21 +273,6 @@ inline bool take_pdl(caten_b200_ctx *ctx) {
   ctx->weights_pending = false;
   return ok;
 }
-
-// Single-kernel decode step for 1..4 sequences (decode_small.cu)
-struct DecodeSmall;
-bool decode_small_supported(const caten_b200_gpt2_desc &c, const caten_b200_weight *const *attn, const caten_b200_weight *const *proj,
-                            const caten_b200_weight *const *fc, const caten_b200_weight *const *mproj);
-// vecs: eight per-layer tables in the order ln1_g, ln1_b, attn_b, proj_b, ln2_g, ln2_b, fc_b, mproj_b
-int decode_small_create(caten_b200_ctx *ctx, const caten_b200_gpt2_desc &c, const std::vector<const caten_b200_weight *> &attn,
-                        const std::vector<const caten_b200_weight *> &proj, const std::vector<const caten_b200_weight *> &fc,
-                        const std::vector<const caten_b200_weight *> &mproj, const std::vector<const float *> *vecs,
-                        const std::vector<float *> &kc, const std::vector<float *> &vc, int64_t *ids_io, int64_t *out_ids, int64_t *hist,
-                        int *d_pos, float *logits, DecodeSmall **out);
-void decode_small_destroy(DecodeSmall *s);
-int decode_small_launch(caten_b200_ctx *ctx, DecodeSmall *s);
-// after a kernel-side failure the exchange words of the interrupted step are stale: forget them
-int decode_small_reset(caten_b200_ctx *ctx, DecodeSmall *s);
 
 // Kernel launch with programmatic dependent launch allowed: the next kernel in the stream may be
 // scheduled (and run its prologue) while this one drains; every kernel launched this way calls

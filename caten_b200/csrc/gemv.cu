@@ -8,6 +8,48 @@
 
 namespace cb {
 
+// LayerNorm of the rows of x where they lie in shared memory (float4 i of row m at at(m, i)): every CTA does it for itself,
+// which costs a linear about 0.6 us where a kernel of its own, one CTA and one more hand-off, cost 1.8 to 2.9.  gamma and beta
+// (2 x K floats of shared memory) are staged before the wait for x.  The order of a row's statistics is one warp's.
+__device__ __forceinline__ void gemv_stage_norm(const GemvNorm &n, float *gb, int K) {
+  if (!n.g) return;
+  for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
+    reinterpret_cast<float4 *>(gb)[i] = reinterpret_cast<const float4 *>(n.g)[i];
+    reinterpret_cast<float4 *>(gb + K)[i] = reinterpret_cast<const float4 *>(n.b)[i];
+  }
+}
+
+template <class At>
+__device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const float *gb, int M, int K, At at) {
+  if (!n.g) return;
+  __shared__ float stat[4][2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K4 = K / 4;
+  for (int m = warp; m < M; m += blockDim.x >> 5) {
+    const float invd = 1.0f / (float)K;
+    float sum = 0.0f, sq = 0.0f;
+    for (int i = lane; i < K4; i += 32) {
+      const float4 v = *at(m, i);
+      sum += (v.x + v.y) + (v.z + v.w);
+    }
+    const float u = warp_sum(sum) * invd;
+    for (int i = lane; i < K4; i += 32) {
+      const float4 v = *at(m, i);
+      const float x = v.x - u, y = v.y - u, z = v.z - u, w = v.w - u;
+      sq += (x * x + y * y) + (z * z + w * w);
+    }
+    const float var = warp_sum(sq) * invd;
+    if (lane == 0) { stat[m][0] = u; stat[m][1] = 1.0f / sqrtf(var + n.eps); }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < M * K4; i += blockDim.x) {
+    const int m = i / K4, j = i - m * K4;
+    const float u = stat[m][0], rs = stat[m][1];
+    const float4 v = *at(m, j), gg = reinterpret_cast<const float4 *>(gb)[j], bb = reinterpret_cast<const float4 *>(gb + K)[j];
+    *at(m, j) = make_float4(((v.x - u) * rs) * gg.x + bb.x, ((v.y - u) * rs) * gg.y + bb.y, ((v.z - u) * rs) * gg.z + bb.z, ((v.w - u) * rs) * gg.w + bb.w);
+  }
+  __syncthreads();
+}
+
 struct GemvArgs {
   const void *qs;
   const __half *d, *m;   // scales; minima (Q4_1, Q5_1)
@@ -15,6 +57,7 @@ struct GemvArgs {
   const float *x, *bias, *res;
   float *y;
   int act, N, nkb, G, M;
+  GemvNorm norm;
 };
 
 constexpr int GEMV_MAX_THREADS = 512;
@@ -38,6 +81,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   const int tid = threadIdx.x, nkb = a.nkb, G = a.G;
   float *xs = gemv_smem;                              // [M][nkb][GEMV_XPAD]
   float *red = gemv_smem + a.M * nkb * GEMV_XPAD;     // two buffers of [G * RI][nkb]
+  float *gb = red + 2 * G * RI * nkb;                 // norm: gamma and beta
   const bool active = tid < G * nkb;
   const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
   const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
@@ -66,6 +110,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   };
   int64_t base = (int64_t)blockIdx.x * rows_per_iter;
   load(base);
+  gemv_stage_norm(a.norm, gb, nkb * 32);
   pdl_wait();
   for (int i = tid; i < a.M * nkb * 8; i += blockDim.x)
     *reinterpret_cast<float4 *>(xs + (i >> 3) * GEMV_XPAD + (i & 7) * 4) = reinterpret_cast<const float4 *>(a.x)[i];
@@ -79,6 +124,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   float bz, rz;
   addends(0, &bz, &rz);
   __syncthreads();
+  gemv_norm_rows(a.norm, gb, a.M, nkb * 32, [&](int m, int i) { return reinterpret_cast<float4 *>(xs + (m * nkb + (i >> 3)) * GEMV_XPAD + (i & 7) * 4); });
   BLK blk;
   int buf = 0;
   for (bool again = false; base < a.N; base += stride, again = true) {
@@ -192,6 +238,7 @@ struct GemvDense {
   int64_t xplane, ygroup, ldy;   // ldy: between the outputs of two rows of x
   const int *expert;
   const float *weight;
+  GemvNorm norm;
 };
 
 template <typename T, int RI, int NR, bool EXPERTS>
@@ -236,7 +283,11 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   int64_t base = ((int64_t)blockIdx.x * slots + slot) * RI;
   const int64_t stride = (int64_t)gridDim.x * slots * RI;
   load(base, c0);
-  if (!EXPERTS) pdl_wait();
+  float *gb = xs + NR * K;
+  if (!EXPERTS) {
+    gemv_stage_norm(a.norm, gb, K);
+    pdl_wait();
+  }
   // the lane that finishes output (row base + i, row m of x) is lane i * NR + m of the slot's first warp
   const int fi = lane / NR, fm = lane % NR;
   const bool glu_rows = RI == 2 && act_is_glu(a.act);
@@ -250,6 +301,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   for (int i = threadIdx.x; i < NR * K / 4; i += 256)
     reinterpret_cast<float4 *>(xs)[i] = NR == 1 || i < a.M * K / 4 ? reinterpret_cast<const float4 *>(x)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
+  if (!EXPERTS) gemv_norm_rows(a.norm, gb, a.M, K, [&](int m, int i) { return reinterpret_cast<float4 *>(xs + (size_t)m * K) + i; });
   const int64_t rounds = ((int64_t)N + stride - 1) / stride;   // the same for every warp: the slots' warps meet at barriers
   for (int64_t it = 0; it < rounds; ++it) {
     float acc[RI][NR];
@@ -319,7 +371,7 @@ template <class BLK, int RI, bool LOOP, int THREADS>
 static int launch_blocked_t(caten_b200_ctx *ctx, GemvArgs a) {
   a.G = THREADS / a.nkb;
   const int threads = (a.G * a.nkb + 31) / 32 * 32;
-  const size_t smem = ((size_t)a.M * a.nkb * GEMV_XPAD + 2 * (size_t)a.G * RI * a.nkb) * sizeof(float);
+  const size_t smem = ((size_t)a.M * a.nkb * GEMV_XPAD + 2 * (size_t)a.G * RI * a.nkb + (a.norm.g ? 2 * 32 * (size_t)a.nkb : 0)) * sizeof(float);
   auto kernel = gemv_blocked_kernel<BLK, RI, LOOP, THREADS>;
   if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t grid = ((int64_t)a.N + a.G * RI - 1) / (a.G * RI);
@@ -342,6 +394,7 @@ static int launch_blocked(caten_b200_ctx *ctx, const GemvArgs &a) {
   const int deep = 16 / BLK::WORDS;   // loads per thread with three CTAs
   if (a.N <= (small ? 3 : 1) * slab) return launch_blocked_t<BLK, 1, false, 256>(ctx, a);
   if (a.N <= (small ? 3 : 1) * 2 * slab) return launch_blocked_t<BLK, 2, false, 256>(ctx, a);
+  if (a.N <= (small ? deep >= 4 ? 3 : 2 : 1) * 3 * slab) return launch_blocked_t<BLK, 3, false, 256>(ctx, a);
   if (a.N <= (small ? deep >= 4 ? 3 : 2 : 1) * 4 * slab) return launch_blocked_t<BLK, 4, false, 256>(ctx, a);
   return launch_blocked_t<BLK, 4, true, 256>(ctx, a);
 }
@@ -355,7 +408,7 @@ static int launch_dense_t(caten_b200_ctx *ctx, GemvDense g, int groups) {
   while (ks < 8 && (nvec > 32 * GEMV_PRE * ks || (nvec > 64 * ks && ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI) * groups < 2 * ctx->sm_count))) ks *= 2;
   g.ks = ks;
   const int64_t ctas = ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI);
-  const size_t smem = (size_t)NR * g.K * sizeof(float);
+  const size_t smem = ((size_t)NR + (g.norm.g ? 2 : 0)) * g.K * sizeof(float);
   auto kernel = gemv_dense_kernel<T, RI, NR, EXPERTS>;
   if (smem > 47 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t grid = ((int64_t)ctx->sm_count * (smem > 72 * 1024 || RI == 2 ? 2 : 3) + groups - 1) / groups;   // resident at once
@@ -380,21 +433,22 @@ static int launch_dense(caten_b200_ctx *ctx, const GemvDense &g, int groups) {
 
 // M rows of x, 1 to 4
 int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x, const float *bias,
-                const float *res, int act, float *y, int64_t M, LinGroups grp) {
+                const float *res, int act, float *y, int64_t M, LinGroups grp, GemvNorm norm) {
   if (w->rows > 0x7fffffff || w->cols > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: dimension too large");
   const int N = (int)w->rows, K = (int)w->cols;
+  if (norm.g && (K % 4 || K > 2400)) return fail(ctx, CATEN_B200_EUNSUPPORTED, "layernorm: d=%d (need d%%4==0, d<=2400)", K);
   if (!type_is_packed(w->type) && (size_t)K * sizeof(float) > 160 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide", K);
   if (M > 1 && (M > 4 || (size_t)K * 4 * sizeof(float) > 160 * 1024)) {   // rows of x that do not fit shared memory together: one by one
     const int64_t ny = grp.ldy ? grp.ldy : act_is_glu(act) ? N / 2 : N;
     for (int64_t m = 0; m < M; ++m)
-      if (int rc = launch_gemv(ctx, w, x + m * K, bias, res ? res + m * ny : nullptr, act, y + m * ny, 1, grp)) return rc;
+      if (int rc = launch_gemv(ctx, w, x + m * K, bias, res ? res + m * ny : nullptr, act, y + m * ny, 1, grp, norm)) return rc;
     return 0;
   }
   if (type_is_packed(w->type)) {
     if (grp.group_rows || act_is_glu(act)) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: input groups and the gated activation take dense weights");
     GemvArgs a;
     a.qs = w->qs; a.d = w->d; a.m = w->m; a.qh = w->qh; a.x = x; a.bias = bias; a.res = res; a.y = y; a.act = act; a.N = N;
-    a.nkb = (int)w->nkb; a.M = (int)M;
+    a.nkb = (int)w->nkb; a.M = (int)M; a.norm = norm;
     if (a.nkb > GEMV_MAX_THREADS) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide (max %d)", K, GEMV_MAX_THREADS * 32);
     switch (w->type) {
       case CATEN_B200_Q4_0: return launch_blocked<BlkQ4>(ctx, a);
@@ -409,7 +463,7 @@ int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x,
   g.group_rows = grp.group_rows > 0 ? (int)grp.group_rows : N;
   g.xplane = grp.xplane; g.ygroup = grp.ygroup ? grp.ygroup : act_is_glu(act) ? g.group_rows / 2 : g.group_rows;
   g.ldy = grp.ldy ? grp.ldy : act_is_glu(act) ? N / 2 : N;
-  g.expert = nullptr; g.weight = nullptr;
+  g.expert = nullptr; g.weight = nullptr; g.norm = norm;
   const int ng = grp.group_rows > 0 ? (int)((N + grp.group_rows - 1) / grp.group_rows) : 1;
   switch (w->type) {
     case CATEN_B200_F32: return launch_dense<float, false>(ctx, g, ng);

@@ -503,7 +503,7 @@ int caten_b200_eval_expr(caten_b200_ctx *ctx, const caten_b200_expr *e);
 enum {
   CATEN_B200_K_EMBED = 0, CATEN_B200_K_LAYERNORM = 1, CATEN_B200_K_GEMV = 2, CATEN_B200_K_GEMM = 3,
   CATEN_B200_K_ATTN_DECODE = 4, CATEN_B200_K_ATTN_PREFILL = 5, CATEN_B200_K_ARGMAX = 6,
-  CATEN_B200_K_DECODE_STEP = 7,   /* the whole single-token step of 1..4 sequences, which is one kernel */
+  CATEN_B200_K_DECODE_STEP = 7,   /* the whole single-token step of 1..4 sequences over Q4_0 / Q8_0 layers (with this class the step's kernels are not timed by themselves) */
   CATEN_B200_K_WKV = 8,           /* recurrence of a time-mixing or retention layer */
   CATEN_B200_K_PREP = 9,          /* rotation, q/k norm and cache append; token-shift mixes; expert routing */
   CATEN_B200_K_EXPERTS = 10,      /* linears of a mixture of experts */
