@@ -126,14 +126,16 @@ struct caten_b200_ctx {
   bool pin_busy[2] = {false, false};
   long long attn_prefetch_bytes = 64ll << 20;  // L2 budget of the decode attention's K / V history hint (CATEN_B200_ATTN_PREFETCH_MB; 0 = off)
   bool dense_gemm = true;    // many-row linears expand the weights once and run the TMA-fed GEMM (CATEN_B200_DENSE_GEMM=0: off)
+  bool dense_pair = true;    // its tiles by pairs of CTAs where that is expected to be faster (CATEN_B200_DENSE_PAIR=0: off)
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   int64_t launches = 0;
   int64_t device_failures = 0;   // kernel-side check failures reported so far
-  // split-K partial tiles: reduced by a second kernel through global scratch (default: it overlaps
-  // with its neighbours under programmatic dependent launch and measured faster), or inside a
-  // thread-block cluster through distributed shared memory (CATEN_B200_SPLITK_CLUSTER=1: every split-K
-  // launch; =2: only launches whose epilogue cannot be handed to the consuming kernel)
-  int splitk_cluster = 0;
+  // split-K partial tiles of the converting GEMM: reduced by a second kernel through global scratch, or inside a thread-block
+  // cluster through distributed shared memory.  By default (-1) the cluster for up to 128 rows where the consumer cannot sum
+  // the tiles itself (GPT-2 medium, 64 sequences: 1345 us a step with the second kernel, 1327 us so; GPT-2 XL, 256 sequences:
+  // 0.7 % slower in a cluster).  CATEN_B200_SPLITK_CLUSTER=0: never; 1: every split-K launch; 2: every launch whose epilogue
+  // cannot be handed to the consuming kernel
+  int splitk_cluster = -1;
   int attn_tc = 1;           // prefill attention of a tensor-core model on the tensor cores (CATEN_B200_ATTN_TC=0: SIMT kernel)
   bool use_pdl = true;       // programmatic dependent launch between consecutive kernels (CATEN_B200_PDL=0 turns it off)
   // A weight upload queued copy / re-layout kernels on the stream.  The Linear kernels read their

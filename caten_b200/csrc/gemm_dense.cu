@@ -11,6 +11,9 @@
 //               activation and the residual, store — while the next tile's MMAs run
 // Tile = 128 output features (TMEM lanes) x 256 rows (TMEM columns); a stage holds 64 k (bf16) or 32 k (split bf16).
 // Split-bf16 (NSPLIT = 3) issues W_hi.x_hi + W_lo.x_hi + W_hi.x_lo per k-step, as the decode GEMM.
+// PAIR: two CTAs of a cluster work on 256 features x bn rows (cta_group::2): each loads its 128 features and half of the rows
+// of x, the even one issues the MMAs for both, and each has the accumulators of its features in its own tensor memory.  Both
+// CTAs' loads complete on the leader's barriers, commits arrive in both CTAs, and the epilogues of both free the accumulators.
 // EXPERTS (mixture of experts): the rows of x are sorted by expert; expert e's rows [offsets[e], offsets[e + 1]), read on
 // the device, are multiplied with its own rows of W.  The tile list is formed from the offsets in every CTA; a row tile
 // may reach into the next expert's rows, whose products are not stored.  The row tile is as narrow as the experts' rows
@@ -62,8 +65,9 @@ constexpr int GD_SPLIT_ROWS = 512;     // rows up to which k is shared among CTA
 struct GdTile {
   int f0, f_end, m0, m_end, x0, shift;
 };
-template <bool EXPERTS>
-__device__ __forceinline__ GdTile gd_tile(const GdArgs &a, int tile, const int *first) {
+// (rank: of a CTA in its pair, which takes 128 features and half of the x rows to load each)
+template <bool EXPERTS, bool PAIR>
+__device__ __forceinline__ GdTile gd_tile(const GdArgs &a, int tile, const int *first, int rank) {
   GdTile t;
   if (EXPERTS) {   // first[e] = index of expert e's first tile
     int lo = 0, hi = a.er.experts;   // the last e with first[e] <= tile (an expert without rows has no tiles)
@@ -79,12 +83,12 @@ __device__ __forceinline__ GdTile gd_tile(const GdArgs &a, int tile, const int *
     t.shift = lo * a.group_rows;
   } else {
     const int f = tile % a.tiles_f, g = f / a.tiles_per_group;
-    t.f0 = g * a.group_rows + (f % a.tiles_per_group) * GD_BM;
-    t.f_end = min(a.N, (g + 1) * a.group_rows);
+    t.f0 = PAIR ? (2 * f + rank) * GD_BM : g * a.group_rows + (f % a.tiles_per_group) * GD_BM;
+    t.f_end = PAIR ? a.N : min(a.N, (g + 1) * a.group_rows);
     t.m0 = (tile / a.tiles_f) * a.bn;
     t.m_end = a.M;
-    t.x0 = t.m0 + g * a.xplane;
-    t.shift = g * (a.group_rows - a.ygroup);
+    t.x0 = PAIR ? t.m0 + rank * (a.bn / 2) : t.m0 + g * a.xplane;
+    t.shift = PAIR ? 0 : g * (a.group_rows - a.ygroup);
   }
   return t;
 }
@@ -232,7 +236,7 @@ __device__ __forceinline__ uint64_t gd_desc(uint32_t saddr) {
   return d;
 }
 
-template <int NSPLIT, bool EXPERTS, bool WLO>
+template <int NSPLIT, bool EXPERTS, bool WLO, bool PAIR>
 __global__ void __launch_bounds__(GD_THREADS, 1)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_constant__ CUtensorMap tw_lo,
                   const __grid_constant__ CUtensorMap tx_hi, const __grid_constant__ CUtensorMap tx_lo, const GdArgs a) {
@@ -240,7 +244,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
   constexpr uint32_t ROW_BYTES = BK * 2u;
   const int BN = a.bn;
   constexpr uint32_t W_BYTES = GD_BM * ROW_BYTES;
-  const uint32_t X_BYTES = (uint32_t)BN * ROW_BYTES;
+  const uint32_t X_BYTES = (uint32_t)(PAIR ? BN / 2 : BN) * ROW_BYTES;
   const uint32_t STAGE_BYTES = W_BYTES * (WLO ? 2u : 1u) + X_BYTES * (NSPLIT == 3 ? 2u : 1u);
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -264,6 +268,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int num_k = a.K / BK;
+  const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   // work item i: tile i % tiles, k-stages [i / tiles * cps, ..) of it
   auto k_of = [&](int z, int *k0) {
     *k0 = z * a.cps;
@@ -277,18 +282,24 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full(b), 1);
-      mbar_init(acc_empty(b), GD_EPI_WARPS);
+      mbar_init(acc_empty(b), PAIR ? 2 * GD_EPI_WARPS : GD_EPI_WARPS);
     }
     abort_flag[0] = 0;
     abort_flag[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(a.tmem_cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(a.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(a.tmem_cols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();   // both CTAs' barriers are initialised
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
@@ -300,16 +311,24 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       tma_prefetch_map(&tx_lo);
     }
   }
+  // a stage's bytes, those of both CTAs of a pair, complete on the leader's barrier
+  auto expect = [&](int s) {
+    if (rank == 0) mbar_expect_tx(full(s), PAIR ? 2 * STAGE_BYTES : STAGE_BYTES);
+  };
+  auto load = [&](uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
+    if (PAIR) tma_load_2d_pair(dst, map, bar, x, y);
+    else tma_load_2d(dst, map, bar, x, y);
+  };
   // Weights that no kernel writes are on their way before the wait below: in a decode step that is most of what this CTA
   // reads, and it arrives while the kernel that produces x still runs.
   int ahead = 0;   // stages whose W tiles have been asked for
   if (!EXPERTS && a.static_w && warp == 0 && lane == 0) {
-    const GdTile t = gd_tile<EXPERTS>(a, (int)(blockIdx.x % a.tiles), nullptr);
+    const GdTile t = gd_tile<EXPERTS, PAIR>(a, worker % a.tiles, nullptr, rank);
     int k0;
-    const int nk = k_of(blockIdx.x / a.tiles, &k0);
+    const int nk = k_of(worker / a.tiles, &k0);
     for (; ahead < nk && ahead < S; ++ahead) {
-      mbar_expect_tx(full(ahead), STAGE_BYTES);
-      tma_load_2d(st_whi(ahead), &tw_hi, full(ahead), (k0 + ahead) * BK, t.f0);
+      expect(ahead);
+      load(st_whi(ahead), &tw_hi, full(ahead), (k0 + ahead) * BK, t.f0);
     }
   }
   // the activations, the residual and (otherwise) the weights were written by preceding kernels
@@ -344,9 +363,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       int issued = 0, s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      for (int item = worker; item < items && ok; item += workers) {
         const int tile = item % tiles;
-        const GdTile t = gd_tile<EXPERTS>(a, tile, first);
+        const GdTile t = gd_tile<EXPERTS, PAIR>(a, tile, first, rank);
         int k0;
         const int nk = k_of(item / tiles, &k0);
         for (int kc = k0; kc < k0 + nk; ++kc) {
@@ -356,27 +375,40 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
             break;
           }
           if (issued >= ahead) {
-            mbar_expect_tx(full(s), STAGE_BYTES);
-            tma_load_2d(st_whi(s), &tw_hi, full(s), kc * BK, t.f0);
+            expect(s);
+            load(st_whi(s), &tw_hi, full(s), kc * BK, t.f0);
           }
-          if (WLO) tma_load_2d(st_wlo(s), &tw_lo, full(s), kc * BK, t.f0);
-          tma_load_2d(st_xhi(s), &tx_hi, full(s), kc * BK, t.x0);
-          if (NSPLIT == 3) tma_load_2d(st_xlo(s), &tx_lo, full(s), kc * BK, t.x0);
+          if (WLO) load(st_wlo(s), &tw_lo, full(s), kc * BK, t.f0);
+          load(st_xhi(s), &tx_hi, full(s), kc * BK, t.x0);
+          if (NSPLIT == 3) load(st_xlo(s), &tx_lo, full(s), kc * BK, t.x0);
           ++issued;
           if (++s == S) { s = 0; ph ^= 1u; }
         }
       }
       if (*abort_flag) {
-        // let the copies this thread started land before the CTA's shared memory is released
+        // let the copies this thread started land before the CTA's shared memory is released (those of a pair's second CTA
+        // complete on the other's barrier: they are given a millisecond, a thousand times what a load takes)
+        if (PAIR)
+          for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+        else
         for (int i = issued > S ? issued - S : 0; i < issued; ++i) mbar_wait(full(i % S), (uint32_t)(i / S) & 1u, abort_flag + 1);
       }
     }
   } else if (warp == 1) {
+    if (rank == 0) {
     // ---------------- MMA issuer (uniform control flow, one elected lane issues) ----------------
+    auto mma = [&](uint32_t acc, uint64_t da, uint64_t db, uint32_t accumulate) {
+      if (PAIR) umma_bf16_pair(acc, da, db, a.idesc, accumulate);
+      else umma_bf16(acc, da, db, a.idesc, accumulate);
+    };
+    auto commit = [&](uint32_t bar) {
+      if (PAIR) umma_commit_pair(bar);
+      else umma_commit(bar);
+    };
     int s = 0, it = 0;
     uint32_t ph = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+    for (int item = worker; item < items && ok; item += workers, ++it) {
       const int b = it & 1, tile = item % tiles;
       int k0;
       const int nk = k_of(item / tiles, &k0);
@@ -401,19 +433,20 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
 #pragma unroll
           for (int k4 = 0; k4 < BK / 16; ++k4) {
             const uint64_t adv = (uint64_t)(k4 * 2);  // 16 bf16 = 32 bytes = 2 descriptor units
-            umma_bf16(acc, dwh + adv, dxh + adv, a.idesc, (kc > 0 || k4 > 0) ? 1u : 0u);
+            mma(acc, dwh + adv, dxh + adv, (kc > 0 || k4 > 0) ? 1u : 0u);
             if (NSPLIT == 3) {
-              if (WLO) umma_bf16(acc, dwl + adv, dxh + adv, a.idesc, 1u);
-              umma_bf16(acc, dwh + adv, dxl + adv, a.idesc, 1u);
+              if (WLO) mma(acc, dwl + adv, dxh + adv, 1u);
+              mma(acc, dwh + adv, dxl + adv, 1u);
             }
           }
-          umma_commit(empty(s));  // frees the stage when these MMAs have read it
+          commit(empty(s));  // frees the stage when these MMAs have read it
         }
         __syncwarp();
         if (++s == S) { s = 0; ph ^= 1u; }
       }
-      if (ok && elect_one()) umma_commit(acc_full(b));
+      if (ok && elect_one()) commit(acc_full(b));
       __syncwarp();
+    }
     }
   } else {
     // ---------------- epilogue ----------------
@@ -424,9 +457,9 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     float *stg = reinterpret_cast<float *>(smem + (size_t)S * STAGE_BYTES) + (warp - 2) * 512;  // 16 rows x 32 features
     int it = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++it) {
+    for (int item = worker; item < items && ok; item += workers, ++it) {
       const int b = it & 1, tile = item % tiles;
-      const GdTile t = gd_tile<EXPERTS>(a, tile, first);
+      const GdTile t = gd_tile<EXPERTS, PAIR>(a, tile, first, rank);
       // after the transpose a lane owns features o0 .. o0 + 3 (N % 4 == 0: all inside or all outside)
       const int64_t o0 = (int64_t)t.f0 + quad * 32 + 4 * (lane & 7);
       const bool o_ok = o0 < t.f_end;
@@ -469,14 +502,19 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty(b));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(acc_empty(b));
+        else mbar_arrive(acc_empty(b));
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();   // the other CTA signals into this one's shared memory, and reads it
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols) : "memory");
+    if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(a.tmem_cols) : "memory");
   }
 }
 
@@ -511,14 +549,18 @@ static int launch_wsplit(caten_b200_ctx *ctx, const WSrc &ws, int64_t N, int64_t
 // How a launch is cut: rows of x per tile and shares of k.
 struct GdPlan {
   int bn, splits, cps;
+  bool pair;
 };
 
 // The cut with the shortest expected time.  A CTA's stage takes as long as its MMAs (bn / 2 cycles each, at least 40) or as
 // long as its operands need from L2 (about 60 bytes a cycle and SM with every SM at work; measured: 128 x 256 tiles of
 // plain bf16 run at 0.85 of the burst rate of the tensor cores, 48 KB in 870 cycles).  Wide tiles read least, narrow ones
-// leave no SM without work and the last wave short; shares of k pay for a pass over their partial sums.
-static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums) {
-  GdPlan best = {256, 1, (int)(K / bk)};
+// leave no SM without work and the last wave short; shares of k pay for a pass over their partial sums.  A pair of CTAs on
+// 256 features loads 32 KB per CTA where a CTA alone loads 48, and has more stages in flight; it starts later (both CTAs
+// meet twice), and narrower tiles gain nothing from it (1665 rows, split bf16, 6400 x 1600, 224 rows wide: 91 us alone, 97).  us a call with the conversion of x, alone -> pair: 8192 rows, plain bf16,
+// 11264 x 2048 328 -> 297, 2048 x 5632 187 -> 170; split bf16, 6400 x 1600 361 -> 341; 777 rows, 4096 x 1024 13.6 -> 14.8.
+static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums, bool can_pair) {
+  GdPlan best = {256, 1, (int)(K / bk), false};
   double least = 1e30;
   const int nk = (int)(K / bk), products = nsplit == 1 ? 1 : wlo ? 3 : 2, parts = nsplit == 1 ? 1 : 2;
   for (int bn = 16; bn <= GD_BN; bn = bn < 32 ? 32 : bn + 32) {
@@ -538,7 +580,14 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
       double t = 1500 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
       if (s > 1) t += (consumer_sums ? 500.0 : 5000.0) + (double)M * N * 4 * s / (sm * 30.0);
       t *= 1.0 + 0.0003 * (GD_BN - bn);   // traffic costs power too, which is what limits long launches
-      if (t < least) { least = t; best = {bn, s, cps}; }
+      if (t < least) { least = t; best = {bn, s, cps, false}; }
+    }
+    if (can_pair && bn == GD_BN) {
+      const int64_t items = (M + bn - 1) / bn * ((N + 2 * GD_BM - 1) / (2 * GD_BM)), waves = (items + sm / 2 - 1) / (sm / 2);
+      const double need = ((double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)bn / 2 * parts)) / 60.0, body = nk * (mma > need ? mma : need);
+      const double t = 4000 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
+      // (a tile of a short K alone is mostly epilogue, which a wave more or less decides: 1665 rows, 3072 x 1024, plain bf16)
+      if (t < least && (body >= 16000 || waves >= 4)) { least = t; best = {bn, 1, nk, true}; }
     }
     if (bn >= M) break;
   }
@@ -619,12 +668,14 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   a.ldy = grp.ldy ? (int)grp.ldy : (int)(act_is_glu(act) ? N / 2 : N);
   if (res && !grp.plain_output()) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: a residual needs the plain output layout");
   const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && grp.plain_output() && grp.group_rows % GD_BM == 0;
-  const GdPlan p = gd_plan(ctx->sm_count, M, N, a.tiles_f, K, nsplit, wlo != nullptr, bk, M <= GD_SPLIT_ROWS, can_defer);
+  const bool can_pair = ctx->dense_pair && M > GD_SPLIT_ROWS && !grp.group_rows && ctx->sm_count % 2 == 0;
+  const GdPlan p = gd_plan(ctx->sm_count, M, N, a.tiles_f, K, nsplit, wlo != nullptr, bk, M <= GD_SPLIT_ROWS, can_defer, can_pair);
+  if (p.pair) a.tiles_f = a.tiles_per_group = (int)((N + 2 * GD_BM - 1) / (2 * GD_BM));
   a.bn = p.bn; a.splits = p.splits; a.cps = p.cps; a.part = nullptr;
   a.static_w = as_is && !ctx->weights_pending;
-  if ((rc = make_map(ctx, &txh, xhi, xrows, K, p.bn, bk))) return rc;
+  if ((rc = make_map(ctx, &txh, xhi, xrows, K, p.pair ? p.bn / 2 : p.bn, bk))) return rc;
   txl = txh;
-  if (nsplit == 3 && (rc = make_map(ctx, &txl, xlo, xrows, K, p.bn, bk))) return rc;
+  if (nsplit == 3 && (rc = make_map(ctx, &txl, xlo, xrows, K, p.pair ? p.bn / 2 : p.bn, bk))) return rc;
   const int64_t tiles = (int64_t)a.tiles_f * ((M + p.bn - 1) / p.bn), items = tiles * p.splits;
   if (items > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: too many tiles");
   a.tiles = (int)tiles;
@@ -632,8 +683,8 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
     if ((rc = scratch_reserve(ctx, &ctx->wtmp, (size_t)items * p.bn * GD_BM * sizeof(float)))) return rc;
     a.part = (float *)ctx->wtmp.ptr;
   }
-  const size_t stage = (size_t)(GD_BM * (wlo ? 2 : 1) + p.bn * parts) * (size_t)bk * 2;
-  const int grid = items < ctx->sm_count ? (int)items : ctx->sm_count;
+  const size_t stage = (size_t)(GD_BM * (wlo ? 2 : 1) + (p.pair ? p.bn / 2 : p.bn) * parts) * (size_t)bk * 2;
+  const int workers = p.pair ? ctx->sm_count / 2 : ctx->sm_count, busy = items < workers ? (int)items : workers, grid = p.pair ? 2 * busy : busy;
   // A CTA with one item leaves room on its SM for one of the next linear, which starts to load its weights meanwhile; a
   // CTA that walks over items takes what there is: 1 KB slack + 1 KB barriers + stages + 32 KB of staging fit 227 KB.
   const size_t staging = 2048 * 4 * (size_t)(p.bn < 64 ? p.bn / 16 : 4);   // of the epilogue warps that have columns to store
@@ -642,9 +693,9 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   if (stages > p.cps) stages = p.cps;
   if (stages < 2) stages = 2;
   a.stages = stages;
-  a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(GD_BM >> 4) << 24);
-  a.tmem_cols = 32;
-  while (a.tmem_cols < (uint32_t)(p.bn * (items > grid ? 2 : 1))) a.tmem_cols *= 2;
+  a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)((p.pair ? 2 * GD_BM : GD_BM) >> 4) << 24);
+  a.tmem_cols = p.pair ? 512 : 32;   // (a pair: all, so that its accumulators have the same columns in both CTAs)
+  while (a.tmem_cols < (uint32_t)(p.bn * (items > busy ? 2 : 1))) a.tmem_cols *= 2;
   const size_t smem = 2048 + stage * stages + staging;
 
   cudaLaunchConfig_t cfg = {};
@@ -652,12 +703,23 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   cfg.blockDim = dim3(GD_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int na = 0;
+  if (take_pdl(ctx)) {
+    at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  if (p.pair) {
+    at[na].id = cudaLaunchAttributeClusterDimension;
+    at[na].val.clusterDim.x = 2;
+    at[na].val.clusterDim.y = at[na].val.clusterDim.z = 1;
+    ++na;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = take_pdl(ctx) ? 1 : 0;
-  auto kernel = nsplit == 1 ? gemm_dense_kernel<1, false, false> : wlo ? gemm_dense_kernel<3, false, true> : gemm_dense_kernel<3, false, false>;
+  cfg.numAttrs = na;
+  auto kernel = p.pair ? (nsplit == 1 ? gemm_dense_kernel<1, false, false, true> : wlo ? gemm_dense_kernel<3, false, true, true> : gemm_dense_kernel<3, false, false, true>)
+                       : (nsplit == 1 ? gemm_dense_kernel<1, false, false, false> : wlo ? gemm_dense_kernel<3, false, true, false> : gemm_dense_kernel<3, false, false, false>);
   CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, twh, twl, txh, txl, a));
   CB_LAUNCH_CHECK(ctx, "gemm_dense_kernel");
@@ -705,11 +767,11 @@ int launch_gemm_experts(caten_b200_ctx *ctx, const caten_b200_weight *w, const E
   const int64_t most = (er.pairs / bn + (er.pairs < er.experts ? er.pairs : er.experts)) * a.tiles_f;
   const int grid = most < ctx->sm_count ? (int)most : ctx->sm_count;
   if (nsplit == 3) {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<3, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_k(ctx, gemm_dense_kernel<3, true, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
+    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<3, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(ctx, gemm_dense_kernel<3, true, false, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
   } else {
-    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_k(ctx, gemm_dense_kernel<1, true, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
+    CB_CUDA(ctx, cudaFuncSetAttribute(gemm_dense_kernel<1, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(ctx, gemm_dense_kernel<1, true, false, false>, dim3((unsigned)grid), dim3(GD_THREADS), smem, tw, tw, txh, txl, a);
   }
   CB_LAUNCH_CHECK(ctx, "gemm_dense_kernel");
   return 0;

@@ -886,10 +886,12 @@ static int run_tc(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x,
   const uintptr_t align_bits = (uintptr_t)bias | (uintptr_t)res | (uintptr_t)y | (uintptr_t)ybf.hi | (uintptr_t)ybf.lo;
   if (gemm_dense_applies(ctx, wt, M, N, K) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp, defer);
   TcPlan p;
-  // reduce inside a cluster: always (mode 1) or only when this launch needs its own epilogue (mode 2)
+  // reduce inside a cluster: always (mode 1), when this launch needs its own epilogue (mode 2), or, with few rows, when
+  // no consumer could have done it
   const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && N % 4 == 0 && grp.plain_output() && grp.group_rows % TC_BM == 0;
   const bool own_epilogue = !can_defer;
-  const bool want_cluster = ctx->splitk_cluster == 1 || (ctx->splitk_cluster == 2 && own_epilogue);
+  const bool want_cluster = ctx->splitk_cluster == 1 || (ctx->splitk_cluster == 2 && own_epilogue) ||
+                            (ctx->splitk_cluster < 0 && M <= 128 && (act != CATEN_B200_ACT_NONE || ybf.hi));
   if (int rc = tc_plan(ctx, "gemm_tc", M, N, K, nsplit, want_cluster ? 8 : 32, &p, grp.group_rows)) return rc;  // 8 = portable cluster size
   uint8_t *xhi, *xlo;
   if (xhi_pre) {

@@ -326,6 +326,27 @@ def test_gemm_many_rows_matches_the_tile_per_cta_kernel(oracle, monkeypatch):
     np.testing.assert_allclose(outs[0][1][:64], ref, atol=1e-5, rtol=1e-5)   # test-gemm.lisp:3-22
 
 
+@pytest.mark.parametrize("wtype", ["q8_0", "f16"])
+@pytest.mark.parametrize("prec,tol", [(L.PREC_BF16X3, 1e-4), (L.PREC_BF16, 4e-2)])
+@pytest.mark.parametrize("M,N,K", [(2400, 2052, 2048), (2561, 4100, 1088)])
+def test_gemm_pairs_of_ctas(rt, monkeypatch, wtype, prec, tol, M, N, K):
+    """Tiles of 256 features by two CTAs, the second one partly or wholly past the last feature, rows that end within a half;
+    and the same linear with one CTA per tile.  Sums of K products of unit variance over sqrt(K): rounding errors of a few
+    2^-16, or of 2^-9 with both operands in bf16."""
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    up, _, _ = make_weight(rng, N, K, wtype, std=K ** -0.5)
+    x, bias, res = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M, N), dtype=np.float32)
+    from caten_b200.runtime import B200Runtime
+    monkeypatch.setenv("CATEN_B200_DENSE_PAIR", "0")
+    with B200Runtime(0) as alone:
+        for r in (rt, alone):
+            w = r.upload_weight(up)
+            want = res + (x.astype(np.float64) @ w.dequantize().astype(np.float64).T + bias)
+            got = r.linear(w, r.transfer_from_array(x), r.transfer_from_array(bias), r.transfer_from_array(res), precision=prec).numpy()
+            assert np.abs(got - want).max() < tol
+            w.close()
+
+
 def test_gemm_tensor_core_split_k_is_deterministic(rt):
     """Few output tiles and a long inner dimension: several CTAs share a tile (split-K) and the
     last one to finish adds the partial tiles in a fixed order, so repeated runs give equal bits."""
