@@ -54,17 +54,20 @@ __device__ __forceinline__ void st_cache(void *cache, bool bf16, int64_t at, flo
 // ---------------------------------------------------------------------------------------------
 constexpr int LP_THREADS = 256;
 
+template <bool FEW>
 __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(const LatentArgs a, const float *__restrict__ y, const PartIn pin, int64_t ld,
                                                                  float *__restrict__ cq, BfOut cq_bf) {
-  extern __shared__ __align__(16) float row[];   // [Qr + Kp + Pp], then the norms' gains [Qr + Kp]
+  extern __shared__ __align__(16) float row[];   // [Qr + Kp + Pp], then (FEW) the norms' gains [Qr + Kp]
   __shared__ float red[2][LP_THREADS / 32];
   const int64_t r = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cols = a.Qr + a.Kp + a.Pp;
+  // gains are written at load: with few rows, whose time is latency, they arrive before the wait instead of behind the sums
   float *gain = row + cols;
-  // gains are written at load: they arrive before the wait instead of behind the sums
-  for (int c = tid; c < a.Qr; c += LP_THREADS) gain[c] = a.q_norm[c];
-  for (int c = tid; c < a.Kp; c += LP_THREADS) gain[a.Qr + c] = a.kv_norm[c];
+  if (FEW) {
+    for (int c = tid; c < a.Qr; c += LP_THREADS) gain[c] = a.q_norm[c];
+    for (int c = tid; c < a.Kp; c += LP_THREADS) gain[a.Qr + c] = a.kv_norm[c];
+  }
   pdl_enter();
   const int pos = (a.d_n ? *a.d_n : a.n) + (int)(r % a.s);
   float sq = 0.0f, sc = 0.0f;   // (padding is zero)
@@ -78,7 +81,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(const LatentArg
   // the angle of this thread's first rotated column, while the sums are formed
   const int half = a.P / 2;
   float sn = 0.0f, cs = 1.0f;
-  if (tid < a.P) sincosf((float)pos * a.freq[tid < half ? tid : tid - half], &sn, &cs);
+  if (FEW && tid < a.P) sincosf((float)pos * a.freq[tid < half ? tid : tid - half], &sn, &cs);
   sq = warp_sum(sq);
   sc = warp_sum(sc);
   if (lane == 0) { red[0][warp] = sq; red[1][warp] = sc; }
@@ -87,15 +90,15 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prep_kernel(const LatentArg
 #pragma unroll
   for (int w = 0; w < LP_THREADS / 32; ++w) { sq += red[0][w]; sc += red[1][w]; }
   const float rq = 1.0f / sqrtf(sq / (float)a.Q + a.eps), rc = 1.0f / sqrtf(sc / (float)a.K + a.eps);
-  for (int c = tid; c < a.Qr; c += LP_THREADS) st1(cq, cq_bf, r * a.Qr + c, row[c] * rq * gain[c]);
+  for (int c = tid; c < a.Qr; c += LP_THREADS) st1(cq, cq_bf, r * a.Qr + c, row[c] * rq * (FEW ? gain[c] : a.q_norm[c]));
   const int64_t seq = r / a.s;
   const float *lat = row + a.Qr, *key = lat + a.Kp;
-  for (int c = tid; c < a.Kp; c += LP_THREADS) st_cache(a.cache, a.cache_bf16, a.at(seq, pos, c), lat[c] * rc * gain[a.Qr + c]);
+  for (int c = tid; c < a.Kp; c += LP_THREADS) st_cache(a.cache, a.cache_bf16, a.at(seq, pos, c), lat[c] * rc * (FEW ? gain[a.Qr + c] : a.kv_norm[c]));
   for (int i = tid; i < a.Pp; i += LP_THREADS) {
     float v = 0.0f;
     if (i < a.P) {
       const int f = i < half ? i : i - half;
-      if (i != tid) sincosf((float)pos * a.freq[f], &sn, &cs);
+      if (!FEW || i != tid) sincosf((float)pos * a.freq[f], &sn, &cs);
       v = i < half ? key[i] * cs - key[i + half] * sn : key[i] * cs + key[f] * sn;
     }
     st_cache(a.cache, a.cache_bf16, a.at(seq, pos, a.Kp + i), v);
@@ -114,9 +117,11 @@ static int check_latent(caten_b200_ctx *ctx, const LatentArgs &a) {
 
 int launch_latent_prep(caten_b200_ctx *ctx, const LatentArgs &a, const float *y, PartIn pin, int64_t ld, float *cq, BfOut cq_bf) {
   if (int rc = check_latent(ctx, a)) return rc;
-  const size_t smem = (size_t)(2 * a.Qr + a.Kp + a.KC()) * sizeof(float);
-  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(latent_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_k(ctx, latent_prep_kernel, dim3((unsigned)(a.B * a.s)), dim3(LP_THREADS), smem, a, y, pin, ld, cq, cq_bf);
+  const bool few = (int64_t)a.B * a.s <= 4 * ctx->sm_count;
+  auto kernel = few ? latent_prep_kernel<true> : latent_prep_kernel<false>;
+  const size_t smem = (size_t)(a.Qr + a.KC() + (few ? a.Qr + a.Kp : 0)) * sizeof(float);
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_k(ctx, kernel, dim3((unsigned)(a.B * a.s)), dim3(LP_THREADS), smem, a, y, pin, ld, cq, cq_bf);
   CB_LAUNCH_CHECK(ctx, "latent_prep_kernel");
   return 0;
 }

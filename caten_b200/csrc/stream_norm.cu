@@ -57,13 +57,13 @@ __device__ __forceinline__ float4 mix4(float4 h, float4 p, float4 mu) {
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 
-template <int IN, int OUT, int MAXV>
+template <int IN, int OUT, int MAXV, bool FEW>
 __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArgs a) {
   __shared__ float red[SN_THREADS / 32];
   const int d4 = a.d4;
-  // The kernel is a chain of latencies when the rows are few, so what does not depend on the kernels before it (gains and the
+  // The kernel is a chain of latencies when the rows are few (FEW), so what does not depend on the kernels before it (gains and the
   // pass's step, written at load) is asked for before the wait, and the places of the experts' rows beside the row itself.
-  constexpr bool EARLY = OUT == SN_NORM2 && MAXV <= 2;
+  constexpr bool EARLY = FEW && OUT == SN_NORM2 && MAXV <= 2;   // (with many rows the registers are worth more: 18 us against 20)
   float4 g1[EARLY ? MAXV : 1], g2[EARLY ? MAXV : 1], st[EARLY ? MAXV : 1];
   if (EARLY) {
 #pragma unroll
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArg
   pdl_enter();
   const int64_t row = blockIdx.x;
   const int64_t src = a.rows ? a.rows[row] : (a.src_stride > 1 ? (row + 1) * a.src_stride - 1 : row);
-  constexpr int SUM_U = 4;   // experts' rows in flight
+  constexpr int SUM_U = FEW ? 4 : 1;   // experts' rows in flight
   int64_t place[SUM_U];
   auto places = [&](int k0) {
 #pragma unroll
@@ -238,10 +238,15 @@ __global__ void __launch_bounds__(SN_THREADS) stream_norm_kernel(const StreamArg
 template <int IN, int OUT>
 static int launch_sn(caten_b200_ctx *ctx, const StreamArgs &a, int64_t rows) {
   const dim3 g((unsigned)rows), b(SN_THREADS);
-  if (a.d4 <= SN_THREADS) launch_k(ctx, stream_norm_kernel<IN, OUT, 1>, g, b, 0, a);
-  else if (a.d4 <= 2 * SN_THREADS) launch_k(ctx, stream_norm_kernel<IN, OUT, 2>, g, b, 0, a);
-  else if (a.d4 <= 4 * SN_THREADS) launch_k(ctx, stream_norm_kernel<IN, OUT, 4>, g, b, 0, a);
-  else launch_k(ctx, stream_norm_kernel<IN, OUT, 8>, g, b, 0, a);
+  const bool few = OUT == SN_NORM2 && rows <= 4 * ctx->sm_count;
+#define SN_LAUNCH(MAXV)                                                                              \
+  if (few) launch_k(ctx, stream_norm_kernel<IN, OUT, MAXV, OUT == SN_NORM2>, g, b, 0, a);            \
+  else launch_k(ctx, stream_norm_kernel<IN, OUT, MAXV, false>, g, b, 0, a)
+  if (a.d4 <= SN_THREADS) { SN_LAUNCH(1); }
+  else if (a.d4 <= 2 * SN_THREADS) { SN_LAUNCH(2); }
+  else if (a.d4 <= 4 * SN_THREADS) launch_k(ctx, stream_norm_kernel<IN, OUT, 4, false>, g, b, 0, a);
+  else launch_k(ctx, stream_norm_kernel<IN, OUT, 8, false>, g, b, 0, a);
+#undef SN_LAUNCH
   CB_LAUNCH_CHECK(ctx, "stream_norm_kernel");
   return 0;
 }
