@@ -546,7 +546,7 @@ struct caten_b200_gpt2 {
   cb::StepLoop loop;
   int *h_pos_pinned = nullptr;
   // 1..4 sequences over Q4_0 / Q8_0 layers: profiling times a single-token step as a whole (class DECODE_STEP), and the
-  // device entry replays the captured step too.  CATEN_B200_PERSISTENT=0: per kernel, and launch by launch
+  // device entry advances the device-side position.  CATEN_B200_PERSISTENT=0: timed per kernel
   bool whole_step = false;
   bool defer_reduce = true;  // CATEN_B200_DEFER_REDUCE=0 keeps a reduction kernel behind every split-K linear
 };
@@ -719,6 +719,7 @@ static int head(caten_b200_gpt2 *m, int64_t s) {
 }
 
 static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps);
+static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host);
 
 int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, const int64_t *d_ids_i64, int64_t s, int64_t n,
                                 int64_t *d_out_ids) {
@@ -733,7 +734,7 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
   const int64_t B = c.batch;
   if (s == 1 && m->whole_step) {
     if (int rc = launch_begin_steps(ctx, d_ids_f32, d_ids_i64, m->loop.ids_io, m->loop.d_pos, n, B)) return rc;
-    if (int rc = decode_run(m, n, 1)) return rc;
+    if (int rc = decode_step_device_pos(m, n)) return rc;   // (launch by launch: a caller may be capturing the stream)
     if (d_out_ids != m->loop.out_ids)
       CB_CUDA(ctx, cudaMemcpyAsync(d_out_ids, m->loop.out_ids, (size_t)B * sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
     return 0;
