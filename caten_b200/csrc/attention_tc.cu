@@ -100,8 +100,9 @@ __host__ __device__ inline int at_first_tile(const AttnArgs &p) {
 
 }  // namespace
 
-// One CTA = one tile of one key/value head: 64 rows of K and V -> hi and lo operand tiles; rows past the context and
-// columns past the head are zero.  PLAIN (GPT-2): rows of this step come from the projections and go to the cache as well.
+// One CTA = one tile of one key/value head: 64 rows of K and V -> hi and lo operand tiles; columns past the head are zero, and
+// so are rows past the context up to a multiple of 16.  Rows above that are not written: their scores are masked, and the
+// second product does not take them (prompts of a dozen tokens would write four times what they hold).  PLAIN (GPT-2): rows of this step come from the projections and go to the cache as well.
 template <int NQ, int NE, bool PLAIN>
 __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b0, uint8_t *__restrict__ tiles) {
   using Lay = AtLayout<NQ, NE>;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b
   const float *kx = !PLAIN && p.kx ? p.kx + b * p.cap * p.kx_ld - p.kx_from : nullptr;   // column c of the key, c >= kx_from
   constexpr int KP = AT_K * NQ * 8, PIECES = KP + AT_K * NE * 8;   // pieces of eight floats
   constexpr int IT = PIECES / 256;
+  const int rows = min(AT_K, (t - j0 + 15) / 16 * 16);
   float4 v[IT][2];   // all of this thread's loads are in flight together: the stores below may alias them
 #pragma unroll
   for (int it = 0; it < IT; ++it) {
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b
     const bool key = i < KP;
     const int nb = key ? NQ : NE, at = key ? i : i - KP;
     const int row = at / (8 * nb), c8 = at % (8 * nb), j = j0 + row;
+    if (row >= rows) continue;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int c = 8 * c8 + 4 * u;
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b
     const bool key = i < KP;
     const int nb = key ? NQ : NE, at = key ? i : i - KP;
     const int row = at / (8 * nb), c8 = at % (8 * nb), j = j0 + row;
+    if (row >= rows) continue;
     if (PLAIN && j >= p.n && j < t) {
       float4 *keep = reinterpret_cast<float4 *>((key ? p.kc : p.vc) + (head * p.cap + j) * 64 + 8 * c8);
       keep[0] = v[it][0];
@@ -297,11 +301,13 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       ok = mbar_wait(v_full(st), (uint32_t)(i >> 1) & 1u, abort_flag) && mbar_wait(p_full, (uint32_t)i & 1u, abort_flag);
       if (!ok) break;
       tc_fence_after();
+      const int groups = (kend - kbeg - i * AT_K + 15) / 16;   // of 16 keys that some query of the tile sees
       if (elect_one()) {
         const uint32_t acc = tmem_base + Lay::COL_O;
         const uint64_t dv_hi = dv0 + (uint64_t)(st * (Lay::V_BYTES >> 4)), dv_lo = dv_hi + 512;
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
+          if (k4 >= groups) break;
           const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
           const uint32_t p_hi = tmem_base + Lay::COL_P + 8 * k4, p_lo = p_hi + 32;
           umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u);

@@ -257,7 +257,7 @@ struct WSrc {
 };
 constexpr int WT_F32_T = 100;  // pseudo weight type: fp32 operand given as [K, N] row-major (relu_matmul's b)
 // many-row GEMM with both operands from shared memory (gemm_dense.cu)
-bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K);
+bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K, int nsplit);
 int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x, const __nv_bfloat16 *xhi, const __nv_bfloat16 *xlo,
                       const float *bias, const float *res, int act, float *y, BfOut ybf, int64_t M, int64_t N, int64_t K, int nsplit,
                       LinGroups grp = LinGroups(), PartIn *defer = nullptr);

@@ -594,14 +594,16 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
   return best;
 }
 
-// Which linears run here.  bf16 weights are the operand as they are: every one whose shape fits (us a call, other kernel ->
+// Which linears run here.  In plain bf16, bf16 weights are the operand as they are: every one whose shape fits (us a call, other kernel ->
 // this, plain bf16, 11264 x 2048: 16 rows 29 -> 13, 256 rows 42 -> 27, 777 rows 108 -> 39; 1024 x 4096: 1665 rows 45 -> 28).
+// In split bf16 they follow the rule below: with few rows the other kernel, whose one MMA takes both parts of x and whose shares
+// of k are shorter, is faster (27 rows of GPT-2 XL: a prompt 3.38 ms there, 3.77 here) and rounds less.
 // Other formats are expanded once per call, which pays when the converting producers of the other kernel (one per output
 // tile) repeat it often: with full waves of the widest tiles from 1024 rows on, otherwise from 1536 (split bf16, Q4_0,
 // 1600 x 6400: 777 rows 65 here 87, 1024 rows 69 here 90, 1665 rows 113 here 106; 1600 x 1600: 1665 rows 38 here 32).
-bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K) {
+bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K, int nsplit) {
   if (!ctx->dense_gemm || N % 4 || K % GD_BK || K < GD_BK) return false;
-  if (wt == CATEN_B200_BF16 || M >= GD_EXPAND_ROWS) return true;
+  if ((wt == CATEN_B200_BF16 && nsplit == 1) || M >= GD_EXPAND_ROWS) return true;
   return M >= 1024 && (M + GD_BN - 1) / GD_BN * ((N + GD_BM - 1) / GD_BM) >= ctx->sm_count;
 }
 

@@ -884,7 +884,7 @@ static int run_tc(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x,
   // thousands of rows (prefill): expand the weights once, both operands through TMA
   // (its epilogue moves 16 bytes at a time: bias, residual and outputs must be aligned for that)
   const uintptr_t align_bits = (uintptr_t)bias | (uintptr_t)res | (uintptr_t)y | (uintptr_t)ybf.hi | (uintptr_t)ybf.lo;
-  if (gemm_dense_applies(ctx, wt, M, N, K) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp, defer);
+  if (gemm_dense_applies(ctx, wt, M, N, K, nsplit) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp, defer);
   TcPlan p;
   // reduce inside a cluster: always (mode 1), when this launch needs its own epilogue (mode 2), or, with few rows, when
   // no consumer could have done it
