@@ -199,6 +199,7 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(Lay::COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  __syncthreads();   // the barriers are initialised
   pdl_wait();
 
   const int Dp = PLAIN ? 64 : p.Dp, Ep = PLAIN ? 64 : p.Ep;
@@ -211,6 +212,23 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
     if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, DEV_WAIT_TIMEOUT); status[1] = code; }
   };
 
+  // the copies of step i; those of the first two steps, whose stages are free, start while Q is converted
+  const uint8_t *src0 = tiles + (((int64_t)blockIdx.y * p.G + (PLAIN ? h : h / (p.H / p.G))) * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;   // of the key/value head this query head reads
+  auto copy_k = [&](int i) {
+    const int st = i & 1;
+    mbar_expect_tx(k_full(st), Lay::K_BYTES);
+    bulk_load(smem_u32(sm + Lay::OFF_K) + st * Lay::K_BYTES, src0 + (int64_t)i * Lay::TILE, Lay::K_BYTES, k_full(st));
+  };
+  auto copy_v = [&](int i) {
+    const int st = i & 1;
+    mbar_expect_tx(v_full(st), Lay::V_BYTES);
+    bulk_load(smem_u32(sm + Lay::OFF_V) + st * Lay::V_BYTES, src0 + (int64_t)i * Lay::TILE + Lay::K_BYTES, Lay::V_BYTES, v_full(st));
+  };
+  if (warp == 8 && lane == 0)
+    for (int i = 0; i < min(nblk, 2); ++i) {
+      copy_k(i);
+      copy_v(i);
+    }
   // Q tiles: rows [0,128) hi, [128,256) lo per block; GPT-2's 1/8 score scale is folded in (a power of two: exact)
   if (warp < AT_SOFTMAX_WARPS) {
     const bool okq = q0 + r < s;
@@ -240,19 +258,14 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   if (warp == 8) {
     // ---------------- tiles ----------------
     if (lane == 0) {
-      const int64_t kv = (int64_t)blockIdx.y * p.G + (PLAIN ? h : h / (p.H / p.G));  // the key/value head this query head reads
-      const uint8_t *src = tiles + (kv * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;
-      int ki = 0, vi = 0;   // copies asked for
-      for (int i = 0; i < nblk; ++i, src += Lay::TILE) {
-        const int st = i & 1;
-        const uint32_t ph = ((uint32_t)(i >> 1) & 1u) ^ 1u;   // (the first use of a stage passes at once)
-        if (!mbar_wait(k_empty(st), ph, abort_flag)) break;
-        mbar_expect_tx(k_full(st), Lay::K_BYTES);
-        bulk_load(smem_u32(sm + Lay::OFF_K) + st * Lay::K_BYTES, src, Lay::K_BYTES, k_full(st));
+      int ki = min(nblk, 2), vi = ki;   // copies asked for
+      for (int i = 2; i < nblk; ++i) {
+        const uint32_t ph = ((uint32_t)(i >> 1) & 1u) ^ 1u;
+        if (!mbar_wait(k_empty(i & 1), ph, abort_flag)) break;
+        copy_k(i);
         ++ki;
-        if (!mbar_wait(v_empty(st), ph, abort_flag)) break;
-        mbar_expect_tx(v_full(st), Lay::V_BYTES);
-        bulk_load(smem_u32(sm + Lay::OFF_V) + st * Lay::V_BYTES, src + Lay::K_BYTES, Lay::V_BYTES, v_full(st));
+        if (!mbar_wait(v_empty(i & 1), ph, abort_flag)) break;
+        copy_v(i);
         ++vi;
       }
       if (vi < nblk) give_up(16);
