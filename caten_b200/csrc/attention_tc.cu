@@ -22,8 +22,8 @@
 //                memory as the A operand of the second product
 // so that the scores of step i + 1 and the output of step i - 1 are computed while the softmax of step i runs.  The softmax is
 // what a step waits for (about 2.5 k cycles against 1.8 k of MMAs); with the phases one after the other, conversion included,
-// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 166 us and 13 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
-// 40 us for the append -> 136 us and 67 us for append and tiles.
+// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 159 us and 14 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
+// 40 us for the append -> 140 us and 67 us for append and tiles.
 // The softmax is single-pass with a lazily moved reference maximum: each step exchanges the
 // maximum of its visible scores between the row's two threads; the reference only moves (and O and
 // the row sum are rescaled, O by a TMEM load / multiply / store) when a step exceeds it by more
