@@ -42,6 +42,15 @@ int scratch_reserve(caten_b200_ctx *ctx, Scratch *s, size_t bytes) {
   return 0;
 }
 
+// Whether work queued on `s` goes into a graph that the caller is capturing.
+bool stream_is_capturing(cudaStream_t s) {
+  if (s == cudaStreamLegacy) return false;   // (it cannot be, and the query fails there while another stream is)
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();
+  return true;
+}
+
 static int check_status(caten_b200_ctx *ctx) {
   if (ctx->h_status[0] != DEV_OK) {
     const int code = ctx->h_status[0], where = ctx->h_status[1], detail = ctx->h_status[2];

@@ -169,6 +169,7 @@ namespace cb {
 int fail(caten_b200_ctx *ctx, int code, const char *fmt, ...);
 int cuda_fail(caten_b200_ctx *ctx, cudaError_t e, const char *what);
 int scratch_reserve(caten_b200_ctx *ctx, Scratch *s, size_t bytes);
+bool stream_is_capturing(cudaStream_t s);
 
 #define CB_CUDA(ctx, call)                                          \
   do {                                                              \

@@ -30,12 +30,42 @@ inline void step_loop_free(StepLoop *l) {
   *l = StepLoop();
 }
 
+// Captures one step's launches.  They are captured on the context's own stream, wherever the steps run: a caller's stream may
+// be the legacy default stream, which cannot be captured, or one that synchronises with it.  Without a graph (l->graph stays
+// NULL) the steps are launched one by one.
+template <class Step>
+void step_loop_capture(caten_b200_ctx *ctx, StepLoop *l, Step step, int64_t pos) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // of this thread: a capture of the caller's elsewhere forbids nothing here
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { (void)cudaGetLastError(); return; }
+  const cudaStream_t caller = ctx->stream;
+  const int64_t before = ctx->launches;
+  cudaGraph_t g = nullptr;
+  ctx->stream = ctx->own_stream;
+  if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    const int rc = step(pos);
+    if (cudaStreamEndCapture(ctx->stream, &g) != cudaSuccess || rc) l->graph = nullptr;
+    else if (cudaGraphInstantiate(&l->graph, g, 0) != cudaSuccess) l->graph = nullptr;
+  }
+  if (g) cudaGraphDestroy(g);
+  if (!l->graph) (void)cudaGetLastError();
+  ctx->stream = caller;
+  l->launches_per_step = ctx->launches - before;
+  ctx->launches = before;  // captured, not launched
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  l->graph_xbf = ctx->xbf.ptr;
+  l->graph_wtmp = ctx->wtmp.ptr;
+  l->graph_wbf = ctx->wbf.ptr;
+  l->graph_side = ctx->wtmp_side.ptr;
+}
+
 // Runs `steps` single-token steps from the device-side state (ids_io and d_pos already loaded).  `step(n)` queues one
 // step's kernels, which read ids and position from device memory; the host-side n only feeds argument checks.  With
-// use_graph its launch sequence is captured the first time and replayed.
+// use_graph its launch sequence is captured the first time and replayed; into a stream that the caller is capturing the
+// steps are launched one by one.
 template <class Step>
 int step_loop_run(caten_b200_ctx *ctx, StepLoop *l, int64_t n, int64_t steps, int64_t T, bool use_graph, Step step) {
   int64_t done = 0;
+  use_graph = use_graph && !stream_is_capturing(ctx->stream) && !stream_is_capturing(ctx->own_stream);
   if (use_graph && l->graph && (l->graph_xbf != ctx->xbf.ptr || l->graph_wtmp != ctx->wtmp.ptr || l->graph_wbf != ctx->wbf.ptr || l->graph_side != ctx->wtmp_side.ptr)) {
     cudaGraphExecDestroy(l->graph);  // scratch was re-allocated since the capture: its pointers are stale
     l->graph = nullptr;
@@ -45,22 +75,7 @@ int step_loop_run(caten_b200_ctx *ctx, StepLoop *l, int64_t n, int64_t steps, in
     // must not happen during capture
     if (int rc = step(n)) return rc;
     done = 1;
-    cudaGraph_t g = nullptr;
-    CB_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int64_t before = ctx->launches;
-    const int rc = step(n + 1 < T ? n + 1 : T - 1);
-    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-    l->launches_per_step = ctx->launches - before;
-    ctx->launches = before;  // captured, not launched
-    if (rc) { if (g) cudaGraphDestroy(g); return rc; }
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamEndCapture");
-    const cudaError_t e2 = cudaGraphInstantiate(&l->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e2 != cudaSuccess) { l->graph = nullptr; return cuda_fail(ctx, e2, "cudaGraphInstantiate"); }
-    l->graph_xbf = ctx->xbf.ptr;
-    l->graph_wtmp = ctx->wtmp.ptr;
-    l->graph_wbf = ctx->wbf.ptr;
-    l->graph_side = ctx->wtmp_side.ptr;
+    step_loop_capture(ctx, l, step, n + 1 < T ? n + 1 : T - 1);
   }
   for (; done < steps; ++done) {
     if (use_graph && l->graph) {

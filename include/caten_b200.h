@@ -274,8 +274,8 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
  * starting from d_first_ids [B] at position n.  The launch sequence of one step is captured in a
  * CUDA graph on first use and replayed, so the host issues one call per token instead of several
  * hundred launches.  d_out_ids: NULL or [steps, B] int64 (row i = ids produced by step i).
- * Asynchronous.  While per-kernel timing is on (caten_b200_profile_begin) the steps are launched
- * one kernel at a time instead. */
+ * Asynchronous.  While per-kernel timing is on (caten_b200_profile_begin), and into a stream that the
+ * caller is capturing, the steps are launched one kernel at a time instead. */
 int caten_b200_gpt2_decode(caten_b200_gpt2 *m, const int64_t *d_first_ids, int64_t n, int64_t steps,
                            int64_t *d_out_ids);
 /* Device pointer to the [B, V] fp32 logits of the last step (valid until the next step). */

@@ -301,3 +301,59 @@ def test_single_kernel_decode_step_matches_kernel_per_operation_path(rt, oracle,
     got = new.decode_device(first, 70, 5)
     np.testing.assert_array_equal(got, np.stack(want[1:], axis=1))
     old.close(); new.close(); ref.close()
+
+
+@pytest.mark.parametrize("wtype,precision,batch", [("q4_0", "bf16x3", 1), ("f32", "fp32", 4), ("q8_0", "bf16x3", 6)])
+@pytest.mark.parametrize("warm", [False, True])
+def test_device_resident_decode_into_a_captured_stream(rt, wtype, precision, batch, warm):
+    """The loop queues plain launches into a graph that the caller captures, also when it has a graph of its own already."""
+    import torch
+    from caten_b200 import _lib as L
+    sd = S.synth_state_dict(TINY, wtype, seed=5, max_seq_len=40, trivial_affine=False, weight_std=0.08)
+    prompt = S.synth_prompts(batch, 9, TINY.vocab_size, seed=2)
+    m = GPT2(rt, TINY, sd, max_seq_len=40, batch=batch, precision=precision)
+    first = m.forward(prompt, 9, 0)
+    if batch > 4 or warm:   # scratch memory is sized before a capture, by any step of the same rows
+        m.decode_device(first, 9, 2)
+    if not warm:
+        m.close()
+        m = GPT2(rt, TINY, sd, max_seq_len=40, batch=batch, precision=precision)
+        m.forward(prompt, 9, 0)
+    ids, out = rt.transfer_from_array(first.astype(np.int64)), rt.open_buffer((6, batch), np.int64)
+    rt.sync()
+    host = torch.cuda.Stream()
+    L.check(rt.ctx, rt.lib.caten_b200_set_stream(rt.ctx, host.cuda_stream))
+    try:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=host, capture_error_mode="thread_local"):
+            m.decode_device_buffers(ids, 9, 6, out)
+        with torch.cuda.stream(host):
+            g.replay()
+            g.replay()
+        got = out.numpy()
+    finally:
+        L.check(rt.ctx, rt.lib.caten_b200_set_stream(rt.ctx, None))
+    np.testing.assert_array_equal(got.T, m.decode_device(first, 9, 6))
+    del g
+    ids.close(); out.close(); m.close()
+
+
+@pytest.mark.parametrize("wtype,precision,batch", [("q4_0", "bf16x3", 1), ("f32", "fp32", 2), ("q8_0", "bf16x3", 6)])
+def test_decode_on_the_legacy_default_stream(rt, wtype, precision, batch):
+    """A stream that cannot be captured: the steps' graph is made on the context's own stream and replayed there."""
+    from caten_b200 import _lib as L
+    sd = S.synth_state_dict(TINY, wtype, seed=5, max_seq_len=40, trivial_affine=False, weight_std=0.08)
+    prompt = S.synth_prompts(batch, 9, TINY.vocab_size, seed=2)
+    want = GPT2(rt, TINY, sd, max_seq_len=40, batch=batch, precision=precision)
+    ids = want.forward(prompt, 9, 0)
+    rows = want.decode_device(ids, 9, 6)
+    want.close()
+    m = GPT2(rt, TINY, sd, max_seq_len=40, batch=batch, precision=precision)
+    L.check(rt.ctx, rt.lib.caten_b200_set_stream(rt.ctx, 1))   # cudaStreamLegacy
+    try:
+        np.testing.assert_array_equal(m.forward(prompt, 9, 0), ids)
+        np.testing.assert_array_equal(m.forward(ids.reshape(-1, 1), 1, 9), rows[:, 0])
+        np.testing.assert_array_equal(m.decode_device(ids, 9, 6), rows)
+    finally:
+        L.check(rt.ctx, rt.lib.caten_b200_set_stream(rt.ctx, None))
+    m.close()
