@@ -403,7 +403,10 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     return 0;
   }
   if (d_n) return fail(ctx, CATEN_B200_EINVAL, "attention: a device-side position is only supported for single-token steps");
-  if (tensor_cores) return launch_attention_tc(ctx, qkv, kc, vc, out, B, s, n, H, T, bf);
+  if (tensor_cores) {
+    const int rc = launch_attention_tc(ctx, qkv, kc, vc, out, B, s, n, H, T, bf);
+    if (rc != AT_NO_ROOM) return rc;
+  }
   launch_k(ctx, kv_append_kernel, dim3((unsigned)(B * s)), dim3(128), 0, qkv, kc, vc, (int)s, (int)n, (int)H, (int)T);
   CB_LAUNCH_CHECK(ctx, "kv_append_kernel");
   const size_t smem = 4 * 64 * PF_LD * sizeof(float);

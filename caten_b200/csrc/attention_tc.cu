@@ -44,7 +44,6 @@ constexpr int AT_Q = 128;                        // queries per CTA (MMA M)
 constexpr int AT_K = 64;                         // keys per step
 constexpr float AT_TAU = 8.0f;                   // slack of the running maximum, in units of the score
 constexpr int AT_SOFTMAX_WARPS = 8, AT_THREADS = (AT_SOFTMAX_WARPS + 2) * 32;
-constexpr size_t AT_TILES_BYTES = (size_t)256 << 20;   // tiles of as many sequences as fit here are made at a time
 template <int NQ, int NE> struct AtLayout {
   static constexpr int CTAS = NQ == 1 && NE == 1 ? 2 : 1;  // per SM
   // Where one CTA has the SM and its tensor memory to itself the rows of K_hi and K_lo are one operand of 128 rows: two MMAs of
@@ -107,8 +106,8 @@ template <int NQ, int NE, bool PLAIN>
 __global__ void __launch_bounds__(256) attn_tiles_kernel(const AttnArgs p, int b0, uint8_t *__restrict__ tiles) {
   using Lay = AtLayout<NQ, NE>;
   pdl_enter();
-  const int g = blockIdx.y, b = b0 + blockIdx.z, t = p.n + p.s, j0 = (at_first_tile(p) + blockIdx.x) * AT_K;
-  uint8_t *dst = tiles + (((int64_t)blockIdx.z * p.G + g) * gridDim.x + blockIdx.x) * Lay::TILE;
+  const int g = p.g0 + blockIdx.y, b = b0 + blockIdx.z, t = p.n + p.s, j0 = (at_first_tile(p) + blockIdx.x) * AT_K;
+  uint8_t *dst = tiles + (((int64_t)blockIdx.z * p.gn + blockIdx.y) * gridDim.x + blockIdx.x) * Lay::TILE;
   const int64_t head = (int64_t)b * p.G + g;
   const float *kx = !PLAIN && p.kx ? p.kx + b * p.cap * p.kx_ld - p.kx_from : nullptr;   // column c of the key, c >= kx_from
   constexpr int KP = AT_K * NQ * 8, PIECES = KP + AT_K * NE * 8;   // pieces of eight floats
@@ -177,7 +176,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   const int hf = warp >> 2;   // which half (of a step's keys / of a block's head dims) this thread takes
   const int r = quad * 32 + lane;  // query row within the tile = TMEM lane
   const int q0 = (int)(gridDim.z - 1 - blockIdx.z) * AT_Q;  // of all heads, the tiles with the longest history first
-  const int h = blockIdx.x, b = b0 + blockIdx.y;
+  const int rep = PLAIN ? 1 : p.H / p.G;   // query heads per key/value head
+  const int h = p.g0 * rep + blockIdx.x, b = b0 + blockIdx.y;
   const int s = p.s, n = p.n, t = n + s;
 
   if (tid == 0) {
@@ -213,7 +213,7 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   };
 
   // the copies of step i; those of the first two steps, whose stages are free, start while Q is converted
-  const uint8_t *src0 = tiles + (((int64_t)blockIdx.y * p.G + (PLAIN ? h : h / (p.H / p.G))) * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;   // of the key/value head this query head reads
+  const uint8_t *src0 = tiles + (((int64_t)blockIdx.y * p.gn + blockIdx.x / rep) * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;   // of the key/value head this query head reads
   auto copy_k = [&](int i) {
     const int st = i & 1;
     mbar_expect_tx(k_full(st), Lay::K_BYTES);
@@ -487,28 +487,34 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
 }
 
 template <int NQ, int NE, bool PLAIN = false>
-static int launch_at(caten_b200_ctx *ctx, const AttnArgs &a, float qscale) {
+static int launch_at(caten_b200_ctx *ctx, AttnArgs a, float qscale) {
   using Lay = AtLayout<NQ, NE>;
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_Q >> 4) << 24);  // fp32 accumulate, bf16 x bf16, M = 128
   constexpr size_t smem = Lay::SMEM;
   CB_CUDA(ctx, cudaFuncSetAttribute(attn_prefill_tc_kernel<NQ, NE, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int ntiles = (a.n + a.s + AT_K - 1) / AT_K - at_first_tile(a);
-  // The tiles are as large as the visible keys and values in fp32.  Sequences are taken in groups whose tiles stay within
-  // AT_TILES_BYTES (a prompt of 8192 tokens of GPT-2 XL, the largest portion by default, needs 105 MB), one at least.
-  const size_t per_seq = (size_t)a.G * ntiles * Lay::TILE;
-  int group = per_seq < AT_TILES_BYTES ? (int)(AT_TILES_BYTES / per_seq) : 1;
-  if (group > a.B) group = a.B;
-  if (int rc = scratch_reserve(ctx, &ctx->attn_tiles, per_seq * group)) return rc;
-  uint8_t *tiles = (uint8_t *)ctx->attn_tiles.ptr;
   const unsigned qtiles = (unsigned)((a.s + AT_Q - 1) / AT_Q);
   if (qtiles > 65535) return fail(ctx, CATEN_B200_EUNSUPPORTED, "attention: %d tokens in one step", a.s);
+  // The tiles are as large as the visible keys and values in fp32 (a prompt of 8192 tokens of GPT-2 XL, the largest portion by
+  // default, needs 105 MB).  As many whole sequences are taken at a time as attn_tiles_most or the memory that is free
+  // allows, otherwise as many key/value heads of one.
+  const size_t per_head = (size_t)ntiles * Lay::TILE, per_seq = per_head * a.G, most = ctx->attn_tiles_most;
+  const size_t want = per_seq <= most ? per_seq * (most / per_seq < (size_t)a.B ? most / per_seq : (size_t)a.B) : per_head * (most > per_head ? most / per_head : 1);
+  const size_t room = most ? tiles_reserve(ctx, per_head, want) : 0;
+  if (room < per_head) return AT_NO_ROOM;
+  uint8_t *tiles = (uint8_t *)ctx->attn_tiles.ptr;
+  const int group = room >= per_seq ? (int)(room / per_seq < (size_t)a.B ? room / per_seq : (size_t)a.B) : 1;
+  const int heads = room >= per_seq ? a.G : (int)(room / per_head);
   for (int b0 = 0; b0 < a.B; b0 += group) {
     const int nb = a.B - b0 < group ? a.B - b0 : group;
-    launch_k(ctx, attn_tiles_kernel<NQ, NE, PLAIN>, dim3((unsigned)ntiles, (unsigned)a.G, (unsigned)nb), dim3(256), 0, a, b0, tiles);
-    CB_LAUNCH_CHECK(ctx, "attn_tiles_kernel");
-    launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)a.H, (unsigned)nb, qtiles), dim3(AT_THREADS), smem, a, qscale, ctx->d_status, idesc, b0,
-             (const uint8_t *)tiles, ntiles);
-    CB_LAUNCH_CHECK(ctx, "attn_prefill_tc_kernel");
+    for (a.g0 = 0; a.g0 < a.G; a.g0 += heads) {
+      a.gn = a.G - a.g0 < heads ? a.G - a.g0 : heads;
+      launch_k(ctx, attn_tiles_kernel<NQ, NE, PLAIN>, dim3((unsigned)ntiles, (unsigned)a.gn, (unsigned)nb), dim3(256), 0, a, b0, tiles);
+      CB_LAUNCH_CHECK(ctx, "attn_tiles_kernel");
+      launch_k(ctx, attn_prefill_tc_kernel<NQ, NE, PLAIN>, dim3((unsigned)(a.H / a.G * a.gn), (unsigned)nb, qtiles), dim3(AT_THREADS), smem, a, qscale, ctx->d_status, idesc,
+               b0, (const uint8_t *)tiles, ntiles);
+      CB_LAUNCH_CHECK(ctx, "attn_prefill_tc_kernel");
+    }
   }
   return 0;
 }

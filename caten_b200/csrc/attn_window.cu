@@ -265,7 +265,10 @@ int launch_attn_window_prefill(caten_b200_ctx *ctx, const AttnArgs &args, int te
   // every key the step's queries may see is still in the ring
   const int64_t span = a.window > 0 && (int64_t)a.window - 1 < a.n ? (int64_t)a.window - 1 + a.s : (int64_t)a.n + a.s;
   if (span > a.cap) return fail(ctx, CATEN_B200_EINVAL, "attention: %lld live positions in a ring of %lld", (long long)span, (long long)a.cap);
-  if (tensor_cores && a.Dp <= 128 && a.Ep <= 128) return launch_attention_tc_ex(ctx, a, 1.0f);
+  if (tensor_cores && a.Dp <= 128 && a.Ep <= 128) {
+    const int rc = launch_attention_tc_ex(ctx, a, 1.0f);
+    if (rc != AT_NO_ROOM) return rc;
+  }
   const size_t smem = ((size_t)2 * AW_T * (a.Dp + 4) + (size_t)AW_T * (a.Ep + 4) + (size_t)AW_T * (AW_T + 1)) * sizeof(float);
   CB_CUDA(ctx, cudaFuncSetAttribute(attn_window_simt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_k(ctx, attn_window_simt_kernel, dim3((unsigned)((a.s + AW_T - 1) / AW_T), (unsigned)a.H, (unsigned)a.B), dim3(256), smem, a);

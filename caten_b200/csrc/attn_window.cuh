@@ -32,6 +32,7 @@ struct AttnArgs {
   const float *freq = nullptr;
   int qk_norm = 0;                  // q and k divided by their root mean square over D after the rotation
   float eps = 0.0f, scale = 1.0f;   // score = q . k * scale
+  int g0 = 0, gn = 0;               // attention_tc.cu: the key/value heads [g0, g0 + gn) of one launch
 
   void fill_strides() {
     if (k_ld == 0) { k_ld = Dp; k_head = cap * Dp; k_seq = G * k_head; }
@@ -47,6 +48,7 @@ int launch_attn_window_prefill(caten_b200_ctx *ctx, const AttnArgs &a, int tenso
 // Single-token step: rotation, q/k norm, cache append, attention and output gate in one kernel.
 int launch_attn_window_decode(caten_b200_ctx *ctx, const AttnArgs &a);
 // Tensor-core kernel (attention_tc.cu): Dp, Ep <= 128.  q is multiplied by qscale as it is loaded.
+// (AT_NO_ROOM as of launch_attention_tc)
 int launch_attention_tc_ex(caten_b200_ctx *ctx, const AttnArgs &a, float qscale);
 
 }  // namespace cb

@@ -37,7 +37,7 @@ int scratch_reserve(caten_b200_ctx *ctx, Scratch *s, size_t bytes) {
   s->ptr = nullptr;
   s->bytes = 0;
   const size_t want = bytes + bytes / 4;
-  CB_CUDA(ctx, cudaMalloc(&s->ptr, want));
+  CB_CUDA(ctx, device_malloc(ctx, &s->ptr, want));
   s->bytes = want;
   return 0;
 }
@@ -49,6 +49,40 @@ bool stream_is_capturing(cudaStream_t s) {
   if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
   (void)cudaGetLastError();
   return true;
+}
+
+static void tiles_release(caten_b200_ctx *ctx) {
+  if (ctx->attn_tiles_in_graph) ctx->attn_tiles_old.push_back(ctx->attn_tiles.ptr);   // (replays of that graph still use it)
+  else cudaFree(ctx->attn_tiles.ptr);   // waits for work that may still read it
+  ctx->attn_tiles = Scratch();
+  ctx->attn_tiles_in_graph = false;
+}
+
+cudaError_t device_malloc(caten_b200_ctx *ctx, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !ctx->attn_tiles.ptr || ctx->attn_tiles_in_graph) return e;
+  (void)cudaGetLastError();
+  tiles_release(ctx);
+  return cudaMalloc(p, bytes);
+}
+
+// Room for operand tiles of a multi-token step's attention: `want` bytes if they can be had, otherwise the largest half,
+// quarter, .. of it, at least `least`; 0 if that is not there either.  Nothing is allocated while the stream is being captured
+// (what is there then is used), and a buffer that a captured graph uses stays where it is.
+size_t tiles_reserve(caten_b200_ctx *ctx, size_t least, size_t want) {
+  Scratch &s = ctx->attn_tiles;
+  const bool capturing = stream_is_capturing(ctx->stream);
+  if (s.bytes < want && !capturing) {
+    if (s.ptr) tiles_release(ctx);
+    for (size_t size = want; size >= least && !s.ptr; size /= 2) {
+      const size_t more = size == want && want + want / 4 <= ctx->attn_tiles_most ? want / 4 : 0;   // the next step's context is longer
+      if (cudaMalloc(&s.ptr, size + more) == cudaSuccess) s.bytes = size + more;
+      else { s.ptr = nullptr; (void)cudaGetLastError(); }
+    }
+  }
+  if (s.bytes < least) return 0;
+  if (capturing) ctx->attn_tiles_in_graph = true;
+  return s.bytes;
 }
 
 static int check_status(caten_b200_ctx *ctx) {
@@ -120,6 +154,7 @@ int caten_b200_init(int device, caten_b200_ctx **out) {
   if (const char *e = getenv("CATEN_B200_DENSE_GEMM")) ctx->dense_gemm = atoi(e) != 0;
   if (const char *e = getenv("CATEN_B200_ATTN_PREFETCH_MB")) ctx->attn_prefetch_bytes = (long long)atoi(e) << 20;
   if (const char *e = getenv("CATEN_B200_ATTN_TC")) ctx->attn_tc = atoi(e);
+  if (const char *e = getenv("CATEN_B200_ATTN_TILES_MB")) ctx->attn_tiles_most = (size_t)(atoi(e) > 0 ? atoi(e) : 0) << 20;
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) { delete ctx; return cuda_fail(nullptr, e, "cudaStreamCreate"); }
   ctx->own_stream = ctx->stream;
   if ((e = cudaMalloc(&ctx->d_status, 4 * sizeof(int))) != cudaSuccess) { delete ctx; return cuda_fail(nullptr, e, "cudaMalloc"); }
@@ -150,6 +185,7 @@ int caten_b200_destroy(caten_b200_ctx *ctx) {
   if (ctx->wkv_tmp.ptr) cudaFree(ctx->wkv_tmp.ptr);
   if (ctx->chunk_states.ptr) cudaFree(ctx->chunk_states.ptr);
   if (ctx->attn_tiles.ptr) cudaFree(ctx->attn_tiles.ptr);
+  for (void *p : ctx->attn_tiles_old) cudaFree(p);
   if (ctx->upload_stage.ptr) cudaFree(ctx->upload_stage.ptr);
   for (int k = 0; k < 2; ++k) {
     if (ctx->pin[k]) cudaFreeHost(ctx->pin[k]);
@@ -176,7 +212,7 @@ int caten_b200_malloc(caten_b200_ctx *ctx, size_t bytes, void **d_ptr) {
   if (!d_ptr) return fail(ctx, CATEN_B200_EINVAL, "malloc: out pointer is NULL");
   *d_ptr = nullptr;
   if (bytes == 0) bytes = 16;
-  CB_CUDA(ctx, cudaMalloc(d_ptr, bytes));
+  CB_CUDA(ctx, device_malloc(ctx, d_ptr, bytes));
   CB_CUDA(ctx, cudaMemsetAsync(*d_ptr, 0, bytes, ctx->stream));
   return 0;
 }
@@ -305,11 +341,11 @@ int caten_b200_weight_upload_device(caten_b200_ctx *ctx, int type, const void *d
     // a block format the kernels do not consume packed: expand to fp32 now, keep an fp32 weight
     w->type = CATEN_B200_F32;
     w->device_bytes = rows * cols * (int64_t)sizeof(float);
-    if ((e = cudaMalloc(&w->qs, (size_t)(rows * cols) * sizeof(float))) != cudaSuccess) { delete w; return cuda_fail(ctx, e, "cudaMalloc(weight)"); }
+    if ((e = device_malloc(ctx, &w->qs, (size_t)(rows * cols) * sizeof(float))) != cudaSuccess) { delete w; return cuda_fail(ctx, e, "cudaMalloc(weight)"); }
     if (int rc = launch_dequant_extra(ctx, type, (const uint8_t *)d_blocks, rows * cols, (float *)w->qs)) { cudaFree(w->qs); delete w; return rc; }
   } else if (type == CATEN_B200_F32 || type == CATEN_B200_F16 || type == CATEN_B200_BF16) {
     w->device_bytes = nbytes;
-    if ((e = cudaMalloc(&w->qs, (size_t)nbytes)) != cudaSuccess) { delete w; return cuda_fail(ctx, e, "cudaMalloc(weight)"); }
+    if ((e = device_malloc(ctx, &w->qs, (size_t)nbytes)) != cudaSuccess) { delete w; return cuda_fail(ctx, e, "cudaMalloc(weight)"); }
     if ((e = cudaMemcpyAsync(w->qs, d_blocks, (size_t)nbytes, cudaMemcpyDeviceToDevice, ctx->stream)) != cudaSuccess) {
       cudaFree(w->qs); delete w; return cuda_fail(ctx, e, "cudaMemcpyAsync(weight)");
     }
@@ -319,17 +355,17 @@ int caten_b200_weight_upload_device(caten_b200_ctx *ctx, int type, const void *d
     const int64_t nblocks = rows * w->nkb;
     const size_t qbytes = (size_t)nblocks * cb::type_code_bytes(type);
     auto drop = [&]() { cudaFree(w->qs); cudaFree(w->d); cudaFree(w->m); cudaFree(w->qh); delete w; };
-    if ((e = cudaMalloc(&w->qs, qbytes)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight codes)"); }
+    if ((e = device_malloc(ctx, &w->qs, qbytes)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight codes)"); }
     // 16 spare bytes: scales may be fetched in whole 16-byte pieces
-    if ((e = cudaMalloc((void **)&w->d, (size_t)nblocks * 2 + 16)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight scales)"); }
+    if ((e = device_malloc(ctx, (void **)&w->d, (size_t)nblocks * 2 + 16)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight scales)"); }
     cudaMemsetAsync((uint8_t *)w->d + (size_t)nblocks * 2, 0, 16, ctx->stream);
     w->device_bytes = (int64_t)qbytes + nblocks * 2;
     if (cb::type_has_min(type)) {
-      if ((e = cudaMalloc((void **)&w->m, (size_t)nblocks * 2)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight minima)"); }
+      if ((e = device_malloc(ctx, (void **)&w->m, (size_t)nblocks * 2)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight minima)"); }
       w->device_bytes += nblocks * 2;
     }
     if (cb::type_has_qh(type)) {
-      if ((e = cudaMalloc((void **)&w->qh, (size_t)nblocks * 4)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight fifth bits)"); }
+      if ((e = device_malloc(ctx, (void **)&w->qh, (size_t)nblocks * 4)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight fifth bits)"); }
       w->device_bytes += nblocks * 4;
     }
     if (int rc = launch_repack(ctx, type, (const uint8_t *)d_blocks, nblocks, w->qs, w->d, w->m, w->qh)) { drop(); return rc; }

@@ -119,7 +119,10 @@ struct caten_b200_ctx {
   cb::Scratch wbf;           // bf16 copy (hi, lo) of the weight operand of the many-row GEMM
   cb::Scratch chunk_states;    // per-chunk states of a recurrent layer's prompt
   cb::Scratch wkv_tmp;       // intermediates of a stand-alone time-mixing call
-  cb::Scratch attn_tiles;    // keys and values of a multi-token step as operand tiles
+  cb::Scratch attn_tiles;    // keys and values of a multi-token step as operand tiles: taken only from memory that is free, given back when an allocation fails
+  size_t attn_tiles_most = (size_t)256 << 20;  // its bound (CATEN_B200_ATTN_TILES_MB)
+  bool attn_tiles_in_graph = false;            // a captured graph holds its address
+  std::vector<void *> attn_tiles_old;          // such buffers, outgrown
   cb::Scratch upload_stage;  // raw blocks of the weight being uploaded, before their re-layout
   void *pin[2] = {nullptr, nullptr};          // pinned bounce buffers for large copies from pageable host memory
   cudaEvent_t pin_ev[2] = {nullptr, nullptr};
@@ -169,6 +172,8 @@ namespace cb {
 int fail(caten_b200_ctx *ctx, int code, const char *fmt, ...);
 int cuda_fail(caten_b200_ctx *ctx, cudaError_t e, const char *what);
 int scratch_reserve(caten_b200_ctx *ctx, Scratch *s, size_t bytes);
+cudaError_t device_malloc(caten_b200_ctx *ctx, void **p, size_t bytes);   // cudaMalloc, once more without the operand tiles' buffer
+size_t tiles_reserve(caten_b200_ctx *ctx, size_t least, size_t want);
 bool stream_is_capturing(cudaStream_t s);
 
 #define CB_CUDA(ctx, call)                                          \
@@ -211,6 +216,8 @@ int launch_sample(caten_b200_ctx *ctx, const float *logits, int64_t rows, int64_
 int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B,
                      int64_t s, int64_t n, int64_t H, int64_t T, const int *d_n = nullptr, cb::BfOut bf = cb::BfOut(),
                      const cb::PartIn *pending_qkv = nullptr, int tensor_cores = 0);
+// AT_NO_ROOM: there is no device memory for the operand tiles of even one head; nothing was launched
+constexpr int AT_NO_ROOM = -1;
 int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B,
                         int64_t s, int64_t n, int64_t H, int64_t T, cb::BfOut bf);
 // LayerNorm of a linear's input rows, done by the linear itself (up to four rows)

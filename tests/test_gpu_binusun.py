@@ -216,6 +216,18 @@ def test_attention_decode_launch_shapes(rt, B, G, rep):
     np.testing.assert_allclose(c.run([93, 1, 1, 1], "bf16x3"), c.want, atol=4e-5, rtol=0)
 
 
+@pytest.mark.parametrize("H,G,D,E,window", [(8, 4, 64, 64, 0), (12, 6, 96, 128, 70)])
+def test_attention_in_whatever_room_there_is(rt, monkeypatch, H, G, D, E, window):
+    """Operand tiles of some of the key/value heads at a time, and none at all."""
+    from caten_b200.runtime import B200Runtime
+    s = 420
+    for mb in ("1", "0"):   # 7 tiles of 32 to 64 KB a head
+        monkeypatch.setenv("CATEN_B200_ATTN_TILES_MB", mb)
+        with B200Runtime(0) as r:
+            c = AttnCase(r, H, G, D, E, window, s, B=2, rot=0)
+            np.testing.assert_allclose(c.run([350, 70], "bf16x3"), c.want, atol=4e-5, rtol=0)
+
+
 # ---- time mixing --------------------------------------------------------------------------------------
 class WkvCase:
     def __init__(self, rt, H, D, s, B=1, low=64, seed=0, w0=-2.0, spread=1.5):

@@ -357,3 +357,94 @@ def test_decode_on_the_legacy_default_stream(rt, wtype, precision, batch):
     finally:
         L.check(rt.ctx, rt.lib.caten_b200_set_stream(rt.ctx, None))
     m.close()
+
+
+@pytest.mark.parametrize("batch,s", [(3, 300), (5, 100)])
+def test_prompt_attention_in_whatever_room_there_is(rt, monkeypatch, batch, s):
+    """Operand tiles of some sequences, or of some heads of one, at a time: equal bits.  Without any room: the kernel that needs none."""
+    from caten_b200.runtime import B200Runtime
+    sd = S.synth_state_dict(WIDE, "q8_0", seed=5, max_seq_len=320, trivial_affine=False, weight_std=0.08)
+    prompt = S.synth_prompts(batch, s, WIDE.vocab_size, seed=2)
+    outs = []
+    for mb in ("256", "1", "0"):   # a head's tiles take 160 (64) KB, a sequence's 1.3 (0.5) MB
+        monkeypatch.setenv("CATEN_B200_ATTN_TILES_MB", mb)
+        with B200Runtime(0) as r:
+            m = GPT2(r, WIDE, sd, max_seq_len=320, batch=batch, precision="bf16x3")
+            m.forward(prompt[:, :s - 20], s - 20, 0)
+            m.forward(prompt[:, s - 20:], 20, s - 20)
+            outs.append((m.logits(), *m.kv_cache(1)))
+            m.close()
+    for a, b, c in zip(*outs):
+        np.testing.assert_array_equal(a, b)
+        np.testing.assert_allclose(a, c, atol=1e-3, rtol=0)   # the bar of every path that holds fp32 (split bf16 keeps 2^-16 of a sum)
+
+
+def test_captured_prompt_over_a_longer_history(rt):
+    """A step that sees more than the scratch memory was sized for, into a captured stream; replayed after a longer one has
+    made that memory grow."""
+    import torch
+    from caten_b200 import _lib as L
+    from caten_b200.runtime import B200Runtime
+    B, T = 2, 1024
+    sd = S.synth_state_dict(TINY, "q8_0", seed=5, max_seq_len=T, trivial_affine=False, weight_std=0.08)
+    prompt = S.synth_prompts(B, T, TINY.vocab_size, seed=2)
+    with B200Runtime(0) as r:
+        m = GPT2(r, TINY, sd, max_seq_len=T, batch=B, precision="bf16x3")
+        step = lambda ids, s, n, out: m.forward_device(ids, s, n, out)
+        dev = [r.transfer_from_array(np.ascontiguousarray(prompt[:, i:i + 128]).astype(np.int64)) for i in range(0, T, 128)]
+        outs = [r.open_buffer((B,), np.int64) for _ in range(2)]
+        step(dev[0], 128, 0, outs[0])
+        r.sync()
+        host = torch.cuda.Stream()
+        L.check(r.ctx, r.lib.caten_b200_set_stream(r.ctx, host.cuda_stream))
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=host, capture_error_mode="thread_local"):
+            step(dev[1], 128, 128, outs[0])
+        for i in range(1, 8):
+            step(dev[i], 128, 128 * i, outs[1])
+        r.sync()
+        step(dev[1], 128, 128, outs[1])
+        want = m.logits().copy()
+        with torch.cuda.stream(host):
+            g.replay()
+        np.testing.assert_allclose(m.logits(), want, atol=1e-3, rtol=0)   # (another kernel may have done the attention)
+        np.testing.assert_array_equal(outs[0].numpy(), outs[1].numpy())
+        L.check(r.ctx, r.lib.caten_b200_set_stream(r.ctx, None))
+        del g
+        m.close()
+
+
+def test_prompt_on_a_gpu_that_is_nearly_full(rt):
+    """What a model does not hold from its creation on, a prompt takes only if it is there: tiles of 64 MB with 16 MB left; and an
+    allocation that fails for want of memory gets what the tiles hold."""
+    import torch
+    from caten_b200.runtime import B200Runtime
+    p = S.GPT2Params(n_layers=1, n_heads=8, dim=512, vocab_size=1003)
+    sd = S.synth_state_dict(p, "q8_0", seed=5, max_seq_len=1024, trivial_affine=False, weight_std=0.08)
+    prompt = S.synth_prompts(16, 1000, p.vocab_size, seed=2)
+
+    def run(r, leave):
+        m = GPT2(r, p, sd, max_seq_len=1024, batch=16, precision="bf16x3", max_rows=16384)
+        ids = m.forward(prompt[:, :500], 500, 0)   # (the other scratch buffers)
+        full = []
+        if leave:
+            r.sync()
+            torch.cuda.empty_cache()
+            for left in (1 << 30, leave):
+                free = torch.cuda.mem_get_info()[0]
+                if free > left:
+                    full.append(r.open_buffer(((free - left) // 4,)))
+        m.forward(prompt, 1000, 0)
+        out = m.logits().copy()
+        if leave:   # more than is left without the tiles' buffer
+            more = [r.open_buffer((1 << 20,)) for _ in range(10)]
+            for b in more: b.close()
+        for b in full: b.close()
+        m.close()
+        return out
+
+    with B200Runtime(0) as r:
+        want = run(r, 0)
+    with B200Runtime(0) as r:
+        got = run(r, 16 << 20)
+    np.testing.assert_allclose(got, want, atol=1e-3, rtol=0)
