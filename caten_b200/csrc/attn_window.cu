@@ -737,6 +737,7 @@ extern "C" int caten_b200_attn_window(caten_b200_ctx *ctx, const caten_b200_attn
                                       float *d_vcache, int64_t cap, float *d_out, int64_t B, int64_t s, int64_t n, int precision) {
   if (!ctx) return fail(nullptr, CATEN_B200_EINVAL, "attn_window: ctx is NULL");
   cudaSetDevice(ctx->device);
+  ctx->work_outside = true;
   if (!c || !d_qkv || !d_kcache || !d_vcache || !d_out) return fail(ctx, CATEN_B200_EINVAL, "attn_window: NULL argument");
   if (B < 0 || s < 0 || n < 0 || cap <= 0 || cap % 64 || cap > 0x3fffffff || n + s > 0x3fffffff || c->heads <= 0 || c->kv_heads <= 0 || c->heads % c->kv_heads || c->dim <= 0 || c->vdim <= 0 ||
       c->window < 0 || c->rot_dims < 0 || c->rot_dims % 2 || c->rot_dims > c->dim || (c->rot_dims && !c->rot_freq))

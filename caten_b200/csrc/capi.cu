@@ -123,6 +123,7 @@ using namespace cb;
   do {                                                                             \
     if (!(ctx)) return cb::fail(nullptr, CATEN_B200_EINVAL, "%s: ctx is NULL", __func__); \
     cudaSetDevice((ctx)->device);                                                  \
+    (ctx)->work_outside = true;                                                    \
   } while (0)
 
 extern "C" {
@@ -771,6 +772,7 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "gpt2_step: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   const caten_b200_gpt2_desc &c = m->desc;
   if ((d_ids_f32 == nullptr) == (d_ids_i64 == nullptr)) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: pass exactly one id array");
   if (!d_out_ids) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: out ids is NULL");
@@ -802,6 +804,7 @@ int caten_b200_gpt2_step(caten_b200_gpt2 *m, const float *h_ids_f32, int64_t s, 
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "gpt2_step: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   const int64_t B = m->desc.batch;
   if (!h_ids_f32 || !h_out_ids) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: NULL host buffer");
   if (s < 1 || s > m->desc.max_seq_len) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: s=%lld", (long long)s);
@@ -853,6 +856,7 @@ int caten_b200_gpt2_decode(caten_b200_gpt2 *m, const int64_t *d_first_ids, int64
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "gpt2_decode: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   const caten_b200_gpt2_desc &c = m->desc;
   const int64_t B = c.batch;
   if (!d_first_ids) return fail(ctx, CATEN_B200_EINVAL, "gpt2_decode: ids is NULL");

@@ -145,6 +145,9 @@ struct caten_b200_ctx {
   // weights BEFORE waiting for the preceding kernel (weights are assumed static), so the next launch
   // after an upload is made as an ordinary stream-ordered launch, which completes everything before it.
   bool weights_pending = false;
+  // The models' kernels likewise read gains and biases of norms early.  Those are plain device memory, which any entry point
+  // outside the models may have queued a kernel to write: a step that follows one begins with such a launch too.
+  bool work_outside = false;
   // multi-GPU group (caten_b200_dist_init): an NCCL communicator, bound at run time
   void *dist_comm = nullptr;
   int dist_rank = 0, dist_world = 1;
@@ -276,6 +279,12 @@ int launch_splitk_reduce(caten_b200_ctx *ctx, const float *part, int splits, int
 // xbf when it is set (written by its producer), and the output can be requested the same way (ybf)
 int model_linear(caten_b200_ctx *ctx, int prec, const caten_b200_weight *w, const float *x, BfOut xbf, const float *bias, const float *res,
                  int act, float *y, BfOut ybf, int64_t M, PartIn *defer = nullptr, LinGroups grp = LinGroups(), GemvNorm norm = GemvNorm());
+
+// At the beginning of a model's step.
+inline void model_begins(caten_b200_ctx *ctx) {
+  if (ctx->work_outside) ctx->weights_pending = true;
+  ctx->work_outside = false;
+}
 
 // Whether the next launch may be a programmatic dependent launch; clears the pending-upload mark.
 inline bool take_pdl(caten_b200_ctx *ctx) {

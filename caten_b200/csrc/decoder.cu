@@ -839,6 +839,7 @@ int caten_b200_decoder_step_device(caten_b200_decoder *m, const int64_t *d_ids, 
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "decoder_step: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   if (!d_ids) return fail(ctx, CATEN_B200_EINVAL, "decoder_step: ids is NULL");
   if (int rc = check_step(m, "decoder_step", s, n)) return rc;
   if (int rc = run_step(m, d_ids, s, n, nullptr, 0, nullptr, d_out_ids != nullptr)) return rc;
@@ -853,6 +854,7 @@ int caten_b200_decoder_step(caten_b200_decoder *m, const int64_t *h_ids, int64_t
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "decoder_step: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   const int64_t B = m->desc.batch, V = m->desc.vocab;
   if (!h_ids || n_want < 0 || (n_want > 0 && (!h_want || !h_logits))) return fail(ctx, CATEN_B200_EINVAL, "decoder_step: NULL host buffer");
   if (int rc = check_step(m, "decoder_step", s, n)) return rc;
@@ -883,6 +885,7 @@ int caten_b200_decoder_decode(caten_b200_decoder *m, const int64_t *d_first_ids,
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "decoder_decode: model is NULL");
   caten_b200_ctx *ctx = m->ctx;
   cudaSetDevice(ctx->device);
+  model_begins(ctx);
   const int64_t B = m->desc.batch;
   if (!d_first_ids || steps < 0) return fail(ctx, CATEN_B200_EINVAL, "decoder_decode: bad argument");
   if (steps == 0) return 0;

@@ -137,6 +137,7 @@ int caten_b200_dist_bcast_weights(caten_b200_ctx *ctx, void *d_arena, size_t byt
 int caten_b200_dist_gather_ids(caten_b200_ctx *ctx, const int64_t *d_local, int64_t n_per_rank, int64_t *d_all) {
   if (!ctx) return fail(nullptr, CATEN_B200_EINVAL, "dist_gather_ids: ctx is NULL");
   cudaSetDevice(ctx->device);
+  ctx->work_outside = true;
   if (n_per_rank < 0 || (n_per_rank && (!d_local || !d_all))) return fail(ctx, CATEN_B200_EINVAL, "dist_gather_ids: bad argument");
   if (ctx->dist_world == 1) {
     if (d_all != d_local) CB_CUDA(ctx, cudaMemcpyAsync(d_all, d_local, (size_t)n_per_rank * sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));

@@ -106,6 +106,7 @@ extern "C" {
 int caten_b200_rmsnorm(caten_b200_ctx *ctx, const float *d_x, const float *d_weight, float *d_y, int64_t rows, int64_t d, float eps) {
   if (!ctx) return fail(nullptr, CATEN_B200_EINVAL, "rmsnorm: ctx is NULL");
   cudaSetDevice(ctx->device);
+  ctx->work_outside = true;
   if (!d_x || !d_y) return fail(ctx, CATEN_B200_EINVAL, "rmsnorm: NULL argument");
   if (rows < 0 || d <= 0) return fail(ctx, CATEN_B200_EINVAL, "rmsnorm: bad shape");
   return launch_rmsnorm(ctx, d_x, d_weight, d_y, rows, d, eps);
@@ -115,6 +116,7 @@ int caten_b200_rope(caten_b200_ctx *ctx, const float *d_x, float *d_y, int64_t B
                     int64_t pos0) {
   if (!ctx) return fail(nullptr, CATEN_B200_EINVAL, "rope: ctx is NULL");
   cudaSetDevice(ctx->device);
+  ctx->work_outside = true;
   if (!d_x || !d_y) return fail(ctx, CATEN_B200_EINVAL, "rope: NULL argument");
   if (B < 0 || S < 0 || H < 0) return fail(ctx, CATEN_B200_EINVAL, "rope: bad shape");
   return launch_rope(ctx, d_x, d_y, B, S, H, head_dim, base, pos0);

@@ -716,6 +716,7 @@ extern "C" int caten_b200_wkv(caten_b200_ctx *ctx, const caten_b200_wkv_desc *c,
                               int64_t s, int64_t n, int precision) {
   if (!ctx) return fail(nullptr, CATEN_B200_EINVAL, "wkv: ctx is NULL");
   cudaSetDevice(ctx->device);
+  ctx->work_outside = true;
   if (!c || !d_y || !d_state || !d_out || !c->w0 || !c->u || !c->norm || !c->w2) return fail(ctx, CATEN_B200_EINVAL, "wkv: NULL argument");
   WkvArgs a;
   a.H = c->heads; a.D = c->dim; a.Dp = (c->dim + 15) / 16 * 16;

@@ -448,3 +448,31 @@ def test_prompt_on_a_gpu_that_is_nearly_full(rt):
     with B200Runtime(0) as r:
         got = run(r, 16 << 20)
     np.testing.assert_allclose(got, want, atol=1e-3, rtol=0)
+
+
+@pytest.mark.parametrize("wtype,precision,batch", [("q4_0", "bf16x3", 1), ("f32", "fp32", 3), ("q8_0", "bf16x3", 6)])
+def test_step_after_a_kernel_that_writes_a_parameter(rt, wtype, precision, batch):
+    """A norm's gain that a slow schedule item, queued just before the step, is still computing."""
+    from caten_b200 import expr as E
+    sd = S.synth_state_dict(TINY, wtype, seed=5, max_seq_len=40, trivial_affine=False, weight_std=0.08)
+    m = GPT2(rt, TINY, sd, max_seq_len=40, batch=batch, precision=precision)
+    first = m.forward(S.synth_prompts(batch, 9, TINY.vocab_size, seed=2), 9, 0)
+    ids, out = rt.transfer_from_array(first.astype(np.int64)), rt.open_buffer((batch,), np.int64)
+    old = sd["h.1.ln_2.affine"]
+    gain = next(b for b in m._bufs if b.shape == old.shape and (b.numpy() == old).all())
+    x = rt.transfer_from_array(np.linspace(-2, 3, TINY.dim).astype(np.float32) * 1e-4)
+    def new_gain(turns):   # every thread adds one element `turns` times
+        E.run(rt, E.Program(E.load(E.View(x, strides=(1, 0)))), E.View(gain, strides=(1, 0)), (TINY.dim, turns), 1, "sum")
+    logits = []
+    for wait in (True, False):
+        for turns in (1000, 100000):
+            new_gain(turns)
+            if wait:
+                rt.sync()
+            m.forward_device(ids, 1, 9, out)
+            logits.append(m.logits().copy())
+    np.testing.assert_array_equal(logits[0], logits[2])
+    np.testing.assert_array_equal(logits[1], logits[3])
+    assert np.abs(logits[0] - logits[1]).max() > 1e-3
+    for b in (x, ids, out): b.close()
+    m.close()
