@@ -150,7 +150,7 @@ int caten_b200_init(int device, caten_b200_ctx **out) {
   ctx->device = device;
   ctx->sm_count = prop.multiProcessorCount;
   if (const char *e = getenv("CATEN_B200_PDL")) ctx->use_pdl = atoi(e) != 0;
-  if (const char *e = getenv("CATEN_B200_DENSE_PAIR")) ctx->dense_pair = atoi(e) != 0;
+  if (const char *e = getenv("CATEN_B200_DENSE_PAIR")) ctx->dense_pair = atoi(e);
   if (const char *e = getenv("CATEN_B200_SPLITK_CLUSTER")) ctx->splitk_cluster = atoi(e);
   if (const char *e = getenv("CATEN_B200_DENSE_GEMM")) ctx->dense_gemm = atoi(e) != 0;
   if (const char *e = getenv("CATEN_B200_ATTN_PREFETCH_MB")) ctx->attn_prefetch_bytes = (long long)atoi(e) << 20;

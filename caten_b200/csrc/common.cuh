@@ -129,7 +129,7 @@ struct caten_b200_ctx {
   bool pin_busy[2] = {false, false};
   long long attn_prefetch_bytes = 64ll << 20;  // L2 budget of the decode attention's K / V history hint (CATEN_B200_ATTN_PREFETCH_MB; 0 = off)
   bool dense_gemm = true;    // many-row linears expand the weights once and run the TMA-fed GEMM (CATEN_B200_DENSE_GEMM=0: off)
-  bool dense_pair = true;    // its tiles by pairs of CTAs where that is expected to be faster (CATEN_B200_DENSE_PAIR=0: off)
+  int dense_pair = 1;        // its tiles by pairs of CTAs: 1 where that is expected to be faster, 0 never, 2 wherever it can be (CATEN_B200_DENSE_PAIR)
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   int64_t launches = 0;
   int64_t device_failures = 0;   // kernel-side check failures reported so far

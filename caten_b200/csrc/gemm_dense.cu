@@ -559,7 +559,7 @@ struct GdPlan {
 // 256 features loads 32 KB per CTA where a CTA alone loads 48, and has more stages in flight; it starts later (both CTAs
 // meet twice), and narrower tiles gain nothing from it (1665 rows, split bf16, 6400 x 1600, 224 rows wide: 91 us alone, 97).  us a call with the conversion of x, alone -> pair: 8192 rows, plain bf16,
 // 11264 x 2048 328 -> 297, 2048 x 5632 187 -> 170; split bf16, 6400 x 1600 361 -> 341; 777 rows, 4096 x 1024 13.6 -> 14.8.
-static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums, bool can_pair) {
+static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums, bool can_pair, bool must_pair) {
   GdPlan best = {256, 1, (int)(K / bk), false};
   double least = 1e30;
   const int nk = (int)(K / bk), products = nsplit == 1 ? 1 : wlo ? 3 : 2, parts = nsplit == 1 ? 1 : 2;
@@ -587,7 +587,7 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
       const double need = ((double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)bn / 2 * parts)) / 60.0, body = nk * (mma > need ? mma : need);
       const double t = 4000 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
       // (a tile of a short K alone is mostly epilogue, which a wave more or less decides: 1665 rows, 3072 x 1024, plain bf16)
-      if (t < least && (body >= 16000 || waves >= 4)) { least = t; best = {bn, 1, nk, true}; }
+      if (must_pair || (t < least && (body >= 16000 || waves >= 4))) { least = t; best = {bn, 1, nk, true}; }
     }
     if (bn >= M) break;
   }
@@ -671,7 +671,7 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   if (res && !grp.plain_output()) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: a residual needs the plain output layout");
   const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && grp.plain_output() && grp.group_rows % GD_BM == 0;
   const bool can_pair = ctx->dense_pair && M > GD_SPLIT_ROWS && !grp.group_rows && ctx->sm_count % 2 == 0;
-  const GdPlan p = gd_plan(ctx->sm_count, M, N, a.tiles_f, K, nsplit, wlo != nullptr, bk, M <= GD_SPLIT_ROWS, can_defer, can_pair);
+  const GdPlan p = gd_plan(ctx->sm_count, M, N, a.tiles_f, K, nsplit, wlo != nullptr, bk, M <= GD_SPLIT_ROWS, can_defer, can_pair, ctx->dense_pair == 2);
   if (p.pair) a.tiles_f = a.tiles_per_group = (int)((N + 2 * GD_BM - 1) / (2 * GD_BM));
   a.bn = p.bn; a.splits = p.splits; a.cps = p.cps; a.part = nullptr;
   a.static_w = as_is && !ctx->weights_pending;

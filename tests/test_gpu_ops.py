@@ -326,24 +326,39 @@ def test_gemm_many_rows_matches_the_tile_per_cta_kernel(oracle, monkeypatch):
     np.testing.assert_allclose(outs[0][1][:64], ref, atol=1e-5, rtol=1e-5)   # test-gemm.lisp:3-22
 
 
-@pytest.mark.parametrize("wtype", ["q8_0", "f16"])
+@pytest.mark.parametrize("wtype", ["q8_0", "f16", "bf16"])
 @pytest.mark.parametrize("prec,tol", [(L.PREC_BF16X3, 1e-4), (L.PREC_BF16, 4e-2)])
-@pytest.mark.parametrize("M,N,K", [(2400, 2052, 2048), (2561, 4100, 1088)])
+@pytest.mark.parametrize("M,N,K", [(2400, 2052, 2048), (2561, 4100, 1088), (1793, 260, 64), (1537, 508, 320)])
 def test_gemm_pairs_of_ctas(rt, monkeypatch, wtype, prec, tol, M, N, K):
-    """Tiles of 256 features by two CTAs, the second one partly or wholly past the last feature, rows that end within a half;
-    and the same linear with one CTA per tile.  Sums of K products of unit variance over sqrt(K): rounding errors of a few
-    2^-16, or of 2^-9 with both operands in bf16."""
-    rng = np.random.Generator(np.random.PCG64(M + N))
-    up, _, _ = make_weight(rng, N, K, wtype, std=K ** -0.5)
-    x, bias, res = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M, N), dtype=np.float32)
+    """Tiles of 256 features by two CTAs, the second one partly or wholly past the last feature, rows that end within a half, one
+    stage of k and more than the ring holds; every instance of the kernel, whatever the expected time, and the same linear with
+    one CTA per tile.  Sums of K products of unit variance over sqrt(K): rounding errors of a few 2^-16, or of 2^-9 with both
+    operands in bf16."""
+    import re
+    import torch
+    from torch.profiler import ProfilerActivity, profile
     from caten_b200.runtime import B200Runtime
-    monkeypatch.setenv("CATEN_B200_DENSE_PAIR", "0")
-    with B200Runtime(0) as alone:
-        for r in (rt, alone):
+    rng = np.random.Generator(np.random.PCG64(M + N))
+    if wtype == "bf16":
+        raw = (rng.standard_normal((N, K), dtype=np.float32) * K ** -0.5).view(np.uint32) >> 16
+        up = S.Packed(L.BF16, N, K, np.ascontiguousarray(raw.astype(np.uint16)).view(np.uint8).reshape(-1))
+    else:
+        up, _, _ = make_weight(rng, N, K, wtype, std=K ** -0.5)
+    x, bias, res = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M, N), dtype=np.float32)
+    for mode in ("2", "0"):
+        monkeypatch.setenv("CATEN_B200_DENSE_PAIR", mode)
+        with B200Runtime(0) as r:
             w = r.upload_weight(up)
+            dx, db, dr = r.transfer_from_array(x), r.transfer_from_array(bias), r.transfer_from_array(res)
             want = res + (x.astype(np.float64) @ w.dequantize().astype(np.float64).T + bias)
-            got = r.linear(w, r.transfer_from_array(x), r.transfer_from_array(bias), r.transfer_from_array(res), precision=prec).numpy()
+            r.sync()
+            with profile(activities=[ProfilerActivity.CUDA]) as p:
+                got = r.linear(w, dx, db, dr, precision=prec).numpy()
+                torch.cuda.synchronize()
             assert np.abs(got - want).max() < tol
+            kernels = [m.groups() for m in (re.search(r"gemm_dense_kernel<(\d), (\w+), (\w+), (\w+)>", e.name) for e in p.events()) if m]
+            split, lo = ("3", "false" if wtype == "bf16" else "true") if prec == L.PREC_BF16X3 else ("1", "false")
+            assert kernels == [(split, "false", lo, "true" if mode == "2" else "false")]
             w.close()
 
 
