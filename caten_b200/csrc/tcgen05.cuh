@@ -101,7 +101,11 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
 }
 // ---- pairs: two CTAs of a cluster on one tile (the even one leads) ----
 // the leader's address of a shared-memory object of this CTA
-__device__ __forceinline__ uint32_t pair_leader(uint32_t saddr) { return saddr & 0xFEFFFFFFu; }
+__device__ __forceinline__ uint32_t pair_leader(uint32_t saddr) {
+  uint32_t at;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(saddr));
+  return at;
+}
 // a load of either CTA that completes on the leader's mbarrier
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
   asm volatile(
@@ -122,9 +126,7 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-  uint32_t at;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(bar), "r"(0));
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at) : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(pair_leader(bar)) : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
