@@ -18,20 +18,23 @@ constexpr float kInvLn2 = 1.0f / 0.6931472f;  // (/ (log 2)) in single float, ap
 // form (max, then exp and sum), not an online rescaling.
 // SPLIT: with few heads and sequences a cluster of CTAs shares a history (contiguous parts of the positions); each forms the
 // two-pass softmax of its part, and the first CTA joins the parts through distributed shared memory.  One sequence of 25
-// heads at 640 positions: 12.4 us with one CTA per head, 6.3 us with eight; at 128 positions and fewer one is as fast.
+// heads at 640 positions: 12.4 us with one CTA per head, 6.3 us with eight.  Below 96 positions one CTA does it, also where the
+// launch, which for a device-side position is made for the longest context, has clusters: the cut depends on the position alone,
+// and every entry gives the same bits (GPT-2 medium Q4_0, one sequence, us a step at 10 positions: all eight 473, one 436; at 130: 476, two 494).
 // ---------------------------------------------------------------------------------------------
 #ifndef ATT_U
 #define ATT_U 4  // rows in flight per half-warp
 #endif
 constexpr int ATT_PARTS = 8;
+__host__ __device__ inline int att_parts(int64_t t, int most) { return t >= 96 ? most : 1; }
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc,
                                                           float *__restrict__ vc, float *__restrict__ out, int H,
                                                           int T, int n, const int *__restrict__ d_n,
                                                           __nv_bfloat16 *__restrict__ ohi, __nv_bfloat16 *__restrict__ olo,
-                                                          const PartIn pin, long long prefetch_bytes, int parts) {
-  const int h = SPLIT ? blockIdx.x / parts : blockIdx.x, rank = SPLIT ? blockIdx.x % parts : 0, b = blockIdx.y, tid = threadIdx.x;
+                                                          const PartIn pin, long long prefetch_bytes, const int cluster) {
+  const int h = SPLIT ? blockIdx.x / cluster : blockIdx.x, rank = SPLIT ? blockIdx.x % cluster : 0, b = blockIdx.y, tid = threadIdx.x;
   if (SPLIT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "my shared memory may be written to"
   float *kb = kc + ((int64_t)b * H + h) * T * 64;
   float *vb = vc + ((int64_t)b * H + h) * T * 64;
@@ -47,8 +50,9 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
     constexpr long long PIECE = 32 << 10;
     int np = d_n ? *d_n : n;
     np = np < 0 ? 0 : (np > T - 1 ? T - 1 : np);
-    const int p0 = SPLIT ? (int)((long long)np * rank / parts) : 0;
-    const long long stream_bytes = 256ll * ((SPLIT ? (int)((long long)np * (rank + 1) / parts) : np) - p0);
+    const int share = SPLIT ? att_parts(np + 1, cluster) : 1;
+    const int p0 = SPLIT ? (int)((long long)np * rank / share) : 0;
+    const long long stream_bytes = rank < share ? 256ll * ((SPLIT ? (int)((long long)np * (rank + 1) / share) : np) - p0) : 0;
     const int pieces = (int)((stream_bytes + PIECE - 1) / PIECE);
     if (tid < 2 * pieces && ((long long)b * H + h + 1) * 2 * 256ll * np <= prefetch_bytes) {
       const int which = tid >= pieces ? 1 : 0, i = tid - which * pieces;
@@ -66,6 +70,14 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
   float *red = part + 1024;   // 32
   float *sc = red + 32;       // t
   const int d = H * 64, t = n + 1;
+  const int parts = SPLIT ? att_parts(t, cluster) : 1;
+  if (SPLIT && rank >= parts) {   // (whole CTAs) not needed at this length; the others still meet at the barriers
+    if (parts > 1) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    return;
+  }
   const int j_first = SPLIT ? (int)((long long)t * rank / parts) : 0, j_end = SPLIT ? (int)((long long)t * (rank + 1) / parts) : t;
   const bool newest = !SPLIT || rank == parts - 1;   // position n is in the last part, which is never empty
   __shared__ float join[SPLIT ? ATT_PARTS * 66 : 1];  // of the first CTA: each part's maximum, sum and 64 outputs
@@ -130,7 +142,7 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
   ss = red[0];
 #pragma unroll
   for (int w = 1; w < 8; ++w) ss += red[w];
-  const float inv = SPLIT ? 1.0f : 1.0f / ss;   // (parts are joined before they are divided by the sum)
+  const float inv = parts > 1 ? 1.0f : 1.0f / ss;   // (parts are joined before they are divided by the sum)
   // O = P.V
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int j0 = j_first; j0 < j_end; j0 += 16 * ATT_U) {
@@ -158,7 +170,7 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
 #pragma unroll
     for (int w = 0; w < 16; ++w) o += part[w * 64 + tid];
   }
-  if (SPLIT) {
+  if (parts > 1) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (tid < 66) {
       uint32_t at;
@@ -371,10 +383,14 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     // with a device-side position the launch is sized for the longest context the cache allows
     const size_t smem = (64 + 1024 + 32 + (size_t)(d_n ? T : n + 1)) * sizeof(float);
     if (smem > 200 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "attention: context too long for the decode kernel");
-    // CTAs per history: as many as are resident twice per SM at most, each with 64 positions or more at the longest context
-    const int64_t longest = d_n ? T : n + 1;
-    int parts = 1;
-    while (parts < ATT_PARTS && B * H * parts * 2 <= 2 * ctx->sm_count && longest >= 128 * parts) parts *= 2;
+    // CTAs per history: as many as are resident twice per SM at most.  Two are not worth a cluster, whose CTAs start later beside the
+    // linear before (us a step, one / two, at 10, 300, 640 and 1000 positions: medium Q4_0, 8 sequences 755 / 811, 895 / 952, 1076 /
+    // 1119, 1258 / 1223; XL, 5 sequences 1982 / 2071, 2238 / 2301, 2581 / 2627, 2942 / 2930; small Q8_0, 8 sequences 424 / 423, 467 / 461, 557 / 525, 643 / 579);
+    // and behind the fp32 GEMM more waiting CTAs cost that GEMM more than they save (small, 5 sequences, 300 positions: 5684 / 5900 with four).
+    int most = 1;
+    while (most < ATT_PARTS && B * H * most * 2 <= 2 * ctx->sm_count) most *= 2;
+    if (most == 2 || (B > 4 && !tensor_cores)) most = 1;
+    const int parts = att_parts(d_n ? T : n + 1, most);
     auto kernel = parts > 1 ? attn_decode_kernel<true> : attn_decode_kernel<false>;
     if (smem > 44 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     cudaLaunchConfig_t cfg = {};

@@ -476,3 +476,24 @@ def test_step_after_a_kernel_that_writes_a_parameter(rt, wtype, precision, batch
     assert np.abs(logits[0] - logits[1]).max() > 1e-3
     for b in (x, ids, out): b.close()
     m.close()
+
+
+@pytest.mark.parametrize("wtype,precision,batch", [("q4_0", "bf16x3", 1), ("f32", "fp32", 2), ("q8_0", "fp32", 4), ("q5_0", "bf16x3", 6), ("f32", "fp32", 5)])
+def test_single_token_steps_give_the_same_bits_from_every_entry(rt, wtype, precision, batch):
+    """gpt2_step replays a graph with the position on the device, gpt2_step_device launches with the position given, gpt2_decode
+    does several: histories are cut alike, at the lengths where the number of parts changes too."""
+    T = 600
+    sd = S.synth_state_dict(TINY, wtype, seed=5, max_seq_len=T, trivial_affine=False, weight_std=0.08)
+    m = GPT2(rt, TINY, sd, max_seq_len=T, batch=batch, precision=precision)
+    m.forward(S.synth_prompts(batch, 520, TINY.vocab_size, seed=2), 520, 0)
+    tok = S.synth_prompts(batch, 1, TINY.vocab_size, seed=9).reshape(batch, 1)
+    ids, out = rt.transfer_from_array(tok.reshape(-1).astype(np.int64)), rt.open_buffer((batch,), np.int64)
+    for n in (0, 5, 126, 127, 128, 254, 255, 256, 400, 511, 512):
+        a = m.forward(tok, 1, n)
+        la = m.logits().copy()
+        m.forward_device(ids, 1, n, out)
+        np.testing.assert_array_equal(m.logits(), la)
+        np.testing.assert_array_equal(out.numpy(), a)
+        np.testing.assert_array_equal(m.decode_device(tok, n, 1)[:, 0], a)
+        np.testing.assert_array_equal(m.logits(), la)
+    ids.close(); out.close(); m.close()
