@@ -89,7 +89,6 @@ static int check_status(caten_b200_ctx *ctx) {
   if (ctx->h_status[0] != DEV_OK) {
     const int code = ctx->h_status[0], where = ctx->h_status[1], detail = ctx->h_status[2];
     ctx->h_status[0] = 0;
-    ctx->device_failures++;
     cudaMemsetAsync(ctx->d_status, 0, 4 * sizeof(int), ctx->stream);
     return fail(ctx, CATEN_B200_EDEVICE, "kernel-side check failed: code %d (%s) at site %d, detail %d", code,
                 code == DEV_WAIT_TIMEOUT ? "bounded wait ran out" : "bad index", where, detail);
@@ -357,9 +356,7 @@ int caten_b200_weight_upload_device(caten_b200_ctx *ctx, int type, const void *d
     const size_t qbytes = (size_t)nblocks * cb::type_code_bytes(type);
     auto drop = [&]() { cudaFree(w->qs); cudaFree(w->d); cudaFree(w->m); cudaFree(w->qh); delete w; };
     if ((e = device_malloc(ctx, &w->qs, qbytes)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight codes)"); }
-    // 16 spare bytes: scales may be fetched in whole 16-byte pieces
-    if ((e = device_malloc(ctx, (void **)&w->d, (size_t)nblocks * 2 + 16)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight scales)"); }
-    cudaMemsetAsync((uint8_t *)w->d + (size_t)nblocks * 2, 0, 16, ctx->stream);
+    if ((e = device_malloc(ctx, (void **)&w->d, (size_t)nblocks * 2)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight scales)"); }
     w->device_bytes = (int64_t)qbytes + nblocks * 2;
     if (cb::type_has_min(type)) {
       if ((e = device_malloc(ctx, (void **)&w->m, (size_t)nblocks * 2)) != cudaSuccess) { drop(); return cuda_fail(ctx, e, "cudaMalloc(weight minima)"); }
@@ -591,15 +588,28 @@ struct caten_b200_gpt2 {
   // decode replayed from a CUDA graph: position and ids live on the device
   cb::StepLoop loop;
   int *h_pos_pinned = nullptr;
-  // 1..4 sequences over Q4_0 / Q8_0 layers: profiling times a single-token step as a whole (class DECODE_STEP), and the
-  // device entry advances the device-side position.  CATEN_B200_PERSISTENT=0: timed per kernel
-  bool whole_step = false;
+  // 1..4 sequences over Q4_0 / Q8_0 layers: profiling times a single-token step as a whole (class DECODE_STEP).
+  // CATEN_B200_PERSISTENT=0: timed per kernel
+  bool time_whole = false;
   bool defer_reduce = true;  // CATEN_B200_DEFER_REDUCE=0 keeps a reduction kernel behind every split-K linear
 };
 
 static int model_linear(caten_b200_gpt2 *m, const caten_b200_weight *w, const float *x, cb::BfOut xbf, const float *bias,
                         const float *res, int act, float *y, cb::BfOut ybf, int64_t M, cb::PartIn *defer = nullptr, cb::GemvNorm norm = cb::GemvNorm()) {
   return cb::model_linear(m->ctx, m->desc.precision, w, x, xbf, bias, res, act, y, ybf, M, defer, cb::LinGroups(), norm);
+}
+
+// Queues the launches of one single-token step, bracketed as a whole where profiling asks for that.
+template <class F>
+static int single_token_step(caten_b200_gpt2 *m, F step) {
+  caten_b200_ctx *ctx = m->ctx;
+  if (!m->time_whole || !(ctx->prof_mask & (1u << CATEN_B200_K_DECODE_STEP))) return step();
+  ProfScope prof(ctx, CATEN_B200_K_DECODE_STEP);
+  const unsigned mask = ctx->prof_mask;
+  ctx->prof_mask = 0;   // the step's kernels are part of it
+  const int rc = step();
+  ctx->prof_mask = mask;
+  return rc;
 }
 
 extern "C" {
@@ -672,11 +682,11 @@ int caten_b200_gpt2_create(caten_b200_ctx *ctx, const caten_b200_gpt2_desc *dsc,
   if (!rc && cudaMallocHost(&m->h_pos_pinned, sizeof(int)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(pos)");
   if (!rc && cudaMallocHost(&m->h_ids_pinned, (size_t)B * T * sizeof(float)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(ids)");
   if (!rc && cudaMallocHost(&m->h_out_pinned, (size_t)B * sizeof(int64_t)) != cudaSuccess) rc = fail(ctx, CATEN_B200_ECUDA, "cudaMallocHost(out ids)");
-  m->whole_step = B <= 4;
+  m->time_whole = B <= 4;
   for (int64_t l = 0; l < L; ++l)
     for (const caten_b200_weight *w : {m->attn_w[l], m->proj_w[l], m->fc_w[l], m->mproj_w[l]})
-      m->whole_step = m->whole_step && (w->type == CATEN_B200_Q4_0 || w->type == CATEN_B200_Q8_0);
-  if (const char *e = getenv("CATEN_B200_PERSISTENT")) m->whole_step = m->whole_step && atoi(e) != 0;
+      m->time_whole = m->time_whole && (w->type == CATEN_B200_Q4_0 || w->type == CATEN_B200_Q8_0);
+  if (const char *e = getenv("CATEN_B200_PERSISTENT")) m->time_whole = m->time_whole && atoi(e) != 0;
   if (rc) { caten_b200_gpt2_destroy(m); return rc; }
   m->launches0 = ctx->launches;
   *out = m;
@@ -765,7 +775,6 @@ static int head(caten_b200_gpt2 *m, int64_t s) {
 }
 
 static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps);
-static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host);
 
 int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, const int64_t *d_ids_i64, int64_t s, int64_t n,
                                 int64_t *d_out_ids) {
@@ -779,26 +788,21 @@ int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, cons
   if (s < 1 || n < 0 || n + s > c.max_seq_len)
     return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: s=%lld n=%lld outside the cache (max_seq_len=%d)", (long long)s, (long long)n, c.max_seq_len);
   const int64_t B = c.batch;
-  if (s == 1 && m->whole_step) {
-    if (int rc = launch_begin_steps(ctx, d_ids_f32, d_ids_i64, m->loop.ids_io, m->loop.d_pos, n, B)) return rc;
-    if (int rc = decode_step_device_pos(m, n)) return rc;   // (launch by launch: a caller may be capturing the stream)
-    if (d_out_ids != m->loop.out_ids)
-      CB_CUDA(ctx, cudaMemcpyAsync(d_out_ids, m->loop.out_ids, (size_t)B * sizeof(int64_t), cudaMemcpyDeviceToDevice, ctx->stream));
-    return 0;
-  }
   int64_t per = m->max_rows / s;
   if (per < 1) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gpt2_step: s=%lld exceeds max_rows=%lld", (long long)s, (long long)m->max_rows);
   if (per > B) per = B;
-  for (int64_t b0 = 0; b0 < B; b0 += per) {
-    const int64_t nb = B - b0 < per ? B - b0 : per;
-    if (int rc = run_chunk(m, d_ids_f32, d_ids_i64, b0, nb, s, n)) return rc;
-  }
-  // lm_head + argmax over the vocabulary
-  if (int rc = head(m, s)) return rc;
-  ProfScope prof(ctx, CATEN_B200_K_ARGMAX);
-  return launch_argmax(ctx, m->logits, B, c.vocab, d_out_ids);
+  auto step = [&]() {
+    for (int64_t b0 = 0; b0 < B; b0 += per) {
+      const int64_t nb = B - b0 < per ? B - b0 : per;
+      if (int rc = run_chunk(m, d_ids_f32, d_ids_i64, b0, nb, s, n)) return rc;
+    }
+    // lm_head + argmax over the vocabulary
+    if (int rc = head(m, s)) return rc;
+    ProfScope prof(ctx, CATEN_B200_K_ARGMAX);
+    return launch_argmax(ctx, m->logits, B, c.vocab, d_out_ids);
+  };
+  return s == 1 ? single_token_step(m, step) : step();
 }
-
 
 int caten_b200_gpt2_step(caten_b200_gpt2 *m, const float *h_ids_f32, int64_t s, int64_t n, int64_t *h_out_ids) {
   if (!m) return fail(nullptr, CATEN_B200_EINVAL, "gpt2_step: model is NULL");
@@ -837,13 +841,7 @@ static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host) {
     if (int rc = launch_argmax(ctx, m->logits, c.batch, c.vocab, m->loop.out_ids)) return rc;
     return launch_finish_step(ctx, m->loop.out_ids, m->loop.ids_io, m->loop.hist, m->loop.d_pos, c.batch);
   };
-  if (!m->whole_step || !(ctx->prof_mask & (1u << CATEN_B200_K_DECODE_STEP))) return step();
-  ProfScope prof(ctx, CATEN_B200_K_DECODE_STEP);
-  const unsigned mask = ctx->prof_mask;
-  ctx->prof_mask = 0;   // the step's kernels are part of it
-  const int rc = step();
-  ctx->prof_mask = mask;
-  return rc;
+  return single_token_step(m, step);
 }
 
 // Runs `steps` single-token steps from the device-side state.

@@ -132,7 +132,6 @@ struct caten_b200_ctx {
   int dense_pair = 1;        // its tiles by pairs of CTAs: 1 where that is expected to be faster, 0 never, 2 wherever it can be (CATEN_B200_DENSE_PAIR)
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   int64_t launches = 0;
-  int64_t device_failures = 0;   // kernel-side check failures reported so far
   // split-K partial tiles of the converting GEMM: reduced by a second kernel through global scratch, or inside a thread-block
   // cluster through distributed shared memory.  By default (-1) the cluster for up to 128 rows where the consumer cannot sum
   // the tiles itself (GPT-2 medium, 64 sequences: 1345 us a step with the second kernel, 1327 us so; GPT-2 XL, 256 sequences:
