@@ -248,14 +248,14 @@ __device__ __forceinline__ ExprAcc expr_acc_init(const caten_b200_expr &e, const
   return a;
 }
 
-// acc <- acc (op) x; `first` = no value has entered a MAX yet
-__device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const bool is_f, const bool is_sum, const bool first) {
+// acc <- acc (op) x (the least value that a MAX starts from gives way to any x)
+__device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const bool is_f, const bool is_sum) {
   if (is_f) {
     const float xf = __uint_as_float(x);
-    a.f = is_sum ? a.f + xf : (first ? xf : (a.f > xf ? a.f : xf));
+    a.f = is_sum ? a.f + xf : (a.f > xf ? a.f : xf);
   } else {
     const int32_t xi = (int32_t)x;
-    a.i = is_sum ? a.i + xi : (first ? xi : (a.i > xi ? a.i : xi));
+    a.i = is_sum ? a.i + xi : (a.i > xi ? a.i : xi);
   }
 }
 
@@ -265,7 +265,7 @@ __device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const
 // paid once per warp.  Reduced loops (if any) are walked by each thread in loop order, exactly
 // like the rendered loop nest, so a float sum is added in the reference's order.
 template <int ND, int EV, bool HEAVY>
-__global__ void __launch_bounds__(EXPR_THREADS, HEAVY ? 2 : 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int spw,
+__global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int spw,
                                                             const int64_t n_red, const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
   pdl_enter();
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(EXPR_THREADS, HEAVY ? 2 : 4) expr_kernel(const
       expr_decode(e, r, nd_out, e.ndim, ix);
       expr_run<ND, EV, EXPR_THREADS, HEAVY>(e, ix, va, lanes, val, sm);
 #pragma unroll
-      for (int j = 0; j < EV; ++j) expr_acc_add(acc[j], val[j], is_f, is_sum, !e.accumulate && r == 0);
+      for (int j = 0; j < EV; ++j) expr_acc_add(acc[j], val[j], is_f, is_sum);
     }
 #pragma unroll
     for (int j = 0; j < EV; ++j)
@@ -325,7 +325,7 @@ constexpr int RR_EV = 8, RR_WARPS = 8, RR_THREADS = (RR_WARPS + 1) * 32;
 __host__ __device__ constexpr int rr_cols(int R) { return R >= RR_WARPS ? 32 * RR_EV : 32 * RR_EV * RR_WARPS / R; }
 
 template <int ND, bool HEAVY>
-__global__ void __launch_bounds__(RR_THREADS, HEAVY ? 1 : 3) expr_rowreduce_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out, const int R,
+__global__ void __launch_bounds__(RR_THREADS, 3) expr_rowreduce_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out, const int R,
                                                                     const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
   pdl_enter();
@@ -371,23 +371,104 @@ __global__ void __launch_bounds__(RR_THREADS, HEAVY ? 1 : 3) expr_rowreduce_kern
             if (j < n) to[32 * j] = val[j];
         }
       }
-    } else if (t > 0 && lane < rows) {
-      const uint32_t *src = tile + ((t - 1) & 1) * R * (C + 1) + lane * (C + 1);
+    } else if (t > 0) {
       const int64_t left = n_red - (int64_t)(t - 1) * C;
       const int n = left < C ? (int)left : C;
-      int i = 0;
-      if (t == 1) { expr_acc_add(acc, src[0], is_f, is_sum, !e.accumulate); i = 1; }
+      const uint32_t *last = tile + ((t - 1) & 1) * R * (C + 1);
       if (is_f && is_sum) {
+        if (lane < rows) {
+          const uint32_t *src = last + lane * (C + 1);
 #pragma unroll 16
-        for (; i < n; ++i) acc.f = acc.f + __uint_as_float(src[i]);
-      } else {
+          for (int i = 0; i < n; ++i) acc.f = acc.f + __uint_as_float(src[i]);
+        }
+      } else if (R == 32) {
+        if (lane < rows) {
+          const uint32_t *src = last + lane * (C + 1);
 #pragma unroll 8
-        for (; i < n; ++i) expr_acc_add(acc, src[i], is_f, is_sum, false);
+          for (int i = 0; i < n; ++i) expr_acc_add(acc, src[i], is_f, is_sum);
+        }
+      } else {
+        // A maximum and an integer sum may be formed in parts: up to 32 / R lanes take consecutive pieces of a row (of odd length, for
+        // the banks), which are joined in order.  A NaN forgets the values before it, as `acc > x ? acc : x` does.
+        const int row = lane & (R - 1);
+        int pieces = 32 / R;
+        while (pieces > 1 && n < 32 * pieces) pieces >>= 1;
+        const int len = ((n + pieces - 1) / pieces) | 1, i0 = min(n, lane / R * len), i1 = min(n, i0 + len);
+        const uint32_t *src = last + row * (C + 1);
+        ExprAcc a = {-INFINITY, is_sum ? 0 : INT32_MIN};
+        bool forgets = false;
+        if (row < rows) {
+          if (is_f) {
+#pragma unroll 8
+            for (int i = i0; i < i1; ++i) {
+              const float x = __uint_as_float(src[i]);
+              a.f = a.f > x ? a.f : x;
+              forgets = forgets || x != x;
+            }
+          } else {
+#pragma unroll 8
+            for (int i = i0; i < i1; ++i) expr_acc_add(a, src[i], false, is_sum);
+          }
+        }
+        for (int p = 0; p < pieces; ++p) {
+          const int from = row + p * R;
+          const float f = __shfl_sync(0xffffffffu, a.f, from);
+          const int i = __shfl_sync(0xffffffffu, a.i, from), any = __shfl_sync(0xffffffffu, (int)(i1 > i0), from), nan = __shfl_sync(0xffffffffu, (int)forgets, from);
+          if (!any) continue;
+          if (!is_f) expr_acc_add(acc, (uint32_t)i, false, is_sum);
+          else acc.f = nan || !(acc.f > f) ? f : acc.f;
+        }
       }
     }
     __syncthreads();
   }
   if (warp == RR_WARPS && lane < rows) expr_store(e.out, e.out_dtype, out_at, is_f ? __float_as_uint(acc.f) : (uint32_t)acc.i, result_cls);
+}
+
+// The same for short rows, which would leave most of a tile's strips empty: one warp per output element, lanes along the reduced
+// loop; a warp evaluates 128 elements at a time and adds them in loop order by walking the lanes with shuffles.
+constexpr int RW_EV = 4;
+template <int ND, bool HEAVY>
+__global__ void __launch_bounds__(EXPR_THREADS, 4) expr_rowwarp_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out, const int result_cls) {
+  extern __shared__ uint32_t expr_smem[];
+  pdl_enter();
+  const int64_t o_idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (o_idx >= n_out) return;  // whole warps leave together
+  uint32_t *sm = expr_smem + threadIdx.x;
+  const int lane = threadIdx.x & 31, nd_out = e.ndim - 1, ra = e.ndim - 1;
+  const int64_t n_red = e.shape[ra];
+  ExprIx<ND> ix;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) ix.v[d] = 0;
+  expr_decode(e, o_idx, 0, nd_out, ix);
+  const int64_t out_at = expr_out_at(e, ix, nd_out);
+  const bool is_f = result_cls == CATEN_B200_CLS_F32, is_sum = e.reduce_op == CATEN_B200_RED_SUM;
+  ExprAcc acc = expr_acc_init(e, is_f, out_at, true);
+  uint32_t val[RW_EV];
+  for (int64_t r0 = 0; r0 < n_red; r0 += 32 * RW_EV) {
+    const int64_t mine = r0 + lane;  // this lane's elements: mine, mine + 32, ...
+    const int n = mine >= n_red ? 0 : (int)((n_red - mine + 31) / 32 < RW_EV ? (n_red - mine + 31) / 32 : RW_EV);
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if (d == ra) ix.v[d] = n > 0 ? (int)mine : 0;   // a lane past the end reads element 0 of the row
+    expr_run<ND, RW_EV, EXPR_THREADS, HEAVY>(e, ix, ra, n, val, sm);
+#pragma unroll
+    for (int j = 0; j < RW_EV; ++j) {
+      const int64_t first = r0 + 32 * j;  // element of lane 0
+      if (first >= n_red) break;
+      const int n_here = (int)(n_red - first < 32 ? n_red - first : 32);
+      auto walk = [&](auto add) {          // loop order: lane 0, 1, ..., 31
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+          const uint32_t x = __shfl_sync(0xffffffffu, val[j], k);
+          if (k < n_here) add(x);
+        }
+      };
+      if (is_f && !is_sum) walk([&](uint32_t x) { expr_acc_add(acc, x, true, false); });
+      else walk([&](uint32_t x) { expr_acc_add(acc, x, is_f, is_sum); });
+    }
+  }
+  if (lane == 0) expr_store(e.out, e.out_dtype, out_at, is_f ? __float_as_uint(acc.f) : (uint32_t)acc.i, result_cls);
 }
 
 // Checks the program on the host (operand indices, stack discipline, classes) and returns the
@@ -547,9 +628,22 @@ static int launch_expr_elements(caten_b200_ctx *ctx, const caten_b200_expr &e, i
 
 template <int ND, bool HEAVY>
 static int launch_expr_rows(caten_b200_ctx *ctx, const caten_b200_expr &e, int depth, int64_t n_out, int result_cls) {
-  // output elements per CTA: 32 keep the adding warp full; fewer when that would leave SMs without a CTA
+  // Short rows by a warp each (us, a warp each / tiles): 1000 rows of 64 sum 2.4 / 3.1, maximum 2.6 / 3.5, of 130 3.4 / 3.5, 3.9 /
+  // 3.6; 12800 rows of 64 7.9 / 6.6.  With the heavy words, whose tiles have fewer warps: 12800 rows of 64 11 / 17, of 130 21 / 17.
+  const int64_t n_red = e.shape[e.ndim - 1];
+  if (n_red <= (HEAVY ? 128 : 96) && (HEAVY || n_out <= 8192)) {
+    const int64_t blocks = (n_out + EXPR_THREADS / 32 - 1) / (EXPR_THREADS / 32);
+    if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
+    const size_t smem = (size_t)(depth > 1 ? depth - 1 : 1) * RW_EV * EXPR_THREADS * sizeof(uint32_t);
+    if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(expr_rowwarp_kernel<ND, HEAVY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(ctx, expr_rowwarp_kernel<ND, HEAVY>, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_out, result_cls);
+    CB_LAUNCH_CHECK(ctx, "expr_rowwarp_kernel");
+    return 0;
+  }
+  // output elements per CTA: 32 keep the adding warp full; fewer while the CTAs are resident all at once (1000 rows of 768: two
+  // per CTA are 500 CTAs and a second, short wave: 9.9 -> 11.5 us)
   int R = 32;
-  while (R > 1 && (n_out + R - 1) / R < 2 * ctx->sm_count) R >>= 1;
+  while (R > 1 && (n_out + R / 2 - 1) / (R / 2) <= 3 * ctx->sm_count) R >>= 1;
   const int64_t blocks = (n_out + R - 1) / R;
   if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
   const size_t smem = (2 * (size_t)R * (rr_cols(R) + 1) + (size_t)(depth > 1 ? depth - 1 : 1) * RR_EV * RR_THREADS) * sizeof(uint32_t);
@@ -590,12 +684,12 @@ int launch_expr(caten_b200_ctx *ctx, const caten_b200_expr *given) {
       if (nd_out > 0 && e->operand_stride[i][nd_out - 1] == 1) unit_kept = true;
     }
     if (nd_out == 0 || (unit_red && !unit_kept)) {
-      if (heavy) return launch_expr_rows<MAXD, true>(ctx, *e, depth, n_out, result_cls);
+      if (heavy) return e->ndim <= 2 ? launch_expr_rows<2, true>(ctx, *e, depth, n_out, result_cls) : launch_expr_rows<MAXD, true>(ctx, *e, depth, n_out, result_cls);
       return e->ndim <= 2 ? launch_expr_rows<2, false>(ctx, *e, depth, n_out, result_cls) : launch_expr_rows<MAXD, false>(ctx, *e, depth, n_out, result_cls);
     }
   }
   const int64_t vlen = nd_out > 0 ? e->shape[nd_out - 1] : 1, rows = n_out / vlen;
-  if (heavy) return launch_expr_elements<MAXD, 4, true>(ctx, *e, depth, rows, vlen, n_red, result_cls);
+  if (heavy) return e->ndim <= 2 ? launch_expr_elements<2, 4, true>(ctx, *e, depth, rows, vlen, n_red, result_cls) : launch_expr_elements<MAXD, 4, true>(ctx, *e, depth, rows, vlen, n_red, result_cls);
   // Elements per thread: decoding a word costs about as much as applying it to four values, so eight, where that pads the
   // rows no further than four would and still gives every SM 16 warps; one where a row fits the lanes of a warp.
   const bool wide = (vlen + 255) / 256 * 256 == (vlen + 127) / 128 * 128 && rows * (vlen / 256) >= (int64_t)ctx->sm_count * 16;

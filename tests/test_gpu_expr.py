@@ -213,6 +213,27 @@ def test_row_reductions_at_tile_edges(rt, rows, cols, op):
     check(rt, E.load(x.view) - 1.0, s, shape=(rows, cols), n_reduce=1, reduce_op=op, accumulate=True, pairs=(x,))
 
 
+@pytest.mark.parametrize("rows,cols", [(5, 96), (5, 97), (8192, 96), (8193, 96), (900, 128), (900, 129), (1200, 700), (2, 700)])
+@pytest.mark.parametrize("op", ["sum", "max"])
+def test_row_reductions_of_short_rows_integers_and_heavy_words(rt, rows, cols, op):
+    """A warp per row and tiles, maxima formed in pieces that NaNs cut, integers, and programs of the heavy kind."""
+    shape = (rows, cols)
+    rng = np.random.Generator(np.random.PCG64(rows + cols))
+    a = rng.standard_normal(shape, dtype=np.float32)
+    for at in (0, 1, cols // 3, cols // 2, cols - 2):
+        a[rng.integers(0, rows, rows // 4 + 1), at] = np.nan
+    a[0] = -np.inf
+    a[-1, cols // 2:] = np.nan
+    x, s = Pair(rt, a), Pair(rt, np.zeros((rows, 1), np.float32), strides=(1, 0))
+    i, t = Pair(rt, rng.integers(-2 ** 30, 2 ** 30, shape, dtype=np.int32)), Pair(rt, np.zeros((rows, 1), np.int32), strides=(1, 0))
+    check(rt, E.load(x.view), s, shape=shape, n_reduce=1, reduce_op=op, pairs=(x,))
+    check(rt, E.load(i.view) + E.const(1), t, shape=shape, n_reduce=1, reduce_op=op, pairs=(i,))
+    t.host[:] = t.dev.numpy()
+    check(rt, E.load(i.view), t, shape=shape, n_reduce=1, reduce_op=op, accumulate=True, pairs=(i,))
+    check(rt, E.mod(E.load(i.view), E.const(7)), t, shape=shape, n_reduce=1, reduce_op=op, pairs=(i,))
+    check(rt, E.sqrt(E.load(x.view) * E.load(x.view)), s, shape=shape, n_reduce=1, reduce_op=op, pairs=(x,))
+
+
 @pytest.mark.parametrize("shape", [(3, 32), (2400, 511), (2400, 256), (5, 7, 300)])
 def test_words_joined_with_their_right_operand(rt, shape):
     """A load or a constant, negated or reciprocal, on either side of a binary word; one, four and eight elements a thread."""
