@@ -392,6 +392,33 @@ __global__ void __launch_bounds__(AM_CLASSES * AM_PARTS) argmax_kernel(const flo
   if (tid == 0) out[row] = c.i == V ? 0 : c.i;
 }
 
+// The walk itself, one block per row, for rows too short or too many to be cut.
+__global__ void __launch_bounds__(AM_CLASSES) argmax_walk_kernel(const float *__restrict__ x, int64_t V, int64_t *__restrict__ out) {
+  __shared__ float sv[AM_CLASSES];
+  __shared__ int64_t si[AM_CLASSES];
+  pdl_enter();
+  const int tid = threadIdx.x;
+  const float *xr = x + (int64_t)blockIdx.x * V;
+  float best = -INFINITY;
+  int64_t at = V;  // V = "nothing seen"
+  for (int64_t v = tid; v < V; v += AM_CLASSES) {
+    const float f = xr[v];
+    if (f > best || at == V) { best = f; at = v; }
+  }
+  sv[tid] = best;
+  si[tid] = at;
+  __syncthreads();
+  for (int o = AM_CLASSES / 2; o > 0; o >>= 1) {
+    if (tid < o) {
+      const float ov = sv[tid + o], mv = sv[tid];
+      const int64_t oi = si[tid + o], mi = si[tid];
+      if (oi < V && (mi == V || ov > mv || (ov == mv && oi < mi))) { sv[tid] = ov; si[tid] = oi; }
+    }
+    __syncthreads();
+  }
+  if (tid == 0) out[blockIdx.x] = si[0] == V ? 0 : si[0];
+}
+
 // End of a graph-replayed decode step: the new ids become the next step's input, are recorded in
 // the per-position history, and the device-side position advances.
 __global__ void finish_step_kernel(const int64_t *__restrict__ out_ids, int64_t *__restrict__ ids_io,
@@ -443,7 +470,18 @@ int launch_argmax(caten_b200_ctx *ctx, const float *x, int64_t rows, int64_t V, 
   // CTAs of 1024 threads while one per SM holds all rows, and a cluster per row while there are SMs to spare; above that two
   // parts per CTA, so that more CTAs are resident.  (us at V = 50257 for cluster x parts, a first version: 1 row 4x4 6.1, 2x4 7.5, 8x4 6.3;
   // 64 rows 2x4 8.0, 4x4 12.2, 1x4 10.3; 128 rows 1x4 10.4, 2x4 15.1; 256 rows 1x2 17.7, 1x4 20.0.)
-  const int cluster = rows * 8 <= ctx->sm_count ? 4 : rows * 2 <= ctx->sm_count ? 2 : 1, parts = rows <= ctx->sm_count ? 4 : 2;
+  // us, walked / cut: 1 row of 300 1.9 / 2.0, 148 rows of 5000 3.3 / 3.1; with more rows than SMs 300 of 5000 3.8 / 5.8, 5000 of 8000 40 / 42, 1000 of 16000
+  // 17.4 / 14.6; 300 of 50257, three CTAs on some SMs, 18.5 / 20.7
+  if (V <= 512 || (rows > ctx->sm_count && V < 12288) || (rows > 2 * ctx->sm_count && rows <= 3 * ctx->sm_count && V < 65536)) {
+    if (rows > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "argmax: %lld rows", (long long)rows);
+    launch_k(ctx, argmax_walk_kernel, dim3((unsigned)rows), dim3(AM_CLASSES), 0, x, V, out);
+    CB_LAUNCH_CHECK(ctx, "argmax_walk_kernel");
+    return 0;
+  }
+  int cluster = rows * 8 <= ctx->sm_count ? 4 : rows * 2 <= ctx->sm_count ? 2 : 1, parts = rows <= ctx->sm_count ? 4 : 2;
+  // a part has four values of each residue or more
+  while (cluster > 1 && V < (int64_t)4 * AM_CLASSES * cluster * parts) cluster /= 2;
+  while (parts > 1 && V < (int64_t)4 * AM_CLASSES * parts) parts /= 2;
   if (V > (int64_t)AM_CLASSES * 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "argmax: rows of %lld", (long long)V);
   if (rows * cluster > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "argmax: %lld rows", (long long)rows);
   cudaLaunchConfig_t cfg = {};

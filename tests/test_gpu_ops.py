@@ -137,9 +137,9 @@ def _argmax_of_256_walkers(row):
     return c[0][1]
 
 
-@pytest.mark.parametrize("rows,V", [(1, 1), (2, 255), (3, 2048), (5, 16385), (74, 8193), (149, 4100)])
+@pytest.mark.parametrize("rows,V", [(1, 1), (2, 255), (1, 512), (1, 513), (3, 2048), (5, 16385), (74, 8193), (149, 4100), (150, 12287), (149, 12289)])
 def test_argmax_however_a_row_is_cut(rt, rows, V):
-    """One, two and four CTAs per row, two and four parts in them; ties, minus infinity only, and NaNs, which stand where no comparison admits them."""
+    """One block that walks a row; one, two and four CTAs per row, one to four parts in them; ties, minus infinity only, and NaNs, which stand where no comparison admits them."""
     rng = np.random.Generator(np.random.PCG64(V))
     x = rng.integers(-40, 40, (rows, V)).astype(np.float32)
     x[0] = -np.inf
