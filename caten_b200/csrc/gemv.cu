@@ -1,7 +1,7 @@
-// Dequant-GEMV for decode with one sequence: y[o] = act(sum_k x[k] * W[o,k] + bias[o]) + res[o]
-// (source/nn/linear.lisp:12-17 with M = 1).  HBM-bound: the packed weights are streamed once
-// with 128-bit loads and unpacked in registers; x lives in registers (quantised types) or
-// shared memory (fp32/fp16 weights).  fp32 accumulation throughout.
+// Dequant-GEMV for decode with one to four sequences: y[m, o] = act(sum_k x[m, k] * W[o,k] + bias[o]) + res[m, o]
+// (source/nn/linear.lisp:12-17 with few rows).  The packed weights are streamed once with 128-bit loads and
+// unpacked in registers; x comes through shared memory, from where a thread keeps its block of it in registers
+// (quantised types) or reads it as it goes (fp32 / fp16 / bf16 weights).  fp32 accumulation throughout.
 #include "common.cuh"
 #include "blocks32.cuh"
 #include "gemv_blocks.cuh"
@@ -186,6 +186,90 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
       buf ^= 1;
     }
     if (!LOOP) break;
+  }
+}
+
+// Many rows for one x: the block of x that a thread multiplies is in its registers from the start, and a CTA of 512 threads, one
+// to an SM, walks down the rows with the next rows' loads ahead.  Where the rows do not fit the CTAs that are resident at once, this
+// is the faster form (us, 20000 x 4128 Q5_1 44 / 55 with the kernel above and as many threads, 16384 x 5632 Q4_0 25 / 28, 4096 x 11008 12.9 / 38; 32000 x 2048 Q5_1 34 / 39).
+template <class BLK, int RI>
+__global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_stream_kernel(const GemvArgs a) {
+  extern __shared__ float red[];   // two buffers of [G * RI][nkb]
+  pdl_launch_dependents();
+  constexpr int W = BLK::WORDS;
+  const int tid = threadIdx.x, nkb = a.nkb, G = a.G;
+  const bool active = tid < G * nkb;
+  const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
+  const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
+  const int rows_per_iter = G * RI, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  const int64_t stride = (int64_t)gridDim.x * rows_per_iter;
+  uint32_t qn[RI][W], qhn[RI];
+  float scn[RI], mnn[RI];
+  auto load = [&](int64_t base) {
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      const int64_t row = base + i * G + ro, bidx = row * nkb + kb;
+      const bool ok = active && row < a.N;
+#pragma unroll
+      for (int j = 0; j < W / 4; ++j) {
+        const uint4 v = ok ? ld_stream(qs + bidx * (W / 4) + j) : make_uint4(0, 0, 0, 0);
+        qn[i][4 * j] = v.x; qn[i][4 * j + 1] = v.y; qn[i][4 * j + 2] = v.z; qn[i][4 * j + 3] = v.w;
+      }
+      scn[i] = ok ? __half2float(a.d[bidx]) : 0.0f;
+      if (BLK::HAS_M) mnn[i] = ok ? __half2float(a.m[bidx]) : 0.0f;
+      if (BLK::HAS_QH) qhn[i] = ok ? a.qh[bidx] : 0u;
+    }
+  };
+  int64_t base = (int64_t)blockIdx.x * rows_per_iter;
+  load(base);
+  pdl_wait();
+  BLK blk;
+  {
+    float xv[32];
+    const float4 *xp = reinterpret_cast<const float4 *>(a.x + (int64_t)kb * 32);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 v = xp[i];
+      xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
+    }
+    blk.prep(xv);
+  }
+  for (int buf = 0; base < a.N; base += stride, buf ^= 1) {
+    uint32_t q[RI][W], qhc[RI];
+    float sc[RI], mn[RI];
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+      sc[i] = scn[i];
+      mn[i] = BLK::HAS_M ? mnn[i] : 0.0f;
+      qhc[i] = BLK::HAS_QH ? qhn[i] : 0u;
+#pragma unroll
+      for (int j = 0; j < W; ++j) q[i][j] = qn[i][j];
+    }
+    if (base + stride < a.N) load(base + stride);
+    float *rb = red + buf * rows_per_iter * nkb;
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < RI; ++i) {
+        float r;
+        if constexpr (BLK::HAS_M || BLK::HAS_QH) r = blk.dotx(q[i], sc[i], mn[i], qhc[i]);
+        else r = blk.dot(q[i], sc[i]);
+        rb[(i * G + ro) * nkb + kb] = r;
+      }
+    }
+    __syncthreads();
+    for (int r = warp; r < rows_per_iter; r += nwarps) {
+      const int64_t row = base + r;
+      if (row >= a.N) break;
+      float s = 0.0f;
+      for (int k = lane; k < nkb; k += 32) s += rb[r * nkb + k];
+      s = warp_sum(s);
+      if (lane == 0) {
+        if (a.bias) s = s + a.bias[row];
+        s = apply_act(s, a.act);
+        if (a.res) s = a.res[row] + s;
+        a.y[row] = s;
+      }
+    }
   }
 }
 
@@ -384,9 +468,30 @@ static int launch_blocked_t(caten_b200_ctx *ctx, GemvArgs a) {
   return 0;
 }
 
+template <class BLK, int RI>
+static int launch_stream_t(caten_b200_ctx *ctx, GemvArgs a) {
+  a.G = GEMV_MAX_THREADS / a.nkb;
+  const int threads = (a.G * a.nkb + 31) / 32 * 32;
+  const size_t smem = 2 * (size_t)a.G * RI * a.nkb * sizeof(float);
+  int occ = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gemv_stream_kernel<BLK, RI>, threads, smem);
+  int64_t grid = ((int64_t)a.N + a.G * RI - 1) / (a.G * RI);
+  if (grid > (int64_t)ctx->sm_count * (occ < 1 ? 1 : occ)) grid = (int64_t)ctx->sm_count * (occ < 1 ? 1 : occ);
+  launch_k(ctx, gemv_stream_kernel<BLK, RI>, dim3((unsigned)grid), dim3(threads), smem, a);
+  CB_LAUNCH_CHECK(ctx, "gemv_stream_kernel");
+  return 0;
+}
+
 template <class BLK>
 static int launch_blocked(caten_b200_ctx *ctx, const GemvArgs &a) {
-  if (a.nkb > 256) return launch_blocked_t<BLK, 1, true, 512>(ctx, a);
+  // a handful of blocks per row: more threads leave fewer rows to each warp's sums (64 x 64: 3.4 us, 4.4 with 256)
+  if (a.nkb < 8) return launch_blocked_t<BLK, 1, true, 512>(ctx, a);
+  const bool alone = a.M == 1 && !a.norm.g;
+  if (a.nkb > 256) {
+    const bool deep = (int64_t)a.N >= (int64_t)4 * ctx->sm_count;   // few rows: keep every SM busy with single rows
+    if (alone) return deep ? launch_stream_t<BLK, 4>(ctx, a) : launch_stream_t<BLK, 1>(ctx, a);
+    return deep ? launch_blocked_t<BLK, 4, true, 512>(ctx, a) : launch_blocked_t<BLK, 1, true, 512>(ctx, a);
+  }
   // one pass while the rows fit the resident CTAs (three to an SM where the blocks in flight leave the registers for it) with
   // up to eight loads per thread; more rows: CTAs that go on
   const int64_t slab = (int64_t)(256 / a.nkb) * ctx->sm_count;
@@ -396,7 +501,11 @@ static int launch_blocked(caten_b200_ctx *ctx, const GemvArgs &a) {
   if (a.N <= (small ? 3 : 1) * 2 * slab) return launch_blocked_t<BLK, 2, false, 256>(ctx, a);
   if (a.N <= (small ? deep >= 4 ? 3 : 2 : 1) * 3 * slab) return launch_blocked_t<BLK, 3, false, 256>(ctx, a);
   if (a.N <= (small ? deep >= 4 ? 3 : 2 : 1) * 4 * slab) return launch_blocked_t<BLK, 4, false, 256>(ctx, a);
-  return launch_blocked_t<BLK, 4, true, 256>(ctx, a);
+  // (Q8_0: 32000 x 2048 30 us there, 26 here, 20000 x 4128 40 and 38)
+  // (Q4: 4096 x 4096 6.5 and 5.9, 11264 x 2048 9.4 and 9.1, 32000 x 2048 18.8 and 19.7, 50257 x 1600 25 and 27)
+  if (alone && BLK::WORDS == 4 && (BLK::HAS_QH || a.nkb > 128 || a.N > 24 * slab)) return launch_stream_t<BLK, 4>(ctx, a);
+  // over 128 blocks a CTA of 256 threads holds one row at a time (16384 x 5632 Q4_0, 4 rows of x: 143 us, 87 with 512 threads)
+  return a.nkb > 128 ? launch_blocked_t<BLK, 4, true, 512>(ctx, a) : launch_blocked_t<BLK, 4, true, 256>(ctx, a);
 }
 
 template <typename T, int RI, int NR, bool EXPERTS>

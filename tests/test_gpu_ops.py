@@ -177,6 +177,28 @@ def test_gemv(rt, oracle, wtype, N, K):
     w.close()
 
 
+@pytest.mark.parametrize("wtype", ["q4_0", "q4_1", "q5_0", "q5_1", "q8_0"])
+@pytest.mark.parametrize("N,K", [(9, 32), (50, 224), (2000, 4128), (1900, 8192), (591, 8224), (592, 8224), (700, 10240), (593, 11008), (100, 16384)])
+def test_gemv_packed_formats_and_launch_shapes(rt, wtype, N, K):
+    """A handful of 32-wide blocks per row and up to the most there may be, rows that fit the resident CTAs and rows that do not, one
+    to four rows of x.  A product passes through at most 38 roundings: two chains of 16 in its block and their sum, 16 blocks of a
+    lane, 5 across lanes."""
+    rng = np.random.Generator(np.random.PCG64(N + K))
+    up, _, _ = make_weight(rng, N, K, wtype)
+    w = rt.upload_weight(up)
+    W = w.dequantize().astype(np.float64)
+    x, bias, res = rng.standard_normal((4, K), dtype=np.float32), rng.standard_normal(N, dtype=np.float32), rng.standard_normal((4, N), dtype=np.float32)
+    bound = 42 * 2.0 ** -24 * (np.abs(x.astype(np.float64)) @ np.abs(W).T + np.abs(bias) + np.abs(res))
+    # (minima enter as m times the sum of a block's x, and codes without their offset: products are larger than their sum)
+    slack = 4.0 if wtype in ("q4_1", "q5_1") else 1.0
+    want = res + (x.astype(np.float64) @ W.T + bias)
+    db = rt.transfer_from_array(bias)
+    for M in (1, 2, 3, 4):
+        got = rt.linear(w, rt.transfer_from_array(x[:M]), db, rt.transfer_from_array(res[:M])).numpy()
+        assert (np.abs(got - want[:M]) <= slack * bound[:M]).all()
+    w.close()
+
+
 def test_gemv_up_to_four_rows(rt, oracle):
     rng = np.random.Generator(np.random.PCG64(8))
     up, t, raw = make_weight(rng, 300, 1024, "q4_0")
