@@ -486,6 +486,287 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// GPT-2, steps of few tokens: where one or two tiles are all the queries of a head, tiles of keys made by a kernel of their own
+// would be read once or twice; here the CTA splits the rows itself.  The step's rows come straight from the projections, and the
+// last tile's CTA, which sees all of them, brings them to the cache; older ones come from the cache.  All eight warps do the
+// same, step after step of 64 keys:
+//   copy the NEXT step's K and V rows into a staging buffer in shared memory (cp.async, in flight during this step's products
+//   and softmax); split the current step's into operand tiles as above; one lane issues S = (Q_hi + Q_lo) . (K_hi + K_lo)^T;
+//   softmax as above; one lane issues O += P_hi.V_hi + P_lo.V_hi + P_hi.V_lo
+// with block-wide barriers between (two CTAs share an SM and one's products run under the other's softmax).
+// TMEM columns: [0, 64) scores, [128, 192) P (hi 32, lo 32), [192, 256) O.
+// ---------------------------------------------------------------------------------------------
+namespace {
+constexpr uint32_t A1_COL_S = 0, A1_COL_P = 128, A1_COL_O = 192, A1_COLS = 256;
+// Q: 128 rows hi, 128 rows lo; K, V: 64 rows hi, 64 rows lo; staging: raw fp32 rows of 256 bytes, padded by 16, so that threads
+// reading one row each spread over all banks
+constexpr uint32_t A1_OFF_Q = 0, A1_OFF_K = 32768, A1_OFF_V = A1_OFF_K + 16384, A1_LD = 256 + 16, A1_OFF_SK = A1_OFF_V + 16384, A1_OFF_SV = A1_OFF_SK + AT_K * A1_LD, A1_OFF_MISC = A1_OFF_SV + AT_K * A1_LD;
+constexpr size_t A1_SMEM = A1_OFF_MISC + 1024 + 64 + 1024;   // + exchange of the rows' maxima, barrier, TMEM slot, abort flag, alignment slack
+static_assert(2 * (A1_SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes) {  // src_bytes 0: zero fill
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+}  // namespace
+
+__global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t idesc) {
+  extern __shared__ unsigned char at_raw[];
+  unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(at_raw) + 1023) & ~(uintptr_t)1023);
+  float *red = reinterpret_cast<float *>(sm + A1_OFF_MISC);
+  const uint32_t bar = smem_u32(sm + A1_OFF_MISC + 1024);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + A1_OFF_MISC + 1024 + 8);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + A1_OFF_MISC + 1024 + 12);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int quad = warp & 3, hf = warp >> 2, r = quad * 32 + lane;   // quadrant of tensor memory; half of a step's keys or dims; query
+  const int ck = tid & 63, cq = tid >> 6;                            // conversion: key row of the step, and which 16 dims
+  const int h = blockIdx.x, b = blockIdx.y, q0 = (int)(gridDim.z - 1 - blockIdx.z) * AT_Q, s = p.s, n = p.n, t = n + s;
+
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(A1_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot, tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
+  pdl_enter();
+
+  const int64_t head = ((int64_t)b * p.G + h) * p.cap * 64;
+  float *kb = p.kc + head, *vb = p.vc + head;
+  const float *xb = p.qkv + ((int64_t)b * s - n) * p.ld + h * 64;   // row j >= n of the step at xb + j * ld
+  const int nblk = (min(t, n + q0 + AT_Q) + AT_K - 1) / AT_K;
+  const int jmax = n + min(q0 + r, s - 1);   // last key this query sees (rows past the step's end mask like its last: their output is dropped)
+
+  const uint64_t dq = umma_desc(smem_u32(sm + A1_OFF_Q)), dk = umma_desc(smem_u32(sm + A1_OFF_K)), dv = umma_desc(smem_u32(sm + A1_OFF_V));
+  const uint32_t idesc_s = idesc | ((64u >> 3) << 17), idesc_pv = idesc_s | (1u << 16);  // second product: B MN-major, V rows (keys) with the dims contiguous
+  uint32_t ph = 0;
+  int ok = 1;
+
+  // the 64 rows [j0, j0 + 64) of K and V, zeros past the end of the context; a thread's pieces are 16 rows apart
+  const int frow = tid >> 4, fcol = (tid & 15) * 4;
+  auto fetch = [&](int j0) {
+    const uint32_t dst = smem_u32(sm + A1_OFF_SK + frow * A1_LD + fcol * 4);
+    if (j0 + AT_K <= n) {
+      const float *k = kb + (int64_t)(j0 + frow) * 64 + fcol, *v = vb + (int64_t)(j0 + frow) * 64 + fcol;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        cp_async16(dst + i * 16 * A1_LD, k + i * 16 * 64, 16u);
+        cp_async16(dst + (A1_OFF_SV - A1_OFF_SK) + i * 16 * A1_LD, v + i * 16 * 64, 16u);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int j = j0 + frow + 16 * i;
+        const float *k = kb, *v = vb;
+        if (j < n) { k += (int64_t)j * 64 + fcol; v += (int64_t)j * 64 + fcol; }
+        else if (j < t) { k = xb + (int64_t)j * p.ld + p.k_off + fcol; v = xb + (int64_t)j * p.ld + p.v_off + fcol; }
+        cp_async16(dst + i * 16 * A1_LD, k, j < t ? 16u : 0u);
+        cp_async16(dst + (A1_OFF_SV - A1_OFF_SK) + i * 16 * A1_LD, v, j < t ? 16u : 0u);
+      }
+    }
+    cp_async_commit();
+  };
+  auto staged_row = [&](uint32_t off, float4 *v) {  // this thread's 16 dims of its key row
+    const float4 *src = reinterpret_cast<const float4 *>(sm + off + ck * A1_LD + 64 * cq);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = src[i];
+  };
+  // one warp polls the mbarrier; the others park at the block barrier instead of spinning
+  auto wait_mma = [&]() {
+    if (warp == 0 && !mbar_wait(bar, ph, abort_flag)) {
+      ok = 0;
+      *abort_flag = 1;
+    }
+    ph ^= 1u;
+    ok = __syncthreads_and(ok);
+  };
+
+  fetch(0);
+  {   // Q tiles: rows [0,128) hi, [128,256) lo; the score scale 1/8 is folded in (a power of two: exact)
+    const float4 *src = reinterpret_cast<const float4 *>(p.qkv + ((int64_t)b * s + (q0 + r < s ? q0 + r : 0)) * p.ld + p.q_off + (int64_t)h * 64);
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = q0 + r < s ? scale4(src[8 * hf + i], qscale) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) st_split8(sm + A1_OFF_Q, r, 128 + r, 4 * hf + c, v[2 * c], v[2 * c + 1]);
+  }
+  cp_async_wait_all();
+  __syncthreads();  // step 0 of K and V is staged (and the Q tile is written)
+
+  float m = -INFINITY;  // the row's reference maximum: the same value in both threads of a row
+  float lsum = 0.0f;    // this thread's part of the row sum, relative to m
+  for (int blk = 0; blk < nblk && ok; ++blk) {
+    const int j0 = blk * AT_K;
+    {
+      // split this thread's part of the staged rows in registers, then (once the previous step's P.V has read the V tile and
+      // P) store it into the tiles
+      float4 kv[4], vv[4];
+      staged_row(A1_OFF_SK, kv);
+      staged_row(A1_OFF_SV, vv);
+      if (q0 + AT_Q >= s && j0 + AT_K > n) {   // rows of this step: to the cache
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = frow + 16 * i, j = j0 + row;
+          if (j < n || j >= t) continue;
+          const unsigned char *src = sm + A1_OFF_SK + row * A1_LD + fcol * 4;
+          *reinterpret_cast<float4 *>(kb + (int64_t)j * 64 + fcol) = *reinterpret_cast<const float4 *>(src);
+          *reinterpret_cast<float4 *>(vb + (int64_t)j * 64 + fcol) = *reinterpret_cast<const float4 *>(src + (A1_OFF_SV - A1_OFF_SK));
+        }
+      }
+      uint4 khi[2], klo[2], vhi[2], vlo[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        khi[c] = pack8(kv[2 * c], kv[2 * c + 1]);
+        klo[c] = pack8_lo(kv[2 * c], kv[2 * c + 1]);
+        vhi[c] = pack8(vv[2 * c], vv[2 * c + 1]);
+        vlo[c] = pack8_lo(vv[2 * c], vv[2 * c + 1]);
+      }
+      if (blk > 0) wait_mma();
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        *reinterpret_cast<uint4 *>(sm + A1_OFF_K + sw128(ck, 2 * cq + c)) = khi[c];
+        *reinterpret_cast<uint4 *>(sm + A1_OFF_K + sw128(64 + ck, 2 * cq + c)) = klo[c];
+        *reinterpret_cast<uint4 *>(sm + A1_OFF_V + sw128(ck, 2 * cq + c)) = vhi[c];
+        *reinterpret_cast<uint4 *>(sm + A1_OFF_V + 8192 + sw128(ck, 2 * cq + c)) = vlo[c];
+      }
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);  // tiles complete, staging buffers free
+    if (!ok) break;
+    if (warp == 0) {  // converged warp, one elected lane: the descriptors stay in uniform registers
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint64_t aq = dq + (uint64_t)(2 * k), ak = dk + (uint64_t)(2 * k);   // 16 bf16 = 32 bytes = 2 descriptor units
+          umma_bf16(tmem_base + A1_COL_S, aq, ak, idesc_s, k > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak, idesc_s, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq, ak + 512, idesc_s, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak + 512, idesc_s, 1u);
+        }
+        umma_commit(bar);
+      }
+      __syncwarp();
+    }
+    if (blk + 1 < nblk) fetch(j0 + AT_K);   // (after the MMAs: they are the critical path)
+    wait_mma();
+    tc_fence_after();
+    {
+      uint32_t a[32];
+      tmem_ld16(tlane + A1_COL_S + 32 * hf, a);
+      tmem_ld16(tlane + A1_COL_S + 32 * hf + 16, a + 16);
+      tmem_ld_wait();
+      const int lim = jmax - j0 - 32 * hf;  // key e of this thread is visible iff e <= lim
+      float mloc = -INFINITY;
+#pragma unroll
+      for (int e = 0; e < 32; ++e)
+        if (e <= lim) mloc = fmaxf(mloc, __uint_as_float(a[e]));
+      red[hf * 128 + r] = mloc;
+      __syncthreads();
+      const float mstep = fmaxf(red[r], red[128 + r]);
+      const bool move = mstep > m + AT_TAU;  // also true at the first step (m = -inf), which sees key 0
+      const float m_new = move ? mstep : m;
+      if (blk > 0 && __any_sync(0xffffffffu, move)) {
+        const float scale = move ? exp2f((m - m_new) * kAtInvLn2) : 1.0f;
+        lsum *= scale;
+        uint32_t o[32];
+        tmem_ld16(tlane + A1_COL_O + 32 * hf, o);
+        tmem_ld16(tlane + A1_COL_O + 32 * hf + 16, o + 16);
+        tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * scale);
+        tmem_st16(tlane + A1_COL_O + 32 * hf, o);
+        tmem_st16(tlane + A1_COL_O + 32 * hf + 16, o + 16);
+      }
+      m = m_new;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t phi[8], plo[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int e0 = 16 * c + 2 * e;
+          const float p0 = e0 <= lim ? ex2_approx((__uint_as_float(a[e0]) - m) * kAtInvLn2) : 0.0f;
+          const float p1 = e0 + 1 <= lim ? ex2_approx((__uint_as_float(a[e0 + 1]) - m) * kAtInvLn2) : 0.0f;
+          lsum += p0;
+          lsum += p1;
+          phi[e] = pack_bf16(p0, p1);
+          plo[e] = pack_bf16(bf16_lo(p0), bf16_lo(p1));
+        }
+        tmem_st8(tlane + A1_COL_P + 16 * hf + 8 * c, phi);   // key k of the step sits in column k / 2
+        tmem_st8(tlane + A1_COL_P + 32 + 16 * hf + 8 * c, plo);
+      }
+    }
+    tmem_st_wait();
+    tc_fence_before();
+    cp_async_wait_all();
+    ok = __syncthreads_and(ok);  // P is written; the next step's rows are staged
+    if (!ok) break;
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+          const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
+          const uint32_t p_hi = tmem_base + A1_COL_P + 8 * k4, p_lo = p_hi + 32;
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_lo, dv + adv, idesc_pv, 1u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + 512 + adv, idesc_pv, 1u);
+        }
+        umma_commit(bar);
+      }
+      __syncwarp();
+    }
+  }
+  if (ok) wait_mma();
+  cp_async_wait_all();   // (left early: the copies land before the shared memory is released)
+  tc_fence_after();
+  red[hf * 128 + r] = lsum;
+  ok = __syncthreads_and(ok);
+  if (ok) {
+    const float inv = 1.0f / (red[r] + red[128 + r]);
+    uint32_t a[32];
+    tmem_ld16(tlane + A1_COL_O + 32 * hf, a);
+    tmem_ld16(tlane + A1_COL_O + 32 * hf + 16, a + 16);
+    tmem_ld_wait();
+    if (q0 + r < s) {
+      const int64_t at = ((int64_t)b * s + q0 + r) * p.out_ld + (int64_t)h * 64 + 32 * hf;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(a[8 * i + e]) * inv;
+        if (p.bf.hi) {
+          *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+          if (p.bf.lo)
+            *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) = make_uint4(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])),
+                                                                          pack_bf16(bf16_lo(v[4]), bf16_lo(v[5])), pack_bf16(bf16_lo(v[6]), bf16_lo(v[7])));
+        } else {
+          *reinterpret_cast<float4 *>(p.out + at + 8 * i) = make_float4(v[0], v[1], v[2], v[3]);
+          *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        }
+      }
+    }
+  } else if (tid == 0) {
+    atomicCAS(status, 0, DEV_WAIT_TIMEOUT);
+    status[1] = 10;
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(A1_COLS) : "memory");
+  }
+}
+
 template <int NQ, int NE, bool PLAIN = false>
 static int launch_at(caten_b200_ctx *ctx, AttnArgs a, float qscale) {
   using Lay = AtLayout<NQ, NE>;
@@ -530,6 +811,17 @@ int launch_attention_tc_ex(caten_b200_ctx *ctx, const AttnArgs &args, float qsca
   return launch_at<1, 1>(ctx, a, qscale);
 }
 
+// Which of GPT-2's steps go without the pass that makes tiles: those of one or two query tiles where the CTAs, one per tile and
+// head, fill the GPU, or where the few blocks of keys that each walks through take less than a kernel and its hand-off.  us,
+// tiles / direct: 25 heads, 64 sequences, 900 positions before 16 tokens 459 / 307 (append and a kernel like this one: 326), 16 sequences, none before 64 tokens 23 / 16, 1
+// sequence, 480 before 64 tokens 21 / 29, 4 sequences, 900 before 64, keys from HBM, 7 less in a step of GPT-2 XL; two tiles: 64 sequences, 480 before 256 627 / 517, 8 sequences 85 / 92, none before 45 / 35.
+static bool at_direct(int sm, int64_t heads, int64_t s, int64_t n) {
+  const int64_t blocks = (n + s + AT_K - 1) / AT_K;
+  const bool some = 16 * heads >= 5 * sm;   // 47 heads on 148 SMs
+  if (s <= AT_Q) return heads >= sm || blocks <= (some ? 4 : 2);
+  return s <= 2 * AT_Q && (2 * heads >= 5 * sm || blocks <= (some ? 8 : 3));
+}
+
 // the step's keys and values are appended to the cache here
 int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc, float *out, int64_t B, int64_t s,
                         int64_t n, int64_t H, int64_t T, BfOut bf) {
@@ -544,6 +836,13 @@ int launch_attention_tc(caten_b200_ctx *ctx, const float *qkv, float *kc, float 
   a.out = out; a.bf = bf; a.out_ld = H * 64;
   a.B = (int)B; a.s = (int)s; a.n = (int)n; a.H = a.G = (int)H;
   a.D = a.Dp = a.E = a.Ep = 64;
+  if (at_direct(ctx->sm_count, B * H, s, n)) {
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_Q >> 4) << 24);   // fp32 accumulate, bf16 x bf16, M = 128
+    CB_CUDA(ctx, cudaFuncSetAttribute(attn_direct_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A1_SMEM));
+    launch_k(ctx, attn_direct_tc_kernel, dim3((unsigned)H, (unsigned)B, (unsigned)((s + AT_Q - 1) / AT_Q)), dim3(256), A1_SMEM, a, 0.125f, ctx->d_status, idesc);
+    CB_LAUNCH_CHECK(ctx, "attn_direct_tc_kernel");
+    return 0;
+  }
   return launch_at<1, 1, true>(ctx, a, 0.125f);
 }
 

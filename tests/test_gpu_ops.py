@@ -526,6 +526,25 @@ def test_attention_prefill_tensor_cores(rt, oracle, B, H, T, s, n):
     np.testing.assert_array_equal(dv.numpy()[:, :, :n + s], _to_gpu_cache(vc)[:, :, :n + s])
 
 
+@pytest.mark.parametrize("B,H,T,s,n", [(1, 1, 128, 128, 0), (1, 2, 130, 63, 1), (2, 50, 300, 2, 130), (4, 25, 330, 65, 191), (4, 25, 400, 128, 200), (2, 48, 200, 64, 64),
+                                       (1, 2, 160, 129, 0), (2, 25, 400, 130, 64), (2, 25, 512, 256, 200), (10, 40, 700, 255, 400)])
+def test_attention_of_few_tokens_without_a_pass_of_tiles(rt, B, H, T, s, n):
+    """One and two query tiles whose CTAs split the keys themselves: steps that begin inside, at and behind a block of 64 keys."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator().manual_seed(s + n)
+    k, v = (torch.randn(B, H, n + s, 64, generator=g) for _ in range(2))
+    q = torch.randn(B, H, s, 64, generator=g)
+    rows = torch.cat([a.transpose(1, 2).reshape(B * s, H * 64) for a in (q, k[:, :, n:], v[:, :, n:])], 1)
+    want = torch.nn.functional.scaled_dot_product_attention(q, k, v, attn_mask=torch.ones(s, n + s, dtype=torch.bool).tril(n))
+    end = torch.full((B, H, T - n, 64), float("nan"))   # (what is past the context must not leak in, and stays)
+    kc, vc = (rt.transfer_from_array(torch.cat([a[:, :, :n], end], 2).numpy()) for a in (k, v))
+    got = rt.attention(rt.transfer_from_array(rows.numpy()), kc, vc, B, s, n, precision=L.PREC_BF16X3).numpy()
+    np.testing.assert_allclose(got, want.transpose(1, 2).reshape(B * s, H * 64).numpy(), atol=2e-5, rtol=2e-5)
+    for cache, a in ((kc, k), (vc, v)):
+        np.testing.assert_array_equal(cache.numpy()[:, :, :n + s], a.numpy())
+        assert np.isnan(cache.numpy()[:, :, n + s:]).all()
+
+
 @pytest.mark.parametrize("B,H,T,s,n,grow", [(2, 2, 600, 300, 0, 1.0), (1, 2, 700, 257, 391, 1.02), (1, 1, 512, 512, 0, 1.01)])
 def test_attention_prefill_tensor_cores_moving_maximum(rt, oracle, B, H, T, s, n, grow):
     """Large scores whose maximum keeps rising along the keys (key j scaled by grow^j on top of
