@@ -603,7 +603,14 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
 // 1600 x 6400: 777 rows 65 here 87, 1024 rows 69 here 90, 1665 rows 113 here 106; 1600 x 1600: 1665 rows 38 here 32).
 bool gemm_dense_applies(const caten_b200_ctx *ctx, int wt, int64_t M, int64_t N, int64_t K, int nsplit) {
   if (!ctx->dense_gemm || N % 4 || K % GD_BK || K < GD_BK) return false;
-  if ((wt == CATEN_B200_BF16 && nsplit == 1) || M >= GD_EXPAND_ROWS) return true;
+  if (wt == CATEN_B200_BF16 && nsplit == 1) return true;
+  if (M >= GD_EXPAND_ROWS) {
+    // .. except, in split bf16, long rows of packed or fp16 weights where equal shares of k of the other kernel's tiles of 128 x 256
+    // about fill its one wave (us there / here, Q4_0: 768 x 3072 2048 rows 37 / 45, 1024 x 4096 1665 rows 51 / 58, 2048 rows 54 / 61, 1280 x 5120
+    // 1665 rows 62 / 75, but 2048 rows, which half fill it, 92 / 78; fp32 weights cost it more: 1024 x 4096 2048 rows 70 / 63)
+    const int64_t tiles = (M + GD_BN - 1) / GD_BN * ((N + GD_BM - 1) / GD_BM), sm = ctx->sm_count;
+    return nsplit != 3 || wt == CATEN_B200_BF16 || wt == CATEN_B200_F32 || wt == WT_F32_T || K <= 2 * N || 2 * tiles > sm || 4 * (sm / tiles * tiles) < 3 * sm;
+  }
   return M >= 1024 && (M + GD_BN - 1) / GD_BN * ((N + GD_BM - 1) / GD_BM) >= ctx->sm_count;
 }
 

@@ -293,7 +293,8 @@ def test_gemm_tensor_core(rt, oracle, wtype, M, N, K, prec):
 # thousands of rows: the weights are expanded to bf16 once and both operands reach the tensor cores through TMA
 # (persistent kernel, two accumulators).  Ragged rows and features, every weight format, both precisions.
 MANY_ROW_CASES = [("q4_0", 2048, 2560, 1600), ("q4_0", 2000, 2500, 768), ("q8_0", 1100, 4800, 128), ("q5_1", 1500, 3200, 256),
-                  ("f32", 1024, 4864, 192), ("f16", 4100, 1200, 64)]
+                  ("f32", 1024, 4864, 192), ("f16", 4100, 1200, 64),
+                  ("q4_0", 1665, 260, 1088), ("q4_0", 1537, 2560, 5184)]   # (long rows: the converting GEMM)
 
 
 @pytest.mark.parametrize("wtype,M,N,K", MANY_ROW_CASES)
