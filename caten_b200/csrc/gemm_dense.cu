@@ -552,9 +552,23 @@ struct GdPlan {
   bool pair;
 };
 
+// Bytes of staging of the epilogue warps that have columns to store, and stages of a launch.  A CTA with one item leaves room on its
+// SM for one of the next linear, which starts to load its weights meanwhile; a CTA that walks over items takes what there is: 1 KB
+// slack + 1 KB barriers + stages + 32 KB of staging fit 227 KB.
+static size_t gd_staging(int bn) { return 2048 * 4 * (size_t)(bn < 64 ? bn / 16 : 4); }
+static int gd_stages(int sm, int64_t M, int64_t items, int bn, int cps, size_t stage) {
+  int stages = (int)((items <= sm && M <= GD_SPLIT_ROWS ? 108 * 1024 - gd_staging(bn) : GD_STAGE_BYTES) / stage);
+  if (stages > 8) stages = 8;
+  if (stages > cps) stages = cps;
+  return stages < 2 ? 2 : stages;
+}
+
 // The cut with the shortest expected time.  A CTA's stage takes as long as its MMAs (bn / 2 cycles each, at least 40) or as
 // long as its operands need from L2 (about 60 bytes a cycle and SM with every SM at work; measured: 128 x 256 tiles of
-// plain bf16 run at 0.85 of the burst rate of the tensor cores, 48 KB in 870 cycles).  Wide tiles read least, narrow ones
+// plain bf16 run at 0.85 of the burst rate of the tensor cores, 48 KB in 870 cycles); a CTA that goes through all of k by itself gets no
+// more than its stages in flight every 2700 cycles (2048 x 2048, 5 rows: 16 CTAs with five stages of 18 KB 12.7 us, seven shares of k and
+// the pass that sums them 8.5, the converting kernel 9.8; up to 32 rows and above 512 this predicts the better cut, between them
+// the plain estimate does: 3072 x 1024, 256 rows 10.2, 13.7 with it).  Wide tiles read least, narrow ones
 // leave no SM without work and the last wave short; shares of k pay for a pass over their partial sums.  A pair of CTAs on
 // 256 features loads 32 KB per CTA where a CTA alone loads 48, and has more stages in flight; it starts later (both CTAs
 // meet twice), and narrower tiles gain nothing from it (1665 rows, split bf16, 6400 x 1600, 224 rows wide: 91 us alone, 97).  us a call with the conversion of x, alone -> pair: 8192 rows, plain bf16,
@@ -574,7 +588,9 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
       if (splits > 1 && (!can_split || tiles * s > sm || cps * bk < 256)) break;
       if (s != splits) continue;
       const int64_t items = tiles * s;
-      const double busy = items < sm ? (double)items : (double)sm, rate = 60.0 * sm / busy < 100.0 ? 60.0 * sm / busy : 100.0;
+      const double busy = items < sm ? (double)items : (double)sm;
+      const double most = splits == 1 && (M <= 32 || M > GD_SPLIT_ROWS) ? bytes * gd_stages(sm, M, items, bn, cps, (size_t)bytes) / 2700.0 : 100.0;
+      const double rate = 60.0 * sm / busy < most ? 60.0 * sm / busy : most;
       const double stage = mma > bytes / rate ? mma : bytes / rate, body = cps * stage;
       const int64_t waves = (items + sm - 1) / sm;
       double t = 1500 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
@@ -694,14 +710,8 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
   }
   const size_t stage = (size_t)(GD_BM * (wlo ? 2 : 1) + (p.pair ? p.bn / 2 : p.bn) * parts) * (size_t)bk * 2;
   const int workers = p.pair ? ctx->sm_count / 2 : ctx->sm_count, busy = items < workers ? (int)items : workers, grid = p.pair ? 2 * busy : busy;
-  // A CTA with one item leaves room on its SM for one of the next linear, which starts to load its weights meanwhile; a
-  // CTA that walks over items takes what there is: 1 KB slack + 1 KB barriers + stages + 32 KB of staging fit 227 KB.
-  const size_t staging = 2048 * 4 * (size_t)(p.bn < 64 ? p.bn / 16 : 4);   // of the epilogue warps that have columns to store
-  int stages = (int)((items <= ctx->sm_count && M <= GD_SPLIT_ROWS ? 108 * 1024 - staging : GD_STAGE_BYTES) / stage);
-  if (stages > 8) stages = 8;
-  if (stages > p.cps) stages = p.cps;
-  if (stages < 2) stages = 2;
-  a.stages = stages;
+  const size_t staging = gd_staging(p.bn);
+  const int stages = a.stages = gd_stages(ctx->sm_count, M, items, p.bn, p.cps, stage);
   a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)((p.pair ? 2 * GD_BM : GD_BM) >> 4) << 24);
   a.tmem_cols = p.pair ? 512 : 32;   // (a pair: all, so that its accumulators have the same columns in both CTAs)
   while (a.tmem_cols < (uint32_t)(p.bn * (items > busy ? 2 : 1))) a.tmem_cols *= 2;
