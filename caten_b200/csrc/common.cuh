@@ -133,10 +133,9 @@ struct caten_b200_ctx {
   void *encode_tiled = nullptr;  // cuTensorMapEncodeTiled, resolved at init
   int64_t launches = 0;
   // split-K partial tiles of the converting GEMM: reduced by a second kernel through global scratch, or inside a thread-block
-  // cluster through distributed shared memory.  By default (-1) the cluster for up to 128 rows where the consumer cannot sum
-  // the tiles itself (GPT-2 medium, 64 sequences: 1345 us a step with the second kernel, 1327 us so; GPT-2 XL, 256 sequences:
-  // 0.7 % slower in a cluster).  CATEN_B200_SPLITK_CLUSTER=0: never; 1: every split-K launch; 2: every launch whose epilogue
-  // cannot be handed to the consuming kernel
+  // cluster through distributed shared memory.  -1: the cluster for linears of few rows with an activation or a bf16 output (run_tc
+  // says how few); CATEN_B200_SPLITK_CLUSTER=0: never; 1: every split-K launch; 2: every launch whose epilogue cannot be handed
+  // to the consuming kernel
   int splitk_cluster = -1;
   int attn_tc = 1;           // prefill attention of a tensor-core model on the tensor cores (CATEN_B200_ATTN_TC=0: SIMT kernel)
   bool use_pdl = true;       // programmatic dependent launch between consecutive kernels (CATEN_B200_PDL=0 turns it off)

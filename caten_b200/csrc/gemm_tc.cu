@@ -886,12 +886,15 @@ static int run_tc(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *x,
   const uintptr_t align_bits = (uintptr_t)bias | (uintptr_t)res | (uintptr_t)y | (uintptr_t)ybf.hi | (uintptr_t)ybf.lo;
   if (gemm_dense_applies(ctx, wt, M, N, K, nsplit) && !(align_bits & 15)) return launch_gemm_dense(ctx, wt, ws, x, xhi_pre, xlo_pre, bias, res, act, y, ybf, M, N, K, nsplit, grp, defer);
   TcPlan p;
-  // reduce inside a cluster: always (mode 1), when this launch needs its own epilogue (mode 2), or, with few rows, when
-  // no consumer could have done it
+  // Reduce inside a cluster: always (mode 1), when this launch needs its own epilogue (mode 2), or, by default, for linears with an
+  // activation or a bf16 output of up to 64 rows, up to 16 only with short rows of weights.  us a step at 100 positions, second kernel / cluster:
+  // GPT-2 medium Q4_0 16 sequences 840 / 856, 32 931 / 903, 64 1120 / 1102, 96 1391 / 1405; XL Q4_0 32 2391 / 2335, 96 3784 / 3874; small fp32
+  // weights 5 579 / 524, 64 685 / 662, 128 892 / 906; small Q4_0 8 385 / 376, 48 494 / 482, 64 503 / 507, 128 704 / 723; small Q8_0 8 451 / 422;
+  // medium Q8_0 8 896 / 920, f16 8 861 / 890; large Q4_0 8 1339 / 1363
   const bool can_defer = defer && act == CATEN_B200_ACT_NONE && !ybf.hi && N % 4 == 0 && grp.plain_output() && grp.group_rows % TC_BM == 0;
   const bool own_epilogue = !can_defer;
   const bool want_cluster = ctx->splitk_cluster == 1 || (ctx->splitk_cluster == 2 && own_epilogue) ||
-                            (ctx->splitk_cluster < 0 && M <= 128 && (act != CATEN_B200_ACT_NONE || ybf.hi));
+                            (ctx->splitk_cluster < 0 && M <= 64 && (M > 16 || K < 1024) && (act != CATEN_B200_ACT_NONE || ybf.hi));
   if (int rc = tc_plan(ctx, "gemm_tc", M, N, K, nsplit, want_cluster ? 8 : 32, &p, grp.group_rows)) return rc;  // 8 = portable cluster size
   uint8_t *xhi, *xlo;
   if (xhi_pre) {
