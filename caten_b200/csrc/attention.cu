@@ -27,6 +27,8 @@ constexpr float kInvLn2 = 1.0f / 0.6931472f;  // (/ (log 2)) in single float, ap
 #endif
 constexpr int ATT_PARTS = 8;
 __host__ __device__ inline int att_parts(int64_t t, int most) { return t >= 96 ? most : 1; }
+// where part `rank` of `parts`, a power of two, begins
+__device__ __forceinline__ int att_cut(int t, int rank, int parts) { return (int)(((long long)t * rank) >> (__ffs(parts) - 1)); }
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc,
@@ -51,8 +53,8 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
     int np = d_n ? *d_n : n;
     np = np < 0 ? 0 : (np > T - 1 ? T - 1 : np);
     const int share = SPLIT ? att_parts(np + 1, cluster) : 1;
-    const int p0 = SPLIT ? (int)((long long)np * rank / share) : 0;
-    const long long stream_bytes = rank < share ? 256ll * ((SPLIT ? (int)((long long)np * (rank + 1) / share) : np) - p0) : 0;
+    const int p0 = SPLIT ? att_cut(np, rank, share) : 0;
+    const long long stream_bytes = rank < share ? 256ll * ((SPLIT ? att_cut(np, rank + 1, share) : np) - p0) : 0;
     const int pieces = (int)((stream_bytes + PIECE - 1) / PIECE);
     if (tid < 2 * pieces && ((long long)b * H + h + 1) * 2 * 256ll * np <= prefetch_bytes) {
       const int which = tid >= pieces ? 1 : 0, i = tid - which * pieces;
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
     }
     return;
   }
-  const int j_first = SPLIT ? (int)((long long)t * rank / parts) : 0, j_end = SPLIT ? (int)((long long)t * (rank + 1) / parts) : t;
+  const int j_first = SPLIT ? att_cut(t, rank, parts) : 0, j_end = SPLIT ? att_cut(t, rank + 1, parts) : t;
   const bool newest = !SPLIT || rank == parts - 1;   // position n is in the last part, which is never empty
   __shared__ float join[SPLIT ? ATT_PARTS * 66 : 1];  // of the first CTA: each part's maximum, sum and 64 outputs
   const float *row = qkv + (int64_t)b * 3 * d;
