@@ -348,8 +348,28 @@ __device__ __forceinline__ float gelu_ref(float x) {
   return l * r;
 }
 
+// x / e for e >= 1 (infinity included), without the branch to a subroutine that an IEEE division carries: in the unrolled loops
+// of an epilogue that branch keeps the elements' chains from overlapping.  The quotient of an approximate reciprocal, corrected
+// once by its own remainder (the bound on e and the test of q keep infinities out of that); every quotient tried is the rounded one.
+__device__ __forceinline__ float div_by_sum(float x, float e) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e));
+  const float q = x * r;
+  const float c = fmaf(r, fmaf(-fminf(e, 0x1p120f), q, x), q);
+  return fabsf(q) < INFINITY ? c : q;
+}
+// The same function as x / (1 + exp(-2 sqrt(2 / pi) (x + 0.044715 x^3))): for the epilogues of the tensor-core kernels.  Error
+// against 64 bits (2-norm) over 4 M normal inputs of deviation 0.3, 1 and 3: 4.3e-8, 4.2e-8, 3.3e-8; of the composition above
+// 5.2e-8, 4.8e-8, 3.6e-8.  c_fc of 1665 rows, 4096 x 1024, plain bf16: 25.7 us with the composition, 20.5 with this.
+__device__ __forceinline__ float gelu_fast(float x) {
+  const float c0 = -2.302208198f, c1 = -2.302208198f * 0.044715f;   // -2 sqrt(2 / pi) / ln 2
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * fmaf(x * x, c1, c0)));
+  return div_by_sum(x, 1.0f + e);
+}
+
 __host__ __device__ constexpr bool act_is_glu(int act) { return act == CATEN_B200_ACT_RELU_GLU || act == CATEN_B200_ACT_SILU_GLU; }
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return div_by_sum(z, 1.0f + expf(-z)); }
 // the gated activations
 __device__ __forceinline__ float glu(int act, float gate, float up) {
   return (act == CATEN_B200_ACT_SILU_GLU ? silu(gate) : (gate > 0.0f ? gate : 0.0f)) * up;

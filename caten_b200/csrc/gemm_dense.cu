@@ -35,6 +35,7 @@ constexpr int GD_BK = 64;    // k granularity of the operands (K % 64 == 0)
 template <int NSPLIT> struct GdStage { static constexpr int BK = NSPLIT == 3 ? 32 : 64; };
 constexpr int GD_EPI_WARPS = 16;
 constexpr int GD_THREADS = (2 + GD_EPI_WARPS) * 32;
+constexpr int GD_REGS = 72;  // a thread: what the epilogue would like beyond these is room that the next launch starts in
 
 struct GdArgs {
   const float *bias, *res;
@@ -169,8 +170,18 @@ __global__ void __launch_bounds__(256) xsplit_kernel(const float *__restrict__ x
 // shared-memory tile of the warp and comes back transposed: a lane then owns four consecutive features of
 // four rows and moves 16 bytes per instruction (bias, activation, residual and the optional split-bf16
 // output are applied on that side).
+// The residual of the block, rr, is asked for beforehand (gd_load_res): loads placed between the stores would each wait for
+// the one before, since y may be the residual's own memory.  1665 rows, 1024 x 1024, plain bf16: 14.1 us, 10.6 with them ahead.
+__device__ __forceinline__ void gd_load_res(const GdArgs &a, float4 *rr, int lane, int64_t o0, bool o_ok, int m_first, int m_end) {
+  if (!a.res) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int64_t m = (int64_t)m_first + 4 * j + (lane >> 3);
+    if (o_ok && m < m_end) rr[j] = *reinterpret_cast<const float4 *>(a.res + m * a.ldy + o0);
+  }
+}
 template <int ACT, bool EXPERTS>
-__device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg, int lane, float4 bias4, int64_t o0, bool o_ok, int m_first, int m_end) {
+__device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg, const float4 *rr, int lane, float4 bias4, int64_t o0, bool o_ok, int m_first, int m_end) {
   const int fg = lane & 7, tr = lane >> 3;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -198,11 +209,11 @@ __device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg
     const int64_t at = m * a.ldy + o0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      if (ACT == CATEN_B200_ACT_GELU) v[e] = gelu_ref(v[e]);
+      if (ACT == CATEN_B200_ACT_GELU) v[e] = gelu_fast(v[e]);
       if (ACT == CATEN_B200_ACT_RELU) v[e] = v[e] > 0.0f ? v[e] : 0.0f;
     }
     if (a.res) {
-      const float4 r = *reinterpret_cast<const float4 *>(a.res + at);
+      const float4 r = rr[j];
       v[0] = r.x + v[0]; v[1] = r.y + v[1]; v[2] = r.z + v[2]; v[3] = r.w + v[3];
     }
     if (a.yhi) {
@@ -237,7 +248,7 @@ __device__ __forceinline__ uint64_t gd_desc(uint32_t saddr) {
 }
 
 template <int NSPLIT, bool EXPERTS, bool WLO, bool PAIR>
-__global__ void __launch_bounds__(GD_THREADS, 1)
+__global__ void __maxnreg__(GD_REGS)
 gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_constant__ CUtensorMap tw_lo,
                   const __grid_constant__ CUtensorMap tx_hi, const __grid_constant__ CUtensorMap tx_lo, const GdArgs a) {
   constexpr int BK = GdStage<NSPLIT>::BK;
@@ -466,6 +477,8 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       const int64_t oc = o0 - t.shift;   // output column
       float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f);
       if (a.bias && o_ok) bias4 = *reinterpret_cast<const float4 *>(a.bias + o0);
+      float4 rr[4];
+      if (16 * turn < BN) gd_load_res(a, rr, lane, oc, o_ok, t.m0 + 16 * turn, t.m_end);
       int got = 0;
       if (lane == 0) {
         got = mbar_wait(acc_full(b), ((uint32_t)it >> 1) & 1u, abort_flag) ? 1 : 0;
@@ -494,11 +507,12 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
         for (int i = 0; i < 16; ++i) stg[i * 32 + lane] = __uint_as_float(r[i]);
         __syncwarp();
         const int m_first = t.m0 + c;
-        if (a.act == CATEN_B200_ACT_SILU_GLU) gd_store_block<CATEN_B200_ACT_SILU_GLU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
-        else if (a.act == CATEN_B200_ACT_RELU_GLU) gd_store_block<CATEN_B200_ACT_RELU_GLU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
-        else if (!EXPERTS && a.act == CATEN_B200_ACT_GELU) gd_store_block<CATEN_B200_ACT_GELU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
-        else if (!EXPERTS && a.act == CATEN_B200_ACT_RELU) gd_store_block<CATEN_B200_ACT_RELU, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
-        else gd_store_block<CATEN_B200_ACT_NONE, EXPERTS>(a, stg, lane, bias4, oc, o_ok, m_first, t.m_end);
+        if (a.act == CATEN_B200_ACT_SILU_GLU) gd_store_block<CATEN_B200_ACT_SILU_GLU, EXPERTS>(a, stg, rr, lane, bias4, oc, o_ok, m_first, t.m_end);
+        else if (a.act == CATEN_B200_ACT_RELU_GLU) gd_store_block<CATEN_B200_ACT_RELU_GLU, EXPERTS>(a, stg, rr, lane, bias4, oc, o_ok, m_first, t.m_end);
+        else if (!EXPERTS && a.act == CATEN_B200_ACT_GELU) gd_store_block<CATEN_B200_ACT_GELU, EXPERTS>(a, stg, rr, lane, bias4, oc, o_ok, m_first, t.m_end);
+        else if (!EXPERTS && a.act == CATEN_B200_ACT_RELU) gd_store_block<CATEN_B200_ACT_RELU, EXPERTS>(a, stg, rr, lane, bias4, oc, o_ok, m_first, t.m_end);
+        else gd_store_block<CATEN_B200_ACT_NONE, EXPERTS>(a, stg, rr, lane, bias4, oc, o_ok, m_first, t.m_end);
+        if (c + 4 * GD_EPI_WARPS < BN) gd_load_res(a, rr, lane, oc, o_ok, m_first + 4 * GD_EPI_WARPS, t.m_end);
       }
       tc_fence_before();
       __syncwarp();

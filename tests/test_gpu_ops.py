@@ -643,6 +643,27 @@ def test_large_copies_through_the_pinned_bounce_buffers(rt, oracle):
     w.close()
 
 
+@pytest.mark.parametrize("act", [L.ACT_GELU, L.ACT_NONE])
+@pytest.mark.parametrize("M,N,K,offset", [(5, 128, 512, 0), (40, 260, 768, 0), (40, 257, 768, 0), (40, 260, 768, 1), (200, 388, 1024, 0), (300, 132, 512, 2), (1601, 260, 192, 0)])
+def test_tensor_core_epilogues_in_fours_and_one_by_one(rt, act, M, N, K, offset):
+    """Bias, activation and residual behind every way a sum can end: by a cluster, by the second kernel and in the tile's own
+    CTA, with features in aligned fours or not (a width that is no multiple of four, a residual that starts between), large and
+    small arguments of GELU.  Split-bf16 products are within 2^-16 of sum |x w|; the activation's slope is at most 1.13."""
+    rng = np.random.Generator(np.random.PCG64(M + N + K + offset))
+    W = rng.standard_normal((N, K), dtype=np.float32) * np.float32(K ** -0.5)
+    x = rng.standard_normal((M, K), dtype=np.float32) * rng.choice(np.float32([0.05, 1.0, 6.0]), (M, 1))
+    bias, res = rng.standard_normal(N, dtype=np.float32), rng.standard_normal((M, N), dtype=np.float32)
+    w = rt.upload_weight(W)
+    dres = rt.transfer_from_array(np.concatenate([np.zeros(offset, np.float32), res.ravel()])).view(offset, (M, N))
+    got = rt.linear(w, rt.transfer_from_array(x), rt.transfer_from_array(bias), dres, act, L.PREC_BF16X3).numpy()
+    z = x.astype(np.float64) @ W.T.astype(np.float64) + bias
+    with np.errstate(over="ignore"):
+        want = z / (1 + np.exp(-2 * np.sqrt(2 / np.pi) * (z + 0.044715 * z ** 3))) if act == L.ACT_GELU else z
+    bound = 2.0 ** -15 * (np.abs(x).astype(np.float64) @ np.abs(W.T).astype(np.float64)) + 1e-6 * (np.abs(z) + np.abs(res))
+    assert (np.abs(got - (want + res)) <= bound).all()
+    w.close()
+
+
 def test_gemm_split_k_cluster_reduction_matches_global_reduction(oracle, monkeypatch):
     """CATEN_B200_SPLITK_CLUSTER=1 reduces split-K partial tiles inside a thread-block cluster
     (distributed shared memory) instead of a second kernel: same splits order, same epilogue."""
