@@ -368,6 +368,12 @@ __device__ __forceinline__ float gelu_fast(float x) {
   return div_by_sum(x, 1.0f + e);
 }
 
+__device__ __forceinline__ float act_fast(float v, int act) {
+  if (act == CATEN_B200_ACT_GELU) return gelu_fast(v);
+  if (act == CATEN_B200_ACT_RELU) return v > 0.0f ? v : 0.0f;
+  return v;
+}
+
 __host__ __device__ constexpr bool act_is_glu(int act) { return act == CATEN_B200_ACT_RELU_GLU || act == CATEN_B200_ACT_SILU_GLU; }
 __device__ __forceinline__ float silu(float z) { return div_by_sum(z, 1.0f + expf(-z)); }
 // the gated activations

@@ -348,11 +348,6 @@ __device__ __forceinline__ void store_glu4(int act, const float *r, float4 b4, c
   }
 }
 
-__device__ __forceinline__ float epi_act(float v, int act) {
-  if (act == CATEN_B200_ACT_GELU) return gelu_fast(v);
-  if (act == CATEN_B200_ACT_RELU) return v > 0.0f ? v : 0.0f;
-  return v;
-}
 // Four consecutive features o .. o + 3 of a row, summed: bias, activation, residual, output.  at: the first one's place in y.
 // VEC: all four exist and every pointer is aligned for them together (tc_vec4), bias and residual (b4, r4) were asked for beforehand.
 template <bool VEC>
@@ -363,7 +358,7 @@ __device__ __forceinline__ void store_out4(int act, float *v, float4 b4, float4 
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (bias) v[e] = v[e] + b[e];
-      v[e] = epi_act(v[e], act);
+      v[e] = act_fast(v[e], act);
       if (res) v[e] = r[e] + v[e];
     }
     if (yhi) {
@@ -379,7 +374,7 @@ __device__ __forceinline__ void store_out4(int act, float *v, float4 b4, float4 
     if (o + e < N) {
       float t = v[e];
       if (bias) t = t + bias[o + e];
-      t = epi_act(t, act);
+      t = act_fast(t, act);
       if (res) t = res[at + e] + t;
       if (yhi) {
         const __nv_bfloat16 h = __float2bfloat16_rn(t);

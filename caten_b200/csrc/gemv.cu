@@ -8,9 +8,6 @@
 
 namespace cb {
 
-// LayerNorm of the rows of x where they lie in shared memory (float4 i of row m at at(m, i)): every CTA does it for itself,
-// which costs a linear about 0.6 us where a kernel of its own, one CTA and one more hand-off, cost 1.8 to 2.9.  gamma and beta
-// (2 x K floats of shared memory) are staged before the wait for x.  The order of a row's statistics is one warp's.
 __device__ __forceinline__ void gemv_stage_norm(const GemvNorm &n, float *gb, int K) {
   if (!n.g) return;
   for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
@@ -19,35 +16,97 @@ __device__ __forceinline__ void gemv_stage_norm(const GemvNorm &n, float *gb, in
   }
 }
 
-template <class At>
-__device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const float *gb, int M, int K, At at) {
-  if (!n.g) return;
-  __shared__ float stat[4][2];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K4 = K / 4;
-  for (int m = warp; m < M; m += blockDim.x >> 5) {
-    const float invd = 1.0f / (float)K;
+// The rows of x, M x K4 float4 one after the other, on their way to shared memory: put(f, v, ok) takes float4 f (ok: it exists;
+// the whole warp calls it).  All of a thread's loads are under way before it uses the first.
+// With a norm every CTA normalises the rows for itself, which costs a linear less than a kernel of its own would (one more
+// hand-off).  gamma and beta (2 x K floats of shared memory) are staged before the wait for x.  A row is in the threads'
+// registers meanwhile: each warp has the mean and the squared deviations of its own part, and the parts are joined behind one
+// barrier.  (By one warp a row, from shared memory, GPT-2 XL's row took 1.3 to 1.8 us of a linear's 6; so, and with the sums of a row's parts by 8 to 32 lanes a row
+// instead of a warp for several, a step with 640 positions went from 1370 to 1258 us.)
+constexpr int GEMV_NORM_K = 2400;   // the longest row that is normalised: three float4 of each of at least 200 threads (launch_blocked's CTAs have 224)
+// MOST: M is at most that.  ASYNC: put is the plain copy to `to`, rows without a norm go there without passing through registers.
+template <int MOST, bool ASYNC, class Put>
+__device__ __forceinline__ void gemv_rows_to_shared(const GemvNorm &n, const float *gb, const float *x, int M, int K4, Put put, float *to = nullptr) {
+  const float4 *x4 = reinterpret_cast<const float4 *>(x);
+  const int tid = threadIdx.x, T = blockDim.x;
+  if (!n.g) {
+    const int total = M * K4;
+    if (ASYNC) {
+      for (int f = tid; f < total; f += T) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 4 * f)), "l"(x4 + f) : "memory");
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      return;
+    }
+    for (int f0 = 0; f0 < total; f0 += 8 * T) {
+      float4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int f = f0 + u * T + tid;
+        v[u] = f < total ? x4[f] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (f0 + u * T >= total) break;   // (the same for the whole CTA)
+        put(f0 + u * T + tid, v[u], f0 + u * T + tid < total);
+      }
+    }
+    return;
+  }
+  __shared__ float4 stat[2][16];   // of a warp's part: sum, squared deviations from its mean, mean, elements
+  const int warp = tid >> 5, lane = tid & 31, nw = T >> 5;
+  const float invd = 1.0f / (float)(K4 * 4);
+  int have = 0;
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    const int left = K4 - (warp * 32 + u * T);
+    have += left <= 0 ? 0 : left < 32 ? left : 32;
+  }
+  const float cnt = (float)(4 * have), inv = have ? 1.0f / cnt : 0.0f;
+  float4 v[3], nx[3];
+  auto load = [&](int m, float4 *d) {
+#pragma unroll
+    for (int u = 0; u < 3; ++u) d[u] = m < M && u * T + tid < K4 ? x4[m * K4 + u * T + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  load(0, v);
+  for (int m = 0; m < M; ++m) {
+    if (MOST > 1) load(m + 1, nx);
     float sum = 0.0f, sq = 0.0f;
-    for (int i = lane; i < K4; i += 32) {
-      const float4 v = *at(m, i);
-      sum += (v.x + v.y) + (v.z + v.w);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) sum += (v[u].x + v[u].y) + (v[u].z + v[u].w);
+    sum = warp_sum(sum);
+    const float mw = sum * inv;
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (u * T + tid < K4) {
+        const float a = v[u].x - mw, b = v[u].y - mw, c = v[u].z - mw, d = v[u].w - mw;
+        sq += (a * a + b * b) + (c * c + d * d);
+      }
+    sq = warp_sum(sq);
+    if (lane == 0) stat[m & 1][warp] = make_float4(sum, sq, mw, cnt);
+    __syncthreads();
+    float all = 0.0f, dev = 0.0f;
+    for (int w = 0; w < nw; ++w) all += stat[m & 1][w].x;
+    const float u = all * invd;
+    for (int w = 0; w < nw; ++w) {
+      const float4 s = stat[m & 1][w];
+      dev += s.y + s.w * ((s.z - u) * (s.z - u));
     }
-    const float u = warp_sum(sum) * invd;
-    for (int i = lane; i < K4; i += 32) {
-      const float4 v = *at(m, i);
-      const float x = v.x - u, y = v.y - u, z = v.z - u, w = v.w - u;
-      sq += (x * x + y * y) + (z * z + w * w);
+    const float rs = 1.0f / sqrtf(dev * invd + n.eps);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (q * T >= K4) break;
+      const int i = q * T + tid;
+      const bool ok = i < K4;
+      float4 y = v[q];
+      if (ok) {
+        const float4 gg = reinterpret_cast<const float4 *>(gb)[i], bb = reinterpret_cast<const float4 *>(gb)[K4 + i];
+        y = make_float4(((y.x - u) * rs) * gg.x + bb.x, ((y.y - u) * rs) * gg.y + bb.y, ((y.z - u) * rs) * gg.z + bb.z, ((y.w - u) * rs) * gg.w + bb.w);
+      }
+      put(m * K4 + i, y, ok);
     }
-    const float var = warp_sum(sq) * invd;
-    if (lane == 0) { stat[m][0] = u; stat[m][1] = 1.0f / sqrtf(var + n.eps); }
+    if (MOST == 1) break;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) v[q] = nx[q];
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < M * K4; i += blockDim.x) {
-    const int m = i / K4, j = i - m * K4;
-    const float u = stat[m][0], rs = stat[m][1];
-    const float4 v = *at(m, j), gg = reinterpret_cast<const float4 *>(gb)[j], bb = reinterpret_cast<const float4 *>(gb + K)[j];
-    *at(m, j) = make_float4(((v.x - u) * rs) * gg.x + bb.x, ((v.y - u) * rs) * gg.y + bb.y, ((v.z - u) * rs) * gg.z + bb.z, ((v.w - u) * rs) * gg.w + bb.w);
-  }
-  __syncthreads();
 }
 
 struct GemvArgs {
@@ -61,7 +120,7 @@ struct GemvArgs {
 };
 
 constexpr int GEMV_MAX_THREADS = 512;
-constexpr int GEMV_XPAD = 36;   // floats between the 32-wide blocks of x in shared memory: eight threads' 16-byte reads cover all banks
+constexpr int GEMV_XPAD = 36;   // floats between the 32-wide blocks of x in shared memory (eight threads' 16-byte reads cover all banks); [32]: the block's sum
 
 __device__ __forceinline__ uint4 ld_stream(const uint4 *p) { return __ldcs(p); }
 
@@ -86,7 +145,6 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
   const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
   const int rows_per_iter = G * RI;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
   const int64_t stride = (int64_t)gridDim.x * rows_per_iter;
 
   uint32_t qn[RI][W];
@@ -112,19 +170,28 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   load(base);
   gemv_stage_norm(a.norm, gb, nkb * 32);
   pdl_wait();
-  for (int i = tid; i < a.M * nkb * 8; i += blockDim.x)
-    *reinterpret_cast<float4 *>(xs + (i >> 3) * GEMV_XPAD + (i & 7) * 4) = reinterpret_cast<const float4 *>(a.x)[i];
-  // what the warp adds to its rows (lane i: its i-th) is asked for before their sums are formed
+  // lpr lanes (a power of two) add up one row; the first of them finishes it, having asked for bias and residual beforehand
+  int lpr = 32;
+  while (lpr * rows_per_iter > (int)blockDim.x) lpr >>= 1;
+  const int rr = tid / lpr, rl = tid - rr * lpr;
   auto addends = [&](int m, float *b, float *r) {
-    const int at = warp + lane * nwarps;
-    const bool has = at < rows_per_iter && base + at < a.N;
-    *b = has && a.bias ? a.bias[base + at] : 0.0f;
-    *r = has && a.res ? a.res[(int64_t)m * a.N + base + at] : 0.0f;
+    const bool has = rl == 0 && rr < rows_per_iter && base + rr < a.N;
+    *b = has && a.bias ? a.bias[base + rr] : 0.0f;
+    *r = has && a.res ? a.res[(int64_t)m * a.N + base + rr] : 0.0f;
   };
   float bz, rz;
   addends(0, &bz, &rz);
+  gemv_rows_to_shared<4, false>(a.norm, gb, a.x, a.M, nkb * 8, [&](int f, float4 v, bool ok) {
+    float *to = xs + (f >> 3) * GEMV_XPAD;
+    if (BLK::SUMS) {
+      float s = (v.x + v.y) + (v.z + v.w);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (ok && (f & 7) == 0) to[32] = s;
+    }
+    if (ok) *reinterpret_cast<float4 *>(to + (f & 7) * 4) = BLK::stage(v, f & 7);
+  });
   __syncthreads();
-  gemv_norm_rows(a.norm, gb, a.M, nkb * 32, [&](int m, int i) { return reinterpret_cast<float4 *>(xs + (m * nkb + (i >> 3)) * GEMV_XPAD + (i & 7) * 4); });
   BLK blk;
   int buf = 0;
   for (bool again = false; base < a.N; base += stride, again = true) {
@@ -155,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
           const float4 v = xp[i];
           xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
         }
-        blk.prep(xv);
+        blk.prep(xv, BLK::SUMS ? xs[(m * nkb + kb) * GEMV_XPAD + 32] : 0.0f);
       }
       float *rb = red + buf * rows_per_iter * nkb;
       if (active) {
@@ -168,20 +235,16 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
         }
       }
       __syncthreads();
-      int t = 0;
-      for (int r = warp; r < rows_per_iter; r += nwarps, ++t) {
-        const int64_t row = base + r;
-        if (row >= a.N) break;
-        float s = 0.0f;
-        for (int k = lane; k < nkb; k += 32) s += rb[r * nkb + k];
-        s = warp_sum(s);
-        const float bt = __shfl_sync(0xffffffffu, bz, t & 31), rt = __shfl_sync(0xffffffffu, rz, t & 31);
-        if (lane == 0) {
-          if (a.bias) s = s + (t < 32 ? bt : a.bias[row]);
-          s = apply_act(s, a.act);
-          if (a.res) s = (t < 32 ? rt : a.res[(int64_t)m * a.N + row]) + s;
-          a.y[(int64_t)m * a.N + row] = s;
-        }
+      float s = 0.0f;
+      if (rr < rows_per_iter) {
+        const float *rp = rb + rr * nkb;
+#pragma unroll 4
+        for (int k = rl; k < nkb; k += lpr) s += rp[k];
+      }
+      for (int o = lpr >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (rl == 0 && rr < rows_per_iter && base + rr < a.N) {
+        s = act_fast(a.bias ? s + bz : s, a.act);
+        a.y[(int64_t)m * a.N + base + rr] = a.res ? rz + s : s;
       }
       buf ^= 1;
     }
@@ -201,7 +264,10 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_stream_kernel(const Gem
   const bool active = tid < G * nkb;
   const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
   const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
-  const int rows_per_iter = G * RI, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  const int rows_per_iter = G * RI;
+  int lpr = 32;   // lanes that add up one row
+  while (lpr * rows_per_iter > (int)blockDim.x) lpr >>= 1;
+  const int rr = tid / lpr, rl = tid - rr * lpr;
   const int64_t stride = (int64_t)gridDim.x * rows_per_iter;
   uint32_t qn[RI][W], qhn[RI];
   float scn[RI], mnn[RI];
@@ -225,14 +291,15 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_stream_kernel(const Gem
   pdl_wait();
   BLK blk;
   {
-    float xv[32];
+    float xv[32], sum = 0.0f;
     const float4 *xp = reinterpret_cast<const float4 *>(a.x + (int64_t)kb * 32);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float4 v = xp[i];
-      xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
+      const float4 v = xp[i], w = BLK::stage(v, i);
+      sum += (v.x + v.y) + (v.z + v.w);
+      xv[4 * i] = w.x; xv[4 * i + 1] = w.y; xv[4 * i + 2] = w.z; xv[4 * i + 3] = w.w;
     }
-    blk.prep(xv);
+    blk.prep(xv, sum);
   }
   for (int buf = 0; base < a.N; base += stride, buf ^= 1) {
     uint32_t q[RI][W], qhc[RI];
@@ -257,18 +324,17 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_stream_kernel(const Gem
       }
     }
     __syncthreads();
-    for (int r = warp; r < rows_per_iter; r += nwarps) {
-      const int64_t row = base + r;
-      if (row >= a.N) break;
-      float s = 0.0f;
-      for (int k = lane; k < nkb; k += 32) s += rb[r * nkb + k];
-      s = warp_sum(s);
-      if (lane == 0) {
-        if (a.bias) s = s + a.bias[row];
-        s = apply_act(s, a.act);
-        if (a.res) s = a.res[row] + s;
-        a.y[row] = s;
-      }
+    float s = 0.0f;
+    if (rr < rows_per_iter) {
+      const float *rp = rb + rr * nkb;
+#pragma unroll 4
+      for (int k = rl; k < nkb; k += lpr) s += rp[k];
+    }
+    for (int o = lpr >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (rl == 0 && rr < rows_per_iter && base + rr < a.N) {
+      const int64_t row = base + rr;
+      s = act_fast(a.bias ? s + a.bias[row] : s, a.act);
+      a.y[row] = a.res ? a.res[row] + s : s;
     }
   }
 }
@@ -382,10 +448,9 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   };
   float bz, rz;
   addends(base, &bz, &rz);
-  for (int i = threadIdx.x; i < NR * K / 4; i += 256)
-    reinterpret_cast<float4 *>(xs)[i] = NR == 1 || i < a.M * K / 4 ? reinterpret_cast<const float4 *>(x)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = a.M * K / 4 + threadIdx.x; i < NR * K / 4; i += 256) reinterpret_cast<float4 *>(xs)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  gemv_rows_to_shared<NR, true>(a.norm, gb, x, a.M, K / 4, [&](int f, float4 v, bool ok) { if (ok) reinterpret_cast<float4 *>(xs)[f] = v; }, xs);
   __syncthreads();
-  if (!EXPERTS) gemv_norm_rows(a.norm, gb, a.M, K, [&](int m, int i) { return reinterpret_cast<float4 *>(xs + (size_t)m * K) + i; });
   const int64_t rounds = ((int64_t)N + stride - 1) / stride;   // the same for every warp: the slots' warps meet at barriers
   for (int64_t it = 0; it < rounds; ++it) {
     float acc[RI][NR];
@@ -442,7 +507,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
         const float up = __shfl_sync(0xffffffffu, s, (lane + NR) & 31);
         if (lane < NR && fin && row < N) y[fm * a.ldy + (row >> 1)] = glu(a.act, s, up);
       } else if (fin && row < N) {
-        s = apply_act(s, a.act);
+        s = act_fast(s, a.act);
         if (res) s = r + s;
         y[fm * a.ldy + row] = s;
       }
@@ -512,9 +577,12 @@ template <typename T, int RI, int NR, bool EXPERTS>
 static int launch_dense_t(caten_b200_ctx *ctx, GemvDense g, int groups) {
   const int nvec = g.K / DenseLoad<T>::VEC;
   // warps per RI rows: so many that a lane's share of a row is loaded at once, and more while the CTAs do not fill the
-  // GPU twice and every lane still has two vectors
+  // GPU twice, every lane still has two vectors and all CTAs stay resident at once (2304 x 768 fp32: with two warps a row 576
+  // CTAs on 444 places, 5.2 us; with one 4.4)
   int ks = 1;
-  while (ks < 8 && (nvec > 32 * GEMV_PRE * ks || (nvec > 64 * ks && ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI) * groups < 2 * ctx->sm_count))) ks *= 2;
+  const auto ctas_of = [&](int k) { return ((int64_t)g.group_rows * k + 8 * RI - 1) / (8 * RI) * groups; };
+  while (ks < 8 && (nvec > 32 * GEMV_PRE * ks ||
+                    (nvec > 64 * ks && ctas_of(ks) < 2 * ctx->sm_count && ctas_of(2 * ks) <= (RI == 2 ? 2 : 3) * ctx->sm_count))) ks *= 2;
   g.ks = ks;
   const int64_t ctas = ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI);
   const size_t smem = ((size_t)NR + (g.norm.g ? 2 : 0)) * g.K * sizeof(float);
@@ -545,7 +613,7 @@ int launch_gemv(caten_b200_ctx *ctx, const caten_b200_weight *w, const float *x,
                 const float *res, int act, float *y, int64_t M, LinGroups grp, GemvNorm norm) {
   if (w->rows > 0x7fffffff || w->cols > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: dimension too large");
   const int N = (int)w->rows, K = (int)w->cols;
-  if (norm.g && (K % 4 || K > 2400)) return fail(ctx, CATEN_B200_EUNSUPPORTED, "layernorm: d=%d (need d%%4==0, d<=2400)", K);
+  if (norm.g && (K % 4 || K > GEMV_NORM_K)) return fail(ctx, CATEN_B200_EUNSUPPORTED, "layernorm: d=%d (need d%%4==0, d<=%d)", K, GEMV_NORM_K);
   if (!type_is_packed(w->type) && (size_t)K * sizeof(float) > 160 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemv: cols=%d too wide", K);
   if (M > 1 && (M > 4 || (size_t)K * 4 * sizeof(float) > 160 * 1024)) {   // rows of x that do not fit shared memory together: one by one
     const int64_t ny = grp.ldy ? grp.ldy : act_is_glu(act) ? N / 2 : N;

@@ -16,27 +16,28 @@ namespace cb {
 // Q4_0 is folded into the accumulator's start value -8*sum(x)*2^-85, and 2^85 into the block
 // scale.  Nibbles of the top byte (bits 24..31 overlap the exponent field) are taken from
 // w >> 8.  Valid for |x| < 2^62; FMA with subnormal operands runs at full rate.
+//
+// x is scaled on its way to shared memory (stage: four consecutive elements, the j-th such group of their block), once for all
+// the threads that use it, and the sum of each block lies beside it.
 struct BlkQ4 {
-  static constexpr bool HAS_M = false, HAS_QH = false;
+  static constexpr bool HAS_M = false, HAS_QH = false, SUMS = true;
   static constexpr int WORDS = 4;
   float xs[32];
   float c0;
-  __device__ __forceinline__ void prep(const float *xv) {
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) sum += xv[j];
+  static __device__ __forceinline__ float4 stage(float4 v, int j) {
+    // elements 0..15 are the low nibbles of bytes 0..15 (p = 0, 8, 16 and, of w >> 8, 16), 16..31 the high ones (p = 4, 12, 20, 20)
+    const float up = j < 4 ? 0x1p64f : 0x1p60f;
+    return make_float4(v.x * up, v.y * (up * 0x1p-8f), v.z * (up * 0x1p-16f), v.w * (up * 0x1p-16f));
+  }
+  __device__ __forceinline__ void prep(const float *xv, float sum) {
     c0 = sum * -0x1p-82f;  // -8 * 2^-85
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      xs[8 * i + 0] = xv[4 * i + 0] * 0x1p64f;        // byte 0 low  nibble, p = 0
-      xs[8 * i + 1] = xv[16 + 4 * i + 0] * 0x1p60f;   // byte 0 high nibble, p = 4
-      xs[8 * i + 2] = xv[4 * i + 1] * 0x1p56f;        // byte 1 low,  p = 8
-      xs[8 * i + 3] = xv[16 + 4 * i + 1] * 0x1p52f;   // byte 1 high, p = 12
-      xs[8 * i + 4] = xv[4 * i + 2] * 0x1p48f;        // byte 2 low,  p = 16
-      xs[8 * i + 5] = xv[16 + 4 * i + 2] * 0x1p44f;   // byte 2 high, p = 20
-      xs[8 * i + 6] = xv[4 * i + 3] * 0x1p48f;        // byte 3 low  (of w >> 8), p = 16
-      xs[8 * i + 7] = xv[16 + 4 * i + 3] * 0x1p44f;   // byte 3 high (of w >> 8), p = 20
-    }
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        xs[8 * i + 2 * e] = xv[4 * i + e];
+        xs[8 * i + 2 * e + 1] = xv[16 + 4 * i + e];
+      }
   }
   __device__ __forceinline__ float dot(const uint32_t *w, float scale) const {
     float a0 = c0, a1 = 0.0f;
@@ -64,10 +65,11 @@ __device__ __forceinline__ float code_to_float(uint32_t magic, float offset) { r
 // Q8_0: byte (biased by 128) -> float -> FMA; (float)q * scale is exact in fp32 (8 + 11 bits), so
 // scaling the 32-term sum once per block only changes where the roundings of the sum fall.
 struct BlkQ8 {
-  static constexpr bool HAS_M = false, HAS_QH = false;
+  static constexpr bool HAS_M = false, HAS_QH = false, SUMS = false;
   static constexpr int WORDS = 8;
   float xs[32];
-  __device__ __forceinline__ void prep(const float *xv) {
+  static __device__ __forceinline__ float4 stage(float4 v, int) { return v; }
+  __device__ __forceinline__ void prep(const float *xv, float) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) xs[j] = xv[j];
   }
@@ -88,16 +90,14 @@ struct BlkQ8 {
 // Q4_1: w = q * d + m.  The nibble arithmetic of BlkQ4 without the -8 offset; the minimum enters
 // once per block as m * sum(x).
 struct BlkQ41 {
-  static constexpr bool HAS_M = true, HAS_QH = false;
+  static constexpr bool HAS_M = true, HAS_QH = false, SUMS = true;
   static constexpr int WORDS = 4;
   BlkQ4 nib;
   float sumx;
-  __device__ __forceinline__ void prep(const float *xv) {
-    nib.prep(xv);
+  static __device__ __forceinline__ float4 stage(float4 v, int j) { return BlkQ4::stage(v, j); }
+  __device__ __forceinline__ void prep(const float *xv, float sum) {
+    nib.prep(xv, sum);
     nib.c0 = 0.0f;
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) sum += xv[j];
     sumx = sum;
   }
   __device__ __forceinline__ float dotx(const uint32_t *w, float scale, float mn, uint32_t) const {
@@ -109,17 +109,14 @@ struct BlkQ41 {
 // with an integer-to-float instruction per weight.
 template <bool WITH_MIN>
 struct BlkQ5 {
-  static constexpr bool HAS_M = WITH_MIN, HAS_QH = true;
+  static constexpr bool HAS_M = WITH_MIN, HAS_QH = true, SUMS = WITH_MIN;
   static constexpr int WORDS = 4;
   float xs[32];
   float sumx;
-  __device__ __forceinline__ void prep(const float *xv) {
-    float sum = 0.0f;
+  static __device__ __forceinline__ float4 stage(float4 v, int) { return v; }
+  __device__ __forceinline__ void prep(const float *xv, float sum) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      xs[j] = xv[j];
-      sum += xv[j];
-    }
+    for (int j = 0; j < 32; ++j) xs[j] = xv[j];
     sumx = sum;
   }
   __device__ __forceinline__ float dotx(const uint32_t *w, float scale, float mn, uint32_t qh) const {
