@@ -8,104 +8,121 @@
 
 namespace cb {
 
-__device__ __forceinline__ void gemv_stage_norm(const GemvNorm &n, float *gb, int K) {
-  if (!n.g) return;
-  for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
-    reinterpret_cast<float4 *>(gb)[i] = reinterpret_cast<const float4 *>(n.g)[i];
-    reinterpret_cast<float4 *>(gb + K)[i] = reinterpret_cast<const float4 *>(n.b)[i];
-  }
-}
-
 // The rows of x, M x K4 float4 one after the other, on their way to shared memory: put(f, v, ok) takes float4 f (ok: it exists;
 // the whole warp calls it).  All of a thread's loads are under way before it uses the first.
 // With a norm every CTA normalises the rows for itself, which costs a linear less than a kernel of its own would (one more
-// hand-off).  gamma and beta (2 x K floats of shared memory) are staged before the wait for x.  A row is in the threads'
-// registers meanwhile: each warp has the mean and the squared deviations of its own part, and the parts are joined behind one
-// barrier.  (By one warp a row, from shared memory, GPT-2 XL's row took 1.3 to 1.8 us of a linear's 6; so, and with the sums of a row's parts by 8 to 32 lanes a row
-// instead of a warp for several, a step with 640 positions went from 1370 to 1258 us.)
+// hand-off).  A row is in the threads' registers meanwhile, SLOTS float4 of each; gamma and beta are there before the wait for x
+// (GemvGain).  Each warp has the mean and the squared deviations of its own part, and the parts are joined behind one barrier.
+// What counts are latencies (by one warp a row, from shared memory, GPT-2 XL's row took 1.3 to 1.8 us of a linear's 6, with the parts
+// joined in a loop over the warps 1.6, so 0.9: a step with 640 positions
+// 1370, 1258 and 1198 us).
 constexpr int GEMV_NORM_K = 2400;   // the longest row that is normalised: three float4 of each of at least 200 threads (launch_blocked's CTAs have 224)
-// MOST: M is at most that.  ASYNC: put is the plain copy to `to`, rows without a norm go there without passing through registers.
-template <int MOST, bool ASYNC, class Put>
-__device__ __forceinline__ void gemv_rows_to_shared(const GemvNorm &n, const float *gb, const float *x, int M, int K4, Put put, float *to = nullptr) {
-  const float4 *x4 = reinterpret_cast<const float4 *>(x);
-  const int tid = threadIdx.x, T = blockDim.x;
-  if (!n.g) {
-    const int total = M * K4;
-    if (ASYNC) {
-      for (int f = tid; f < total; f += T) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 4 * f)), "l"(x4 + f) : "memory");
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      return;
-    }
-    for (int f0 = 0; f0 < total; f0 += 8 * T) {
-      float4 v[8];
+struct GemvGain {
+  float4 g[2], b[2];   // (a third float4 of very long rows is read when it is needed)
+  __device__ __forceinline__ void load(const GemvNorm &n, int K4) {
+    if (!n.g) return;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int f = f0 + u * T + tid;
-        v[u] = f < total ? x4[f] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (f0 + u * T >= total) break;   // (the same for the whole CTA)
-        put(f0 + u * T + tid, v[u], f0 + u * T + tid < total);
+    for (int u = 0; u < 2; ++u) {
+      const int i = u * blockDim.x + threadIdx.x;
+      if (i < K4) {
+        g[u] = reinterpret_cast<const float4 *>(n.g)[i];
+        b[u] = reinterpret_cast<const float4 *>(n.b)[i];
       }
     }
-    return;
   }
+};
+
+template <int SLOTS, int MOST, class Put>
+__device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const GemvGain &gain, const float4 *x4, int M, int K4, Put put) {
   __shared__ float4 stat[2][16];   // of a warp's part: sum, squared deviations from its mean, mean, elements
-  const int warp = tid >> 5, lane = tid & 31, nw = T >> 5;
+  const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31;
   const float invd = 1.0f / (float)(K4 * 4);
   int have = 0;
 #pragma unroll
-  for (int u = 0; u < 3; ++u) {
+  for (int u = 0; u < SLOTS; ++u) {
     const int left = K4 - (warp * 32 + u * T);
     have += left <= 0 ? 0 : left < 32 ? left : 32;
   }
   const float cnt = (float)(4 * have), inv = have ? 1.0f / cnt : 0.0f;
-  float4 v[3], nx[3];
+  float4 v[SLOTS], nx[SLOTS];
   auto load = [&](int m, float4 *d) {
 #pragma unroll
-    for (int u = 0; u < 3; ++u) d[u] = m < M && u * T + tid < K4 ? x4[m * K4 + u * T + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < SLOTS; ++u) d[u] = m < M && u * T + tid < K4 ? x4[m * K4 + u * T + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   load(0, v);
   for (int m = 0; m < M; ++m) {
     if (MOST > 1) load(m + 1, nx);
     float sum = 0.0f, sq = 0.0f;
 #pragma unroll
-    for (int u = 0; u < 3; ++u) sum += (v[u].x + v[u].y) + (v[u].z + v[u].w);
+    for (int u = 0; u < SLOTS; ++u) sum += (v[u].x + v[u].y) + (v[u].z + v[u].w);
     sum = warp_sum(sum);
     const float mw = sum * inv;
 #pragma unroll
-    for (int u = 0; u < 3; ++u)
-      if (u * T + tid < K4) {
-        const float a = v[u].x - mw, b = v[u].y - mw, c = v[u].z - mw, d = v[u].w - mw;
-        sq += (a * a + b * b) + (c * c + d * d);
-      }
+    for (int u = 0; u < SLOTS; ++u) {
+      const float a = v[u].x - mw, b = v[u].y - mw, c = v[u].z - mw, d = v[u].w - mw;
+      sq += u * T + tid < K4 ? (a * a + b * b) + (c * c + d * d) : 0.0f;
+    }
     sq = warp_sum(sq);
     if (lane == 0) stat[m & 1][warp] = make_float4(sum, sq, mw, cnt);
     __syncthreads();
-    float all = 0.0f, dev = 0.0f;
-    for (int w = 0; w < nw; ++w) all += stat[m & 1][w].x;
-    const float u = all * invd;
-    for (int w = 0; w < nw; ++w) {
-      const float4 s = stat[m & 1][w];
-      dev += s.y + s.w * ((s.z - u) * (s.z - u));
-    }
-    const float rs = 1.0f / sqrtf(dev * invd + n.eps);
+    const float4 s = lane < (T >> 5) ? stat[m & 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);   // at most 16 warps
+    float all = s.x;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      if (q * T >= K4) break;
+    for (int o = 8; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+    const float u = __shfl_sync(0xffffffffu, all, 0) * invd;
+    float dev = s.y + s.w * ((s.z - u) * (s.z - u));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) dev += __shfl_xor_sync(0xffffffffu, dev, o);
+    const float rs = 1.0f / sqrtf(__shfl_sync(0xffffffffu, dev, 0) * invd + n.eps);
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
       const int i = q * T + tid;
-      const bool ok = i < K4;
-      float4 y = v[q];
-      if (ok) {
-        const float4 gg = reinterpret_cast<const float4 *>(gb)[i], bb = reinterpret_cast<const float4 *>(gb)[K4 + i];
-        y = make_float4(((y.x - u) * rs) * gg.x + bb.x, ((y.y - u) * rs) * gg.y + bb.y, ((y.z - u) * rs) * gg.z + bb.z, ((y.w - u) * rs) * gg.w + bb.w);
+      float4 gg, bb;
+      if (q < 2) {
+        gg = gain.g[q];
+        bb = gain.b[q];
+      } else if (i < K4) {
+        gg = reinterpret_cast<const float4 *>(n.g)[i];
+        bb = reinterpret_cast<const float4 *>(n.b)[i];
       }
-      put(m * K4 + i, y, ok);
+      const float4 y = v[q];
+      put(m * K4 + i, make_float4(((y.x - u) * rs) * gg.x + bb.x, ((y.y - u) * rs) * gg.y + bb.y, ((y.z - u) * rs) * gg.z + bb.z, ((y.w - u) * rs) * gg.w + bb.w), i < K4);
     }
     if (MOST == 1) break;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) v[q] = nx[q];
+    for (int q = 0; q < SLOTS; ++q) v[q] = nx[q];
+  }
+}
+
+// MOST: M is at most that.  ASYNC: put is the plain copy to `to`, rows without a norm go there without passing through registers.
+template <int MOST, bool ASYNC, class Put>
+__device__ __forceinline__ void gemv_rows_to_shared(const GemvNorm &n, const GemvGain &gain, const float *x, int M, int K4, Put put, float *to = nullptr) {
+  const float4 *x4 = reinterpret_cast<const float4 *>(x);
+  const int tid = threadIdx.x, T = blockDim.x;
+  if (n.g) {
+    if (K4 <= T) gemv_norm_rows<1, MOST>(n, gain, x4, M, K4, put);
+    else if (K4 <= 2 * T) gemv_norm_rows<2, MOST>(n, gain, x4, M, K4, put);
+    else gemv_norm_rows<3, MOST>(n, gain, x4, M, K4, put);
+    return;
+  }
+  const int total = M * K4;
+  if (ASYNC) {
+    for (int f = tid; f < total; f += T) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 4 * f)), "l"(x4 + f) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  for (int f0 = 0; f0 < total; f0 += 8 * T) {
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int f = f0 + u * T + tid;
+      v[u] = f < total ? x4[f] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (f0 + u * T >= total) break;   // (the same for the whole CTA)
+      put(f0 + u * T + tid, v[u], f0 + u * T + tid < total);
+    }
   }
 }
 
@@ -124,7 +141,8 @@ constexpr int GEMV_XPAD = 36;   // floats between the 32-wide blocks of x in sha
 
 __device__ __forceinline__ uint4 ld_stream(const uint4 *p) { return __ldcs(p); }
 
-// Thread t < G*nkb owns column block kb = t % nkb and row offset ro = t / nkb; a CTA covers G*RI consecutive rows (RI
+// Thread t < G*nkb owns column block kb = t / G and row offset ro = t % G (the G threads of a block are neighbours and read
+// their x from shared memory together: an eighth to a half of the reads that G passes over all blocks would be); a CTA covers G*RI consecutive rows (RI
 // independent 16/32-byte loads in flight per thread), once, or (LOOP) again and again with the next rows' loads ahead.  The
 // per-(row, block) partial sums go through shared memory and are added in a fixed order (lane
 // strided, then a butterfly), so results do not depend on scheduling.
@@ -140,9 +158,8 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   const int tid = threadIdx.x, nkb = a.nkb, G = a.G;
   float *xs = gemv_smem;                              // [M][nkb][GEMV_XPAD]
   float *red = gemv_smem + a.M * nkb * GEMV_XPAD;     // two buffers of [G * RI][nkb]
-  float *gb = red + 2 * G * RI * nkb;                 // norm: gamma and beta
   const bool active = tid < G * nkb;
-  const int kb = active ? tid % nkb : 0, ro = active ? tid / nkb : 0;
+  const int kb = active ? tid / G : 0, ro = active ? tid - kb * G : 0;
   const uint4 *qs = reinterpret_cast<const uint4 *>(a.qs);
   const int rows_per_iter = G * RI;
   const int64_t stride = (int64_t)gridDim.x * rows_per_iter;
@@ -168,7 +185,8 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   };
   int64_t base = (int64_t)blockIdx.x * rows_per_iter;
   load(base);
-  gemv_stage_norm(a.norm, gb, nkb * 32);
+  GemvGain gain;
+  gain.load(a.norm, nkb * 8);
   pdl_wait();
   // lpr lanes (a power of two) add up one row; the first of them finishes it, having asked for bias and residual beforehand
   int lpr = 32;
@@ -181,7 +199,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   };
   float bz, rz;
   addends(0, &bz, &rz);
-  gemv_rows_to_shared<4, false>(a.norm, gb, a.x, a.M, nkb * 8, [&](int f, float4 v, bool ok) {
+  gemv_rows_to_shared<4, false>(a.norm, gain, a.x, a.M, nkb * 8, [&](int f, float4 v, bool ok) {
     float *to = xs + (f >> 3) * GEMV_XPAD;
     if (BLK::SUMS) {
       float s = (v.x + v.y) + (v.z + v.w);
@@ -433,9 +451,9 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   int64_t base = ((int64_t)blockIdx.x * slots + slot) * RI;
   const int64_t stride = (int64_t)gridDim.x * slots * RI;
   load(base, c0);
-  float *gb = xs + NR * K;
+  GemvGain gain;
   if (!EXPERTS) {
-    gemv_stage_norm(a.norm, gb, K);
+    gain.load(a.norm, K / 4);
     pdl_wait();
   }
   // the lane that finishes output (row base + i, row m of x) is lane i * NR + m of the slot's first warp
@@ -449,7 +467,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   float bz, rz;
   addends(base, &bz, &rz);
   for (int i = a.M * K / 4 + threadIdx.x; i < NR * K / 4; i += 256) reinterpret_cast<float4 *>(xs)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  gemv_rows_to_shared<NR, true>(a.norm, gb, x, a.M, K / 4, [&](int f, float4 v, bool ok) { if (ok) reinterpret_cast<float4 *>(xs)[f] = v; }, xs);
+  gemv_rows_to_shared<NR, true>(a.norm, gain, x, a.M, K / 4, [&](int f, float4 v, bool ok) { if (ok) reinterpret_cast<float4 *>(xs)[f] = v; }, xs);
   __syncthreads();
   const int64_t rounds = ((int64_t)N + stride - 1) / stride;   // the same for every warp: the slots' warps meet at barriers
   for (int64_t it = 0; it < rounds; ++it) {
@@ -520,7 +538,7 @@ template <class BLK, int RI, bool LOOP, int THREADS>
 static int launch_blocked_t(caten_b200_ctx *ctx, GemvArgs a) {
   a.G = THREADS / a.nkb;
   const int threads = (a.G * a.nkb + 31) / 32 * 32;
-  const size_t smem = ((size_t)a.M * a.nkb * GEMV_XPAD + 2 * (size_t)a.G * RI * a.nkb + (a.norm.g ? 2 * 32 * (size_t)a.nkb : 0)) * sizeof(float);
+  const size_t smem = ((size_t)a.M * a.nkb * GEMV_XPAD + 2 * (size_t)a.G * RI * a.nkb) * sizeof(float);
   auto kernel = gemv_blocked_kernel<BLK, RI, LOOP, THREADS>;
   if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t grid = ((int64_t)a.N + a.G * RI - 1) / (a.G * RI);
@@ -585,7 +603,7 @@ static int launch_dense_t(caten_b200_ctx *ctx, GemvDense g, int groups) {
                     (nvec > 64 * ks && ctas_of(ks) < 2 * ctx->sm_count && ctas_of(2 * ks) <= (RI == 2 ? 2 : 3) * ctx->sm_count))) ks *= 2;
   g.ks = ks;
   const int64_t ctas = ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI);
-  const size_t smem = ((size_t)NR + (g.norm.g ? 2 : 0)) * g.K * sizeof(float);
+  const size_t smem = (size_t)NR * g.K * sizeof(float);
   auto kernel = gemv_dense_kernel<T, RI, NR, EXPERTS>;
   if (smem > 47 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t grid = ((int64_t)ctx->sm_count * (smem > 72 * 1024 || RI == 2 ? 2 : 3) + groups - 1) / groups;   // resident at once
