@@ -16,28 +16,17 @@ constexpr float kInvLn2 = 1.0f / 0.6931472f;  // (/ (log 2)) in single float, ap
 // this step's k and v rows at position n, so no separate append kernel runs in decode.
 // Scores are kept in shared memory (t <= T floats) and the softmax is the reference's two-pass
 // form (max, then exp and sum), not an online rescaling.
-// SPLIT: with few heads and sequences a cluster of CTAs shares a history (contiguous parts of the positions); each forms the
-// two-pass softmax of its part, and the first CTA joins the parts through distributed shared memory.  One sequence of 25
-// heads at 640 positions: 12.4 us with one CTA per head, 6.3 us with eight.  Below 96 positions one CTA does it, also where the
-// launch, which for a device-side position is made for the longest context, has clusters: the cut depends on the position alone,
-// and every entry gives the same bits (GPT-2 medium Q4_0, one sequence, us a step at 10 positions: all eight 473, one 436; at 130: 476, two 494).
 // ---------------------------------------------------------------------------------------------
 #ifndef ATT_U
 #define ATT_U 4  // rows in flight per half-warp
 #endif
-constexpr int ATT_PARTS = 8;
-__host__ __device__ inline int att_parts(int64_t t, int most) { return t >= 96 ? most : 1; }
-// where part `rank` of `parts`, a power of two, begins
-__device__ __forceinline__ int att_cut(int t, int rank, int parts) { return (int)(((long long)t * rank) >> (__ffs(parts) - 1)); }
 
-template <bool SPLIT>
 __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__restrict__ qkv, float *__restrict__ kc,
                                                           float *__restrict__ vc, float *__restrict__ out, int H,
                                                           int T, int n, const int *__restrict__ d_n,
                                                           __nv_bfloat16 *__restrict__ ohi, __nv_bfloat16 *__restrict__ olo,
-                                                          const PartIn pin, long long prefetch_bytes, const int cluster) {
-  const int h = SPLIT ? blockIdx.x / cluster : blockIdx.x, rank = SPLIT ? blockIdx.x % cluster : 0, b = blockIdx.y, tid = threadIdx.x;
-  if (SPLIT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "my shared memory may be written to"
+                                                          const PartIn pin, long long prefetch_bytes) {
+  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   float *kb = kc + ((int64_t)b * H + h) * T * 64;
   float *vb = vc + ((int64_t)b * H + h) * T * 64;
   // Under programmatic dependent launch the first CTAs of this grid become resident while the kernels before it
@@ -52,13 +41,11 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
     constexpr long long PIECE = 32 << 10;
     int np = d_n ? *d_n : n;
     np = np < 0 ? 0 : (np > T - 1 ? T - 1 : np);
-    const int share = SPLIT ? att_parts(np + 1, cluster) : 1;
-    const int p0 = SPLIT ? att_cut(np, rank, share) : 0;
-    const long long stream_bytes = rank < share ? 256ll * ((SPLIT ? att_cut(np, rank + 1, share) : np) - p0) : 0;
+    const long long stream_bytes = 256ll * np;
     const int pieces = (int)((stream_bytes + PIECE - 1) / PIECE);
     if (tid < 2 * pieces && ((long long)b * H + h + 1) * 2 * 256ll * np <= prefetch_bytes) {
       const int which = tid >= pieces ? 1 : 0, i = tid - which * pieces;
-      const char *src = reinterpret_cast<const char *>(which ? vb : kb) + 256ll * p0 + (long long)i * PIECE;
+      const char *src = reinterpret_cast<const char *>(which ? vb : kb) + (long long)i * PIECE;
       const long long left = stream_bytes - (long long)i * PIECE;
       const unsigned bytes = (unsigned)(left < PIECE ? left : PIECE);
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
@@ -72,42 +59,29 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
   float *red = part + 1024;   // 32
   float *sc = red + 32;       // t
   const int d = H * 64, t = n + 1;
-  const int parts = SPLIT ? att_parts(t, cluster) : 1;
-  if (SPLIT && rank >= parts) {   // (whole CTAs) not needed at this length; the others still meet at the barriers
-    if (parts > 1) {
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    }
-    return;
-  }
-  const int j_first = SPLIT ? att_cut(t, rank, parts) : 0, j_end = SPLIT ? att_cut(t, rank + 1, parts) : t;
-  const bool newest = !SPLIT || rank == parts - 1;   // position n is in the last part, which is never empty
-  __shared__ float join[SPLIT ? ATT_PARTS * 66 : 1];  // of the first CTA: each part's maximum, sum and 64 outputs
   const float *row = qkv + (int64_t)b * 3 * d;
   if (pin.splits > 0) {
     // the qkv linear left split-K partial tiles: sum this head's q, k, v entries here
-    if (tid < (newest ? 192 : 64)) {
+    if (tid < 192) {
       const int which = tid >> 6, e = tid & 63;
       const float val = partin_load1(pin, b, which * d + h * 64 + e);
       if (which == 0) q[e] = val;
-      else if (newest) (which == 1 ? kb : vb)[(int64_t)n * 64 + e] = val;
+      else (which == 1 ? kb : vb)[(int64_t)n * 64 + e] = val;
     }
   } else if (tid < 64) {
     q[tid] = row[h * 64 + tid];
-    if (newest) {
-      kb[(int64_t)n * 64 + tid] = row[d + h * 64 + tid];
-      vb[(int64_t)n * 64 + tid] = row[2 * d + h * 64 + tid];
-    }
+    kb[(int64_t)n * 64 + tid] = row[d + h * 64 + tid];
+    vb[(int64_t)n * 64 + tid] = row[2 * d + h * 64 + tid];
   }
   __syncthreads();
   const int hw = tid >> 4, l16 = tid & 15;
   const float4 q4 = reinterpret_cast<const float4 *>(q)[l16];
-  for (int j0 = j_first; j0 < j_end; j0 += 16 * ATT_U) {
+  for (int j0 = 0; j0 < t; j0 += 16 * ATT_U) {
     float4 k4[ATT_U];
 #pragma unroll
     for (int u = 0; u < ATT_U; ++u) {
       const int j = j0 + u * 16 + hw;
-      k4[u] = j < j_end ? __ldcs(reinterpret_cast<const float4 *>(kb + (int64_t)j * 64) + l16) : make_float4(0.f, 0.f, 0.f, 0.f);
+      k4[u] = j < t ? __ldcs(reinterpret_cast<const float4 *>(kb + (int64_t)j * 64) + l16) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < ATT_U; ++u) {
@@ -117,13 +91,13 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
       p += __shfl_xor_sync(0xffffffffu, p, 2);
       p += __shfl_xor_sync(0xffffffffu, p, 1);
       const int j = j0 + u * 16 + hw;
-      if (l16 == 0 && j < j_end) sc[j - j_first] = p * 0.125f;
+      if (l16 == 0 && j < t) sc[j] = p * 0.125f;
     }
   }
   __syncthreads();
   // row max
   float m = -INFINITY;
-  for (int j = tid; j < j_end - j_first; j += 256) m = fmaxf(m, sc[j]);
+  for (int j = tid; j < t; j += 256) m = fmaxf(m, sc[j]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((tid & 31) == 0) red[tid >> 5] = m;
@@ -133,7 +107,7 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
   for (int w = 1; w < 8; ++w) m = fmaxf(m, red[w]);
   __syncthreads();
   float ss = 0.0f;
-  for (int j = tid; j < j_end - j_first; j += 256) {
+  for (int j = tid; j < t; j += 256) {
     const float e = exp2f((sc[j] - m) * kInvLn2);
     sc[j] = e;
     ss += e;
@@ -144,18 +118,18 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
   ss = red[0];
 #pragma unroll
   for (int w = 1; w < 8; ++w) ss += red[w];
-  const float inv = parts > 1 ? 1.0f : 1.0f / ss;   // (parts are joined before they are divided by the sum)
+  const float inv = 1.0f / ss;
   // O = P.V
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int j0 = j_first; j0 < j_end; j0 += 16 * ATT_U) {
+  for (int j0 = 0; j0 < t; j0 += 16 * ATT_U) {
     float4 v4[ATT_U];
     float p[ATT_U];
 #pragma unroll
     for (int u = 0; u < ATT_U; ++u) {
       const int j = j0 + u * 16 + hw;
-      const bool ok = j < j_end;
+      const bool ok = j < t;
       v4[u] = ok ? __ldcs(reinterpret_cast<const float4 *>(vb + (int64_t)j * 64) + l16) : make_float4(0.f, 0.f, 0.f, 0.f);
-      p[u] = ok ? sc[j - j_first] * inv : 0.0f;
+      p[u] = ok ? sc[j] * inv : 0.0f;
     }
 #pragma unroll
     for (int u = 0; u < ATT_U; ++u) {
@@ -172,27 +146,195 @@ __global__ void __launch_bounds__(256, 6) attn_decode_kernel(const float *__rest
 #pragma unroll
     for (int w = 0; w < 16; ++w) o += part[w * 64 + tid];
   }
+  if (tid < 64) {
+    const int64_t at = (int64_t)b * d + h * 64 + tid;
+    if (ohi) {  // split bf16 operand of the projection GEMM
+      const __nv_bfloat16 hh = __float2bfloat16_rn(o);
+      ohi[at] = hh;
+      if (olo) olo[at] = __float2bfloat16_rn(o - __bfloat162float(hh));
+    } else {
+      out[at] = o;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Decode with few heads and sequences (two CTAs per SM at most): a launch is a few microseconds of dependent latencies, so
+// the first FEW_U rows of K and V of every half-warp, which are history and depend on nothing in flight, are in registers before
+// the wait for q (early: inside a model's step, where a kernel that waited for everything before the step is already over);
+// a half-warp keeps a softmax of its own rows, running where they are more than it loads at once, and the halves meet
+// behind one barrier.  A cluster of CTAs may share a history (contiguous parts of the positions); the first CTA joins the
+// parts through distributed shared memory.  Below 96 positions one CTA does it, also where the launch, which for a device-side
+// position is made for the longest context, has clusters: the cut depends on the position alone, and every entry gives the same
+// bits (GPT-2 medium Q4_0, one sequence, us a step at 10 positions: all eight 473, one 436; at 130: 476, two 494).
+// us a step with the kernel above (which had clusters too) / this one: XL Q4_0, one sequence at 640 positions 1197 / 1099; medium Q8_0, three
+// at 300 896 / 818; medium Q4_0, 18 at 800 1513 / 1210; small fp32, one at 66 265 / 250.
+// ---------------------------------------------------------------------------------------------
+constexpr int ATT_PARTS = 8;
+constexpr int FEW_U = 6;
+__host__ __device__ inline int att_parts(int64_t t, int most) { return t >= 96 ? most : 1; }
+// where part `rank` of `parts`, a power of two, begins
+__device__ __forceinline__ int att_cut(int t, int rank, int parts) { return (int)(((long long)t * rank) >> (__ffs(parts) - 1)); }
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(256, 3) attn_decode_few_kernel(const float *__restrict__ qkv, float *__restrict__ kc, float *__restrict__ vc,
+                                                                 float *__restrict__ out, int H, int T, int n, const int *__restrict__ d_n,
+                                                                 __nv_bfloat16 *__restrict__ ohi, __nv_bfloat16 *__restrict__ olo, const PartIn pin,
+                                                                 const int cluster, const bool early) {
+  const int h = SPLIT ? blockIdx.x / cluster : blockIdx.x, rank = SPLIT ? blockIdx.x % cluster : 0, b = blockIdx.y, tid = threadIdx.x;
+  if (SPLIT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // "my shared memory may be written to"
+  __shared__ __align__(16) float fresh[192];            // q, k, v of this step where they come as partial tiles
+  __shared__ __align__(16) float part[8][64];           // each warp's outputs
+  __shared__ float2 stat[8];                            // its maximum and sum
+  __shared__ float join[SPLIT ? ATT_PARTS * 66 : 1];    // of the first CTA: each part's maximum, sum and 64 outputs
+  float *kb = kc + ((int64_t)b * H + h) * T * 64;
+  float *vb = vc + ((int64_t)b * H + h) * T * 64;
+  const int hw = tid >> 4, l16 = tid & 15, d = H * 64;
+  float4 k4[FEW_U], v4[FEW_U];
+  int t, parts, j_first, j_end;
+  auto place = [&]() {
+    t = n + 1;
+    parts = SPLIT ? att_parts(t, cluster) : 1;
+    j_first = SPLIT ? att_cut(t, rank, parts) : 0;
+    j_end = SPLIT ? rank < parts ? att_cut(t, rank + 1, parts) : j_first : t;
+  };
+  auto load = [&](int j0) {   // rows of the history among the half-warp's next FEW_U
+#pragma unroll
+    for (int u = 0; u < FEW_U; ++u) {
+      const int j = j0 + u * 16 + hw;
+      const bool ok = j < j_end && j < n;
+      k4[u] = ok ? __ldcs(reinterpret_cast<const float4 *>(kb + (int64_t)j * 64) + l16) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v4[u] = ok ? __ldcs(reinterpret_cast<const float4 *>(vb + (int64_t)j * 64) + l16) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (early) {
+    if (d_n) n = min(max(*d_n, 0), T - 1);  // position kept on the device (decode replayed from a CUDA graph)
+    place();
+    load(j_first);
+    pdl_enter();
+  } else {
+    pdl_enter();
+    if (d_n) n = *d_n;
+    place();
+    load(j_first);
+  }
+  if (SPLIT && rank >= parts) {   // (whole CTAs) not needed at this length; the others still meet at the barriers
+    if (parts > 1) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    return;
+  }
+  const bool newest = !SPLIT || rank == parts - 1;   // position n is in the last part, which is never empty
+  const float4 *qp, *kp, *vp;
+  if (pin.splits > 0) {
+    // the qkv linear left split-K partial tiles: sum this head's q, k, v entries here
+    if (tid < (newest ? 192 : 64)) fresh[tid] = partin_load1(pin, b, (tid >> 6) * d + h * 64 + (tid & 63));
+    __syncthreads();
+    qp = reinterpret_cast<const float4 *>(fresh);
+    kp = qp + 16;
+    vp = qp + 32;
+  } else {
+    qp = reinterpret_cast<const float4 *>(qkv + (int64_t)b * 3 * d + h * 64);
+    kp = qp + d / 4;
+    vp = kp + d / 4;
+  }
+  const float4 q4 = qp[l16];
+  float4 kn = make_float4(0.f, 0.f, 0.f, 0.f), vn = kn;
+  if (newest) {
+    kn = kp[l16];
+    vn = vp[l16];
+    if (hw == 0) {
+      reinterpret_cast<float4 *>(kb + (int64_t)n * 64)[l16] = kn;
+      reinterpret_cast<float4 *>(vb + (int64_t)n * 64)[l16] = vn;
+    }
+  }
+  float m = -INFINITY, ss = 0.0f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j0 = j_first; j0 < j_end; j0 += 16 * FEW_U) {
+    if (j0 > j_first) load(j0);
+    float p[FEW_U], top = m;
+#pragma unroll
+    for (int u = 0; u < FEW_U; ++u) {
+      const int j = j0 + u * 16 + hw;
+      if (j == n) { k4[u] = kn; v4[u] = vn; }
+      p[u] = fmaf(q4.x, k4[u].x, fmaf(q4.y, k4[u].y, fmaf(q4.z, k4[u].z, q4.w * k4[u].w)));
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < FEW_U; ++u) p[u] += __shfl_xor_sync(0xffffffffu, p[u], o);
+#pragma unroll
+    for (int u = 0; u < FEW_U; ++u) {
+      p[u] = j0 + u * 16 + hw < j_end ? p[u] * 0.125f : -INFINITY;
+      top = fmaxf(top, p[u]);
+    }
+    if (top == -INFINITY) continue;   // no row yet
+    const float keep = exp2f((m - top) * kInvLn2);
+    m = top;
+    ss *= keep;
+    acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+#pragma unroll
+    for (int u = 0; u < FEW_U; ++u) {
+      const float e = exp2f((p[u] - top) * kInvLn2);
+      ss += e;
+      acc.x = fmaf(e, v4[u].x, acc.x);
+      acc.y = fmaf(e, v4[u].y, acc.y);
+      acc.z = fmaf(e, v4[u].z, acc.z);
+      acc.w = fmaf(e, v4[u].w, acc.w);
+    }
+  }
+  {   // the two halves of the warp
+    const float mo = __shfl_xor_sync(0xffffffffu, m, 16), top = fmaxf(m, mo), f = m == -INFINITY ? 0.0f : exp2f((m - top) * kInvLn2);
+    m = top;
+    ss *= f;
+    acc.x *= f; acc.y *= f; acc.z *= f; acc.w *= f;
+    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
+    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16);
+    acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+  }
+  if (!(hw & 1)) reinterpret_cast<float4 *>(part[tid >> 5])[l16] = acc;
+  if ((tid & 31) == 0) stat[tid >> 5] = make_float2(m, ss);
+  __syncthreads();
+  float o = 0.0f, sum = 0.0f;
+  m = -INFINITY;
+  if (tid < 96) {   // (whole warps; 64 of them have an output)
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, stat[w].x);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const float2 st = stat[w];
+      const float f = st.x == -INFINITY ? 0.0f : exp2f((st.x - m) * kInvLn2);
+      sum = fmaf(st.y, f, sum);
+      o = fmaf(part[w][tid & 63], f, o);
+    }
+  }
   if (parts > 1) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (tid < 66) {
       uint32_t at;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&join[rank * 66 + tid])), "r"(0));
-      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(tid < 64 ? o : tid == 64 ? m : ss) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(tid < 64 ? o : tid == 64 ? m : sum) : "memory");
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (rank != 0 || tid >= 64) return;
-    float top = -INFINITY, sum = 0.0f;   // an empty part has the maximum -inf, the sum 0 and outputs of 0
-    for (int r = 0; r < parts; ++r) top = fmaxf(top, join[r * 66 + 64]);
-    o = 0.0f;
-    for (int r = 0; r < parts; ++r) {
+    float top = -INFINITY;   // an empty part has the maximum -inf, the sum 0 and outputs of 0
+#pragma unroll
+    for (int r = 0; r < ATT_PARTS; ++r) top = fmaxf(top, r < parts ? join[r * 66 + 64] : -INFINITY);
+    o = sum = 0.0f;
+#pragma unroll
+    for (int r = 0; r < ATT_PARTS; ++r) {
+      if (r >= parts) break;
       const float mr = join[r * 66 + 64], f = mr == -INFINITY ? 0.0f : exp2f((mr - top) * kInvLn2);
       sum = fmaf(join[r * 66 + 65], f, sum);
       o = fmaf(join[r * 66 + tid], f, o);
     }
-    o = o / sum;
   }
   if (tid < 64) {
+    o = o / sum;
     const int64_t at = (int64_t)b * d + h * 64 + tid;
     if (ohi) {  // split bf16 operand of the projection GEMM
       const __nv_bfloat16 hh = __float2bfloat16_rn(o);
@@ -393,12 +535,19 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     while (most < ATT_PARTS && B * H * most * 2 <= 2 * ctx->sm_count) most *= 2;
     if (most == 2 || (B > 4 && !tensor_cores)) most = 1;
     const int parts = att_parts(d_n ? T : n + 1, most);
-    auto kernel = parts > 1 ? attn_decode_kernel<true> : attn_decode_kernel<false>;
-    if (smem > 44 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    // (more CTAs are limited by bytes, and the kernel with more of them on an SM is the better one: us a step, few / other: medium Q4_0, 64
+    // sequences, 200 positions 1358 / 1316; small Q8_0, 64 at 300 724 / 679; XL Q4_0, 16 at 100 2182 / 2118, but 16 at 800 3093 / 3343)
+    if (B * H > 2 * ctx->sm_count) {
+      if (smem > 44 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+      launch_k(ctx, attn_decode_kernel, dim3((unsigned)H, (unsigned)B), dim3(256), smem, qkv, kc, vc, out, (int)H, (int)T, (int)n, d_n, bf.hi, bf.lo,
+               pending_qkv ? *pending_qkv : PartIn(), ctx->attn_prefetch_bytes);
+      CB_LAUNCH_CHECK(ctx, "attn_decode_kernel");
+      return 0;
+    }
+    auto kernel = parts > 1 ? attn_decode_few_kernel<true> : attn_decode_few_kernel<false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(H * parts), (unsigned)B);
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at[2];
     int na = 0;
@@ -415,9 +564,9 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, qkv, kc, vc, out, (int)H, (int)T, (int)n, d_n, bf.hi, bf.lo, pending_qkv ? *pending_qkv : PartIn(),
-                                    ctx->attn_prefetch_bytes, parts));
-    CB_LAUNCH_CHECK(ctx, "attn_decode_kernel");
+    CB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, qkv, (float *)kc, (float *)vc, out, (int)H, (int)T, (int)n, d_n, bf.hi, bf.lo, pending_qkv ? *pending_qkv : PartIn(),
+                                    parts, pending_qkv != nullptr));
+    CB_LAUNCH_CHECK(ctx, "attn_decode_few_kernel");
     return 0;
   }
   if (d_n) return fail(ctx, CATEN_B200_EINVAL, "attention: a device-side position is only supported for single-token steps");

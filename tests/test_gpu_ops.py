@@ -462,9 +462,10 @@ def test_attention_decode_steps(rt, oracle, B, H, T):
     np.testing.assert_array_equal(dv.numpy(), _to_gpu_cache(vc))
 
 
-@pytest.mark.parametrize("B,H,T", [(1, 2, 1030), (1, 25, 515), (2, 3, 259), (5, 30, 130)])
+@pytest.mark.parametrize("B,H,T", [(1, 2, 1030), (1, 25, 515), (2, 3, 259), (5, 30, 130), (4, 74, 103), (3, 99, 103), (1, 4, 99), (2, 60, 1000)])
 def test_attention_decode_shared_histories(rt, oracle, B, H, T):
-    """One to eight CTAs per history, around the lengths where their number changes."""
+    """One to eight CTAs per history, around the lengths and the numbers of heads and sequences where their number and the kernel change;
+    histories of one round of a half-warp's rows and of several."""
     test_attention_decode_steps(rt, oracle, B, H, T)
 
 
