@@ -293,16 +293,16 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
           if (NQ == 1 || k < ksteps) {
             // 16 bf16 = 32 bytes = 2 descriptor units; a Q block is 32 KB = 2048 units, a K block 16 KB = 1024
             const uint64_t aq = dq + (uint64_t)((k >> 2) * 2048 + 2 * (k & 3)), ak = dk + (uint64_t)((k >> 2) * 1024 + 2 * (k & 3));
-            umma_bf16(acc, aq, ak, idesc_s, k > 0 ? 1u : 0u);
-            umma_bf16(acc, aq + 1024, ak, idesc_s, 1u);
+            umma_bf16(acc, aq, ak, idesc_s, k > 0 ? 1u : 0u, 1u);
+            umma_bf16(acc, aq + 1024, ak, idesc_s, 1u, 1u);
             if (!Lay::STACK) {
-              umma_bf16(acc, aq, ak + 512, idesc_s, 1u);
-              umma_bf16(acc, aq + 1024, ak + 512, idesc_s, 1u);
+              umma_bf16(acc, aq, ak + 512, idesc_s, 1u, 1u);
+              umma_bf16(acc, aq + 1024, ak + 512, idesc_s, 1u, 1u);
             }
           }
         }
-        umma_commit(k_empty(st));
-        umma_commit(s_full(st));
+        umma_commit(k_empty(st), 1u);
+        umma_commit(s_full(st), 1u);
       }
       __syncwarp();
       return true;
@@ -323,12 +323,12 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
           if (k4 >= groups) break;
           const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
           const uint32_t p_hi = tmem_base + Lay::COL_P + 8 * k4, p_lo = p_hi + 32;
-          umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u);
-          umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u);
-          umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u);
+          umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u, 1u);
+          umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u, 1u);
+          umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u, 1u);
         }
-        umma_commit(v_empty(st));
-        umma_commit(pv_done);
+        umma_commit(v_empty(st), 1u);
+        umma_commit(pv_done, 1u);
       }
       __syncwarp();
     }
@@ -648,12 +648,12 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint64_t aq = dq + (uint64_t)(2 * k), ak = dk + (uint64_t)(2 * k);   // 16 bf16 = 32 bytes = 2 descriptor units
-          umma_bf16(tmem_base + A1_COL_S, aq, ak, idesc_s, k > 0 ? 1u : 0u);
-          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak, idesc_s, 1u);
-          umma_bf16(tmem_base + A1_COL_S, aq, ak + 512, idesc_s, 1u);
-          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak + 512, idesc_s, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq, ak, idesc_s, k > 0 ? 1u : 0u, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak, idesc_s, 1u, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq, ak + 512, idesc_s, 1u, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak + 512, idesc_s, 1u, 1u);
         }
-        umma_commit(bar);
+        umma_commit(bar, 1u);
       }
       __syncwarp();
     }
@@ -717,11 +717,11 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
         for (int k4 = 0; k4 < 4; ++k4) {
           const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
           const uint32_t p_hi = tmem_base + A1_COL_P + 8 * k4, p_lo = p_hi + 32;
-          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u);
-          umma_bf16_ts(tmem_base + A1_COL_O, p_lo, dv + adv, idesc_pv, 1u);
-          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + 512 + adv, idesc_pv, 1u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u, 1u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_lo, dv + adv, idesc_pv, 1u, 1u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + 512 + adv, idesc_pv, 1u, 1u);
         }
-        umma_commit(bar);
+        umma_commit(bar, 1u);
       }
       __syncwarp();
     }

@@ -277,7 +277,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
   auto st_xhi = [&](int s) { return stage0 + (uint32_t)s * STAGE_BYTES + (WLO ? 2u : 1u) * W_BYTES; };
   auto st_xlo = [&](int s) { return st_xhi(s) + X_BYTES; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int num_k = a.K / BK;
   const int rank = PAIR ? (int)(blockIdx.x & 1) : 0, worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, workers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   // work item i: tile i % tiles, k-stages [i / tiles * cps, ..) of it
@@ -323,23 +323,24 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
     }
   }
   // a stage's bytes, those of both CTAs of a pair, complete on the leader's barrier
-  auto expect = [&](int s) {
-    if (rank == 0) mbar_expect_tx(full(s), PAIR ? 2 * STAGE_BYTES : STAGE_BYTES);
+  auto expect = [&](int s, uint32_t el) {
+    if (rank == 0) mbar_expect_tx(full(s), PAIR ? 2 * STAGE_BYTES : STAGE_BYTES, el);
   };
-  auto load = [&](uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y) {
-    if (PAIR) tma_load_2d_pair(dst, map, bar, x, y);
-    else tma_load_2d(dst, map, bar, x, y);
+  auto load = [&](uint32_t dst, const CUtensorMap *map, uint32_t bar, int x, int y, uint32_t el) {
+    if (PAIR) tma_load_2d_pair(dst, map, bar, x, y, el);
+    else tma_load_2d(dst, map, bar, x, y, el);
   };
   // Weights that no kernel writes are on their way before the wait below: in a decode step that is most of what this CTA
   // reads, and it arrives while the kernel that produces x still runs.
   int ahead = 0;   // stages whose W tiles have been asked for
-  if (!EXPERTS && a.static_w && warp == 0 && lane == 0) {
+  if (!EXPERTS && a.static_w && warp == 0) {
     const GdTile t = gd_tile<EXPERTS, PAIR>(a, worker % a.tiles, nullptr, rank);
     int k0;
     const int nk = k_of(worker / a.tiles, &k0);
     for (; ahead < nk && ahead < S; ++ahead) {
-      expect(ahead);
-      load(st_whi(ahead), &tw_hi, full(ahead), (k0 + ahead) * BK, t.f0);
+      const uint32_t el = elect_one();
+      expect(ahead, el);
+      load(st_whi(ahead), &tw_hi, full(ahead), (k0 + ahead) * BK, t.f0, el);
     }
   }
   // the activations, the residual and (otherwise) the weights were written by preceding kernels
@@ -369,52 +370,52 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
   const int items = tiles * a.splits;
 
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int issued = 0, s = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int item = worker; item < items && ok; item += workers) {
-        const int tile = item % tiles;
-        const GdTile t = gd_tile<EXPERTS, PAIR>(a, tile, first, rank);
-        int k0;
-        const int nk = k_of(item / tiles, &k0);
-        for (int kc = k0; kc < k0 + nk; ++kc) {
-          if (!mbar_wait(empty(s), ph ^ 1u, abort_flag)) {
-            if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 11; a.status[2] = tile; }
-            ok = false;
-            break;
-          }
-          if (issued >= ahead) {
-            expect(s);
-            load(st_whi(s), &tw_hi, full(s), kc * BK, t.f0);
-          }
-          if (WLO) load(st_wlo(s), &tw_lo, full(s), kc * BK, t.f0);
-          load(st_xhi(s), &tx_hi, full(s), kc * BK, t.x0);
-          if (NSPLIT == 3) load(st_xlo(s), &tx_lo, full(s), kc * BK, t.x0);
-          ++issued;
-          if (++s == S) { s = 0; ph ^= 1u; }
+    // ---------------- TMA producer (uniform control flow, one elected lane issues) ----------------
+    int issued = 0, s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int item = worker; item < items && ok; item += workers) {
+      const int tile = item % tiles;
+      const GdTile t = gd_tile<EXPERTS, PAIR>(a, tile, first, rank);
+      int k0;
+      const int nk = k_of(item / tiles, &k0);
+      for (int kc = k0; kc < k0 + nk; ++kc) {
+        if (!mbar_wait(empty(s), ph ^ 1u, abort_flag)) {
+          if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 11; a.status[2] = tile; }
+          ok = false;
+          break;
         }
+        const uint32_t el = elect_one();
+        if (issued >= ahead) {
+          expect(s, el);
+          load(st_whi(s), &tw_hi, full(s), kc * BK, t.f0, el);
+        }
+        if (WLO) load(st_wlo(s), &tw_lo, full(s), kc * BK, t.f0, el);
+        load(st_xhi(s), &tx_hi, full(s), kc * BK, t.x0, el);
+        if (NSPLIT == 3) load(st_xlo(s), &tx_lo, full(s), kc * BK, t.x0, el);
+        ++issued;
+        if (++s == S) { s = 0; ph ^= 1u; }
       }
-      if (*abort_flag) {
-        // let the copies this thread started land before the CTA's shared memory is released (those of a pair's second CTA
-        // complete on the other's barrier: they are given a millisecond, a thousand times what a load takes)
-        if (PAIR)
-          for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-        else
+    }
+    __syncwarp();
+    if (*abort_flag) {
+      // let the copies this warp started land before the CTA's shared memory is released (those of a pair's second CTA
+      // complete on the other's barrier: they are given a millisecond, a thousand times what a load takes)
+      if (PAIR)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+      else
         for (int i = issued > S ? issued - S : 0; i < issued; ++i) mbar_wait(full(i % S), (uint32_t)(i / S) & 1u, abort_flag + 1);
-      }
     }
   } else if (warp == 1) {
     if (rank == 0) {
     // ---------------- MMA issuer (uniform control flow, one elected lane issues) ----------------
-    auto mma = [&](uint32_t acc, uint64_t da, uint64_t db, uint32_t accumulate) {
-      if (PAIR) umma_bf16_pair(acc, da, db, a.idesc, accumulate);
-      else umma_bf16(acc, da, db, a.idesc, accumulate);
+    auto mma = [&](uint32_t acc, uint64_t da, uint64_t db, uint32_t accumulate, uint32_t el) {
+      if (PAIR) umma_bf16_pair(acc, da, db, a.idesc, accumulate, el);
+      else umma_bf16(acc, da, db, a.idesc, accumulate, el);
     };
-    auto commit = [&](uint32_t bar) {
-      if (PAIR) umma_commit_pair(bar);
-      else umma_commit(bar);
+    auto commit = [&](uint32_t bar, uint32_t el) {
+      if (PAIR) umma_commit_pair(bar, el);
+      else umma_commit(bar, el);
     };
     int s = 0, it = 0;
     uint32_t ph = 0;
@@ -440,23 +441,20 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
         tc_fence_after();
         const uint64_t dwh = gd_desc<BK>(st_whi(s)), dwl = gd_desc<BK>(st_wlo(s));
         const uint64_t dxh = gd_desc<BK>(st_xhi(s)), dxl = gd_desc<BK>(st_xlo(s));
-        if (elect_one()) {
+        const uint32_t el = elect_one();
 #pragma unroll
-          for (int k4 = 0; k4 < BK / 16; ++k4) {
-            const uint64_t adv = (uint64_t)(k4 * 2);  // 16 bf16 = 32 bytes = 2 descriptor units
-            mma(acc, dwh + adv, dxh + adv, (kc > 0 || k4 > 0) ? 1u : 0u);
-            if (NSPLIT == 3) {
-              if (WLO) mma(acc, dwl + adv, dxh + adv, 1u);
-              mma(acc, dwh + adv, dxl + adv, 1u);
-            }
+        for (int k4 = 0; k4 < BK / 16; ++k4) {
+          const uint64_t adv = (uint64_t)(k4 * 2);  // 16 bf16 = 32 bytes = 2 descriptor units
+          mma(acc, dwh + adv, dxh + adv, (kc > 0 || k4 > 0) ? 1u : 0u, el);
+          if (NSPLIT == 3) {
+            if (WLO) mma(acc, dwl + adv, dxh + adv, 1u, el);
+            mma(acc, dwh + adv, dxl + adv, 1u, el);
           }
-          commit(empty(s));  // frees the stage when these MMAs have read it
         }
-        __syncwarp();
+        commit(empty(s), el);  // frees the stage when these MMAs have read it
         if (++s == S) { s = 0; ph ^= 1u; }
       }
-      if (ok && elect_one()) commit(acc_full(b));
-      __syncwarp();
+      if (ok) commit(acc_full(b), elect_one());
     }
     }
   } else {
@@ -479,13 +477,13 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       if (a.bias && o_ok) bias4 = *reinterpret_cast<const float4 *>(a.bias + o0);
       float4 rr[4];
       if (16 * turn < BN) gd_load_res(a, rr, lane, oc, o_ok, t.m0 + 16 * turn, t.m_end);
-      int got = 0;
-      if (lane == 0) {
-        got = mbar_wait(acc_full(b), ((uint32_t)it >> 1) & 1u, abort_flag) ? 1 : 0;
-        if (!got && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 14; a.status[2] = tile; }
+      // (by all lanes: sixteen warps whose first lane alone polls slow the issuing warp down)
+      if (!mbar_wait(acc_full(b), ((uint32_t)it >> 1) & 1u, abort_flag)) {
+        if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 14; a.status[2] = tile; }
+        ok = false;
+        break;
       }
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) { ok = false; break; }
+      __syncwarp();
       tc_fence_after();
       const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * BN);
       for (int c = 16 * turn; c < BN; c += 4 * GD_EPI_WARPS) {

@@ -467,7 +467,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
   auto stage_xhi = [&](int s) { return smem + (size_t)s * stage_bytes; };
   auto stage_xlo = [&](int s) { return smem + (size_t)s * stage_bytes + xbytes; };
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int group = blockIdx.x / a.tiles_per_group;
   const int n0 = group * a.group_rows + (blockIdx.x % a.tiles_per_group) * TC_BM, n_end = min(a.N, (group + 1) * a.group_rows), m0 = blockIdx.y * bnx;
   const int shift = group * (a.group_rows - a.ygroup);   // output column = row of W - shift
@@ -607,31 +607,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
     }
     tc_fence_before();
   } else if (warp == TMA_WARP) {
-    // ---------------- activation TMA producer ----------------
-    if (lane == 0) {
+    // ---------------- activation TMA producer (uniform control flow, one elected lane issues) ----------------
+    if (elect_one()) {
       // the tensor maps are fetched while the preceding kernel still runs, not by the first copy after the wait
       tma_prefetch_map(&tm_hi);
       if (NSPLIT == 3) tma_prefetch_map(&tm_lo);
-      pdl_wait();  // x is written by the preceding kernel
-      int issued = 0, s = 0;
-      uint32_t ph = 0;
-      const int y0 = m0 + group * a.xplane;  // first row of the input plane this tile's output rows read
-      for (int kc = 0; kc < num_k; ++kc) {
-        if (!mbar_wait(empty(s), ph ^ 1u, abort_flag)) {
-          if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 3; a.status[2] = kc; }
-          break;
-        }
-        mbar_expect_tx(full(s), stage_bytes);
-        tma_load_2d(smem_u32(stage_xhi(s)), &tm_hi, full(s), (kc0 + kc) * TC_BK, y0);
-        if (NSPLIT == 3) tma_load_2d(smem_u32(stage_xlo(s)), &tm_lo, full(s), (kc0 + kc) * TC_BK, y0);
-        issued = kc + 1;
-        if (++s == S) { s = 0; ph ^= 1u; }
+    }
+    __syncwarp();
+    pdl_wait();  // x is written by the preceding kernel
+    int issued = 0, s = 0;
+    uint32_t ph = 0;
+    const int y0 = m0 + group * a.xplane;  // first row of the input plane this tile's output rows read
+    const uint32_t x0 = smem_u32(smem);
+    for (int kc = 0; kc < num_k; ++kc) {
+      if (!mbar_wait(empty(s), ph ^ 1u, abort_flag)) {
+        if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 3; a.status[2] = kc; }
+        break;
       }
-      if (*abort_flag) {
-        // let the copies this thread started land before the CTA's shared memory is released
-        for (int kc = issued > S ? issued - S : 0; kc < issued; ++kc)
-          mbar_wait(full(kc % S), (uint32_t)(kc / S) & 1u, abort_flag + 1);
-      }
+      const uint32_t el = elect_one();
+      mbar_expect_tx(full(s), stage_bytes, el);
+      const uint32_t dst = x0 + (uint32_t)s * stage_bytes;
+      tma_load_2d(dst, &tm_hi, full(s), (kc0 + kc) * TC_BK, y0, el);
+      if (NSPLIT == 3) tma_load_2d(dst + xbytes, &tm_lo, full(s), (kc0 + kc) * TC_BK, y0, el);
+      issued = kc + 1;
+      if (++s == S) { s = 0; ph ^= 1u; }
+    }
+    __syncwarp();
+    if (*abort_flag) {
+      // let the copies this warp started land before the CTA's shared memory is released
+      for (int kc = issued > S ? issued - S : 0; kc < issued; ++kc)
+        mbar_wait(full(kc % S), (uint32_t)(kc / S) & 1u, abort_flag + 1);
     }
   } else {
     // ---------------- MMA issuer ----------------
@@ -659,31 +664,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
       tc_fence_after();
       const uint32_t a_hi = t_w0 + (uint32_t)s * WCOLS, a_lo = a_hi + 32u;
       const uint64_t dxh = dx0 + (uint64_t)((uint32_t)s * stage16), dxl = dxh + (uint64_t)xlo16;
-      if (elect_one()) {
+      const uint32_t el = elect_one();
 #pragma unroll
-        for (int k4 = 0; k4 < TC_BK / 16; ++k4) {
-          const uint64_t adv = (uint64_t)(k4 * 2);  // 16 bf16 = 32 bytes = 2 descriptor units
-          const uint32_t first = (kc > 0 || k4 > 0) ? 1u : 0u;
-          if (NSPLIT == 3 && a.concat) {
-            // B = [x_hi; x_lo] (2 bnx rows, adjacent in the stage): one MMA per weight part
-            umma_bf16_ts(tmem_base, a_hi + 8u * k4, dxh + adv, a.idesc, first);
-            umma_bf16_ts(tmem_base, a_lo + 8u * k4, dxh + adv, a.idesc, 1u);
-          } else {
-            umma_bf16_ts(tmem_base, a_hi + 8u * k4, dxh + adv, a.idesc, first);
-            if (NSPLIT == 3) {
-              umma_bf16_ts(tmem_base, a_lo + 8u * k4, dxh + adv, a.idesc, 1u);
-              umma_bf16_ts(tmem_base, a_hi + 8u * k4, dxl + adv, a.idesc, 1u);
-            }
-          }
+      for (int k4 = 0; k4 < TC_BK / 16; ++k4) {
+        const uint64_t adv = (uint64_t)(k4 * 2);  // 16 bf16 = 32 bytes = 2 descriptor units
+        const uint32_t first = (kc > 0 || k4 > 0) ? 1u : 0u;
+        // concat: B = [x_hi; x_lo] (2 bnx rows, adjacent in the stage), one MMA per weight part
+        umma_bf16_ts(tmem_base, a_hi + 8u * k4, dxh + adv, a.idesc, first, el);
+        if (NSPLIT == 3) {
+          umma_bf16_ts(tmem_base, a_lo + 8u * k4, dxh + adv, a.idesc, 1u, el);
+          if (!a.concat) umma_bf16_ts(tmem_base, a_hi + 8u * k4, dxl + adv, a.idesc, 1u, el);
         }
-        umma_commit(empty(s));  // frees the stage when these MMAs have read it
       }
-      __syncwarp();
+      umma_commit(empty(s), el);  // frees the stage when these MMAs have read it
       if (lane == 0) TC_MARK(2, 22, mk);
       if (++s == S) { s = 0; ph ^= 1u; }
     }
-    if (ok && elect_one()) umma_commit(accum_bar);
-    __syncwarp();
+    if (ok) umma_commit(accum_bar, elect_one());
   }
   __syncthreads();
   if (a.cluster) {

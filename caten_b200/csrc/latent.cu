@@ -717,8 +717,8 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
           for (int k = 0; k < 8; ++k)   // 16 columns = 32 bytes = 2 descriptor units
             if (k < left)
               umma_bf16(tmem_base + col_s + NH * (i & 1), (2 * p + (k >> 2) == narrow ? dn0 : dk0) + at + (uint64_t)((k >> 2) * (LA_BLOCK >> 4) + 2 * (k & 3)),
-                        db + (uint64_t)((k >> 2) * (QB >> 4) + 2 * (k & 3)), idesc_s, p > 0 || k > 0 ? 1u : 0u);
-          if (p == np - 1) umma_commit(s_full(i & 1));
+                        db + (uint64_t)((k >> 2) * (QB >> 4) + 2 * (k & 3)), idesc_s, p > 0 || k > 0 ? 1u : 0u, 1u);
+          if (p == np - 1) umma_commit(s_full(i & 1), 1u);
         }
         __syncwarp();
       }
@@ -740,12 +740,12 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
           const uint32_t acc = tmem_base + (uint32_t)j * 2 * NH;
 #pragma unroll
           for (int k = 0; k < LA_KEYS / 16; ++k)   // A: 16 keys = 16 rows of 128 bytes = 128 descriptor units
-            umma_bf16(acc, da + (uint64_t)(128 * k), db + (uint64_t)((k >> 2) * (PB >> 5) + 2 * (k & 3)), idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
-          umma_commit(empty(s, j));
+            umma_bf16(acc, da + (uint64_t)(128 * k), db + (uint64_t)((k >> 2) * (PB >> 5) + 2 * (k & 3)), idesc_pv, (i > 0 || k > 0) ? 1u : 0u, 1u);
+          umma_commit(empty(s, j), 1u);
         }
         // (the tile's scores, which also read it, were complete before its probabilities were formed)
-        for (int p = npv; p < np; ++p) umma_commit(empty(s, p));
-        umma_commit(o_done(i & 1));
+        for (int p = npv; p < np; ++p) umma_commit(empty(s, p), 1u);
+        umma_commit(o_done(i & 1), 1u);
       }
       __syncwarp();
       if (++s == stages) s = 0;
