@@ -22,8 +22,8 @@
 //                memory as the A operand of the second product
 // so that the scores of step i + 1 and the output of step i - 1 are computed while the softmax of step i runs.  The softmax is
 // what a step waits for (about 2.5 k cycles against 1.8 k of MMAs); with the phases one after the other, conversion included,
-// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 159 us and 14 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
-// 40 us for the append -> 140 us and 67 us for append and tiles.
+// a step took 11 k.  8 x 1024 tokens, 16 heads of 128 over 4: 378 -> 142 us and 14 us for the tiles; 16 x 512 tokens, 25 heads of 64: 193 us and
+// 40 us for the append -> 92 us and 63 us for append and tiles.
 // The softmax is single-pass with a lazily moved reference maximum: each step exchanges the
 // maximum of its visible scores between the row's two threads; the reference only moves (and O and
 // the row sum are rescaled, O by a TMEM load / multiply / store) when a step exceeds it by more
@@ -71,14 +71,14 @@ __device__ __forceinline__ uint32_t sw128(int row, int chunk) {
 __device__ __forceinline__ uint4 pack8(const float4 a, const float4 b) {
   return make_uint4(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w), pack_bf16(b.x, b.y), pack_bf16(b.z, b.w));
 }
-__device__ __forceinline__ uint4 pack8_lo(const float4 a, const float4 b) {
-  return make_uint4(pack_bf16(bf16_lo(a.x), bf16_lo(a.y)), pack_bf16(bf16_lo(a.z), bf16_lo(a.w)),
-                    pack_bf16(bf16_lo(b.x), bf16_lo(b.y)), pack_bf16(bf16_lo(b.z), bf16_lo(b.w)));
+__device__ __forceinline__ uint4 pack8_lo(const float4 a, const float4 b, const uint4 hi) {
+  return make_uint4(pack_bf16_lo(a.x, a.y, hi.x), pack_bf16_lo(a.z, a.w, hi.y), pack_bf16_lo(b.x, b.y, hi.z), pack_bf16_lo(b.z, b.w, hi.w));
 }
 // 8 consecutive fp32 of one row -> one chunk of the hi row and one of the lo row
 __device__ __forceinline__ void st_split8(unsigned char *tile, int row_hi, int row_lo, int chunk, const float4 a, const float4 b) {
-  *reinterpret_cast<uint4 *>(tile + sw128(row_hi, chunk)) = pack8(a, b);
-  *reinterpret_cast<uint4 *>(tile + sw128(row_lo, chunk)) = pack8_lo(a, b);
+  const uint4 hi = pack8(a, b);
+  *reinterpret_cast<uint4 *>(tile + sw128(row_hi, chunk)) = hi;
+  *reinterpret_cast<uint4 *>(tile + sw128(row_lo, chunk)) = pack8_lo(a, b, hi);
 }
 
 // 2^x by one PTX ex2.approx instruction; results below 2^-126 flush to zero (such probabilities do not
@@ -171,7 +171,7 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + Lay::OFF_MISC + 2048 + 112);
   // [0] some role gave up a wait; [1] never set (for waits that must run their full limit)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Lay::OFF_MISC + 2048 + 120);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   const int quad = warp & 3;  // 32-lane quadrant of tensor memory this warp may access
   const int hf = warp >> 2;   // which half (of a step's keys / of a block's head dims) this thread takes
   const int r = quad * 32 + lane;  // query row within the tile = TMEM lane
@@ -216,33 +216,38 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   const uint8_t *src0 = tiles + (((int64_t)blockIdx.y * p.gn + blockIdx.x / rep) * ntiles + tile0 - at_first_tile(p)) * Lay::TILE;   // of the key/value head this query head reads
   auto copy_k = [&](int i) {
     const int st = i & 1;
-    mbar_expect_tx(k_full(st), Lay::K_BYTES);
-    bulk_load(smem_u32(sm + Lay::OFF_K) + st * Lay::K_BYTES, src0 + (int64_t)i * Lay::TILE, Lay::K_BYTES, k_full(st));
+    const uint32_t el = elect_one();
+    mbar_expect_tx(k_full(st), Lay::K_BYTES, el);
+    bulk_load(smem_u32(sm + Lay::OFF_K) + st * Lay::K_BYTES, src0 + (int64_t)i * Lay::TILE, Lay::K_BYTES, k_full(st), el);
   };
   auto copy_v = [&](int i) {
     const int st = i & 1;
-    mbar_expect_tx(v_full(st), Lay::V_BYTES);
-    bulk_load(smem_u32(sm + Lay::OFF_V) + st * Lay::V_BYTES, src0 + (int64_t)i * Lay::TILE + Lay::K_BYTES, Lay::V_BYTES, v_full(st));
+    const uint32_t el = elect_one();
+    mbar_expect_tx(v_full(st), Lay::V_BYTES, el);
+    bulk_load(smem_u32(sm + Lay::OFF_V) + st * Lay::V_BYTES, src0 + (int64_t)i * Lay::TILE + Lay::K_BYTES, Lay::V_BYTES, v_full(st), el);
   };
-  if (warp == 8 && lane == 0)
+  if (warp == 8)
     for (int i = 0; i < min(nblk, 2); ++i) {
       copy_k(i);
       copy_v(i);
     }
   // Q tiles: rows [0,128) hi, [128,256) lo per block; GPT-2's 1/8 score scale is folded in (a power of two: exact)
   if (warp < AT_SOFTMAX_WARPS) {
-    const bool okq = q0 + r < s;
-    const float4 *src = reinterpret_cast<const float4 *>(p.qkv + ((int64_t)b * s + (okq ? q0 + r : 0)) * p.ld + p.q_off + (int64_t)h * Dp);
+    // eight lanes a row (a thread's own row, piece by piece, takes 4.9 k cycles)
+    const int rq = warp * 16 + (lane >> 3), c8 = lane & 7;
 #pragma unroll
     for (int kb_ = 0; kb_ < NQ; ++kb_) {
-      float4 v[8];
+      float4 v[4][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c4 = 16 * kb_ + 8 * hf + i;
-        v[i] = okq && (PLAIN || 4 * c4 < Dp) ? scale4(src[c4], qscale) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < 4; ++i) {
+        const int row = rq + 4 * i, c = 64 * kb_ + 8 * c8;
+        const bool okq = q0 + row < s;
+        const float4 *src = reinterpret_cast<const float4 *>(p.qkv + ((int64_t)b * s + (okq ? q0 + row : 0)) * p.ld + p.q_off + (int64_t)h * Dp + c);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) v[i][u] = okq && (PLAIN || c + 4 * u < Dp) ? src[u] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) st_split8(sm + Lay::OFF_Q + kb_ * 32768, r, 128 + r, 4 * hf + c, v[2 * c], v[2 * c + 1]);
+      for (int i = 0; i < 4; ++i) st_split8(sm + Lay::OFF_Q + kb_ * 32768, rq + 4 * i, 128 + rq + 4 * i, c8, scale4(v[i][0], qscale), scale4(v[i][1], qscale));
     }
     fence_proxy_async();
   }
@@ -256,8 +261,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
   float lsum = 0.0f;    // this thread's part of the row sum, relative to m
   bool ok = true;
   if (warp == 8) {
-    // ---------------- tiles ----------------
-    if (lane == 0) {
+    // ---------------- tiles (uniform control flow, one elected lane issues) ----------------
+    {
       int ki = min(nblk, 2), vi = ki;   // copies asked for
       for (int i = 2; i < nblk; ++i) {
         const uint32_t ph = ((uint32_t)(i >> 1) & 1u) ^ 1u;
@@ -268,7 +273,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
         copy_v(i);
         ++vi;
       }
-      if (vi < nblk) give_up(16);
+      if (vi < nblk && lane == 0) give_up(16);
+      __syncwarp();
       // the copies this thread started land before the CTA's shared memory is released, whoever gives up
       for (int k = ki > 2 ? ki - 2 : 0; k < ki; ++k) mbar_wait(k_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
       for (int k = vi > 2 ? vi - 2 : 0; k < vi; ++k) mbar_wait(v_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
@@ -285,7 +291,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       const uint32_t ph = (uint32_t)(i >> 1) & 1u;
       if (!mbar_wait(k_full(st), ph, abort_flag) || !mbar_wait(s_empty(st), ph ^ 1u, abort_flag)) return false;
       tc_fence_after();
-      if (elect_one()) {
+      {
+        const uint32_t el = elect_one();
         const uint64_t dk = dk0 + (uint64_t)(st * (Lay::K_BYTES >> 4));
         const uint32_t acc = tmem_base + Lay::S_COLS * st;
 #pragma unroll
@@ -293,18 +300,17 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
           if (NQ == 1 || k < ksteps) {
             // 16 bf16 = 32 bytes = 2 descriptor units; a Q block is 32 KB = 2048 units, a K block 16 KB = 1024
             const uint64_t aq = dq + (uint64_t)((k >> 2) * 2048 + 2 * (k & 3)), ak = dk + (uint64_t)((k >> 2) * 1024 + 2 * (k & 3));
-            umma_bf16(acc, aq, ak, idesc_s, k > 0 ? 1u : 0u, 1u);
-            umma_bf16(acc, aq + 1024, ak, idesc_s, 1u, 1u);
+            umma_bf16(acc, aq, ak, idesc_s, k > 0 ? 1u : 0u, el);
+            umma_bf16(acc, aq + 1024, ak, idesc_s, 1u, el);
             if (!Lay::STACK) {
-              umma_bf16(acc, aq, ak + 512, idesc_s, 1u, 1u);
-              umma_bf16(acc, aq + 1024, ak + 512, idesc_s, 1u, 1u);
+              umma_bf16(acc, aq, ak + 512, idesc_s, 1u, el);
+              umma_bf16(acc, aq + 1024, ak + 512, idesc_s, 1u, el);
             }
           }
         }
-        umma_commit(k_empty(st), 1u);
-        umma_commit(s_full(st), 1u);
+        umma_commit(k_empty(st), el);
+        umma_commit(s_full(st), el);
       }
-      __syncwarp();
       return true;
     };
     ok = scores(0);
@@ -315,7 +321,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       if (!ok) break;
       tc_fence_after();
       const int groups = (kend - kbeg - i * AT_K + 15) / 16;   // of 16 keys that some query of the tile sees
-      if (elect_one()) {
+      {
+        const uint32_t el = elect_one();
         const uint32_t acc = tmem_base + Lay::COL_O;
         const uint64_t dv_hi = dv0 + (uint64_t)(st * (Lay::V_BYTES >> 4)), dv_lo = dv_hi + 512;
 #pragma unroll
@@ -323,14 +330,13 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
           if (k4 >= groups) break;
           const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
           const uint32_t p_hi = tmem_base + Lay::COL_P + 8 * k4, p_lo = p_hi + 32;
-          umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u, 1u);
-          umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u, 1u);
-          umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u, 1u);
+          umma_bf16_ts(acc, p_hi, dv_hi + adv, idesc_pv, (i > 0 || k4 > 0) ? 1u : 0u, el);
+          umma_bf16_ts(acc, p_lo, dv_hi + adv, idesc_pv, 1u, el);
+          umma_bf16_ts(acc, p_hi, dv_lo + adv, idesc_pv, 1u, el);
         }
-        umma_commit(v_empty(st), 1u);
-        umma_commit(pv_done, 1u);
+        umma_commit(v_empty(st), el);
+        umma_commit(pv_done, el);
       }
-      __syncwarp();
     }
     if (!ok && lane == 0) give_up(17);
     // the last products are awaited here too: tensor memory is freed below
@@ -403,14 +409,16 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       m = m_new;
       const float m_ref = m == -INFINITY ? 0.0f : m;   // (nothing visible yet: every score is -inf)
       uint32_t phi[16], plo[16];
+      float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const float p0 = ex2_approx((__uint_as_float(a[2 * e]) - m_ref) * kAtInvLn2), p1 = ex2_approx((__uint_as_float(a[2 * e + 1]) - m_ref) * kAtInvLn2);
-        lsum += p0;
-        lsum += p1;
+        s0 += p0;
+        s1 += p1;
         phi[e] = pack_bf16(p0, p1);
-        plo[e] = pack_bf16(bf16_lo(p0), bf16_lo(p1));
+        plo[e] = pack_bf16_lo(p0, p1, phi[e]);
       }
+      lsum += s0 + s1;
       if (i > 0) {   // the step before has read P and added to O
         wait(pv_done, (uint32_t)(i - 1) & 1u);
         if (!ok) continue;
@@ -442,38 +450,52 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
     float *rd = red + (nblk & 1) * 256;
     rd[hf * 128 + r] = lsum;
     pair_sync();
+    // The rows go out through shared memory (every tile has been read), 128 bytes at a time: a thread's own row in pieces of 16
+    // bytes took 5.1 k cycles.  16 x 512 tokens, 25 heads of 64, with both: 141 -> 92 us.
+    float inv = 1.0f / (rd[r] + rd[128 + r]);
+    if (!PLAIN && p.gate_off >= 0 && q0 + r < s) inv *= 1.0f / (1.0f + expf(-p.qkv[((int64_t)b * s + q0 + r) * p.ld + p.gate_off + h]));
     if (ok) {
-      float inv = 1.0f / (rd[r] + rd[128 + r]);
-      const int64_t orow = (int64_t)b * s + q0 + r;
-      if (!PLAIN && p.gate_off >= 0 && q0 + r < s) inv *= 1.0f / (1.0f + expf(-p.qkv[orow * p.ld + p.gate_off + h]));
 #pragma unroll
       for (int w = 0; w < NE; ++w) {
         uint32_t a[32];
         tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf, a);
         tmem_ld16(tlane + Lay::COL_O + 64 * w + 32 * hf + 16, a + 16);
         tmem_ld_wait();
-        float o[32];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = __uint_as_float(a[e]) * inv;
-        if (q0 + r < s) {
-          const int c0 = 64 * w + 32 * hf;
-          const int64_t at = orow * p.out_ld + (int64_t)h * Ep + c0;
+        for (int i = 0; i < 4; ++i) {
+          float4 v[2];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (!PLAIN && c0 + 8 * i >= Ep) continue;
-            const float *v = o + 8 * i;
-            if (p.bf.hi) {
-              *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) =
-                  make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-              if (p.bf.lo)
-                *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) =
-                    make_uint4(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])),
-                               pack_bf16(bf16_lo(v[4]), bf16_lo(v[5])), pack_bf16(bf16_lo(v[6]), bf16_lo(v[7])));
-            } else {
-              *reinterpret_cast<float4 *>(p.out + at + 8 * i) = make_float4(v[0], v[1], v[2], v[3]);
-              *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
-            }
+          for (int u = 0; u < 2; ++u)
+            v[u] = make_float4(__uint_as_float(a[8 * i + 4 * u]) * inv, __uint_as_float(a[8 * i + 4 * u + 1]) * inv, __uint_as_float(a[8 * i + 4 * u + 2]) * inv, __uint_as_float(a[8 * i + 4 * u + 3]) * inv);
+          unsigned char *rows = sm + w * 32768;   // bf16: high parts of 64 dims, 16 KB on the low ones; fp32: dims 0 .. 31, 32 .. 63
+          if (p.bf.hi) {
+            const uint4 hi = pack8(v[0], v[1]);
+            *reinterpret_cast<uint4 *>(rows + sw128(r, 4 * hf + i)) = hi;
+            if (p.bf.lo) *reinterpret_cast<uint4 *>(rows + 16384 + sw128(r, 4 * hf + i)) = pack8_lo(v[0], v[1], hi);
+          } else {
+            *reinterpret_cast<float4 *>(rows + 16384 * hf + sw128(r, 2 * i)) = v[0];
+            *reinterpret_cast<float4 *>(rows + 16384 * hf + sw128(r, 2 * i + 1)) = v[1];
           }
+        }
+      }
+    }
+    asm volatile("bar.sync 5, 256;" ::: "memory");
+    if (!*abort_flag) {
+      const int c8 = lane & 7;
+#pragma unroll
+      for (int w = 0; w < 2 * NE; ++w) {
+        const bool bf = p.bf.hi != nullptr;
+        if (bf && (w & 1) && !p.bf.lo) continue;
+        const int c = bf ? 64 * (w >> 1) + 8 * c8 : 32 * w + 4 * c8;   // first dim of the lane's 16 bytes
+        if (!PLAIN && c >= Ep) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = warp * 16 + 4 * i + (lane >> 3);
+          if (q0 + row >= s) continue;
+          const uint4 v = *reinterpret_cast<const uint4 *>(sm + w * 16384 + sw128(row, c8));
+          const int64_t at = ((int64_t)b * s + q0 + row) * p.out_ld + (int64_t)h * Ep + c;
+          if (!bf) *reinterpret_cast<uint4 *>(p.out + at) = v;
+          else *reinterpret_cast<uint4 *>(((w & 1) ? p.bf.lo : p.bf.hi) + at) = v;
         }
       }
     }
@@ -625,9 +647,9 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         khi[c] = pack8(kv[2 * c], kv[2 * c + 1]);
-        klo[c] = pack8_lo(kv[2 * c], kv[2 * c + 1]);
+        klo[c] = pack8_lo(kv[2 * c], kv[2 * c + 1], khi[c]);
         vhi[c] = pack8(vv[2 * c], vv[2 * c + 1]);
-        vlo[c] = pack8_lo(vv[2 * c], vv[2 * c + 1]);
+        vlo[c] = pack8_lo(vv[2 * c], vv[2 * c + 1], vhi[c]);
       }
       if (blk > 0) wait_mma();
 #pragma unroll
@@ -699,7 +721,7 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
           lsum += p0;
           lsum += p1;
           phi[e] = pack_bf16(p0, p1);
-          plo[e] = pack_bf16(bf16_lo(p0), bf16_lo(p1));
+          plo[e] = pack_bf16_lo(p0, p1, phi[e]);
         }
         tmem_st8(tlane + A1_COL_P + 16 * hf + 8 * c, phi);   // key k of the step sits in column k / 2
         tmem_st8(tlane + A1_COL_P + 32 + 16 * hf + 8 * c, plo);
@@ -744,14 +766,14 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
         float v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(a[8 * i + e]) * inv;
+        const float4 v0 = make_float4(v[0], v[1], v[2], v[3]), v1 = make_float4(v[4], v[5], v[6], v[7]);
         if (p.bf.hi) {
-          *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-          if (p.bf.lo)
-            *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) = make_uint4(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])),
-                                                                          pack_bf16(bf16_lo(v[4]), bf16_lo(v[5])), pack_bf16(bf16_lo(v[6]), bf16_lo(v[7])));
+          const uint4 hi = pack8(v0, v1);
+          *reinterpret_cast<uint4 *>(p.bf.hi + at + 8 * i) = hi;
+          if (p.bf.lo) *reinterpret_cast<uint4 *>(p.bf.lo + at + 8 * i) = pack8_lo(v0, v1, hi);
         } else {
-          *reinterpret_cast<float4 *>(p.out + at + 8 * i) = make_float4(v[0], v[1], v[2], v[3]);
-          *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+          *reinterpret_cast<float4 *>(p.out + at + 8 * i) = v0;
+          *reinterpret_cast<float4 *>(p.out + at + 8 * i + 4) = v1;
         }
       }
     }

@@ -392,6 +392,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);  // .x = a in the low half
   return *reinterpret_cast<const uint32_t *>(&v);
 }
+// the low parts of two values whose high parts are packed in `hi` (a conversion less per value than each low part by itself)
+__device__ __forceinline__ uint32_t pack_bf16_lo(float a, float b, uint32_t hi) {
+  return pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xFFFF0000u));
+}
 __device__ __forceinline__ float bf16_lo(float w) { return w - __bfloat162float(__float2bfloat16_rn(w)); }
 
 __device__ __forceinline__ float warp_sum(float v) {

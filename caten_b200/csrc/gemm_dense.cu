@@ -100,11 +100,8 @@ __device__ __forceinline__ void store_split8(const float *w, __nv_bfloat16 *hi, 
   uint32_t h[4], l[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    const __nv_bfloat16 h0 = __float2bfloat16_rn(w[2 * e]), h1 = __float2bfloat16_rn(w[2 * e + 1]);
-    h[e] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-    const __nv_bfloat16 l0 = __float2bfloat16_rn(w[2 * e] - __bfloat162float(h0));
-    const __nv_bfloat16 l1 = __float2bfloat16_rn(w[2 * e + 1] - __bfloat162float(h1));
-    l[e] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+    h[e] = pack_bf16(w[2 * e], w[2 * e + 1]);
+    l[e] = pack_bf16_lo(w[2 * e], w[2 * e + 1], h[e]);
   }
   *reinterpret_cast<uint4 *>(hi + at) = make_uint4(h[0], h[1], h[2], h[3]);
   if (lo) *reinterpret_cast<uint4 *>(lo + at) = make_uint4(l[0], l[1], l[2], l[3]);
@@ -199,8 +196,9 @@ __device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg
       const float g0 = glu(ACT, v[0], v[1]), g1 = glu(ACT, v[2], v[3]);
       const int64_t at2 = m * a.ldy + o0 / 2;
       if (a.yhi) {
-        *reinterpret_cast<uint32_t *>(a.yhi + at2) = pack_bf16(g0, g1);
-        if (a.ylo) *reinterpret_cast<uint32_t *>(a.ylo + at2) = pack_bf16(bf16_lo(g0), bf16_lo(g1));
+        const uint32_t h = pack_bf16(g0, g1);
+        *reinterpret_cast<uint32_t *>(a.yhi + at2) = h;
+        if (a.ylo) *reinterpret_cast<uint32_t *>(a.ylo + at2) = pack_bf16_lo(g0, g1, h);
       } else {
         *reinterpret_cast<float2 *>(a.y + at2) = make_float2(g0, g1);
       }
@@ -220,11 +218,8 @@ __device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg
       uint32_t h[2], l[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(v[2 * e]), h1 = __float2bfloat16_rn(v[2 * e + 1]);
-        h[e] = (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
-        const __nv_bfloat16 l0 = __float2bfloat16_rn(v[2 * e] - __bfloat162float(h0));
-        const __nv_bfloat16 l1 = __float2bfloat16_rn(v[2 * e + 1] - __bfloat162float(h1));
-        l[e] = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+        h[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+        l[e] = pack_bf16_lo(v[2 * e], v[2 * e + 1], h[e]);
       }
       *reinterpret_cast<uint2 *>(a.yhi + at) = make_uint2(h[0], h[1]);
       if (a.ylo) *reinterpret_cast<uint2 *>(a.ylo + at) = make_uint2(l[0], l[1]);

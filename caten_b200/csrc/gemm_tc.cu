@@ -97,7 +97,7 @@ __device__ __forceinline__ void emit16(uint32_t t_hi, int col, const float *w) {
   if (NSPLIT == 3) {
     uint32_t l[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) l[e] = pack_bf16(bf16_lo(w[2 * e]), bf16_lo(w[2 * e + 1]));
+    for (int e = 0; e < 8; ++e) l[e] = pack_bf16_lo(w[2 * e], w[2 * e + 1], h[e]);
     tmem_st8(t_hi + 32 + col, l);
   }
 }
@@ -325,8 +325,9 @@ __device__ __forceinline__ void store_glu4(int act, const float *r, float4 b4, c
     const float g0 = glu(act, bias ? r[0] + b4.x : r[0], bias ? r[1] + b4.y : r[1]), g1 = glu(act, bias ? r[2] + b4.z : r[2], bias ? r[3] + b4.w : r[3]);
     const int64_t at = row_at + o / 2;
     if (yhi) {
-      *reinterpret_cast<uint32_t *>(yhi + at) = pack_bf16(g0, g1);
-      if (ylo) *reinterpret_cast<uint32_t *>(ylo + at) = pack_bf16(bf16_lo(g0), bf16_lo(g1));
+      const uint32_t h = pack_bf16(g0, g1);
+      *reinterpret_cast<uint32_t *>(yhi + at) = h;
+      if (ylo) *reinterpret_cast<uint32_t *>(ylo + at) = pack_bf16_lo(g0, g1, h);
     } else {
       *reinterpret_cast<float2 *>(y + at) = make_float2(g0, g1);
     }
@@ -362,8 +363,9 @@ __device__ __forceinline__ void store_out4(int act, float *v, float4 b4, float4 
       if (res) v[e] = r[e] + v[e];
     }
     if (yhi) {
-      *reinterpret_cast<uint2 *>(yhi + at) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
-      if (ylo) *reinterpret_cast<uint2 *>(ylo + at) = make_uint2(pack_bf16(bf16_lo(v[0]), bf16_lo(v[1])), pack_bf16(bf16_lo(v[2]), bf16_lo(v[3])));
+      const uint2 h = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+      *reinterpret_cast<uint2 *>(yhi + at) = h;
+      if (ylo) *reinterpret_cast<uint2 *>(ylo + at) = make_uint2(pack_bf16_lo(v[0], v[1], h.x), pack_bf16_lo(v[2], v[3], h.y));
     } else {
       *reinterpret_cast<float4 *>(y + at) = make_float4(v[0], v[1], v[2], v[3]);
     }
@@ -808,8 +810,9 @@ __global__ void split_bf16_kernel(const float4 *__restrict__ x, uint2 *__restric
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 v = x[i];
-  hi[i] = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
-  if (lo) lo[i] = make_uint2(pack_bf16(bf16_lo(v.x), bf16_lo(v.y)), pack_bf16(bf16_lo(v.z), bf16_lo(v.w)));
+  const uint2 h = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  hi[i] = h;
+  if (lo) lo[i] = make_uint2(pack_bf16_lo(v.x, v.y, h.x), pack_bf16_lo(v.z, v.w, h.y));
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
