@@ -123,29 +123,11 @@ __global__ void __launch_bounds__(256) wsplit_kernel(const void *__restrict__ qs
   store_split8(w, hi, lo, row * K + (int64_t)o8 * 8);
 }
 
-// b[K, N] fp32 -> hi / lo [N, K] bf16 (transposed through a shared-memory tile)
-__global__ void __launch_bounds__(256) bt_split_kernel(const float *__restrict__ b, int64_t K, int64_t N, __nv_bfloat16 *__restrict__ hi,
-                                                       __nv_bfloat16 *__restrict__ lo) {
-  __shared__ float tile[32][33];
-  pdl_enter();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const int64_t k0 = (int64_t)blockIdx.y * 32, n0 = (int64_t)blockIdx.x * 32;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t k = k0 + ty + 8 * i, n = n0 + tx;
-    tile[ty + 8 * i][tx] = (k < K && n < N) ? b[k * N + n] : 0.0f;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t n = n0 + ty + 8 * i, k = k0 + tx;
-    if (n < N && k < K) {
-      const float v = tile[tx][ty + 8 * i];
-      const __nv_bfloat16 h = __float2bfloat16_rn(v);
-      hi[n * K + k] = h;
-      if (lo) lo[n * K + k] = __float2bfloat16_rn(v - __bfloat162float(h));
-    }
-  }
+// 8 consecutive fp32 of x -> bf16 hi (and lo)
+__device__ __forceinline__ void xsplit8(const float *__restrict__ x, int64_t i, __nv_bfloat16 *hi, __nv_bfloat16 *lo) {
+  const float4 a = reinterpret_cast<const float4 *>(x)[2 * i], c = reinterpret_cast<const float4 *>(x)[2 * i + 1];
+  const float w[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+  store_split8(w, hi, lo, i * 8);
 }
 
 // x fp32 [M, K] -> bf16 hi (and lo)
@@ -153,10 +135,38 @@ __global__ void __launch_bounds__(256) xsplit_kernel(const float *__restrict__ x
                                                      __nv_bfloat16 *__restrict__ lo) {
   pdl_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n8) return;
-  const float4 a = reinterpret_cast<const float4 *>(x)[2 * i], c = reinterpret_cast<const float4 *>(x)[2 * i + 1];
-  const float w[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-  store_split8(w, hi, lo, i * 8);
+  if (i < n8) xsplit8(x, i, hi, lo);
+}
+
+// Both operands of relu(a . b) in one launch: the first `tiles` CTAs bring 64 x 64 tiles of b[K, N] fp32 to [N, K] bf16 hi (and lo)
+// through shared memory, the others do as above with a.  4096 x 768 x 3072, split bf16: a launch for each, with two
+// bytes a store for b, 10.9 us of 54; so 8.8 of 52.
+__global__ void __launch_bounds__(256) operands_split_kernel(const float *__restrict__ b, int K, int N, int tiles_n, int tiles, __nv_bfloat16 *__restrict__ bhi,
+                                                             __nv_bfloat16 *__restrict__ blo, const float *__restrict__ x, int64_t n8,
+                                                             __nv_bfloat16 *__restrict__ xhi, __nv_bfloat16 *__restrict__ xlo) {
+  __shared__ float tile[64][65];
+  pdl_enter();
+  if ((int)blockIdx.x >= tiles) {
+    const int64_t i = (int64_t)(blockIdx.x - tiles) * 256 + threadIdx.x;
+    if (i < n8) xsplit8(x, i, xhi, xlo);
+    return;
+  }
+  const int k0 = (int)(blockIdx.x / tiles_n) * 64, n0 = (int)(blockIdx.x % tiles_n) * 64;   // K is a multiple of 64
+  const int tn = threadIdx.x & 63, tk = threadIdx.x >> 6;
+  float v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = n0 + tn < N ? b[(int64_t)(k0 + tk + 4 * i) * N + n0 + tn] : 0.0f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) tile[tk + 4 * i][tn] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int n = (threadIdx.x >> 3) + 32 * i, k = (threadIdx.x & 7) * 8;
+    float w[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[e] = tile[k + e][n];
+    if (n0 + n < N) store_split8(w, bhi, blo, (int64_t)(n0 + n) * K + k0 + k);
+  }
 }
 
 // ---- the GEMM -----------------------------------------------------------------------------------
@@ -661,10 +671,7 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
     case CATEN_B200_Q5_0: rc = launch_wsplit<CATEN_B200_Q5_0>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_Q5_1: rc = launch_wsplit<CATEN_B200_Q5_1>(ctx, ws, N, K, whi, wlo); break;
     case CATEN_B200_Q8_0: rc = launch_wsplit<CATEN_B200_Q8_0>(ctx, ws, N, K, whi, wlo); break;
-    case WT_F32_T:
-      launch_k(ctx, bt_split_kernel, dim3((unsigned)((N + 31) / 32), (unsigned)((K + 31) / 32)), dim3(256), 0, (const float *)ws.qs, K, N, whi, wlo);
-      CB_LAUNCH_CHECK(ctx, "bt_split_kernel");
-      break;
+    case WT_F32_T: break;   // together with x, below
     default: return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: weight type %d", wt);
   }
   if (rc) return rc;
@@ -673,13 +680,19 @@ int launch_gemm_dense(caten_b200_ctx *ctx, int wt, const WSrc &ws, const float *
     const size_t xb = ((size_t)M * K * 2 + 1023) & ~(size_t)1023;
     if (int rc2 = scratch_reserve(ctx, &ctx->xbf, xb * parts)) return rc2;
     __nv_bfloat16 *h = (__nv_bfloat16 *)ctx->xbf.ptr, *l = parts == 2 ? (__nv_bfloat16 *)((uint8_t *)ctx->xbf.ptr + xb) : nullptr;
-    const int64_t n8 = M * K / 8;
-    launch_k(ctx, xsplit_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), 0, x, n8, h, l);
+    const int64_t n8 = M * K / 8, xb_ctas = (n8 + 255) / 256;
+    if (wt == WT_F32_T) {
+      const int64_t tiles_n = (N + 63) / 64, tiles = tiles_n * (K / 64);
+      if (tiles + xb_ctas > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "gemm_dense: shape %lldx%lldx%lld", (long long)M, (long long)N, (long long)K);
+      launch_k(ctx, operands_split_kernel, dim3((unsigned)(tiles + xb_ctas)), dim3(256), 0, (const float *)ws.qs, (int)K, (int)N, (int)tiles_n, (int)tiles, whi, wlo, x, n8, h, l);
+    } else {
+      launch_k(ctx, xsplit_kernel, dim3((unsigned)xb_ctas), dim3(256), 0, x, n8, h, l);
+    }
     CB_LAUNCH_CHECK(ctx, "xsplit_kernel");
     xhi = h;
     xlo = l;
-  } else if (nsplit == 3 && !xlo) {
-    return fail(ctx, CATEN_B200_EINVAL, "gemm_dense: split-bf16 needs the lo part of x");
+  } else if (wt == WT_F32_T || (nsplit == 3 && !xlo)) {
+    return fail(ctx, CATEN_B200_EINVAL, "gemm_dense: split-bf16 needs the lo part of x, relu(matmul) an fp32 x");
   }
   if (((uintptr_t)xhi | (uintptr_t)xlo) & 15) return fail(ctx, CATEN_B200_EINVAL, "gemm_dense: bf16 operand must be 16-byte aligned");
 

@@ -429,6 +429,18 @@ def test_relu_matmul(rt, oracle, prec, tol):
         assert np.abs(got - ref).max() <= tol * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("prec", ["bf16x3", "bf16"])
+@pytest.mark.parametrize("M,K,N", [(1537, 64, 68), (1600, 192, 132), (2100, 128, 64), (1536, 320, 1000)])
+def test_relu_matmul_of_many_rows(rt, prec, M, K, N):
+    """Both operands converted in one launch: partial tiles of b, rows of a that end inside a block of threads.  Products of split
+    bf16 are within 2^-15 of sum |a b|, of plain bf16 within 2^-7."""
+    rng = np.random.Generator(np.random.PCG64(M + K + N))
+    a, b = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((K, N), dtype=np.float32)
+    got = rt.relu_matmul(rt.transfer_from_array(a), rt.transfer_from_array(b), L.PRECISIONS[prec]).numpy()
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    assert (np.abs(got - np.maximum(a64 @ b64, 0)) <= 2.0 ** (-15 if prec == "bf16x3" else -7) * (np.abs(a64) @ np.abs(b64))).all()
+
+
 def test_relu_matmul_golden(rt, golden):
     g = golden["torch_ops"]
     a = np.zeros((37, 64), np.float32); a[:] = g["mm_a"]
