@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
   const uint32_t bar = smem_u32(sm + A1_OFF_MISC + 1024);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(sm + A1_OFF_MISC + 1024 + 8);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + A1_OFF_MISC + 1024 + 12);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   const int quad = warp & 3, hf = warp >> 2, r = quad * 32 + lane;   // quadrant of tensor memory; half of a step's keys or dims; query
   const int ck = tid & 63, cq = tid >> 6;                            // conversion: key row of the step, and which 16 dims
   const int h = blockIdx.x, b = blockIdx.y, q0 = (int)(gridDim.z - 1 - blockIdx.z) * AT_Q, s = p.s, n = p.n, t = n + s;
@@ -666,18 +666,18 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
     if (!ok) break;
     if (warp == 0) {  // converged warp, one elected lane: the descriptors stay in uniform registers
       tc_fence_after();
-      if (elect_one()) {
+      {
+        const uint32_t el = elect_one();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint64_t aq = dq + (uint64_t)(2 * k), ak = dk + (uint64_t)(2 * k);   // 16 bf16 = 32 bytes = 2 descriptor units
-          umma_bf16(tmem_base + A1_COL_S, aq, ak, idesc_s, k > 0 ? 1u : 0u, 1u);
-          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak, idesc_s, 1u, 1u);
-          umma_bf16(tmem_base + A1_COL_S, aq, ak + 512, idesc_s, 1u, 1u);
-          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak + 512, idesc_s, 1u, 1u);
+          umma_bf16(tmem_base + A1_COL_S, aq, ak, idesc_s, k > 0 ? 1u : 0u, el);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak, idesc_s, 1u, el);
+          umma_bf16(tmem_base + A1_COL_S, aq, ak + 512, idesc_s, 1u, el);
+          umma_bf16(tmem_base + A1_COL_S, aq + 1024, ak + 512, idesc_s, 1u, el);
         }
-        umma_commit(bar, 1u);
+        umma_commit(bar, el);
       }
-      __syncwarp();
     }
     if (blk + 1 < nblk) fetch(j0 + AT_K);   // (after the MMAs: they are the critical path)
     wait_mma();
@@ -734,18 +734,18 @@ __global__ void __launch_bounds__(256, 2) attn_direct_tc_kernel(const AttnArgs p
     if (!ok) break;
     if (warp == 0) {
       tc_fence_after();
-      if (elect_one()) {
+      {
+        const uint32_t el = elect_one();
 #pragma unroll
         for (int k4 = 0; k4 < 4; ++k4) {
           const uint64_t adv = (uint64_t)(64 * 2 * k4);  // 16 keys = 16 rows of 128 bytes = 128 descriptor units
           const uint32_t p_hi = tmem_base + A1_COL_P + 8 * k4, p_lo = p_hi + 32;
-          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u, 1u);
-          umma_bf16_ts(tmem_base + A1_COL_O, p_lo, dv + adv, idesc_pv, 1u, 1u);
-          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + 512 + adv, idesc_pv, 1u, 1u);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + adv, idesc_pv, (blk > 0 || k4 > 0) ? 1u : 0u, el);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_lo, dv + adv, idesc_pv, 1u, el);
+          umma_bf16_ts(tmem_base + A1_COL_O, p_hi, dv + 512 + adv, idesc_pv, 1u, el);
         }
-        umma_commit(bar, 1u);
+        umma_commit(bar, el);
       }
-      __syncwarp();
     }
   }
   if (ok) wait_mma();

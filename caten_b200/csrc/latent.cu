@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int flags[2];   // [0] a wait ran out; [1] never set
   volatile int *abort_flag = flags;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   const int h0 = blockIdx.x * NH, hn = min(NH, a.H - h0), split = blockIdx.z;
   const int64_t r = blockIdx.y;
 
@@ -672,20 +672,26 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
 
   bool ok = true;
   if (warp == 8) {
-    if (lane == 0) {
+    {
       int issued = 0, s = 0;
       uint32_t ph = 1;
       const unsigned char *src = reinterpret_cast<const unsigned char *>(a.cache) + (r / a.s) * a.seq_elems() * 2 + (int64_t)tile0 * tile_bytes;
       for (int i = 0; i < nt && ok; ++i, src += tile_bytes) {
         for (int p = 0; p < np; ++p) {
-          if (!mbar_wait(empty(s, p), ph, abort_flag)) { give_up(30); ok = false; break; }
+          if (!mbar_wait(empty(s, p), ph, abort_flag)) {
+            if (lane == 0) give_up(30);
+            ok = false;
+            break;
+          }
           const uint32_t at = (uint32_t)p * 2 * LA_BLOCK, bytes = min(2 * LA_BLOCK, tile_bytes - at);
-          mbar_expect_tx(full(s, p), bytes);
-          bulk_load(smem_u32(kv) + s * tile_bytes + at, src + at, bytes, full(s, p));
+          const uint32_t el = elect_one();
+          mbar_expect_tx(full(s, p), bytes, el);
+          bulk_load(smem_u32(kv) + s * tile_bytes + at, src + at, bytes, full(s, p), el);
           ++issued;
         }
         if (++s == stages) { s = 0; ph ^= 1u; }
       }
+      __syncwarp();
       if (*abort_flag)   // copies in flight land before the CTA's shared memory is released
         for (int i = issued > stages * np ? issued - stages * np : 0; i < issued; ++i)
           mbar_wait(full(i / np % stages, i % np), (uint32_t)(i / np / stages) & 1u, abort_flag + 1);
@@ -710,17 +716,17 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
           break;
         }
         tc_fence_after();
-        if (elect_one()) {
+        {
+          const uint32_t el = elect_one();
           const uint64_t at = (uint64_t)((s * tile_bytes + (uint32_t)p * 2 * LA_BLOCK) >> 4), db = dq + (uint64_t)(2 * p * (int)(QB >> 4));
           const int left = ksteps - 8 * p;
 #pragma unroll
           for (int k = 0; k < 8; ++k)   // 16 columns = 32 bytes = 2 descriptor units
             if (k < left)
               umma_bf16(tmem_base + col_s + NH * (i & 1), (2 * p + (k >> 2) == narrow ? dn0 : dk0) + at + (uint64_t)((k >> 2) * (LA_BLOCK >> 4) + 2 * (k & 3)),
-                        db + (uint64_t)((k >> 2) * (QB >> 4) + 2 * (k & 3)), idesc_s, p > 0 || k > 0 ? 1u : 0u, 1u);
-          if (p == np - 1) umma_commit(s_full(i & 1), 1u);
+                        db + (uint64_t)((k >> 2) * (QB >> 4) + 2 * (k & 3)), idesc_s, p > 0 || k > 0 ? 1u : 0u, el);
+          if (p == np - 1) umma_commit(s_full(i & 1), el);
         }
-        __syncwarp();
       }
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
@@ -733,21 +739,21 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
         break;
       }
       tc_fence_after();
-      if (elect_one()) {
+      {
+        const uint32_t el = elect_one();
         const uint64_t db = dp + (uint64_t)((i & 1) * (int)(PB >> 4));
         for (int j = 0; j < npv; ++j) {
           const uint64_t da = dm + (uint64_t)((s * tile_bytes + (uint32_t)j * 2 * LA_BLOCK) >> 4);
           const uint32_t acc = tmem_base + (uint32_t)j * 2 * NH;
 #pragma unroll
           for (int k = 0; k < LA_KEYS / 16; ++k)   // A: 16 keys = 16 rows of 128 bytes = 128 descriptor units
-            umma_bf16(acc, da + (uint64_t)(128 * k), db + (uint64_t)((k >> 2) * (PB >> 5) + 2 * (k & 3)), idesc_pv, (i > 0 || k > 0) ? 1u : 0u, 1u);
-          umma_commit(empty(s, j), 1u);
+            umma_bf16(acc, da + (uint64_t)(128 * k), db + (uint64_t)((k >> 2) * (PB >> 5) + 2 * (k & 3)), idesc_pv, (i > 0 || k > 0) ? 1u : 0u, el);
+          umma_commit(empty(s, j), el);
         }
         // (the tile's scores, which also read it, were complete before its probabilities were formed)
-        for (int p = npv; p < np; ++p) umma_commit(empty(s, p), 1u);
-        umma_commit(o_done(i & 1), 1u);
+        for (int p = npv; p < np; ++p) umma_commit(empty(s, p), el);
+        umma_commit(o_done(i & 1), el);
       }
-      __syncwarp();
       if (++s == stages) s = 0;
     }
   } else {
