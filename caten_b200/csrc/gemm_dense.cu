@@ -580,49 +580,44 @@ static int gd_stages(int sm, int64_t M, int64_t items, int bn, int cps, size_t s
   return stages < 2 ? 2 : stages;
 }
 
-// The cut with the shortest expected time.  A CTA's stage takes as long as its MMAs (bn / 2 cycles each, at least 40) or as
-// long as its operands need from L2 (about 60 bytes a cycle and SM with every SM at work; measured: 128 x 256 tiles of
-// plain bf16 run at 0.85 of the burst rate of the tensor cores, 48 KB in 870 cycles); a CTA that goes through all of k by itself gets no
-// more than its stages in flight every 2700 cycles (2048 x 2048, 5 rows: 16 CTAs with five stages of 18 KB 12.7 us, seven shares of k and
-// the pass that sums them 8.5, the converting kernel 9.8; up to 32 rows and above 512 this predicts the better cut, between them
-// the plain estimate does: 3072 x 1024, 256 rows 10.2, 13.7 with it).  Wide tiles read least, narrow ones
-// leave no SM without work and the last wave short; shares of k pay for a pass over their partial sums.  A pair of CTAs on
-// 256 features loads 32 KB per CTA where a CTA alone loads 48, and has more stages in flight; it starts later (both CTAs
-// meet twice), and narrower tiles gain nothing from it (1665 rows, split bf16, 6400 x 1600, 224 rows wide: 91 us alone, 97).  us a call with the conversion of x, alone -> pair: 8192 rows, plain bf16,
-// 11264 x 2048 328 -> 297, 2048 x 5632 187 -> 170; split bf16, 6400 x 1600 361 -> 341; 777 rows, 4096 x 1024 13.6 -> 14.8.
+// The cut with the shortest expected time, in cycles.  A CTA's stage takes as long as its MMAs (bn / 2 cycles each, 32 at least, and
+// 110 to 200 a stage that the tensor cores wait between stages), as its operands need from L2 (52 bytes a cycle for each of
+// the SMs, shared by the CTAs that are at work), or as the stages in flight allow, which are back after about 1400 cycles.
+// Wide tiles read least, narrow ones leave no SM without work and the last wave short; shares of k pay for a pass over their
+// partial sums.  A pair of CTAs on 256 features loads half of x per CTA and starts later (both CTAs meet twice).  The constants
+// are those with which this function comes closest to the fastest cut over 740 launches of 62 shapes (5 to 8192 rows, 768 to 11264 features,
+// k of 704 to 6400, both precisions), except for what shares of k cost, which is taken from whole decode steps: on average 0.5 % from it, where the one before, which had pairs 256 rows wide only, was 4.8 %
+// (us, before -> now: 2331 rows, plain bf16, 2048 x 5632 62.6 -> 46.6 by pairs 160 wide, 2048 x 4096 46.9 -> 36.4; 5000 rows, 1280 x 5120 61.4 -> 51.6; 64 rows,
+// 1024 x 2048 9.8 -> 7.3 in four shares of 16 rows; 200 rows, 4096 x 1024 11.3 -> 9.0; split bf16, 5000 rows, 2304 x 768 45.4 -> 41.5).
 static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int nsplit, bool wlo, int bk, bool can_split, bool consumer_sums, bool can_pair, bool must_pair) {
   GdPlan best = {256, 1, (int)(K / bk), false};
   double least = 1e30;
   const int nk = (int)(K / bk), products = nsplit == 1 ? 1 : wlo ? 3 : 2, parts = nsplit == 1 ? 1 : 2;
-  for (int bn = 16; bn <= GD_BN; bn = bn < 32 ? 32 : bn + 32) {
-    if (bn == 16 && M > 16) continue;
-    const int64_t tiles = (M + bn - 1) / bn * tiles_f;
-    const double mma = (double)(bk / 16) * products * (bn > 80 ? bn / 2 : 40);
-    const double bytes = (double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)bn * parts);
-    const double epilogue = 500 + 8.0 * bn;
-    for (int splits = 1; splits <= 32; ++splits) {
-      const int cps = (nk + splits - 1) / splits, s = (nk + cps - 1) / cps;
-      if (splits > 1 && (!can_split || tiles * s > sm || cps * bk < 256)) break;
-      if (s != splits) continue;
-      const int64_t items = tiles * s;
-      const double busy = items < sm ? (double)items : (double)sm;
-      const double most = splits == 1 && (M <= 32 || M > GD_SPLIT_ROWS) ? bytes * gd_stages(sm, M, items, bn, cps, (size_t)bytes) / 2700.0 : 100.0;
-      const double rate = 60.0 * sm / busy < most ? 60.0 * sm / busy : most;
-      const double stage = mma > bytes / rate ? mma : bytes / rate, body = cps * stage;
-      const int64_t waves = (items + sm - 1) / sm;
-      double t = 1500 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
-      if (s > 1) t += (consumer_sums ? 500.0 : 5000.0) + (double)M * N * 4 * s / (sm * 30.0);
-      t *= 1.0 + 0.0003 * (GD_BN - bn);   // traffic costs power too, which is what limits long launches
-      if (t < least) { least = t; best = {bn, s, cps, false}; }
+  for (int pair = must_pair && can_pair ? 1 : 0; pair <= (can_pair ? 1 : 0); ++pair) {
+    const int workers = pair ? sm / 2 : sm;
+    for (int bn = pair ? 96 : 16; bn <= GD_BN; bn = bn < 32 ? 32 : bn + 32) {
+      if (bn == 16 && M > 64) continue;
+      const int64_t tiles = (M + bn - 1) / bn * (pair ? (N + 2 * GD_BM - 1) / (2 * GD_BM) : tiles_f);
+      const double mma = (double)(bk / 16) * products * (bn > 64 ? bn / 2 : 32) + (nsplit == 1 ? 200.0 : 110.0);
+      const double bytes = (double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)(pair ? bn / 2 : bn) * parts);
+      const double epilogue = 1360 + 20.0 * bn;
+      for (int splits = 1; splits <= 32; ++splits) {
+        const int cps = (nk + splits - 1) / splits, s = (nk + cps - 1) / cps;
+        if (splits > 1 && (pair || !can_split || tiles * s > sm || cps * bk < 256)) break;
+        if (s != splits) continue;
+        const int64_t items = tiles * s, waves = (items + workers - 1) / workers;
+        const double busy = (items < workers ? (double)items : (double)workers) * (pair ? 2 : 1);
+        const double in_flight = gd_stages(sm, M, items, bn, cps, (size_t)bytes);
+        double stage = mma > bytes * busy / (52.0 * sm) ? mma : bytes * busy / (52.0 * sm);
+        if (stage < 1400.0 / in_flight) stage = 1400.0 / in_flight;
+        const double body = cps * stage;
+        double t = (pair ? 8900 : 5900) + body + epilogue + (double)(waves - 1) * (body > 0.54 * epilogue ? body : 0.54 * epilogue);
+        if (s > 1) t += (consumer_sums ? 500.0 + 60.0 * s : 6000.0) + (double)M * N * 4 * s / (sm * 17.0);
+        t *= 1.0 + 0.0001 * (GD_BN - bn);   // traffic costs power too, which is what limits long launches
+        if (t < least) { least = t; best = {bn, s, cps, pair != 0}; }
+      }
+      if (bn >= M) break;
     }
-    if (can_pair && bn == GD_BN) {
-      const int64_t items = (M + bn - 1) / bn * ((N + 2 * GD_BM - 1) / (2 * GD_BM)), waves = (items + sm / 2 - 1) / (sm / 2);
-      const double need = ((double)bk * 2 * (GD_BM * (wlo ? 2 : 1) + (double)bn / 2 * parts)) / 60.0, body = nk * (mma > need ? mma : need);
-      const double t = 4000 + body + epilogue + (double)(waves - 1) * (body > epilogue ? body : epilogue);
-      // (a tile of a short K alone is mostly epilogue, which a wave more or less decides: 1665 rows, 3072 x 1024, plain bf16)
-      if (must_pair || (t < least && (body >= 16000 || waves >= 4))) { least = t; best = {bn, 1, nk, true}; }
-    }
-    if (bn >= M) break;
   }
   return best;
 }

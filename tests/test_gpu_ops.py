@@ -351,7 +351,7 @@ def test_gemm_many_rows_matches_the_tile_per_cta_kernel(oracle, monkeypatch):
 
 @pytest.mark.parametrize("wtype", ["q8_0", "f16", "bf16"])
 @pytest.mark.parametrize("prec,tol", [(L.PREC_BF16X3, 1e-4), (L.PREC_BF16, 4e-2)])
-@pytest.mark.parametrize("M,N,K", [(2400, 2052, 2048), (2561, 4100, 1088), (1793, 260, 64), (1537, 508, 320)])
+@pytest.mark.parametrize("M,N,K", [(2400, 2052, 2048), (2561, 4100, 1088), (1793, 260, 64), (1537, 508, 320), (1700, 2052, 192), (2049, 2300, 640)])
 def test_gemm_pairs_of_ctas(rt, monkeypatch, wtype, prec, tol, M, N, K):
     """Tiles of 256 features by two CTAs, the second one partly or wholly past the last feature, rows that end within a half, one
     stage of k and more than the ring holds; every instance of the kernel, whatever the expected time, and the same linear with
