@@ -96,6 +96,11 @@ static int check_status(caten_b200_ctx *ctx) {
   return 0;
 }
 
+int sync_published(caten_b200_ctx *ctx) {
+  CB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return check_status(ctx);
+}
+
 ProfScope::ProfScope(caten_b200_ctx *c, int klass) : ctx(c) {
   if (!(ctx->prof_mask & (1u << klass))) return;
   cudaEvent_t a;
@@ -774,7 +779,7 @@ static int head(caten_b200_gpt2 *m, int64_t s) {
   return model_linear(m, c.lm_head, norm.g ? m->h : m->last, m->last_bf, nullptr, nullptr, CATEN_B200_ACT_NONE, m->logits, cb::BfOut(), c.batch, nullptr, norm);
 }
 
-static int decode_run(caten_b200_gpt2 *m, int64_t n, int64_t steps);
+static int decode_step_device_pos(caten_b200_gpt2 *m, int64_t n_host);
 
 int caten_b200_gpt2_step_device(caten_b200_gpt2 *m, const float *d_ids_f32, const int64_t *d_ids_i64, int64_t s, int64_t n,
                                 int64_t *d_out_ids) {
@@ -813,19 +818,20 @@ int caten_b200_gpt2_step(caten_b200_gpt2 *m, const float *h_ids_f32, int64_t s, 
   if (!h_ids_f32 || !h_out_ids) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: NULL host buffer");
   if (s < 1 || s > m->desc.max_seq_len) return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: s=%lld", (long long)s);
   memcpy(m->h_ids_pinned, h_ids_f32, (size_t)(B * s) * sizeof(float));
-  CB_CUDA(ctx, cudaMemcpyAsync(m->ids_f32, m->h_ids_pinned, (size_t)(B * s) * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   if (s == 1 && ctx->prof_mask == 0) {
     // single-token step: the captured graph of the step is replayed (ids and position are loaded
     // into the device-side state first); the result is the same as the kernel-by-kernel path
     if (n < 0 || n + 1 > m->desc.max_seq_len)
       return fail(ctx, CATEN_B200_EINVAL, "gpt2_step: s=1 n=%lld outside the cache (max_seq_len=%d)", (long long)n, m->desc.max_seq_len);
-    if (int rc = launch_begin_steps(ctx, m->ids_f32, nullptr, m->loop.ids_io, m->loop.d_pos, n, B)) return rc;
-    if (int rc = decode_run(m, n, 1)) return rc;
-  } else if (int rc = caten_b200_gpt2_step_device(m, m->ids_f32, nullptr, s, n, m->loop.out_ids)) {
-    return rc;
+    if (int rc = cb::step_loop_host_step(ctx, &m->loop, n, m->desc.max_seq_len, true,
+          [&](int64_t) { return launch_begin_steps(ctx, m->h_ids_pinned, nullptr, m->loop.ids_io, m->loop.d_pos, n, B, m->loop.h_pos); },
+          [&](int64_t pos) { return decode_step_device_pos(m, pos); }, [&]() { return launch_publish(ctx, m->loop.out_ids, m->h_out_pinned, B); })) return rc;
+  } else {
+    CB_CUDA(ctx, cudaMemcpyAsync(m->ids_f32, m->h_ids_pinned, (size_t)(B * s) * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    if (int rc = caten_b200_gpt2_step_device(m, m->ids_f32, nullptr, s, n, m->loop.out_ids)) return rc;
+    if (int rc = launch_publish(ctx, m->loop.out_ids, m->h_out_pinned, B)) return rc;
   }
-  CB_CUDA(ctx, cudaMemcpyAsync(m->h_out_pinned, m->loop.out_ids, (size_t)B * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  if (int rc = caten_b200_sync(ctx)) return rc;
+  if (int rc = sync_published(ctx)) return rc;
   memcpy(h_out_ids, m->h_out_pinned, (size_t)B * sizeof(int64_t));
   return 0;
 }

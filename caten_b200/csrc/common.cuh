@@ -208,8 +208,11 @@ int launch_embed(caten_b200_ctx *ctx, const float *ids_f32, const int64_t *ids_i
                  const float *wpe, float *out, int64_t B, int64_t s, int64_t n, int64_t d, int64_t V, int64_t T,
                  const int *d_n = nullptr);
 int launch_begin_steps(caten_b200_ctx *ctx, const float *ids_f32, const int64_t *ids_i64, int64_t *ids_io, int *d_pos,
-                       int64_t n, int64_t B);
+                       int64_t n, int64_t B, const int *h_pos = nullptr);
 int launch_finish_step(caten_b200_ctx *ctx, const int64_t *out_ids, int64_t *ids_io, int64_t *hist, int *d_pos, int64_t B);
+// ids (h_ids NULL: none) and the status word to pinned host memory; sync_published waits for them and checks the status
+int launch_publish(caten_b200_ctx *ctx, const int64_t *ids, int64_t *h_ids, int64_t B);
+int sync_published(caten_b200_ctx *ctx);
 int launch_argmax(caten_b200_ctx *ctx, const float *x, int64_t rows, int64_t V, int64_t *out);
 int launch_expr(caten_b200_ctx *ctx, const caten_b200_expr *e);
 int launch_sample(caten_b200_ctx *ctx, const float *logits, int64_t rows, int64_t V, float temperature, int top_k,

@@ -861,22 +861,23 @@ int caten_b200_decoder_step(caten_b200_decoder *m, const int64_t *h_ids, int64_t
   for (int64_t i = 0; i < n_want; ++i)
     if (h_want[i] < 0 || h_want[i] >= s || (i > 0 && h_want[i] <= h_want[i - 1])) return fail(ctx, CATEN_B200_EINVAL, "decoder_step: wanted places must be ascending and inside the step");
   memcpy(m->h_ids, h_ids, (size_t)(B * s) * sizeof(int64_t));
-  CB_CUDA(ctx, cudaMemcpyAsync(m->ids, m->h_ids, (size_t)(B * s) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
   if (s == 1) {
     // the captured graph of a single-token step; it always forms the logits
-    if (int rc = launch_begin_steps(ctx, nullptr, m->ids, m->loop.ids_io, m->loop.d_pos, n, B)) return rc;
-    if (int rc = decode_run(m, n, 1)) return rc;
+    if (int rc = step_loop_host_step(ctx, &m->loop, n, m->desc.max_seq_len, ctx->prof_mask == 0 && !m->capture,
+          [&](int64_t) { return launch_begin_steps(ctx, nullptr, m->h_ids, m->loop.ids_io, m->loop.d_pos, n, B, m->loop.h_pos); },
+          [&](int64_t pos) { return decode_step_device_pos(m, pos); }, [&]() { return launch_publish(ctx, m->loop.out_ids, m->h_out, B); })) return rc;
     if (n_want) CB_CUDA(ctx, cudaMemcpyAsync(h_logits, m->logits, (size_t)(B * V) * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   } else {
+    CB_CUDA(ctx, cudaMemcpyAsync(m->ids, m->h_ids, (size_t)(B * s) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     if (int rc = run_step(m, m->ids, s, n, h_want, n_want, h_logits, h_out_ids != nullptr)) return rc;
     if (h_out_ids) {
       ProfScope prof(ctx, CATEN_B200_K_ARGMAX);
       if (int rc = launch_argmax(ctx, m->logits, B, V, m->loop.out_ids)) return rc;
     }
+    if (int rc = launch_publish(ctx, m->loop.out_ids, h_out_ids ? m->h_out : nullptr, B)) return rc;
   }
   m->pos = n + s;
-  if (h_out_ids) CB_CUDA(ctx, cudaMemcpyAsync(m->h_out, m->loop.out_ids, (size_t)B * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  if (int rc = caten_b200_sync(ctx)) return rc;
+  if (int rc = sync_published(ctx)) return rc;
   if (h_out_ids) memcpy(h_out_ids, m->h_out, (size_t)B * sizeof(int64_t));
   return 0;
 }

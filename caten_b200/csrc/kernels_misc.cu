@@ -437,9 +437,11 @@ __global__ void finish_step_kernel(const int64_t *__restrict__ out_ids, int64_t 
 // Start of a run of graph-replayed steps: loads the input ids (int64, or float32 as the reference's
 // caller passes them; an id that is not an integer selects no embedding row, kept as -1) and the
 // start position into the device-side state.
+// (h_pos: the position is in pinned host memory, as the ids are then)
 __global__ void begin_steps_kernel(const float *__restrict__ ids_f32, const int64_t *__restrict__ ids_i64,
-                                   int64_t *__restrict__ ids_io, int *__restrict__ d_pos, int n, int B) {
+                                   int64_t *__restrict__ ids_io, int *__restrict__ d_pos, int n, int B, const volatile int *h_pos) {
   pdl_enter();
+  if (h_pos && threadIdx.x == 0) n = *h_pos;
   for (int b = threadIdx.x; b < B; b += blockDim.x) {
     if (ids_i64) {
       ids_io[b] = ids_i64[b];
@@ -451,9 +453,23 @@ __global__ void begin_steps_kernel(const float *__restrict__ ids_f32, const int6
   if (threadIdx.x == 0) *d_pos = n;
 }
 
+// What the host waits for at the end of a step: the new ids and the status word, written to pinned host memory.  (Two copies
+// queued behind the step took 18 us of a decode step, one after the other, each started by the one before.)
+__global__ void publish_kernel(const int64_t *__restrict__ ids, int64_t *__restrict__ h_ids, int B, const int *__restrict__ d_status, int *__restrict__ h_status) {
+  pdl_enter();
+  for (int b = threadIdx.x; b < B; b += blockDim.x) h_ids[b] = ids[b];
+  if (threadIdx.x < 4) h_status[threadIdx.x] = d_status[threadIdx.x];
+}
+
+int launch_publish(caten_b200_ctx *ctx, const int64_t *ids, int64_t *h_ids, int64_t B) {
+  launch_k(ctx, publish_kernel, dim3(1), dim3(256), 0, ids, h_ids, h_ids ? (int)B : 0, ctx->d_status, ctx->h_status);
+  CB_LAUNCH_CHECK(ctx, "publish_kernel");
+  return 0;
+}
+
 int launch_begin_steps(caten_b200_ctx *ctx, const float *ids_f32, const int64_t *ids_i64, int64_t *ids_io, int *d_pos,
-                       int64_t n, int64_t B) {
-  launch_k(ctx, begin_steps_kernel, dim3(1), dim3(256), 0, ids_f32, ids_i64, ids_io, d_pos, (int)n, (int)B);
+                       int64_t n, int64_t B, const int *h_pos) {
+  launch_k(ctx, begin_steps_kernel, dim3(1), dim3(256), 0, ids_f32, ids_i64, ids_io, d_pos, (int)n, (int)B, h_pos);
   CB_LAUNCH_CHECK(ctx, "begin_steps_kernel");
   return 0;
 }
