@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
   const uint32_t bar0 = smem_u32(bars);
   auto full = [&](int s) { return bar0 + 8u * s; };
   auto empty = [&](int s) { return bar0 + 8u * (AD_MAX_STAGES + s); };
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = warp_index();
   const int h0 = blockIdx.x * HPC, b = blockIdx.y, rank = blockIdx.z;
   const int rep = a.H / a.G, g = h0 / rep, cap = (int)a.cap;
   float *kb = a.kc + ((int64_t)b * a.G + g) * a.cap * Dp;
@@ -380,7 +380,9 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
     }
   }
   __syncthreads();
-  pdl_enter();
+  // a.early: the copies of the history, which depend on nothing in flight, start at once, and the ring is full when q arrives
+  if (warp != AD_WORK / 32 || !a.early) pdl_wait();
+  pdl_launch_dependents();
   const int n = a.d_n ? *a.d_n : a.n;
   int jb, je;
   range(n, jb, je);
@@ -389,12 +391,12 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
   const int cnt = hist + (own_new ? 1 : 0);
 
   if (warp == AD_WORK / 32) {
-    if (lane == 0) {
+    {   // uniform control flow, one elected lane issues
       int issued = 0, s = 0;
       uint32_t ph = 1;   // (a fresh barrier's previous phase counts as complete)
       for (int i = 0; i < 2 * nc; ++i) {
         if (!mbar_wait(empty(s), ph, abort_flag)) {
-          if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, DEV_WAIT_TIMEOUT); status[1] = 20; }
+          if (lane == 0 && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, DEV_WAIT_TIMEOUT); status[1] = 20; }
           break;
         }
         const bool isv = i >= nc;
@@ -402,12 +404,14 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
         const int rows = min(CH, hist - c * CH), s0 = (jb + c * CH) % cap, r0 = min(rows, cap - s0);
         const float *base = isv ? vb : kb;
         const uint32_t dst = smem_u32(ring + s * CH * wide);
-        mbar_expect_tx(full(s), (uint32_t)(rows * w) * 4u);
-        bulk_load(dst, base + (int64_t)s0 * w, (uint32_t)(r0 * w) * 4u, full(s));
-        if (r0 < rows) bulk_load(dst + (uint32_t)(r0 * w) * 4u, base, (uint32_t)((rows - r0) * w) * 4u, full(s));
+        const uint32_t el = elect_one();
+        mbar_expect_tx(full(s), (uint32_t)(rows * w) * 4u, el);
+        bulk_load(dst, base + (int64_t)s0 * w, (uint32_t)(r0 * w) * 4u, full(s), el);
+        if (r0 < rows) bulk_load(dst + (uint32_t)(r0 * w) * 4u, base, (uint32_t)((rows - r0) * w) * 4u, full(s), el);
         issued = i + 1;
         if (++s == stages) { s = 0; ph ^= 1u; }
       }
+      __syncwarp();
       if (*abort_flag)  // copies in flight land before the CTA's shared memory is released
         for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait(full(i % stages), (uint32_t)(i / stages) & 1u, abort_flag + 1);
     }

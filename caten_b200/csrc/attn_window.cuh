@@ -32,6 +32,7 @@ struct AttnArgs {
   const float *freq = nullptr;
   int qk_norm = 0;                  // q and k divided by their root mean square over D after the rotation
   float eps = 0.0f, scale = 1.0f;   // score = q . k * scale
+  bool early = false;               // single-token steps: position and cache are complete before the kernel in front of this one starts
   int g0 = 0, gn = 0;               // attention_tc.cu: the key/value heads [g0, g0 + gn) of one launch
 
   void fill_strides() {

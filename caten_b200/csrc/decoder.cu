@@ -695,6 +695,7 @@ class StepRunner {
     a.B = (int)p_.nb; a.s = (int)p_.s; a.n = (int)p_.n; a.d_n = p_.d_n;
     a.window = c.window; a.rot_pairs = c.rot_dims / 2; a.freq = c.rot_freq; a.qk_norm = c.qk_norm; a.eps = m_->desc.eps; a.scale = c.scale;
     if (p_.s == 1) {
+      a.early = true;   // (the norm in front of the projections starts nothing before everything in front of it is complete)
       ProfScope prof(ctx_, CATEN_B200_K_ATTN_DECODE);
       return launch_attn_window_decode(ctx_, a);
     }
