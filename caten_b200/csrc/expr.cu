@@ -45,13 +45,39 @@ __device__ __forceinline__ uint32_t expr_cast(uint32_t v, int from, int to) {
   return to == CATEN_B200_CLS_BOOL ? (v != 0u ? 1u : 0u) : v;                          // I32 <-> BOOL
 }
 
+// 2^x rounded once from double: x = n + f with n the nearest integer (the difference is exact), 2^f by 1 + f q(f), q the
+// polynomial of degree 8 through (2^f - 1) / f at the Chebyshev nodes of [-1/2, 1/2] (relative error 2^-44, none at whole
+// numbers), n added to the exponent; past +-160 the conversion gives 0 or inf either way.  Nine fused steps and no branch: an
+// exp2 item over 12800 x 511 takes 18.2 us, with exp2(double) 31.8 (and 26 before words were one class each).
+__device__ __forceinline__ float expr_exp2(float x) {
+  x = x > 160.0f ? 160.0f : x;
+  x = x < -160.0f ? -160.0f : x;
+  const float big = 12582912.0f;           // 1.5 * 2^23: adding it rounds to an integer
+  const float t = x + big;
+  const double f = (double)(x - (t - big));
+  double p = 1.0203121063391729e-07;
+  p = fma(p, f, 1.3255224878668817e-06);
+  p = fma(p, f, 1.525268684626772e-05);
+  p = fma(p, f, 0.00015403455852453838);
+  p = fma(p, f, 0.0013333558179043112);
+  p = fma(p, f, 0.009618129159402558);
+  p = fma(p, f, 0.055504108664760424);
+  p = fma(p, f, 0.2402265069581299);
+  p = fma(p, f, 0.6931471805599453);
+  p = fma(p, f, 1.0);
+  const float y = (float)__hiloint2double(__double2hiint(p) + ((__float_as_int(t) - 0x4b400000) << 20), __double2loint(p));
+  return x != x ? x : y;
+}
+
 constexpr int EXPR_THREADS = 256;
 constexpr int MAXD = CATEN_B200_EXPR_MAX_DIMS;
 
-// Words as the kernels see them (expr_fuse writes them from the caller's program): bits 24..26 say where a word's right
+// Words as the kernels see them (expr_fuse writes them from the caller's program): bits 24..26 say where a binary word's right
 // operand comes from, so that `LOAD b; ADD` or `CONST c; MUL` is one word that touches no stack slot; bit 27 / 28: the right
-// operand is negated / replaced by its reciprocal first (`LOAD b; NEG; ADD` and `LOAD b; RECIP; MUL`, floats).
-enum ExprMode : uint32_t { EXPR_POP = 0, EXPR_WITH_CONST = 1u << 24, EXPR_WITH_LOAD = 2u << 24, EXPR_MODES = 7u << 24, EXPR_NEG_B = 1u << 27, EXPR_RECIP_B = 1u << 28 };
+// operand is negated / replaced by its reciprocal first (`LOAD b; NEG; ADD` and `LOAD b; RECIP; MUL`, floats); bit 29: a binary
+// word.  An op that floats and whole numbers share has a code of its own for the latter, so that a word computes one of the two.
+enum ExprMode : uint32_t { EXPR_POP = 0, EXPR_WITH_CONST = 1u << 24, EXPR_WITH_LOAD = 2u << 24, EXPR_MODES = 7u << 24, EXPR_NEG_B = 1u << 27, EXPR_RECIP_B = 1u << 28, EXPR_BINARY = 1u << 29 };
+constexpr int EXPR_WHOLE = 64;   // added to the code of NEG, RECIP, NOT, ADD, MUL, MAX, NE and LT on whole numbers, and to LOAD of them
 
 // Per-thread state is kept out of local memory: with 2048 threads per SM a few hundred bytes of
 // local arrays each overflow L1 and turn every stack access into L2 traffic.  The loop indices
@@ -65,30 +91,28 @@ template <int ND> struct ExprIx {
 // EV values of operand `arg`: element j is 32 j further along loop `va`; for j >= lanes the last element is re-read, so
 // nothing outside the views is touched.
 template <int ND, int EV>
-__device__ __forceinline__ void expr_load_ev(const caten_b200_expr &e, const int arg, const ExprIx<ND> &ix, const int va, const int lanes, uint32_t *out) {
-  const int dt = e.operand_dtype[arg];
+__device__ __forceinline__ void expr_load_ev(const caten_b200_expr &e, const int arg, const ExprIx<ND> &ix, const int va, const int lanes, const bool whole, uint32_t *out) {
   int64_t o = e.operand_offset[arg];
 #pragma unroll
   for (int d = 0; d < ND; ++d) o += (int64_t)ix.v[d] * e.operand_stride[arg][d];
   const int64_t step = va >= 0 ? 32 * e.operand_stride[arg][va] : 0;
   const int last = lanes > 0 ? lanes - 1 : 0;
-  if (dt == CATEN_B200_DT_F32) {  // the common case without the per-element type switch
+  if (!whole) {
     const float *p = reinterpret_cast<const float *>(e.operand[arg]) + o;
     if (step == 0) {
       const uint32_t v = __float_as_uint(*p);
 #pragma unroll
       for (int j = 0; j < EV; ++j) out[j] = v;
-      return;
-    }
-    if (step == 32) {   // the strip is contiguous
+    } else if (step == 32 && lanes == EV) {   // the strip is contiguous and full
 #pragma unroll
-      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * 32]);
-      return;
-    }
+      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[32 * j]);
+    } else {
 #pragma unroll
-    for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * step]);
+      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * step]);
+    }
     return;
   }
+  const int dt = e.operand_dtype[arg];
 #pragma unroll
   for (int j = 0; j < EV; ++j) out[j] = expr_load(e.operand[arg], dt, o + (j < last ? j : last) * step);
 }
@@ -96,7 +120,7 @@ __device__ __forceinline__ void expr_load_ev(const caten_b200_expr &e, const int
 // Runs the program for EV elements at once: the decode of a word is shared.  Element j of the
 // thread is 32 j further along loop `va` (va < 0: a single element).  HEAVY: with the words whose code takes twice the
 // registers (sines and logarithms in double, integer division); programs without them run in the lean form, of which twice
-// as many warps are resident (exp2 and division items over 12800 x 511: 50 us before, 36 us without the split, 27 us with it).
+// as many warps are resident (exp2 and division items over 12800 x 511: 36 us without the split, 27 us with it, 25 and 19 now).
 template <int ND, int EV, int THREADS, bool HEAVY>
 __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx<ND> &ix, const int va, const int lanes, uint32_t *tos, uint32_t *sm) {
   int sp = 0;  // values on the stack, the top one (registers) included
@@ -108,58 +132,64 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx<
     }
     ++sp;
   };
-#define EXPR_UN(EXPR_F, EXPR_I)                                                    \
+#define EXPR_UN(VALUE)                                                             \
   {                                                                                \
     _Pragma("unroll") for (int j = 0; j < EV; ++j) {                               \
       const uint32_t a = tos[j];                                                   \
       const float fa = __uint_as_float(a);                                         \
       const int32_t ia = (int32_t)a;                                               \
       (void)fa; (void)ia;                                                          \
-      tos[j] = f ? (EXPR_F) : (EXPR_I);                                            \
+      tos[j] = VALUE;                                                              \
     }                                                                              \
     break;                                                                         \
   }
-#define EXPR_BIN(EXPR_F, EXPR_I)                                                   \
+#define EXPR_BIN(VALUE)                                                            \
   {                                                                                \
     _Pragma("unroll") for (int j = 0; j < EV; ++j) {                               \
       const uint32_t a = tos[j], b = r[j];                                         \
       const float fa = __uint_as_float(a), fb = __uint_as_float(b);                \
       const int32_t ia = (int32_t)a, ib = (int32_t)b;                              \
       (void)fa; (void)fb; (void)ia; (void)ib;                                      \
-      tos[j] = f ? (EXPR_F) : (EXPR_I);                                            \
+      tos[j] = VALUE;                                                              \
     }                                                                              \
     break;                                                                         \
   }
   for (int pc = 0; pc < e.n_code; ++pc) {
     const uint32_t w = e.code[pc];
-    const int op = w & 255, arg = (w >> 8) & 255, cls = (w >> 16) & 255;
-    const bool f = cls == CATEN_B200_CLS_F32;
+    const int op = w & 255, arg = (w >> 8) & 255;
     uint32_t r[EV];   // right operand of a binary word; tos becomes the left one
-    if (op >= CATEN_B200_OP_ADD && op <= CATEN_B200_OP_LT) {
+    if (w & EXPR_BINARY) {
       const uint32_t mode = w & EXPR_MODES;
-      if (mode == EXPR_WITH_LOAD) {
-        expr_load_ev<ND, EV>(e, arg, ix, va, lanes, r);
-      } else if (mode == EXPR_WITH_CONST) {
-#pragma unroll
-        for (int j = 0; j < EV; ++j) r[j] = e.consts[arg];
-      } else {
+      if (mode == EXPR_POP) {
         --sp;
 #pragma unroll
         for (int j = 0; j < EV; ++j) { r[j] = tos[j]; tos[j] = slot(sp - 1, j); }
-      }
-      if (w & EXPR_NEG_B) {
+      } else {
+        const bool one = mode == EXPR_WITH_CONST || va < 0 || e.operand_stride[arg][va] == 0;   // one value for all of them
+        if (mode == EXPR_WITH_LOAD) {
+          expr_load_ev<ND, EV>(e, arg, ix, va, lanes, op >= EXPR_WHOLE || (op >= CATEN_B200_OP_MOD && op <= CATEN_B200_OP_XOR), r);
+        } else {
+          r[0] = e.consts[arg];
+        }
+        if (w & EXPR_NEG_B) {
 #pragma unroll
-        for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(-__uint_as_float(r[j]));
-      }
-      if (w & EXPR_RECIP_B) {
+          for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(-__uint_as_float(r[j]));
+        }
+        if (one) {
+          if (w & EXPR_RECIP_B) r[0] = __float_as_uint(1.0f / __uint_as_float(r[0]));
 #pragma unroll
-        for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(1.0f / __uint_as_float(r[j]));
+          for (int j = 1; j < EV; ++j) r[j] = r[0];
+        } else if (w & EXPR_RECIP_B) {
+#pragma unroll
+          for (int j = 0; j < EV; ++j) r[j] = __float_as_uint(1.0f / __uint_as_float(r[j]));
+        }
       }
     }
     switch (op) {
       case CATEN_B200_OP_LOAD:
+      case CATEN_B200_OP_LOAD + EXPR_WHOLE:
         push();
-        expr_load_ev<ND, EV>(e, arg, ix, va, lanes, tos);
+        expr_load_ev<ND, EV>(e, arg, ix, va, lanes, op >= EXPR_WHOLE, tos);
         break;
       case CATEN_B200_OP_CONST:
         push();
@@ -176,28 +206,37 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx<
         for (int j = 0; j < EV; ++j) tos[j] = (uint32_t)(base + (arg == va ? 32 * j : 0));
         break;
       }
-      case CATEN_B200_OP_NEG: EXPR_UN(__float_as_uint(-fa), (uint32_t)(-ia))
-      case CATEN_B200_OP_RECIP: EXPR_UN(__float_as_uint(1.0f / fa), (ia == 1 || ia == -1 ? (uint32_t)ia : 0u))
-      case CATEN_B200_OP_SIN: EXPR_UN(HEAVY ? __float_as_uint((float)sin((double)fa)) : a, a)
-      case CATEN_B200_OP_EXP2: EXPR_UN(__float_as_uint((float)exp2((double)fa)), a)
-      case CATEN_B200_OP_LOG2: EXPR_UN(HEAVY ? __float_as_uint((float)log2((double)fa)) : a, a)
-      case CATEN_B200_OP_SQRT: EXPR_UN(HEAVY ? __float_as_uint((float)sqrt((double)fa)) : a, a)
-      case CATEN_B200_OP_NOT: EXPR_UN((fa == 0.0f ? 1u : 0u), (a == 0u ? 1u : 0u))
+      case CATEN_B200_OP_NEG: EXPR_UN(__float_as_uint(-fa))
+      case CATEN_B200_OP_NEG + EXPR_WHOLE: EXPR_UN((uint32_t)(-ia))
+      case CATEN_B200_OP_RECIP: EXPR_UN(__float_as_uint(1.0f / fa))
+      case CATEN_B200_OP_RECIP + EXPR_WHOLE: EXPR_UN((ia == 1 || ia == -1 ? (uint32_t)ia : 0u))
+      case CATEN_B200_OP_SIN: EXPR_UN(HEAVY ? __float_as_uint((float)sin((double)fa)) : a)
+      case CATEN_B200_OP_EXP2: EXPR_UN(__float_as_uint(expr_exp2(fa)))
+      case CATEN_B200_OP_LOG2: EXPR_UN(HEAVY ? __float_as_uint((float)log2((double)fa)) : a)
+      case CATEN_B200_OP_SQRT: EXPR_UN(HEAVY ? __float_as_uint((float)sqrt((double)fa)) : a)
+      case CATEN_B200_OP_NOT: EXPR_UN((fa == 0.0f ? 1u : 0u))
+      case CATEN_B200_OP_NOT + EXPR_WHOLE: EXPR_UN((a == 0u ? 1u : 0u))
       case CATEN_B200_OP_CAST: {
+        const int cls = (w >> 16) & 255;
 #pragma unroll
         for (int j = 0; j < EV; ++j) tos[j] = expr_cast(tos[j], arg, cls);
         break;
       }
-      case CATEN_B200_OP_ADD: EXPR_BIN(__float_as_uint(fa + fb), (uint32_t)(ia + ib))
-      case CATEN_B200_OP_MUL: EXPR_BIN(__float_as_uint(fa * fb), (uint32_t)(ia * ib))
-      case CATEN_B200_OP_MOD: EXPR_BIN(a, (!HEAVY || ib == 0 ? 0u : (uint32_t)(ia % ib)))
-      case CATEN_B200_OP_IDIV: EXPR_BIN(a, (!HEAVY || ib == 0 ? 0u : (uint32_t)(ia / ib)))
-      case CATEN_B200_OP_AND: EXPR_BIN(a & b, a & b)
-      case CATEN_B200_OP_OR: EXPR_BIN(a | b, a | b)
-      case CATEN_B200_OP_XOR: EXPR_BIN(a ^ b, a ^ b)
-      case CATEN_B200_OP_MAX: EXPR_BIN((fa > fb ? a : b), (ia > ib ? a : b))
-      case CATEN_B200_OP_NE: EXPR_BIN((fa != fb ? 1u : 0u), (a != b ? 1u : 0u))
-      case CATEN_B200_OP_LT: EXPR_BIN((fa < fb ? 1u : 0u), (ia < ib ? 1u : 0u))
+      case CATEN_B200_OP_ADD: EXPR_BIN(__float_as_uint(fa + fb))
+      case CATEN_B200_OP_ADD + EXPR_WHOLE: EXPR_BIN((uint32_t)(ia + ib))
+      case CATEN_B200_OP_MUL: EXPR_BIN(__float_as_uint(fa * fb))
+      case CATEN_B200_OP_MUL + EXPR_WHOLE: EXPR_BIN((uint32_t)(ia * ib))
+      case CATEN_B200_OP_MOD: EXPR_BIN((!HEAVY || ib == 0 ? 0u : (uint32_t)(ia % ib)))
+      case CATEN_B200_OP_IDIV: EXPR_BIN((!HEAVY || ib == 0 ? 0u : (uint32_t)(ia / ib)))
+      case CATEN_B200_OP_AND: EXPR_BIN(a & b)
+      case CATEN_B200_OP_OR: EXPR_BIN(a | b)
+      case CATEN_B200_OP_XOR: EXPR_BIN(a ^ b)
+      case CATEN_B200_OP_MAX: EXPR_BIN((fa > fb ? a : b))
+      case CATEN_B200_OP_MAX + EXPR_WHOLE: EXPR_BIN((ia > ib ? a : b))
+      case CATEN_B200_OP_NE: EXPR_BIN((fa != fb ? 1u : 0u))
+      case CATEN_B200_OP_NE + EXPR_WHOLE: EXPR_BIN((a != b ? 1u : 0u))
+      case CATEN_B200_OP_LT: EXPR_BIN((fa < fb ? 1u : 0u))
+      case CATEN_B200_OP_LT + EXPR_WHOLE: EXPR_BIN((ia < ib ? 1u : 0u))
       default: {  // WHERE: (cond a b) with b on top
         sp -= 2;
 #pragma unroll
@@ -210,14 +249,24 @@ __device__ __forceinline__ void expr_run(const caten_b200_expr &e, const ExprIx<
 #undef EXPR_BIN
 }
 
-// loop indices of flat position `pos` over loops [first, last) -> ix (innermost fastest)
+// loop indices of flat position `pos` over loops [first, last) -> ix (innermost fastest).  The outermost one is what is left;
+// the others divide in 32 bits where the position has no more (a 64-bit division is some 80 instructions, paid per strip).
 template <int ND>
 __device__ __forceinline__ void expr_decode(const caten_b200_expr &e, int64_t pos, const int first, const int last, ExprIx<ND> &ix) {
 #pragma unroll
   for (int d = ND - 1; d >= 0; --d) {
-    if (d >= first && d < last) {
-      ix.v[d] = (int)(pos % e.shape[d]);
-      pos /= e.shape[d];
+    if (d > first && d < last) {
+      const uint32_t n = (uint32_t)e.shape[d];   // (an extent is at most 2^31 - 1)
+      if ((uint64_t)pos >> 32) {
+        ix.v[d] = (int)(pos % n);
+        pos /= n;
+      } else {
+        const uint32_t q = (uint32_t)pos / n;
+        ix.v[d] = (int)((uint32_t)pos - q * n);
+        pos = q;
+      }
+    } else if (d == first && d < last) {
+      ix.v[d] = (int)pos;
     }
   }
 }
@@ -261,11 +310,14 @@ __device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const
 
 // A warp owns strips of 32 * EV consecutive elements of the innermost kept loop; lane l takes
 // elements l, l + 32, ... of a strip, so every load and store of the warp is coalesced.  Each
-// warp takes `spw` consecutive strips of one row, so the index decoding (64-bit divisions) is
-// paid once per warp.  Reduced loops (if any) are walked by each thread in loop order, exactly
-// like the rendered loop nest, so a float sum is added in the reference's order.
+// warp takes `spw` consecutive strips of one row, so the index decoding is paid once per warp.
+// Reduced loops (if any) are walked by each thread in loop order, exactly like the rendered loop
+// nest, so a float sum is added in the reference's order.  What bounds an item is its words: some
+// 2 us each over 12800 x 511 (a copy 10.7 us out of L2, 14.5 out of memory, gelu's 14 words 53;
+// 12.8, 16.0 and 65 with 64-bit divisions per warp, both classes computed by each word and a clamp
+// per element).  Four elements a thread in place of eight: gelu 89 us; three CTAs per SM: 57.
 template <int ND, int EV, bool HEAVY>
-__global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int spw,
+__global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int groups_per_row, const int spw,
                                                             const int64_t n_red, const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
   pdl_enter();
@@ -276,13 +328,12 @@ __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_cons
   const int nd_out = e.ndim - e.n_reduce;
   const int va = nd_out - 1;  // the loop the strips run along (-1: a single output element)
   const int64_t vlen = va >= 0 ? e.shape[va] : 1;
-  const int64_t strips_per_row = (vlen + 32 * EV - 1) / (32 * EV);
-  const int64_t groups_per_row = (strips_per_row + spw - 1) / spw;
   ExprIx<ND> ix;
 #pragma unroll
   for (int d = 0; d < ND; ++d) ix.v[d] = 0;
-  expr_decode(e, group / groups_per_row, 0, va, ix);
-  int64_t j0 = (group % groups_per_row) * spw * (32 * EV) + lane;  // this thread's first element; the others follow 32 apart
+  const int64_t row = (uint64_t)group >> 32 ? group / groups_per_row : (int64_t)((uint32_t)group / (uint32_t)groups_per_row);
+  expr_decode(e, row, 0, va, ix);
+  int64_t j0 = (group - row * groups_per_row) * spw * (32 * EV) + lane;  // this thread's first element; the others follow 32 apart
   const bool is_f = result_cls == CATEN_B200_CLS_F32, is_sum = e.reduce_op == CATEN_B200_RED_SUM;
   const int64_t ovs = va >= 0 ? 32 * e.out_stride[va] : 0;
   for (int s = 0; s < spw && j0 < vlen; ++s, j0 += 32 * EV) {
@@ -294,6 +345,13 @@ __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_cons
     uint32_t val[EV];
     if (e.n_reduce == 0) {
       expr_run<ND, EV, EXPR_THREADS, HEAVY>(e, ix, va, lanes, val, sm);
+      if (is_f && e.out_dtype == CATEN_B200_DT_F32 && ovs == 32) {   // without the type switch per element
+        float *p = reinterpret_cast<float *>(e.out) + out_at;
+#pragma unroll
+        for (int j = 0; j < EV; ++j)
+          if (j < lanes) p[32 * j] = __uint_as_float(val[j]);
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < EV; ++j)
         if (j < lanes) expr_store(e.out, e.out_dtype, out_at + j * ovs, val[j], result_cls);
@@ -319,12 +377,96 @@ __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_cons
 // shuffles spends a warp's instructions on a single sum.  So a CTA takes R output elements: eight warps evaluate tiles of
 // R x C values with lanes along the reduced loop and leave them in shared memory (rows C + 1 apart, no bank conflicts), and a
 // ninth warp, one lane per output element, adds the tile before in loop order meanwhile.  12800 rows of 511: 50 us with
-// the shuffles (issue-bound: 8 instructions per value and row), 17 us with the tiles; 16 rows of 2048: 26 -> 14 us.
+// the shuffles (issue-bound: 8 instructions per value and row), 17 us with the tiles; 16 rows of 2048: 26 -> 14 us.  What is left
+// of it is the chain of additions (4 cycles a value) and, on a cold input, the first tile's way from memory.
 constexpr int RR_EV = 8, RR_WARPS = 8, RR_THREADS = (RR_WARPS + 1) * 32;
 // columns of a tile: one strip, more where there are too few rows to give every warp one
 __host__ __device__ constexpr int rr_cols(int R) { return R >= RR_WARPS ? 32 * RR_EV : 32 * RR_EV * RR_WARPS / R; }
 
-template <int ND, bool HEAVY>
+// The ninth warp's part: adds the n values of each of a tile's rows to the row's accumulator (lane = row, or lanes row + R p).
+__device__ __forceinline__ void rr_add_tile(const uint32_t *tile, const int pitch, const int n, const int R, const int rows, const int lane,
+                                            const bool is_f, const bool is_sum, ExprAcc &acc) {
+  if (is_f && is_sum) {
+    if (lane < rows) {
+      const uint32_t *src = tile + lane * pitch;
+      int i = 0;
+      if (n >= 16) {   // sixteen values on their way while sixteen are added
+        uint32_t x[16], y[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x[j] = src[j];
+        for (; i + 32 <= n; i += 16) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) y[j] = src[i + 16 + j];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc.f = acc.f + __uint_as_float(x[j]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) x[j] = y[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc.f = acc.f + __uint_as_float(x[j]);
+        i += 16;
+      }
+      for (; i < n; ++i) acc.f = acc.f + __uint_as_float(src[i]);
+    }
+    return;
+  }
+  // A maximum and an integer sum may be formed in parts, which are joined in order: up to 32 / R lanes take consecutive pieces of a
+  // row (of odd length, for the banks), and a lane four consecutive parts of its piece side by side, so that its comparisons are
+  // four chains.  A NaN forgets the values before it, as `acc > x ? acc : x` does.
+  const int row = lane & (R - 1);
+  int pieces = 32 / R;
+  while (pieces > 1 && n < 32 * pieces) pieces >>= 1;
+  const int len = ((n + pieces - 1) / pieces) | 1, i0 = min(n, lane / R * len), i1 = min(n, i0 + len);
+  const uint32_t *src = tile + row * pitch;
+  ExprAcc a = {-INFINITY, is_sum ? 0 : INT32_MIN};
+  bool forgets = false;
+  if (row < rows && i0 < i1) {
+    if (is_f) {
+      const int part = (i1 - i0) / 4;
+      float m[4];
+      bool nan[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { m[q] = -INFINITY; nan[q] = false; }
+#pragma unroll 4
+      for (int i = 0; i < part; ++i) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float x = __uint_as_float(src[i0 + q * part + i]);
+          m[q] = m[q] > x ? m[q] : x;
+          nan[q] = nan[q] || x != x;
+        }
+      }
+      if (part > 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          a.f = nan[q] || !(a.f > m[q]) ? m[q] : a.f;
+          forgets = forgets || nan[q];
+        }
+      }
+      for (int i = i0 + 4 * part; i < i1; ++i) {
+        const float x = __uint_as_float(src[i]);
+        a.f = a.f > x ? a.f : x;
+        forgets = forgets || x != x;
+      }
+    } else {
+#pragma unroll 8
+      for (int i = i0; i < i1; ++i) expr_acc_add(a, src[i], false, is_sum);
+    }
+  }
+  for (int p = 0; p < pieces; ++p) {
+    const int from = row + p * R;
+    const float f = __shfl_sync(0xffffffffu, a.f, from);
+    const int i = __shfl_sync(0xffffffffu, a.i, from), any = __shfl_sync(0xffffffffu, (int)(i1 > i0), from), nan = __shfl_sync(0xffffffffu, (int)forgets, from);
+    if (!any) continue;
+    if (!is_f) expr_acc_add(acc, (uint32_t)i, false, is_sum);
+    else acc.f = nan || !(acc.f > f) ? f : acc.f;
+  }
+}
+
+// PLAIN: the program is one LOAD of floats, whose values go from memory to the tile by asynchronous copies, a whole tile ahead of
+// the additions: through registers a warp had eight loads in flight, one strip after the other (12800 rows of 511, not in L2:
+// sum 16.7 -> 13 us, maximum 17.5 -> 15).  Copies of four bytes: rows start anywhere.
+template <int ND, bool HEAVY, bool PLAIN>
 __global__ void __launch_bounds__(RR_THREADS, 3) expr_rowreduce_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_out, const int R,
                                                                     const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
@@ -343,84 +485,80 @@ __global__ void __launch_bounds__(RR_THREADS, 3) expr_rowreduce_kernel(const __g
   ExprIx<ND> ix;
 #pragma unroll
   for (int d = 0; d < ND; ++d) ix.v[d] = 0;
+  const int shift = 31 - __clz(strips);   // (a power of two)
+  auto fill = [&](const int t) {
+    uint32_t *dst = tile + (t & 1) * R * (C + 1);
+    for (int s = warp; s < rows << shift; s += RR_WARPS) {
+      const int row = s >> shift, col = (s & (strips - 1)) * (32 * RR_EV) + lane;   // this thread's first element of the strip, in the tile
+      const uint32_t first = (uint32_t)t * C + col;                                 // and in the row
+      if (first - lane >= (uint32_t)n_red) continue;
+      const int n = first >= (uint32_t)n_red ? 0 : min(RR_EV, (int)(((uint32_t)n_red - first + 31) >> 5));   // its elements
+      expr_decode(e, o0 + row, 0, nd_out, ix);
+#pragma unroll
+      for (int d = 0; d < ND; ++d)
+        if (d == ra) ix.v[d] = n > 0 ? (int)first : 0;   // a lane past the end reads element 0 of the row
+      uint32_t *to = dst + row * (C + 1) + col;
+      if (PLAIN) {
+        const int arg = (e.code[0] >> 8) & 255;
+        int64_t o = e.operand_offset[arg];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) o += (int64_t)ix.v[d] * e.operand_stride[arg][d];
+        const float *p = reinterpret_cast<const float *>(e.operand[arg]) + o;
+        const int64_t step = 32 * e.operand_stride[arg][ra];
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(to);
+        if (n == RR_EV && step == 32) {
+#pragma unroll
+          for (int j = 0; j < RR_EV; ++j) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(at + 128 * j), "l"(p + 32 * j) : "memory");
+          continue;
+        }
+#pragma unroll
+        for (int j = 0; j < RR_EV; ++j)
+          if (j < n) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(at + 128 * j), "l"(p + j * step) : "memory");
+        continue;
+      }
+      uint32_t val[RR_EV];
+      expr_run<ND, RR_EV, RR_THREADS, HEAVY>(e, ix, ra, n, val, sm);
+#pragma unroll
+      for (int j = 0; j < RR_EV; ++j)
+        if (j < n) to[32 * j] = val[j];
+    }
+  };
+  if (PLAIN && warp < RR_WARPS) {
+    for (int t = 0; t < 2; ++t) {
+      fill(t);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  }
   if (warp == RR_WARPS && lane < rows) {
     expr_decode(e, o0 + lane, 0, nd_out, ix);
     out_at = expr_out_at(e, ix, nd_out);
     acc = expr_acc_init(e, is_f, out_at, true);
   }
   const int tiles = n_red / C + (n_red % C != 0);
-  for (int t = 0; t <= tiles; ++t) {
-    if (warp < RR_WARPS) {
-      if (t < tiles) {
-        uint32_t *dst = tile + (t & 1) * R * (C + 1);
-        for (int s = warp; s < R * strips; s += RR_WARPS) {
-          const int row = s / strips;
-          const int64_t at = (int64_t)t * C + (s - row * strips) * (32 * RR_EV);   // first element of the strip along the reduced loop
-          if (row >= rows || at >= n_red) continue;
-          const int64_t mine = at + lane;
-          const int n = mine >= n_red ? 0 : (int)((n_red - mine + 31) / 32 < RR_EV ? (n_red - mine + 31) / 32 : RR_EV);
-          expr_decode(e, o0 + row, 0, nd_out, ix);
-#pragma unroll
-          for (int d = 0; d < ND; ++d)
-            if (d == ra) ix.v[d] = n > 0 ? (int)mine : 0;   // a lane past the end reads element 0 of the row
-          uint32_t val[RR_EV];
-          expr_run<ND, RR_EV, RR_THREADS, HEAVY>(e, ix, ra, n, val, sm);
-          uint32_t *to = dst + row * (C + 1) + (int)(mine - (int64_t)t * C);
-#pragma unroll
-          for (int j = 0; j < RR_EV; ++j)
-            if (j < n) to[32 * j] = val[j];
-        }
+  auto add = [&](const int t) {
+    const int64_t left = n_red - (int64_t)t * C;
+    rr_add_tile(tile + (t & 1) * R * (C + 1), C + 1, left < C ? (int)left : C, R, rows, lane, is_f, is_sum, acc);
+  };
+  if (PLAIN) {
+    for (int t = 0; t < tiles; ++t) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();   // tile t is there
+      if (warp == RR_WARPS) add(t);
+      if (t + 2 < tiles) {
+        __syncthreads();   // its buffer is free
+        if (warp < RR_WARPS) fill(t + 2);
       }
-    } else if (t > 0) {
-      const int64_t left = n_red - (int64_t)(t - 1) * C;
-      const int n = left < C ? (int)left : C;
-      const uint32_t *last = tile + ((t - 1) & 1) * R * (C + 1);
-      if (is_f && is_sum) {
-        if (lane < rows) {
-          const uint32_t *src = last + lane * (C + 1);
-#pragma unroll 16
-          for (int i = 0; i < n; ++i) acc.f = acc.f + __uint_as_float(src[i]);
-        }
-      } else if (R == 32) {
-        if (lane < rows) {
-          const uint32_t *src = last + lane * (C + 1);
-#pragma unroll 8
-          for (int i = 0; i < n; ++i) expr_acc_add(acc, src[i], is_f, is_sum);
-        }
-      } else {
-        // A maximum and an integer sum may be formed in parts: up to 32 / R lanes take consecutive pieces of a row (of odd length, for
-        // the banks), which are joined in order.  A NaN forgets the values before it, as `acc > x ? acc : x` does.
-        const int row = lane & (R - 1);
-        int pieces = 32 / R;
-        while (pieces > 1 && n < 32 * pieces) pieces >>= 1;
-        const int len = ((n + pieces - 1) / pieces) | 1, i0 = min(n, lane / R * len), i1 = min(n, i0 + len);
-        const uint32_t *src = last + row * (C + 1);
-        ExprAcc a = {-INFINITY, is_sum ? 0 : INT32_MIN};
-        bool forgets = false;
-        if (row < rows) {
-          if (is_f) {
-#pragma unroll 8
-            for (int i = i0; i < i1; ++i) {
-              const float x = __uint_as_float(src[i]);
-              a.f = a.f > x ? a.f : x;
-              forgets = forgets || x != x;
-            }
-          } else {
-#pragma unroll 8
-            for (int i = i0; i < i1; ++i) expr_acc_add(a, src[i], false, is_sum);
-          }
-        }
-        for (int p = 0; p < pieces; ++p) {
-          const int from = row + p * R;
-          const float f = __shfl_sync(0xffffffffu, a.f, from);
-          const int i = __shfl_sync(0xffffffffu, a.i, from), any = __shfl_sync(0xffffffffu, (int)(i1 > i0), from), nan = __shfl_sync(0xffffffffu, (int)forgets, from);
-          if (!any) continue;
-          if (!is_f) expr_acc_add(acc, (uint32_t)i, false, is_sum);
-          else acc.f = nan || !(acc.f > f) ? f : acc.f;
-        }
-      }
+      asm volatile("cp.async.commit_group;" ::: "memory");   // (empty at the end: the wait above counts groups)
     }
-    __syncthreads();
+  } else {
+    for (int t = 0; t <= tiles; ++t) {
+      if (warp < RR_WARPS) {
+        if (t < tiles) fill(t);
+      } else if (t > 0) {
+        add(t - 1);
+      }
+      __syncthreads();
+    }
   }
   if (warp == RR_WARPS && lane < rows) expr_store(e.out, e.out_dtype, out_at, is_f ? __float_as_uint(acc.f) : (uint32_t)acc.i, result_cls);
 }
@@ -605,6 +743,14 @@ static int expr_fuse(caten_b200_expr *c) {
     else if (op == CATEN_B200_OP_WHERE) sp -= 2;
     if (sp > depth) depth = sp;
   }
+  for (int pc = 0; pc < n; ++pc) {
+    uint32_t &w = c->code[pc];
+    const int op = w & 255;
+    if (op >= CATEN_B200_OP_ADD && op <= CATEN_B200_OP_LT) w |= EXPR_BINARY;
+    const bool shared = op == CATEN_B200_OP_LOAD || op == CATEN_B200_OP_NEG || op == CATEN_B200_OP_RECIP || op == CATEN_B200_OP_NOT || op == CATEN_B200_OP_ADD ||
+                        op == CATEN_B200_OP_MUL || op == CATEN_B200_OP_MAX || op == CATEN_B200_OP_NE || op == CATEN_B200_OP_LT;
+    if (shared && ((w >> 16) & 255) != CATEN_B200_CLS_F32) w += EXPR_WHOLE;
+  }
   return depth;
 }
 
@@ -618,10 +764,11 @@ static int launch_expr_elements(caten_b200_ctx *ctx, const caten_b200_expr &e, i
   int64_t spw = (rows * strips_per_row) / ((int64_t)ctx->sm_count * 64);
   spw = spw < 1 ? 1 : spw > 16 ? 16 : spw;
   if (spw > strips_per_row) spw = strips_per_row;
-  const int64_t n_groups = rows * ((strips_per_row + spw - 1) / spw);  // one warp each
+  const int64_t groups_per_row = (strips_per_row + spw - 1) / spw;   // (a loop's extent has 31 bits)
+  const int64_t n_groups = rows * groups_per_row;                    // one warp each
   const int64_t blocks = (n_groups + 7) / 8;
   if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)(rows * vlen));
-  launch_k(ctx, expr_kernel<ND, EV, HEAVY>, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_groups, (int)spw, n_red, result_cls);
+  launch_k(ctx, expr_kernel<ND, EV, HEAVY>, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_groups, (int)groups_per_row, (int)spw, n_red, result_cls);
   CB_LAUNCH_CHECK(ctx, "expr_kernel");
   return 0;
 }
@@ -646,9 +793,12 @@ static int launch_expr_rows(caten_b200_ctx *ctx, const caten_b200_expr &e, int d
   while (R > 1 && (n_out + R / 2 - 1) / (R / 2) <= 3 * ctx->sm_count) R >>= 1;
   const int64_t blocks = (n_out + R - 1) / R;
   if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)n_out);
-  const size_t smem = (2 * (size_t)R * (rr_cols(R) + 1) + (size_t)(depth > 1 ? depth - 1 : 1) * RR_EV * RR_THREADS) * sizeof(uint32_t);
-  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(expr_rowreduce_kernel<ND, HEAVY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  launch_k(ctx, expr_rowreduce_kernel<ND, HEAVY>, dim3((unsigned)blocks), dim3(RR_THREADS), smem, e, n_out, R, result_cls);
+  const bool plain = !HEAVY && e.n_code == 1 && (e.code[0] & 255) == CATEN_B200_OP_LOAD;   // (LOAD alone: of floats)
+  const size_t tiles = 2 * (size_t)R * (rr_cols(R) + 1) * sizeof(uint32_t);
+  const size_t smem = tiles + (plain ? 0 : (size_t)(depth > 1 ? depth - 1 : 1) * RR_EV * RR_THREADS * sizeof(uint32_t));
+  auto kernel = plain ? expr_rowreduce_kernel<ND, false, true> : expr_rowreduce_kernel<ND, HEAVY, false>;
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_k(ctx, kernel, dim3((unsigned)blocks), dim3(RR_THREADS), smem, e, n_out, R, result_cls);
   CB_LAUNCH_CHECK(ctx, "expr_rowreduce_kernel");
   return 0;
 }

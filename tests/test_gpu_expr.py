@@ -248,6 +248,43 @@ def test_words_joined_with_their_right_operand(rt, shape):
     check(rt, E.where(lx < lz, E.maximum(ly, lz), E.cast(E.load(i.view) * E.const(3) + E.index(len(shape) - 1), E.F32)), out, pairs=(x, y, z, i))
 
 
+@pytest.mark.parametrize("op", ["sum", "max"])
+@pytest.mark.parametrize("shape", [(7, 13, 511), (40, 33, 513), (3, 2, 1100), (300, 90, 300)])
+def test_plain_row_reductions_over_strided_views(rt, shape, op):
+    """A bare operand's rows, copied to the tiles a tile ahead: one to five tiles, rows that start off any boundary, loops that
+    do not merge, values no comparison admits, a result added to what is there."""
+    a, b, n = shape
+    rng = np.random.Generator(np.random.PCG64(a + n))
+    host = rng.standard_normal((b, a, n + 2), dtype=np.float32)
+    host[rng.integers(0, b, 5), rng.integers(0, a, 5), rng.integers(1, n + 1, 5)] = np.nan
+    host[0, 0] = -np.inf
+    x = Pair(rt, host, strides=(n + 2, a * (n + 2), 1), offset=1)
+    s = Pair(rt, rng.standard_normal((a, b), dtype=np.float32), strides=(b, 1, 0))
+    check(rt, E.load(x.view), s, shape=shape, n_reduce=1, reduce_op=op, pairs=(x,))
+    s.host[:] = s.dev.numpy()
+    check(rt, E.load(x.view), s, shape=shape, n_reduce=1, reduce_op=op, accumulate=True, pairs=(x,))
+
+
+def test_exp2_over_the_whole_range(rt):
+    """Every 4099th bit pattern, whole numbers, and the ends of the range.  The polynomial is within 2^-44 of 2^x, so one value in
+    some 2^20 (two sides of a boundary 2^-24 apart) may round to the other neighbour: a handful of the million here, by one ulp."""
+    bits = np.concatenate([np.arange(0, 2 ** 32, 4099, dtype=np.uint64).astype(np.uint32),
+                           np.array([np.nan, np.inf, -np.inf, 0.0, -0.0, 127.99999, 128.0, -125.5, -126.0, -148.5, -149.0, -149.5, -150.0, -151.0, 160.5, -160.5, 3e38, -3e38],
+                                    np.float32).view(np.uint32), np.arange(-160, 161).astype(np.float32).view(np.uint32)])
+    x = Pair(rt, bits.view(np.float32))
+    out = Pair(rt, np.zeros(len(bits), np.float32))
+    E.run(rt, E.exp2(E.load(x.view)), out.view)
+    got = out.dev.numpy()
+    with np.errstate(all="ignore"):
+        want = np.exp2(x.host.astype(np.float64)).astype(np.float32)
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+    d = np.abs(got.view(np.int32).astype(np.int64) - want.view(np.int32).astype(np.int64))[~np.isnan(want)]
+    assert d.max() <= 1 and (d > 0).sum() <= 20, (d.max(), (d > 0).sum())
+    whole = np.arange(-160, 161)
+    with np.errstate(over="ignore"):
+        np.testing.assert_array_equal(got[-321:], np.ldexp(1.0, whole).astype(np.float32))
+
+
 def test_malformed_programs_are_refused(rt):
     from caten_b200 import _lib as L
     x = Pair(rt, np.zeros(8, np.float32))
