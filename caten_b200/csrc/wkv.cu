@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(WS_THREADS) wkv_scan_kernel(const WkvArgs a, c
 // wkv_out_kernel: adds the state's part, then the head's norm and the gate.
 // ---------------------------------------------------------------------------------------------
 constexpr int WC_T = 64, WC_D = 64, WC_LD = 68, WC_THREADS = 256;   // tokens per chunk, head size, row pitch in shared memory
-constexpr size_t WC_SMEM = (size_t)(6 * WC_T * WC_LD + 2 * 4 * WC_D) * sizeof(float);
+constexpr size_t WC_SMEM = (size_t)(4 * WC_T * WC_LD + 2 * 4 * WC_D) * sizeof(float);
 
 __device__ __forceinline__ float exp_neg(float x) { return exp2f(-1.4426950408889634f * x); }
 
@@ -218,26 +218,44 @@ __device__ __forceinline__ void split_level(const float *ev, const float *r, con
   }
 }
 
-__global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_kernel(const WkvArgs a, float *__restrict__ U, float *__restrict__ decays) {
+// Four tiles of shared memory, so that three CTAs share an SM: xs holds e, then k and r at one segment length after another, then v,
+// which arrives under the products of the subchunks.  8 x 1024 tokens of 32 heads: 325 us with loads one after the other, 236 with all
+// under way at once (six tiles, two CTAs), 227 so; its bytes take 71.  Bound by shared memory and the barriers between the passes.
+__global__ void __launch_bounds__(WC_THREADS, 3) wkv_chunk_kernel(const WkvArgs a, float *__restrict__ U, float *__restrict__ decays) {
   extern __shared__ __align__(16) float sm[];
-  float *rs = sm, *ks = rs + WC_T * WC_LD, *vs = ks + WC_T * WC_LD, *ws = vs + WC_T * WC_LD, *xs = ws + WC_T * WC_LD, *As = xs + WC_T * WC_LD;
+  float *rs = sm, *ks = rs + WC_T * WC_LD, *xs = ks + WC_T * WC_LD, *vs = xs, *As = xs + WC_T * WC_LD;
   float *tot = As + WC_T * WC_LD;   // [4][WC_D] sums of e per subchunk
   float *g = tot + 4 * WC_D;        // [4][WC_D] exp(-tot)
   const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, Dp = a.Dp;
   const int t0 = c * WC_T, tn = min(WC_T, a.s - t0);
   const int64_t row0 = (int64_t)b * a.s + t0;
   pdl_enter();
-  // tokens past the end and channels past the head: r = k = v = 0 and no decay
-  for (int e = tid; e < 4 * WC_T * (WC_D / 4); e += WC_THREADS) {
-    const int which = e >> 10, t = (e >> 4) & 63, c4 = e & 15;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool ok = t < tn && 4 * c4 < Dp;
-    if (ok) {
-      const float *src = which < 3 ? a.y + (row0 + t) * a.ld + (int64_t)which * a.gr + (int64_t)h * Dp : a.d + (row0 + t) * a.d_ld + (int64_t)h * Dp;
-      v = reinterpret_cast<const float4 *>(src)[c4];
-      if (which == 3) v = make_float4(expf(v.x), expf(v.y), expf(v.z), expf(v.w));
+  // tokens past the end and channels past the head: r = k = v = 0 and no decay.  All of a thread's twelve loads are under way
+  // before the first is waited for (one after the other they were 20 k of a CTA's 44 k cycles).
+  const int tx = tid & 15, ty = tid >> 4;
+  const bool in = 4 * tx < Dp;
+  const float *y = a.y + row0 * a.ld + (int64_t)h * Dp + (in ? 4 * tx : 0);
+  auto fetch = [&](float *dst, const float *src) {   // tokens ty + 16 j, channels 4 tx ..
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int t = ty + 16 * j;
+      cp16(dst + t * WC_LD + 4 * tx, src + (t < tn ? t : 0) * a.ld, in && t < tn);
     }
-    *reinterpret_cast<float4 *>((which == 0 ? rs : which == 1 ? ks : which == 2 ? vs : ws) + t * WC_LD + 4 * c4) = v;
+  };
+  {
+    const float *d = a.d + row0 * a.d_ld + (int64_t)h * Dp + (in ? 4 * tx : 0);
+    float4 e4[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int t = ty + 16 * j;
+      e4[j] = in && t < tn ? *reinterpret_cast<const float4 *>(d + t * a.d_ld) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    }
+    fetch(rs, y);
+    fetch(ks, y + a.gr);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4 *>(xs + (ty + 16 * j) * WC_LD + 4 * tx) = make_float4(expf(e4[j].x), expf(e4[j].y), expf(e4[j].z), expf(e4[j].w));
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
   __syncthreads();
   const int sub = tid >> 6, ch = tid & 63;   // this thread's subchunk and channel in the element-wise passes
@@ -247,44 +265,46 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_kernel(const WkvArgs 
     float sum = 0.0f;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      ev[j] = ws[(16 * sub + j) * WC_LD + ch];
+      ev[j] = xs[(16 * sub + j) * WC_LD + ch];
       sum += ev[j];
     }
     tot[sub * WC_D + ch] = sum;
     g[sub * WC_D + ch] = exp_neg(sum);
-    split_level<8>(ev, rc, kc, ws + 16 * sub * WC_LD + ch);   // (a thread's own elements of ws)
-    split_level<4>(ev, rc, kc, xs + 16 * sub * WC_LD + ch);
+    split_level<8>(ev, rc, kc, xs + 16 * sub * WC_LD + ch);   // (a thread's own elements of xs)
   }
   __syncthreads();
   // ---- same subchunk, one pair of tokens (t, s < t) per thread and level ----
   {
     const int bl = tid >> 6, t8 = (tid >> 3) & 7, s8 = tid & 7;
-    As[(16 * bl + 8 + t8) * WC_LD + 16 * bl + s8] = dot_rows(ws + (16 * bl + 8 + t8) * WC_LD, ws + (16 * bl + s8) * WC_LD);
-    if (tid < 128) {
-      const int base = 8 * (tid >> 4), t = base + 4 + ((tid >> 2) & 3), s_ = base + (tid & 3);
-      As[t * WC_LD + s_] = dot_rows(xs + t * WC_LD, xs + s_ * WC_LD);
-    } else if (tid < 192) {   // the token itself, with the bonus
-      const int t = tid - 128;
-      float acc = 0.0f;
-#pragma unroll 4
-      for (int i = 0; i < Dp; i += 4) {
-        const float4 k4 = *reinterpret_cast<const float4 *>(ks + t * WC_LD + i), r4 = *reinterpret_cast<const float4 *>(rs + t * WC_LD + i);
-        const float4 u4 = *reinterpret_cast<const float4 *>(a.u + (int64_t)h * Dp + i);
-        acc = fmaf(r4.x * u4.x, k4.x, fmaf(r4.y * u4.y, k4.y, fmaf(r4.z * u4.z, k4.z, fmaf(r4.w * u4.w, k4.w, acc))));
-      }
-      As[t * WC_LD + t] = acc;
-      for (int s_ = t + 1; s_ < (t | 15) + 1; ++s_) As[t * WC_LD + s_] = 0.0f;   // later tokens of the subchunk do not reach back
-    } else if (tid < 224) {   // neighbours: nothing decays in between
-      const int s_ = 2 * (tid - 192);
-      As[(s_ + 1) * WC_LD + s_] = dot_rows(rs + (s_ + 1) * WC_LD, ks + s_ * WC_LD);
-    }
+    As[(16 * bl + 8 + t8) * WC_LD + 16 * bl + s8] = dot_rows(xs + (16 * bl + 8 + t8) * WC_LD, xs + (16 * bl + s8) * WC_LD);
   }
   __syncthreads();
-  split_level<2>(ev, rc, kc, ws + 16 * sub * WC_LD + ch);
+  split_level<4>(ev, rc, kc, xs + 16 * sub * WC_LD + ch);
+  __syncthreads();
+  if (tid < 128) {
+    const int base = 8 * (tid >> 4), t = base + 4 + ((tid >> 2) & 3), s_ = base + (tid & 3);
+    As[t * WC_LD + s_] = dot_rows(xs + t * WC_LD, xs + s_ * WC_LD);
+  } else if (tid < 192) {   // the token itself, with the bonus
+    const int t = tid - 128;
+    float acc = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < Dp; i += 4) {
+      const float4 k4 = *reinterpret_cast<const float4 *>(ks + t * WC_LD + i), r4 = *reinterpret_cast<const float4 *>(rs + t * WC_LD + i);
+      const float4 u4 = *reinterpret_cast<const float4 *>(a.u + (int64_t)h * Dp + i);
+      acc = fmaf(r4.x * u4.x, k4.x, fmaf(r4.y * u4.y, k4.y, fmaf(r4.z * u4.z, k4.z, fmaf(r4.w * u4.w, k4.w, acc))));
+    }
+    As[t * WC_LD + t] = acc;
+    for (int s_ = t + 1; s_ < (t | 15) + 1; ++s_) As[t * WC_LD + s_] = 0.0f;   // later tokens of the subchunk do not reach back
+  } else if (tid < 224) {   // neighbours: nothing decays in between
+    const int s_ = 2 * (tid - 192);
+    As[(s_ + 1) * WC_LD + s_] = dot_rows(rs + (s_ + 1) * WC_LD, ks + s_ * WC_LD);
+  }
+  __syncthreads();
+  split_level<2>(ev, rc, kc, xs + 16 * sub * WC_LD + ch);
   __syncthreads();
   if (tid < 64) {
     const int base = 4 * (tid >> 2), t = base + 2 + ((tid >> 1) & 1), s_ = base + (tid & 1);
-    As[t * WC_LD + s_] = dot_rows(ws + t * WC_LD, ws + s_ * WC_LD);
+    As[t * WC_LD + s_] = dot_rows(xs + t * WC_LD, xs + s_ * WC_LD);
   }
   // ---- r_t exp(-P_t), k_t exp(-Q_t) ----
   {
@@ -302,7 +322,8 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_kernel(const WkvArgs 
     }
   }
   __syncthreads();
-  const int tx = tid & 15, ty = tid >> 4;
+  fetch(vs, y + 2 * (int64_t)a.gr);   // (the segments have been read)
+  asm volatile("cp.async.commit_group;" ::: "memory");
   // ---- earlier subchunks: thread (ty, tx) owns (token ty of subchunk a, token tx of subchunk b) for all a > b ----
   {
     float a10 = 0.f, a21 = 0.f, a32 = 0.f, a20 = 0.f, a31 = 0.f, a30 = 0.f;
@@ -333,6 +354,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_kernel(const WkvArgs 
     As[(ty + 48) * WC_LD + tx + 16] = a31;
     As[(ty + 48) * WC_LD + tx + 32] = a32;
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   // ---- scale r for the state before the chunk (written over d) and k for the state after it ----
   {
@@ -441,22 +463,27 @@ __global__ void __launch_bounds__(WC_THREADS) wkv_out_kernel(const WkvArgs a, co
   const int t0 = c * WC_T, tn = min(WC_T, a.s - t0);
   const int64_t row0 = (int64_t)b * a.s + t0;
   pdl_enter();
-  const float4 *src = reinterpret_cast<const float4 *>(U + (((int64_t)b * a.H + h) * gridDim.x + c) * (WC_D * WC_D));
-  for (int e = tid; e < WC_T * 16; e += WC_THREADS) {
-    const int t = e >> 4, c4 = e & 15;
-    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t < tn && 4 * c4 < Dp) r = reinterpret_cast<const float4 *>(a.d + (row0 + t) * a.d_ld + (int64_t)h * Dp)[c4];
-    *reinterpret_cast<float4 *>(rs + t * WC_LD + 4 * c4) = r;
-    *reinterpret_cast<float4 *>(S + t * WC_LD + 4 * c4) = src[e];
-  }
-  __syncthreads();
+  const float *src = U + (((int64_t)b * a.H + h) * gridDim.x + c) * (WC_D * WC_D);
   const int tx = tid & 15, ty = tid >> 4;
-  float4 o[4];
+  const bool in = 4 * tx < Dp;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {   // everything that is read is under way before the first of it is waited for
+    const int t = ty + 16 * j;
+    cp16(rs + t * WC_LD + 4 * tx, a.d + (row0 + (t < tn ? t : 0)) * a.d_ld + (int64_t)h * Dp + (in ? 4 * tx : 0), in && t < tn);
+    cp16(S + t * WC_LD + 4 * tx, src + t * WC_D + 4 * tx, true);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 o[4], z[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int t = ty + 16 * j;
-    o[j] = t < tn && 4 * tx < Dp ? *reinterpret_cast<const float4 *>(a.o + (row0 + t) * a.o_ld + (int64_t)h * Dp + 4 * tx) : make_float4(0.f, 0.f, 0.f, 0.f);
+    o[j] = t < tn && in ? *reinterpret_cast<const float4 *>(a.o + (row0 + t) * a.o_ld + (int64_t)h * Dp + 4 * tx) : zero;
+    z[j] = t < tn && in ? *reinterpret_cast<const float4 *>(a.y + (row0 + t) * a.ld + 3 * (int64_t)a.gr + (int64_t)h * Dp + 4 * tx) : zero;
   }
+  const float4 nw = in ? *reinterpret_cast<const float4 *>(a.norm + (int64_t)h * Dp + 4 * tx) : zero;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
 #pragma unroll 4
   for (int i = 0; i < WC_D; i += 4) {
     float4 v[4];
@@ -471,7 +498,6 @@ __global__ void __launch_bounds__(WC_THREADS) wkv_out_kernel(const WkvArgs a, co
       o[j].w = fmaf(r.x, v[0].w, fmaf(r.y, v[1].w, fmaf(r.z, v[2].w, fmaf(r.w, v[3].w, o[j].w))));
     }
   }
-  const float4 nw = 4 * tx < Dp ? *reinterpret_cast<const float4 *>(a.norm + (int64_t)h * Dp + 4 * tx) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     float ss = (o[j].x * o[j].x + o[j].y * o[j].y) + (o[j].z * o[j].z + o[j].w * o[j].w);
@@ -480,8 +506,7 @@ __global__ void __launch_bounds__(WC_THREADS) wkv_out_kernel(const WkvArgs a, co
     const int t = ty + 16 * j;
     if (t < tn && 4 * tx < Dp) {
       const float inv = 1.0f / sqrtf(ss / (float)a.D + a.eps);
-      const float4 z = *reinterpret_cast<const float4 *>(a.y + (row0 + t) * a.ld + 3 * (int64_t)a.gr + (int64_t)h * Dp + 4 * tx);
-      const float4 v = make_float4(o[j].x * inv * nw.x * silu(z.x), o[j].y * inv * nw.y * silu(z.y), o[j].z * inv * nw.z * silu(z.z), o[j].w * inv * nw.w * silu(z.w));
+      const float4 v = make_float4(o[j].x * inv * nw.x * silu(z[j].x), o[j].y * inv * nw.y * silu(z[j].y), o[j].z * inv * nw.z * silu(z[j].z), o[j].w * inv * nw.w * silu(z[j].w));
       const int64_t at = (row0 + t) * a.out_ld + (int64_t)h * Dp + 4 * tx;
       if (a.bf.hi) {
         *reinterpret_cast<uint2 *>(a.bf.hi + at) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
