@@ -276,8 +276,8 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
       if (vi < nblk && lane == 0) give_up(16);
       __syncwarp();
       // the copies this thread started land before the CTA's shared memory is released, whoever gives up
-      for (int k = ki > 2 ? ki - 2 : 0; k < ki; ++k) mbar_wait(k_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
-      for (int k = vi > 2 ? vi - 2 : 0; k < vi; ++k) mbar_wait(v_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
+      for (int k = ki > 2 ? ki - 2 : 0; k < ki; ++k) mbar_wait_thread(k_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
+      for (int k = vi > 2 ? vi - 2 : 0; k < vi; ++k) mbar_wait_thread(v_full(k & 1), (uint32_t)(k >> 1) & 1u, abort_flag + 1);
     }
   } else if (warp == 9) {
     // ---------------- MMAs (uniform control flow, one elected lane issues) ----------------
@@ -351,7 +351,7 @@ attn_prefill_tc_kernel(const AttnArgs p, float qscale, int *status, uint32_t ide
     // the warp's view of a wait; a warp whose wait ran out goes on through the pair barriers and touches nothing else
     auto wait = [&](uint32_t bar, uint32_t ph) {
       if (!ok) return;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, ph, abort_flag));
+      ok = mbar_wait(bar, ph, abort_flag);
       if (!ok && lane == 0) give_up(10);
     };
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };   // warps quad and quad + 4

@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
       }
       __syncwarp();
       if (*abort_flag)  // copies in flight land before the CTA's shared memory is released
-        for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait(full(i % stages), (uint32_t)(i / stages) & 1u, abort_flag + 1);
+        for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait_thread(full(i % stages), (uint32_t)(i / stages) & 1u, abort_flag + 1);
     }
     __syncwarp();
   } else {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
           q4[h][v] = 4 * c < Dp ? reinterpret_cast<const float4 *>(q + h * Dp)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       for (int i = 0; i < nc && ok; ++i) {
-        ok = __all_sync(0xffffffffu, mbar_wait(full(s), ph, abort_flag));
+        ok = mbar_wait(full(s), ph, abort_flag);
         if (!ok) break;
         const float *st = ring + s * CH * wide;
         float d[R];
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(AD_THREADS, NV == 1 ? 3 : 1) attn_window_decod
         acc[h][v] = make_float4(p * x.x, p * x.y, p * x.z, p * x.w);
       }
     for (int i = nc; i < 2 * nc && ok; ++i) {
-      ok = __all_sync(0xffffffffu, mbar_wait(full(s), ph, abort_flag));
+      ok = mbar_wait(full(s), ph, abort_flag);
       if (!ok) break;
       const float *st = ring + s * CH * wide;
 #pragma unroll

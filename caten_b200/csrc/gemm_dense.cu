@@ -409,7 +409,7 @@ gemm_dense_kernel(const __grid_constant__ CUtensorMap tw_hi, const __grid_consta
       if (PAIR)
         for (int i = 0; i < 1000; ++i) __nanosleep(1000);
       else
-        for (int i = issued > S ? issued - S : 0; i < issued; ++i) mbar_wait(full(i % S), (uint32_t)(i / S) & 1u, abort_flag + 1);
+        for (int i = issued > S ? issued - S : 0; i < issued; ++i) mbar_wait_thread(full(i % S), (uint32_t)(i / S) & 1u, abort_flag + 1);
     }
   } else if (warp == 1) {
     if (rank == 0) {

@@ -532,7 +532,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
     for (int kc = g; kc < num_k && alive; kc += ga) {
       int got = 0;
       if (lane == 0) {
-        got = mbar_wait(empty(s), ph ^ 1u, abort_flag) ? 1 : 0;
+        got = mbar_wait_thread(empty(s), ph ^ 1u, abort_flag) ? 1 : 0;
         if (!got && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 1; a.status[2] = kc; }
       }
       got = __shfl_sync(0xffffffffu, got, 0);
@@ -557,7 +557,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
     // ---------------- epilogue ----------------
     pdl_wait();
     if (tid == 0) {
-      const bool got = !*abort_flag && mbar_wait(accum_bar, 0, abort_flag);
+      const bool got = !*abort_flag && mbar_wait_thread(accum_bar, 0, abort_flag);
       if (!got && !*abort_flag) { *abort_flag = 1; atomicCAS(a.status, 0, DEV_WAIT_TIMEOUT); a.status[1] = 2; }
       abort_flag[3] = got ? 1 : 0;
     }
@@ -638,7 +638,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_hi, const __grid_constant_
     if (*abort_flag) {
       // let the copies this warp started land before the CTA's shared memory is released
       for (int kc = issued > S ? issued - S : 0; kc < issued; ++kc)
-        mbar_wait(full(kc % S), (uint32_t)(kc / S) & 1u, abort_flag + 1);
+        mbar_wait_thread(full(kc % S), (uint32_t)(kc / S) & 1u, abort_flag + 1);
     }
   } else {
     // ---------------- MMA issuer ----------------

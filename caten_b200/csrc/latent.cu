@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
       __syncwarp();
       if (*abort_flag)   // copies in flight land before the CTA's shared memory is released
         for (int i = issued > stages * np ? issued - stages * np : 0; i < issued; ++i)
-          mbar_wait(full(i / np % stages, i % np), (uint32_t)(i / np / stages) & 1u, abort_flag + 1);
+          mbar_wait_thread(full(i / np % stages, i % np), (uint32_t)(i / np / stages) & 1u, abort_flag + 1);
     }
     __syncwarp();
   } else if (warp == 9) {
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(LA_THREADS, 1) latent_attn_tc_kernel(const Lat
     // (a warp that gives up stays in the loop, without waiting for anything, so that all warps reach the same block barriers)
     auto wait = [&](uint32_t bar, uint32_t parity, int where) {
       if (!ok) return;
-      ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+      ok = mbar_wait(bar, parity, abort_flag);
       if (!ok && lane == 0) give_up(where);
     };
     for (int i = 0; i < nt; ++i) {

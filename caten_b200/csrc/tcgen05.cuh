@@ -50,8 +50,8 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait. Returns false when the limit ran out or another role already gave up.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+// Bounded wait of a thread by itself.  Returns false when the limit ran out or another role already gave up.
+__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
   for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
     if (mbar_try(bar, parity)) return true;
     if (i > 1024) {
@@ -60,6 +60,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
   return false;
+}
+// The same by a whole warp, with one answer for all lanes: at the limit, or when the flag is raised meanwhile, some lanes may have
+// seen the phase complete and others not, and elect.sync, __syncwarp and the .aligned instructions that follow need every lane.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait_thread(bar, parity, abort_flag));
 }
 // One lane of the (converged) warp; the same lane every time for a full mask.
 __device__ __forceinline__ uint32_t elect_one() {

@@ -88,3 +88,23 @@ def test_product_code_never_touches_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h", ".lisp")):
                 txt = open(os.path.join(dirpath, f)).read()
                 assert "import oracle" not in txt and "from oracle" not in txt and "libcaten_oracle" not in txt, f
+
+
+def test_a_warps_bounded_wait_has_one_answer():
+    """Kernels' loops that a whole warp runs branch on `mbar_wait`, whose answer is voted on: lanes that disagreed at the limit would part
+    in front of instructions that need all of them.  A thread's own answer (`mbar_wait_thread`) decides only where one thread waits."""
+    csrc = os.path.join(ROOT, "caten_b200", "csrc")
+    text = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.endswith((".cu", ".cuh"))}
+    wait = re.search(r"bool mbar_wait\(.*?\n\}", text["tcgen05.cuh"], re.S).group()
+    assert "__all_sync(0xffffffffu, mbar_wait_thread(" in wait
+    calls = 0
+    for name, src in text.items():
+        lines = src.split("\n")
+        for i, line in enumerate(lines):
+            code = line.split("//")[0]
+            calls += "mbar_wait(" in code
+            if name == "tcgen05.cuh" or "mbar_wait_thread(" not in code:
+                continue
+            dropped = re.search(r"(^|\)|;)\s*mbar_wait_thread\(.*\);\s*\}?\s*$", code)   # a copy's landing is awaited, the answer not used
+            assert dropped or re.search(r"\b(lane|tid) == 0\b", lines[i - 1]), f"{name}:{i + 1}: {line.strip()}"
+    assert calls > 20
