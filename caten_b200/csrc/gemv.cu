@@ -32,8 +32,13 @@ struct GemvGain {
   }
 };
 
-template <int SLOTS, int MOST, class Put>
-__device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const GemvGain &gain, const float4 *x4, int M, int K4, Put put) {
+__device__ __forceinline__ void gemv_copy_async(float *to, const float4 *x4, int f) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 4 * f)), "l"(x4 + f) : "memory");
+}
+__device__ __forceinline__ void gemv_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int SLOTS, int MOST, bool ASYNC, class Put>
+__device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const GemvGain &gain, const float4 *x4, int M, int K4, Put put, float *to) {
   __shared__ float4 stat[2][16];   // of a warp's part: sum, squared deviations from its mean, mean, elements
   const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31;
   const float invd = 1.0f / (float)(K4 * 4);
@@ -44,14 +49,26 @@ __device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const GemvGain
     have += left <= 0 ? 0 : left < 32 ? left : 32;
   }
   const float cnt = (float)(4 * have), inv = have ? 1.0f / cnt : 0.0f;
-  float4 v[SLOTS], nx[SLOTS];
+  // Several long rows wait where they will lie, a thread's own float4 brought there by itself: the next row in registers is more than
+  // there are, and the compiler then stores weights that are still on their way (gemv_dense_kernel).
+  constexpr bool STAGED = ASYNC && MOST > 1 && SLOTS > 1;
+  const float4 *from = x4;
+  if (STAGED) {
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int u = 0; u < SLOTS; ++u)
+        if (u * T + tid < K4) gemv_copy_async(to, x4, m * K4 + u * T + tid);
+    gemv_copies_wait();
+    from = reinterpret_cast<const float4 *>(to);
+  }
+  float4 v[SLOTS], nx[STAGED ? 1 : SLOTS];
   auto load = [&](int m, float4 *d) {
 #pragma unroll
-    for (int u = 0; u < SLOTS; ++u) d[u] = m < M && u * T + tid < K4 ? x4[m * K4 + u * T + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < SLOTS; ++u) d[u] = m < M && u * T + tid < K4 ? from[m * K4 + u * T + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   load(0, v);
   for (int m = 0; m < M; ++m) {
-    if (MOST > 1) load(m + 1, nx);
+    if (MOST > 1 && !STAGED) load(m + 1, nx);
     float sum = 0.0f, sq = 0.0f;
 #pragma unroll
     for (int u = 0; u < SLOTS; ++u) sum += (v[u].x + v[u].y) + (v[u].z + v[u].w);
@@ -89,26 +106,31 @@ __device__ __forceinline__ void gemv_norm_rows(const GemvNorm &n, const GemvGain
       put(m * K4 + i, make_float4(((y.x - u) * rs) * gg.x + bb.x, ((y.y - u) * rs) * gg.y + bb.y, ((y.z - u) * rs) * gg.z + bb.z, ((y.w - u) * rs) * gg.w + bb.w), i < K4);
     }
     if (MOST == 1) break;
+    if (STAGED) {
+      load(m + 1, v);
+      continue;
+    }
 #pragma unroll
     for (int q = 0; q < SLOTS; ++q) v[q] = nx[q];
   }
 }
 
 // MOST: M is at most that.  ASYNC: put is the plain copy to `to`, rows without a norm go there without passing through registers.
-template <int MOST, bool ASYNC, class Put>
+// NORM: with the code for rows that have one.
+template <int MOST, bool ASYNC, bool NORM, class Put>
 __device__ __forceinline__ void gemv_rows_to_shared(const GemvNorm &n, const GemvGain &gain, const float *x, int M, int K4, Put put, float *to = nullptr) {
   const float4 *x4 = reinterpret_cast<const float4 *>(x);
   const int tid = threadIdx.x, T = blockDim.x;
-  if (n.g) {
-    if (K4 <= T) gemv_norm_rows<1, MOST>(n, gain, x4, M, K4, put);
-    else if (K4 <= 2 * T) gemv_norm_rows<2, MOST>(n, gain, x4, M, K4, put);
-    else gemv_norm_rows<3, MOST>(n, gain, x4, M, K4, put);
+  if (NORM && n.g) {
+    if (K4 <= T) gemv_norm_rows<1, MOST, ASYNC>(n, gain, x4, M, K4, put, to);
+    else if (K4 <= 2 * T) gemv_norm_rows<2, MOST, ASYNC>(n, gain, x4, M, K4, put, to);
+    else gemv_norm_rows<3, MOST, ASYNC>(n, gain, x4, M, K4, put, to);
     return;
   }
   const int total = M * K4;
   if (ASYNC) {
-    for (int f = tid; f < total; f += T) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + 4 * f)), "l"(x4 + f) : "memory");
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int f = tid; f < total; f += T) gemv_copy_async(to, x4, f);
+    gemv_copies_wait();
     return;
   }
   for (int f0 = 0; f0 < total; f0 += 8 * T) {
@@ -199,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
   };
   float bz, rz;
   addends(0, &bz, &rz);
-  gemv_rows_to_shared<4, false>(a.norm, gain, a.x, a.M, nkb * 8, [&](int f, float4 v, bool ok) {
+  gemv_rows_to_shared<4, false, true>(a.norm, gain, a.x, a.M, nkb * 8, [&](int f, float4 v, bool ok) {
     float *to = xs + (f >> 3) * GEMV_XPAD;
     if (BLK::SUMS) {
       float s = (v.x + v.y) + (v.z + v.w);
@@ -409,7 +431,7 @@ struct GemvDense {
   GemvNorm norm;
 };
 
-template <typename T, int RI, int NR, bool EXPERTS>
+template <typename T, int RI, int NR, bool EXPERTS, bool NORM>
 __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const GemvDense a) {
   constexpr int PRE = GEMV_PRE;
   extern __shared__ float xs[];   // [NR][K]
@@ -453,7 +475,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   load(base, c0);
   GemvGain gain;
   if (!EXPERTS) {
-    gain.load(a.norm, K / 4);
+    if (NORM) gain.load(a.norm, K / 4);
     pdl_wait();
   }
   // the lane that finishes output (row base + i, row m of x) is lane i * NR + m of the slot's first warp
@@ -467,7 +489,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
   float bz, rz;
   addends(base, &bz, &rz);
   for (int i = a.M * K / 4 + threadIdx.x; i < NR * K / 4; i += 256) reinterpret_cast<float4 *>(xs)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  gemv_rows_to_shared<NR, true>(a.norm, gain, x, a.M, K / 4, [&](int f, float4 v, bool ok) { if (ok) reinterpret_cast<float4 *>(xs)[f] = v; }, xs);
+  gemv_rows_to_shared<NR, true, NORM>(a.norm, gain, x, a.M, K / 4, [&](int f, float4 v, bool ok) { if (ok) reinterpret_cast<float4 *>(xs)[f] = v; }, xs);
   __syncthreads();
   const int64_t rounds = ((int64_t)N + stride - 1) / stride;   // the same for every warp: the slots' warps meet at barriers
   for (int64_t it = 0; it < rounds; ++it) {
@@ -604,7 +626,13 @@ static int launch_dense_t(caten_b200_ctx *ctx, GemvDense g, int groups) {
   g.ks = ks;
   const int64_t ctas = ((int64_t)g.group_rows * ks + 8 * RI - 1) / (8 * RI);
   const size_t smem = (size_t)NR * g.K * sizeof(float);
-  auto kernel = gemv_dense_kernel<T, RI, NR, EXPERTS>;
+  // Several rows without a norm run a kernel without its code, whose registers (gamma, beta, a row) made the compiler store weights that
+  // are still on their way, i.e. wait for them before the wait for x.  Two short rows keep the common kernel, which the launch before
+  // left in the instruction cache (us a step, common / without / by this rule: small f32, two sequences 293 / 297 / 281, medium bf16, two
+  // 729 / 740 / 711; XL bf16, two 1924 / 1837 / 1838; large f32, three 1700 / 1556 / 1570, f16, four 1978 / 1900 / 1911, medium
+  // f32, four 1010 / 855 / 879; the middle figure with rows of all lengths staged).  One row: small f32 234 / 238.
+  const bool bare = NR > 1 && !g.norm.g && (NR == 4 || g.K > 1024);
+  auto kernel = bare ? gemv_dense_kernel<T, RI, NR, EXPERTS, NR == 1 && !EXPERTS> : gemv_dense_kernel<T, RI, NR, EXPERTS, !EXPERTS>;
   if (smem > 47 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t grid = ((int64_t)ctx->sm_count * (smem > 72 * 1024 || RI == 2 ? 2 : 3) + groups - 1) / groups;   // resident at once
   if (grid > ctas) grid = ctas;

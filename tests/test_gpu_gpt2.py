@@ -108,6 +108,13 @@ def test_gpt2_xl_width_one_layer(rt, oracle):
     run_parity(rt, oracle, p, "q4_0", "fp32", B=1, prompt_len=5, steps=3, T=32, logit_tol=1e-3)
 
 
+@pytest.mark.parametrize("batch", [2, 3, 4])
+@pytest.mark.parametrize("heads", [1, 16, 17, 32, 33, 37])
+def test_steps_of_few_sequences_over_dense_rows_of_every_length(rt, oracle, heads, batch):
+    """LayerNorm of two to four rows inside the dense GEMV: one, two and three float4 a thread, and linears without one."""
+    run_parity(rt, oracle, S.GPT2Params(n_layers=1, n_heads=heads, dim=64 * heads, vocab_size=307), "f32", "fp32", B=batch, prompt_len=1, steps=4, T=8, logit_tol=1e-3)
+
+
 def test_golden_fixture_float64_torch(rt, golden):
     """Against the committed float64 PyTorch run (tests/golden/gpt2_tiny_f64.npz)."""
     g = golden["gpt2_tiny_f64"]
