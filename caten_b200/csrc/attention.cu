@@ -537,7 +537,8 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
     const int parts = att_parts(d_n ? T : n + 1, most);
     // (more CTAs are limited by bytes, and the kernel with more of them on an SM is the better one: us a step, few / other: medium Q4_0, 64
     // sequences, 200 positions 1358 / 1316; small Q8_0, 64 at 300 724 / 679; XL Q4_0, 16 at 100 2182 / 2118, but 16 at 800 3093 / 3343)
-    if (B * H > 2 * ctx->sm_count) {
+    // A caller's qkv may start at any float; the few-heads kernel reads it 16 bytes at a time.
+    if (B * H > 2 * ctx->sm_count || ((uintptr_t)qkv & 15)) {
       if (smem > 44 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
       launch_k(ctx, attn_decode_kernel, dim3((unsigned)H, (unsigned)B), dim3(256), smem, qkv, kc, vc, out, (int)H, (int)T, (int)n, d_n, bf.hi, bf.lo,
                pending_qkv ? *pending_qkv : PartIn(), ctx->attn_prefetch_bytes);

@@ -481,6 +481,21 @@ def test_attention_decode_shared_histories(rt, oracle, B, H, T):
     test_attention_decode_steps(rt, oracle, B, H, T)
 
 
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_attention_decode_from_any_float(rt, oracle, offset):
+    """qkv may start between two 16-byte boundaries, also where few heads and sequences would be read in such pieces."""
+    B, H, T = 2, 3, 140
+    rng = np.random.Generator(np.random.PCG64(offset))
+    kc, vc = (rng.standard_normal((B, T, H, 64), dtype=np.float32) for _ in range(2))
+    dk, dv = rt.transfer_from_array(_to_gpu_cache(kc)), rt.transfer_from_array(_to_gpu_cache(vc))
+    for n in (0, 17, T - 1):
+        qkv = rng.standard_normal((B, 3 * H * 64), dtype=np.float32)
+        want = oracle.attention(qkv, kc, vc, B, 1, n, H, mode=0)
+        moved = rt.transfer_from_array(np.concatenate([np.zeros(offset, np.float32), qkv.ravel()])).view(offset, qkv.shape)
+        np.testing.assert_allclose(rt.attention(moved, dk, dv, B, 1, n).numpy(), want, atol=1e-5, rtol=1e-5)
+    np.testing.assert_array_equal(dk.numpy(), _to_gpu_cache(kc))
+
+
 def test_attention_prefill_tensor_cores_in_groups(rt):
     """Histories so long that the operand tiles of one sequence fill the memory they are given."""
     torch = pytest.importorskip("torch")
