@@ -269,7 +269,17 @@ __global__ void __launch_bounds__(256, 3) attn_decode_few_kernel(const float *__
       p[u] = j0 + u * 16 + hw < j_end ? p[u] * 0.125f : -INFINITY;
       top = fmaxf(top, p[u]);
     }
-    if (top == -INFINITY) continue;   // no row yet
+    if (top == -INFINITY) {   // no row yet, or none that counts: but a NaN, which the maximum passes over, does
+#pragma unroll
+      for (int u = 0; u < FEW_U; ++u) {
+        ss += p[u] == p[u] ? 0.0f : p[u];
+        acc.x = fmaf(0.0f, v4[u].x, acc.x);
+        acc.y = fmaf(0.0f, v4[u].y, acc.y);
+        acc.z = fmaf(0.0f, v4[u].z, acc.z);
+        acc.w = fmaf(0.0f, v4[u].w, acc.w);
+      }
+      continue;
+    }
     const float keep = exp2f((m - top) * kInvLn2);
     m = top;
     ss *= keep;

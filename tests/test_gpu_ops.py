@@ -496,6 +496,30 @@ def test_attention_decode_from_any_float(rt, oracle, offset):
     np.testing.assert_array_equal(dk.numpy(), _to_gpu_cache(kc))
 
 
+@pytest.mark.parametrize("B,H,n,at", [(1, 4, 5, 5), (1, 4, 5, 2), (1, 4, 20, 3), (1, 4, 140, 130), (1, 4, 140, 5), (2, 30, 140, 77), (5, 30, 139, 130), (5, 70, 20, 3)])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_attention_decode_of_scores_that_are_no_numbers(rt, B, H, n, at, value):
+    """One key with a NaN or an infinity: a NaN score makes its head's output NaN wherever it lies (a half-warp's only row, a part of
+    a cluster's, among others), a score of -inf counts nothing, one of +inf gives NaN; the other heads do not notice."""
+    T = n + 3
+    rng = np.random.Generator(np.random.PCG64(n + at))
+    kc, vc = (rng.standard_normal((B, H, T, 64), dtype=np.float32) for _ in range(2))
+    qkv = np.abs(rng.standard_normal((B, 3, H, 64), dtype=np.float32))
+    b, h = B - 1, H // 2
+    if at == n:
+        qkv[b, 1, h, 7] = value
+    else:
+        kc[b, h, at, 7] = value
+    got = rt.attention(rt.transfer_from_array(qkv.reshape(B, -1)), rt.transfer_from_array(kc), rt.transfer_from_array(vc), B, 1, n).numpy().reshape(B, H, 64)
+    kc[:, :, n], vc[:, :, n] = qkv[:, 1], qkv[:, 2]
+    with np.errstate(invalid="ignore"):
+        s = np.einsum("bhd,bhtd->bht", qkv[:, 0].astype(np.float64), kc[:, :, :n + 1].astype(np.float64)) * 0.125
+        p = np.exp(s - s.max(-1, keepdims=True))
+        want = np.einsum("bht,bhtd->bhd", p / p.sum(-1, keepdims=True), vc[:, :, :n + 1].astype(np.float64))
+    assert np.isnan(want[b, h]).all() == (value != -np.inf)
+    np.testing.assert_allclose(got, want, atol=1e-5, rtol=1e-5)
+
+
 def test_attention_prefill_tensor_cores_in_groups(rt):
     """Histories so long that the operand tiles of one sequence fill the memory they are given."""
     torch = pytest.importorskip("torch")
