@@ -35,6 +35,41 @@ __device__ __forceinline__ void expr_store(void *p, int dtype, int64_t at, uint3
   }
 }
 
+// A strip's values, as above with one switch for all of them (a switch per element, and spilled registers: int add over 12800 x 511 28.0 us, so 17.3).
+template <int EV>
+__device__ __forceinline__ void expr_store_ev(void *out, const int dtype, const int64_t at, const int64_t step, const int lanes, const uint32_t *v, const int cls) {
+  const bool is_f = cls == CATEN_B200_CLS_F32;
+  auto strip = [&](auto *p, auto value) {
+    if (step == 32) {   // contiguous
+#pragma unroll
+      for (int j = 0; j < EV; ++j)
+        if (j < lanes) p[32 * j] = value(v[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < EV; ++j)
+        if (j < lanes) p[j * step] = value(v[j]);
+    }
+  };
+  switch (dtype) {
+    case CATEN_B200_DT_F32:
+      if (is_f) strip(reinterpret_cast<float *>(out) + at, [](uint32_t x) { return __uint_as_float(x); });
+      else strip(reinterpret_cast<float *>(out) + at, [](uint32_t x) { return (float)(int32_t)x; });
+      break;
+    case CATEN_B200_DT_I32:
+      if (is_f) strip(reinterpret_cast<int32_t *>(out) + at, [](uint32_t x) { return (int32_t)__uint_as_float(x); });
+      else strip(reinterpret_cast<int32_t *>(out) + at, [](uint32_t x) { return (int32_t)x; });
+      break;
+    case CATEN_B200_DT_I64:
+      if (is_f) strip(reinterpret_cast<int64_t *>(out) + at, [](uint32_t x) { return (int64_t)__uint_as_float(x); });
+      else strip(reinterpret_cast<int64_t *>(out) + at, [](uint32_t x) { return (int64_t)(int32_t)x; });
+      break;
+    default:
+      if (is_f) strip(reinterpret_cast<uint8_t *>(out) + at, [](uint32_t x) { return (uint8_t)(__uint_as_float(x) != 0.0f); });
+      else strip(reinterpret_cast<uint8_t *>(out) + at, [](uint32_t x) { return (uint8_t)(x != 0u); });
+      break;
+  }
+}
+
 __device__ __forceinline__ uint32_t expr_cast(uint32_t v, int from, int to) {
   if (from == to) return v;
   if (to == CATEN_B200_CLS_F32) return __float_as_uint((float)(int32_t)v);          // I32 / BOOL -> float
@@ -99,22 +134,38 @@ __device__ __forceinline__ void expr_load_ev(const caten_b200_expr &e, const int
   const int last = lanes > 0 ? lanes - 1 : 0;
   if (!whole) {
     const float *p = reinterpret_cast<const float *>(e.operand[arg]) + o;
-    if (step == 0) {
+    if (step == 32 && lanes == EV) {   // the strip is contiguous and full
+#pragma unroll
+      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[32 * j]);
+    } else if (step == 0) {
       const uint32_t v = __float_as_uint(*p);
 #pragma unroll
       for (int j = 0; j < EV; ++j) out[j] = v;
-    } else if (step == 32 && lanes == EV) {   // the strip is contiguous and full
-#pragma unroll
-      for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[32 * j]);
     } else {
 #pragma unroll
       for (int j = 0; j < EV; ++j) out[j] = __float_as_uint(p[(j < last ? j : last) * step]);
     }
     return;
   }
-  const int dt = e.operand_dtype[arg];
+  // (one switch for all of them)
+  auto strip = [&](auto *p, auto value) {
+    if (step == 0) {
+      const uint32_t v = value(*p);
 #pragma unroll
-  for (int j = 0; j < EV; ++j) out[j] = expr_load(e.operand[arg], dt, o + (j < last ? j : last) * step);
+      for (int j = 0; j < EV; ++j) out[j] = v;
+    } else if (step == 32 && lanes == EV) {
+#pragma unroll
+      for (int j = 0; j < EV; ++j) out[j] = value(p[32 * j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < EV; ++j) out[j] = value(p[(j < last ? j : last) * step]);
+    }
+  };
+  switch (e.operand_dtype[arg]) {
+    case CATEN_B200_DT_I32: strip(reinterpret_cast<const int32_t *>(e.operand[arg]) + o, [](int32_t v) { return (uint32_t)v; }); break;
+    case CATEN_B200_DT_I64: strip(reinterpret_cast<const int64_t *>(e.operand[arg]) + o, [](int64_t v) { return (uint32_t)(int32_t)v; }); break;
+    default: strip(reinterpret_cast<const uint8_t *>(e.operand[arg]) + o, [](uint8_t v) { return v ? 1u : 0u; }); break;
+  }
 }
 
 // Runs the program for EV elements at once: the decode of a word is shared.  Element j of the
@@ -313,10 +364,12 @@ __device__ __forceinline__ void expr_acc_add(ExprAcc &a, const uint32_t x, const
 // warp takes `spw` consecutive strips of one row, so the index decoding is paid once per warp.
 // Reduced loops (if any) are walked by each thread in loop order, exactly like the rendered loop
 // nest, so a float sum is added in the reference's order.  What bounds an item is its words: some
-// 2 us each over 12800 x 511 (a copy 10.7 us out of L2, 14.5 out of memory, gelu's 14 words 53;
-// 12.8, 16.0 and 65 with 64-bit divisions per warp, both classes computed by each word and a clamp
-// per element).  Four elements a thread in place of eight: gelu 89 us; three CTAs per SM: 57.
-template <int ND, int EV, bool HEAVY>
+// 2 us each over 12800 x 511 (a copy 10.2 us out of L2, gelu's 14 words 47; 12.8 and 65 with
+// 64-bit divisions per warp, both classes computed by each word and a clamp per element).  Four
+// elements a thread in place of eight: gelu 89 us, three CTAs per SM 57, where eight and four
+// took 53.  Reducing programs are an instance of their own: with both in one, 430 bytes of a
+// thread's registers lay in local memory (gelu 51 us, column sums 6.9 ms, 5.0 so).
+template <int ND, int EV, bool HEAVY, bool REDUCES>
 __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_constant__ caten_b200_expr e, const int64_t n_groups, const int groups_per_row, const int spw,
                                                             const int64_t n_red, const int result_cls) {
   extern __shared__ uint32_t expr_smem[];
@@ -343,18 +396,9 @@ __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_cons
       if (d == va) ix.v[d] = (int)j0;
     const int64_t out_at = expr_out_at(e, ix, nd_out);
     uint32_t val[EV];
-    if (e.n_reduce == 0) {
+    if (!REDUCES) {
       expr_run<ND, EV, EXPR_THREADS, HEAVY>(e, ix, va, lanes, val, sm);
-      if (is_f && e.out_dtype == CATEN_B200_DT_F32 && ovs == 32) {   // without the type switch per element
-        float *p = reinterpret_cast<float *>(e.out) + out_at;
-#pragma unroll
-        for (int j = 0; j < EV; ++j)
-          if (j < lanes) p[32 * j] = __uint_as_float(val[j]);
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < EV; ++j)
-        if (j < lanes) expr_store(e.out, e.out_dtype, out_at + j * ovs, val[j], result_cls);
+      expr_store_ev<EV>(e.out, e.out_dtype, out_at, ovs, lanes, val, result_cls);
       continue;
     }
     ExprAcc acc[EV];
@@ -367,8 +411,8 @@ __global__ void __launch_bounds__(EXPR_THREADS, 4) expr_kernel(const __grid_cons
       for (int j = 0; j < EV; ++j) expr_acc_add(acc[j], val[j], is_f, is_sum);
     }
 #pragma unroll
-    for (int j = 0; j < EV; ++j)
-      if (j < lanes) expr_store(e.out, e.out_dtype, out_at + j * ovs, is_f ? __float_as_uint(acc[j].f) : (uint32_t)acc[j].i, result_cls);
+    for (int j = 0; j < EV; ++j) val[j] = is_f ? __float_as_uint(acc[j].f) : (uint32_t)acc[j].i;
+    expr_store_ev<EV>(e.out, e.out_dtype, out_at, ovs, lanes, val, result_cls);
   }
 }
 
@@ -758,7 +802,8 @@ template <int ND, int EV, bool HEAVY>
 static int launch_expr_elements(caten_b200_ctx *ctx, const caten_b200_expr &e, int depth, int64_t rows, int64_t vlen, int64_t n_red, int result_cls) {
   // values under the top of the stack: [slot][element][thread] in shared memory
   const size_t smem = (size_t)(depth > 1 ? depth - 1 : 1) * EV * EXPR_THREADS * sizeof(uint32_t);
-  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(expr_kernel<ND, EV, HEAVY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kernel = e.n_reduce > 0 ? expr_kernel<ND, EV, HEAVY, true> : expr_kernel<ND, EV, HEAVY, false>;
+  if (smem > 48 * 1024) CB_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t strips_per_row = (vlen + 32 * EV - 1) / (32 * EV);
   // strips per warp: as many as still leave every SM a full complement of warps, at most 16
   int64_t spw = (rows * strips_per_row) / ((int64_t)ctx->sm_count * 64);
@@ -768,7 +813,7 @@ static int launch_expr_elements(caten_b200_ctx *ctx, const caten_b200_expr &e, i
   const int64_t n_groups = rows * groups_per_row;                    // one warp each
   const int64_t blocks = (n_groups + 7) / 8;
   if (blocks > 0x7fffffff) return fail(ctx, CATEN_B200_EUNSUPPORTED, "eval_expr: %lld output elements", (long long)(rows * vlen));
-  launch_k(ctx, expr_kernel<ND, EV, HEAVY>, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_groups, (int)groups_per_row, (int)spw, n_red, result_cls);
+  launch_k(ctx, kernel, dim3((unsigned)blocks), dim3(EXPR_THREADS), smem, e, n_groups, (int)groups_per_row, (int)spw, n_red, result_cls);
   CB_LAUNCH_CHECK(ctx, "expr_kernel");
   return 0;
 }

@@ -248,6 +248,31 @@ def test_words_joined_with_their_right_operand(rt, shape):
     check(rt, E.where(lx < lz, E.maximum(ly, lz), E.cast(E.load(i.view) * E.const(3) + E.index(len(shape) - 1), E.F32)), out, pairs=(x, y, z, i))
 
 
+@pytest.mark.parametrize("shape", [(1300, 512), (60, 511), (7, 1000), (90, 33), (5, 7)])
+@pytest.mark.parametrize("step", [1, 2])
+def test_strips_of_every_type(rt, shape, step):
+    """Loads and stores of whole and broken strips of each element type, contiguous and not: one, four and eight elements a thread,
+    element-wise and under a reduction over the outer loop."""
+    rows, cols = shape
+    rng = np.random.Generator(np.random.PCG64(rows + cols + step))
+    host = {np.float32: lambda: (rng.standard_normal((rows, step * cols)) * 9).astype(np.float32), np.int32: lambda: rng.integers(-99, 99, (rows, step * cols)).astype(np.int32),
+            np.int64: lambda: rng.integers(-99, 99, (rows, step * cols)), np.uint8: lambda: rng.integers(0, 2, (rows, step * cols)).astype(np.uint8)}
+    ins = [Pair(rt, make(), strides=(step * cols, step)) for make in host.values()]
+    for x in ins:
+        lx = E.load(x.view)
+        for make in host.values():
+            out = Pair(rt, np.zeros_like(make()), strides=(step * cols, step))
+            check(rt, lx if x is not ins[3] else E.not_(lx), out, shape=shape, pairs=(x,))
+            out.close()
+        by_column = E.load(E.View(x.dev, (step, step * cols)))
+        total = Pair(rt, np.zeros(cols, np.float32 if x is ins[0] else np.int32), strides=(1, 0))
+        x.view = by_column.value
+        check(rt, by_column if x is not ins[3] else E.cast(by_column, E.I32), total, shape=(cols, rows), n_reduce=1, reduce_op="sum", pairs=(x,))
+        total.close()
+    for x in ins:
+        x.close()
+
+
 @pytest.mark.parametrize("op", ["sum", "max"])
 @pytest.mark.parametrize("shape", [(7, 13, 511), (40, 33, 513), (3, 2, 1100), (300, 90, 300)])
 def test_plain_row_reductions_over_strided_views(rt, shape, op):
