@@ -291,8 +291,8 @@ def test_plain_row_reductions_over_strided_views(rt, shape, op):
 
 
 def test_exp2_over_the_whole_range(rt):
-    """Every 4099th bit pattern, whole numbers, and the ends of the range.  The polynomial is within 2^-44 of 2^x, so one value in
-    some 2^20 (two sides of a boundary 2^-24 apart) may round to the other neighbour: a handful of the million here, by one ulp."""
+    """Every 4099th bit pattern, whole numbers, and the ends of the range.  Numpy's own value in double is within an ulp of 2^x, so
+    a value that lies that close to the middle between two floats may round to the other neighbour."""
     bits = np.concatenate([np.arange(0, 2 ** 32, 4099, dtype=np.uint64).astype(np.uint32),
                            np.array([np.nan, np.inf, -np.inf, 0.0, -0.0, 127.99999, 128.0, -125.5, -126.0, -148.5, -149.0, -149.5, -150.0, -151.0, 160.5, -160.5, 3e38, -3e38],
                                     np.float32).view(np.uint32), np.arange(-160, 161).astype(np.float32).view(np.uint32)])
@@ -308,6 +308,20 @@ def test_exp2_over_the_whole_range(rt):
     whole = np.arange(-160, 161)
     with np.errstate(over="ignore"):
         np.testing.assert_array_equal(got[-321:], np.ldexp(1.0, whole).astype(np.float32))
+
+
+def test_exp2_is_rounded_from_all_of_double(rt):
+    """Arguments whose power lies within 2^-43 of the middle between two floats, on either side: a value of 2^-44 rounds some of
+    them to the other neighbour, double's 2^-53 none.  And the grid above, without an exception."""
+    near = np.array([0x3f4d2720, 0xbf34b452, 0x3fa5a5d7, 0x3fe69390, 0xbf996c70, 0xbfda5a29, 0x403349c8, 0x407349c8, 0xc00cb638, 0xc04cb638, 0x3e96975c, 0x4099a4e4,
+                     0x40b9a4e4, 0x40d9a4e4, 0x40f9a4e4, 0xc0865b1c, 0xc0a65b1c, 0xc0c65b1c, 0xc0e65b1c], np.uint32)
+    bits = np.concatenate([near, np.arange(0x3a000000, 0x43200000, 149, dtype=np.uint32), np.arange(0xba000000, 0xc3200000, 149, dtype=np.uint32)])
+    x = Pair(rt, bits.view(np.float32))
+    out = Pair(rt, np.zeros(len(bits), np.float32))
+    E.run(rt, E.exp2(E.load(x.view)), out.view)
+    with np.errstate(all="ignore"):
+        want = np.exp2(x.host.astype(np.float64)).astype(np.float32)
+    np.testing.assert_array_equal(out.dev.numpy().view(np.uint32), want.view(np.uint32))
 
 
 def test_malformed_programs_are_refused(rt):
