@@ -330,27 +330,6 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_enter() { pdl_wait(); pdl_launch_dependents(); }
 
 
-// GeLU exactly as the reference composes it (source/nn/activations.lisp:202-204 with
-// tanh(z) = 2*sigmoid(2z) - 1 and sigmoid(y) = 1/(1 + exp2(y * -1/ln2))), every step in fp32.
-__device__ __forceinline__ float gelu_ref(float x) {
-  const float kC = 0.7978845608028654f, k044 = 0.044715f, kNegInvLn2 = -1.0f / 0.6931472f;
-  float x3 = x * x;
-  x3 = x3 * x;
-  float in = k044 * x3;
-  in = x + in;
-  const float z = kC * in;
-  float a = 2.0f * z;
-  a = a * kNegInvLn2;
-  float e = exp2f(a);
-  e = 1.0f + e;
-  const float sg = 1.0f / e;
-  float th = 2.0f * sg;
-  th = th + (-1.0f);
-  const float l = 0.5f * x;
-  const float r = 1.0f + th;
-  return l * r;
-}
-
 // x / e for e >= 1 (infinity included), without the branch to a subroutine that an IEEE division carries: in the unrolled loops
 // of an epilogue that branch keeps the elements' chains from overlapping.  The quotient by an approximate reciprocal, corrected
 // once by its own remainder in fused arithmetic (P. W. Markstein, Computation of elementary functions on the IBM RISC
@@ -365,20 +344,16 @@ __device__ __forceinline__ float div_by_sum(float x, float e) {
   const float c = fmaf(r, fmaf(-fminf(e, 0x1.fffffep127f), q, x), q);
   return fabsf(q) < INFINITY ? c : q;
 }
-// The same function as x / (1 + exp(-2 sqrt(2 / pi) (x + 0.044715 x^3))): for the epilogues of the tensor-core kernels.  Error
-// against 64 bits (2-norm) over 4 M normal inputs of deviation 0.3, 1 and 3: 4.3e-8, 4.2e-8, 3.3e-8; of the composition above
-// 5.2e-8, 4.8e-8, 3.6e-8.  c_fc of 1665 rows, 4096 x 1024, plain bf16: 25.7 us with the composition, 20.5 with this.
-__device__ __forceinline__ float gelu_fast(float x) {
+// GELU as the reference defines it (source/nn/activations.lisp:202-204: x / 2 (1 + tanh(sqrt(2 / pi) (x + 0.044715 x^3))), tanh by a
+// sigmoid), in the form x / (1 + exp(-2 sqrt(2 / pi) (x + 0.044715 x^3))), which loses nothing where tanh is near -1: the one form of
+// every kernel.  Error against 64 bits (2-norm) over 4 M normal inputs of deviation 0.3, 1 and 3: 4.3e-8, 4.2e-8, 3.3e-8; of the
+// reference's composition step by step in fp32 5.2e-8, 4.8e-8, 3.6e-8.  c_fc of 1665 rows, 4096 x 1024, plain bf16: 25.7 us with
+// that, 20.5 with this; a step of GPT-2 small, one sequence: 250 and 234.
+__device__ __forceinline__ float gelu(float x) {
   const float c0 = -2.302208198f, c1 = -2.302208198f * 0.044715f;   // -2 sqrt(2 / pi) / ln 2
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * fmaf(x * x, c1, c0)));
   return div_by_sum(x, 1.0f + e);
-}
-
-__device__ __forceinline__ float act_fast(float v, int act) {
-  if (act == CATEN_B200_ACT_GELU) return gelu_fast(v);
-  if (act == CATEN_B200_ACT_RELU) return v > 0.0f ? v : 0.0f;
-  return v;
 }
 
 __host__ __device__ constexpr bool act_is_glu(int act) { return act == CATEN_B200_ACT_RELU_GLU || act == CATEN_B200_ACT_SILU_GLU; }
@@ -389,7 +364,7 @@ __device__ __forceinline__ float glu(int act, float gate, float up) {
 }
 
 __device__ __forceinline__ float apply_act(float v, int act) {
-  if (act == CATEN_B200_ACT_GELU) return gelu_ref(v);
+  if (act == CATEN_B200_ACT_GELU) return gelu(v);
   if (act == CATEN_B200_ACT_RELU) return v > 0.0f ? v : 0.0f;
   return v;
 }

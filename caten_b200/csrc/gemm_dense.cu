@@ -217,7 +217,7 @@ __device__ __forceinline__ void gd_store_block(const GdArgs &a, const float *stg
     const int64_t at = m * a.ldy + o0;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      if (ACT == CATEN_B200_ACT_GELU) v[e] = gelu_fast(v[e]);
+      if (ACT == CATEN_B200_ACT_GELU) v[e] = gelu(v[e]);
       if (ACT == CATEN_B200_ACT_RELU) v[e] = v[e] > 0.0f ? v[e] : 0.0f;
     }
     if (a.res) {

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 256 ? 1 : LOOP || RI * BLK:
       }
       for (int o = lpr >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (rl == 0 && rr < rows_per_iter && base + rr < a.N) {
-        s = act_fast(a.bias ? s + bz : s, a.act);
+        s = apply_act(a.bias ? s + bz : s, a.act);
         a.y[(int64_t)m * a.N + base + rr] = a.res ? rz + s : s;
       }
       buf ^= 1;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(GEMV_MAX_THREADS) gemv_stream_kernel(const Gem
     for (int o = lpr >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (rl == 0 && rr < rows_per_iter && base + rr < a.N) {
       const int64_t row = base + rr;
-      s = act_fast(a.bias ? s + a.bias[row] : s, a.act);
+      s = apply_act(a.bias ? s + a.bias[row] : s, a.act);
       a.y[row] = a.res ? a.res[row] + s : s;
     }
   }
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(256, RI == 2 ? 2 : 3) gemv_dense_kernel(const 
         const float up = __shfl_sync(0xffffffffu, s, (lane + NR) & 31);
         if (lane < NR && fin && row < N) y[fm * a.ldy + (row >> 1)] = glu(a.act, s, up);
       } else if (fin && row < N) {
-        s = act_fast(s, a.act);
+        s = apply_act(s, a.act);
         if (res) s = r + s;
         y[fm * a.ldy + row] = s;
       }

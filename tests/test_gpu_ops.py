@@ -716,11 +716,11 @@ def test_tensor_core_epilogues_in_fours_and_one_by_one(rt, act, M, N, K, offset)
     w.close()
 
 
-@pytest.mark.parametrize("M", [1, 5, 200, 1700])
-def test_activations_over_their_whole_range(rt, M):
+@pytest.mark.parametrize("M,precision", [(1, L.PREC_FP32), (5, L.PREC_FP32), (5, L.PREC_BF16X3), (200, L.PREC_BF16X3), (1700, L.PREC_BF16X3)])
+def test_activations_over_their_whole_range(rt, M, precision):
     """Weights of zero, so that the activation's argument is the bias.  silu: exp within two ulps, one rounding of the sum and at most one
-    ulp of the quotient, down to where exp(-z) overflows; GELU by sums of fp32 (rows of the tensor-core kernels): the exponent has
-    a few roundings of its own size; one row composes it from 1 + tanh, whose error is of the argument's size."""
+    ulp of the quotient, down to where exp(-z) overflows; GELU, one form in every kernel and precision: the exponent has
+    a few roundings of its own size."""
     z = np.concatenate([np.linspace(-104, 104, 4177), -10.0 ** np.linspace(-30, 30, 301), 10.0 ** np.linspace(-30, 30, 301),
                         [0.0, -0.0, np.inf, -np.inf, np.nan, -83.3, -84.0, -86.0, -87.5, -88.6, -9.5, -9.9, -10.1]]).astype(np.float32)
     z = z[np.abs(z + 88.72) > 0.05]
@@ -728,16 +728,15 @@ def test_activations_over_their_whole_range(rt, M):
     N = len(z)
     x = rt.transfer_from_array(np.ones((M, 64), np.float32))
     w, ww = rt.upload_weight(np.zeros((N, 64), np.float32)), rt.upload_weight(np.zeros((2 * N, 64), np.float32))
-    gelu = rt.linear(w, x, rt.transfer_from_array(z), act=L.ACT_GELU, precision=L.PREC_BF16X3).numpy()
-    silu = rt.linear(ww, x, rt.transfer_from_array(np.stack([z, np.ones_like(z)], 1).ravel()), act=L.ACT_SILU_GLU, precision=L.PREC_BF16X3, out=rt.open_buffer((M, N), np.float32)).numpy()
+    gelu = rt.linear(w, x, rt.transfer_from_array(z), act=L.ACT_GELU, precision=precision).numpy()
+    silu = rt.linear(ww, x, rt.transfer_from_array(np.stack([z, np.ones_like(z)], 1).ravel()), act=L.ACT_SILU_GLU, precision=precision, out=rt.open_buffer((M, N), np.float32)).numpy()
     with np.errstate(all="ignore"):
         z64 = z.astype(np.float64)
         e = np.exp(-z64)
         want = z64 / (1 + np.where(e > np.finfo(np.float32).max, np.inf, e))
         a = 2 * np.sqrt(2 / np.pi) * (z64 + 0.044715 * z64 ** 3)
         wg = z64 / (1 + np.where(-a > 127.99 * np.log(2), np.inf, np.exp(-a)))
-        rel = 2.0 ** -20 + 2.0 ** -21 * np.minimum(np.abs(a), 200) if M > 1 else 0.0
-        bound = rel * np.abs(wg) + (2.0 ** -100 if M > 1 else 2.0 ** -21 * np.minimum(np.abs(z64), 20) + 2.0 ** -22 * np.abs(wg))
+        bound = (2.0 ** -20 + 2.0 ** -21 * np.minimum(np.abs(a), 200)) * np.abs(wg) + 2.0 ** -100
         for row in (0, M - 1):
             np.testing.assert_array_equal(np.isnan(silu[row]), np.isnan(want))
             np.testing.assert_array_equal(np.isnan(gelu[row]), np.isnan(wg))
