@@ -95,8 +95,9 @@ def test_a_warps_bounded_wait_has_one_answer():
     in front of instructions that need all of them.  A thread's own answer (`mbar_wait_thread`) decides only where one thread waits."""
     csrc = os.path.join(ROOT, "caten_b200", "csrc")
     text = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.endswith((".cu", ".cuh"))}
-    wait = re.search(r"bool mbar_wait\(.*?\n\}", text["tcgen05.cuh"], re.S).group()
-    assert "__all_sync(0xffffffffu, mbar_wait_thread(" in wait
+    tried = re.search(r"bool mbar_wait\(.*?\n\}", text["tcgen05.cuh"], re.S).group()
+    assert "mbar_try_warp(" in tried and "__any_sync(0xffffffffu, *abort_flag" in tried
+    assert "vote.sync.all.pred" in re.search(r"bool mbar_try_warp\(.*?\n\}", text["tcgen05.cuh"], re.S).group()
     calls = 0
     for name, src in text.items():
         lines = src.split("\n")
