@@ -611,7 +611,9 @@ static GdPlan gd_plan(int sm, int64_t M, int64_t N, int tiles_f, int64_t K, int 
         double stage = mma > bytes * busy / (52.0 * sm) ? mma : bytes * busy / (52.0 * sm);
         if (stage < 1400.0 / in_flight) stage = 1400.0 / in_flight;
         const double body = cps * stage;
-        double t = (pair ? 8900 : 5900) + body + epilogue + (double)(waves - 1) * (body > 0.54 * epilogue ? body : 0.54 * epilogue);
+        // (a single wave of the widest pairs lost where the model had them ahead: us alone / pairs, plain bf16, 1525 rows, 3072 x 1600
+        // 18.0 / 19.5, 909 rows, 4096 x 2816 23.0 / 24.7)
+        double t = (pair ? bn == GD_BN && waves == 1 ? 11900 : 8900 : 5900) + body + epilogue + (double)(waves - 1) * (body > 0.54 * epilogue ? body : 0.54 * epilogue);
         if (s > 1) t += (consumer_sums ? 500.0 + 60.0 * s : 6000.0) + (double)M * N * 4 * s / (sm * 17.0);
         t *= 1.0 + 0.0001 * (GD_BN - bn);   // traffic costs power too, which is what limits long launches
         if (t < least) { least = t; best = {bn, s, cps, pair != 0}; }
