@@ -218,13 +218,7 @@ __global__ void __launch_bounds__(256, 3) attn_decode_few_kernel(const float *__
     place();
     load(j_first);
   }
-  if (SPLIT && rank >= parts) {   // (whole CTAs) not needed at this length; the others still meet at the barriers
-    if (parts > 1) {
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    }
-    return;
-  }
+  if (SPLIT && rank >= parts) return;   // (whole CTAs) one part at this length, whose CTA waits for no other
   const bool newest = !SPLIT || rank == parts - 1;   // position n is in the last part, which is never empty
   const float4 *qp, *kp, *vp;
   if (pin.splits > 0) {
@@ -536,6 +530,7 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
   if (s == 1) {
     // with a device-side position the launch is sized for the longest context the cache allows
     const size_t smem = (64 + 1024 + 32 + (size_t)(d_n ? T : n + 1)) * sizeof(float);
+    // one limit, that of the general kernel's scores, whatever kernel runs: a context that one sequence may have is not refused to many
     if (smem > 200 * 1024) return fail(ctx, CATEN_B200_EUNSUPPORTED, "attention: context too long for the decode kernel");
     // CTAs per history: as many as are resident twice per SM at most.  Two are not worth a cluster, whose CTAs start later beside the
     // linear before (us a step, one / two, at 10, 300, 640 and 1000 positions: medium Q4_0, 8 sequences 755 / 811, 895 / 952, 1076 /
