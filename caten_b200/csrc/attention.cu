@@ -527,6 +527,9 @@ int launch_attention(caten_b200_ctx *ctx, const float *qkv, float *kc, float *vc
   if (pending_qkv && pending_qkv->splits > 0 && s != 1) return fail(ctx, CATEN_B200_EINVAL, "attention: a pending qkv is only supported for single-token steps");
   if (n < 0 || n + s > T) return fail(ctx, CATEN_B200_EINVAL, "attention: positions [%lld,%lld) outside the cache (T=%lld)", (long long)n, (long long)(n + s), (long long)T);
   if (H > 65535 || B > 65535) return fail(ctx, CATEN_B200_EUNSUPPORTED, "attention: B or H > 65535");
+  // (every kernel moves 16 bytes of these at a time; a single token's qkv and output may start at any float)
+  if (((uintptr_t)kc | (uintptr_t)vc | (s > 1 ? (uintptr_t)qkv | (uintptr_t)out : 0)) & 15)
+    return fail(ctx, CATEN_B200_EINVAL, "attention: the caches, and qkv and out of several tokens, must be 16-byte aligned");
   if (s == 1) {
     // with a device-side position the launch is sized for the longest context the cache allows
     const size_t smem = (64 + 1024 + 32 + (size_t)(d_n ? T : n + 1)) * sizeof(float);

@@ -496,6 +496,20 @@ def test_attention_decode_from_any_float(rt, oracle, offset):
     np.testing.assert_array_equal(dk.numpy(), _to_gpu_cache(kc))
 
 
+def test_attention_refuses_addresses_that_its_kernels_cannot_read(rt):
+    """Refused on the host, before anything is launched."""
+    B, H, T = 1, 2, 20
+    cache = [rt.open_buffer((B * H * T * 64 + 4,), np.float32) for _ in range(2)]
+    qkv = rt.open_buffer((2 * 3 * H * 64 + 4,), np.float32)
+    shape = (B, H, T, 64)
+    for s, q, k, v in ((1, 0, 1, 0), (1, 0, 0, 2), (2, 0, 3, 0), (2, 1, 0, 0)):
+        with pytest.raises(B200Error) as e:
+            rt.attention(qkv.view(q, (B * s, 3 * H * 64)), cache[0].view(k, shape), cache[1].view(v, shape), B, s, 0)
+        assert e.value.code == L.EINVAL
+    for b in (*cache, qkv):
+        b.close()
+
+
 @pytest.mark.parametrize("B,H,n,at", [(1, 4, 5, 5), (1, 4, 5, 2), (1, 4, 20, 3), (1, 4, 140, 130), (1, 4, 140, 5), (2, 30, 140, 77), (5, 30, 139, 130), (5, 70, 20, 3)])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 def test_attention_decode_of_scores_that_are_no_numbers(rt, B, H, n, at, value):
