@@ -206,7 +206,8 @@ int caten_b200_embed(caten_b200_ctx *ctx, const float *d_ids_f32, const int64_t 
  * rows (columns [d,2d) and [2d,3d) of qkv) at positions [n, n+s) of the caches, then
  * out = softmax(q.K^T * 0.125 + causal mask) . V over positions [0, n+s).
  * qkv [B*s, 3d]; out [B*s, d]; caches are [B, H, T, 64] fp32 (head-major so one head's history
- * is contiguous; the reference's [B, T, H, 64] holds the same values). */
+ * is contiguous; the reference's [B, T, H, 64] holds the same values).  The caches, and with s > 1
+ * qkv and out, start on a multiple of 16 bytes (CATEN_B200_EINVAL otherwise). */
 int caten_b200_attention(caten_b200_ctx *ctx, const float *d_qkv, float *d_kcache, float *d_vcache,
                          float *d_out, int64_t B, int64_t s, int64_t n, int64_t H, int64_t T);
 /* The same with a precision (CATEN_B200_PREC_*) for steps of more than one token: FP32 is
